@@ -232,6 +232,20 @@ MF_API size_t mf_transition_bwd_workspace_bytes(const mf_transition_bwd_args* ar
 MF_API int mf_transition_bwd(const mf_transition_bwd_args* args, void* stream);
 
 /* ------------------------------------------------------------------------------------------
+ * Type conversion of several contiguous arrays (fp32, bf16, fp16 in any combination) in one launch, for hosts that
+ * hold their parameters in another type than the one they compute in.  n_items <= MF_CAST_MAX.
+ * (No counterpart in the reference, which leaves these conversions to torch: fused_layernorm_linear.py:480.)
+ * ------------------------------------------------------------------------------------------ */
+#define MF_CAST_MAX 8
+typedef struct mf_cast_item {
+  const void* src; void* dst;
+  int64_t n;                     /* elements */
+  int32_t src_dtype, dst_dtype;
+} mf_cast_item;
+
+MF_API int mf_cast_batch(const mf_cast_item* items, int32_t n_items, void* stream);
+
+/* ------------------------------------------------------------------------------------------
  * Library queries.
  * ------------------------------------------------------------------------------------------ */
 MF_API const char* mf_last_error_string(void);   /* thread-local, never NULL */

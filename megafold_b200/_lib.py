@@ -1,11 +1,13 @@
-"""ctypes binding of libmegafold_b200.so (C ABI declared in include/megafold_b200.h).
+"""Loads libmegafold_b200.so (C ABI declared in include/megafold_b200.h) and the torch functions over it.
 
-The structures below mirror the C structs field for field.  There is no CPU fallback: if the
+``lib()`` is the ctypes binding, for the entry points that have no torch function and for tests of the C ABI; its
+structures mirror the C structs field for field.  ``native()`` is what the operators call.  There is no CPU fallback: if the
 library cannot be loaded, or an entry point returns an error, a RuntimeError is raised.
 """
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 import threading
 
@@ -13,6 +15,7 @@ import torch
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libmegafold_b200_trace.so" if os.environ.get("MF_TRACE") == "1" else "libmegafold_b200.so")
+NATIVE_PATH = os.path.join(_PKG, "_native.so")
 
 MF_F32, MF_BF16, MF_F16, MF_U8 = 0, 1, 2, 3
 MF_FLAG_FORCE_SIMT = 1
@@ -75,6 +78,10 @@ class TransitionBwdArgs(C.Structure):
                 ("workspace", _vp), ("workspace_bytes", _sz)]
 
 
+class CastItem(C.Structure):
+    _fields_ = [("src", _vp), ("dst", _vp), ("n", _i64), ("src_dtype", _i32), ("dst_dtype", _i32)]
+
+
 # every symbol include/megafold_b200.h declares: name -> (restype, argtypes)
 SYMBOLS = {
     "mf_evo_fwd": (C.c_int, [C.POINTER(EvoFwdArgs), _vp]),
@@ -91,6 +98,7 @@ SYMBOLS = {
     "mf_transition_fwd": (C.c_int, [C.POINTER(TransitionFwdArgs), _vp]),
     "mf_transition_bwd_workspace_bytes": (_sz, [C.POINTER(TransitionBwdArgs)]),
     "mf_transition_bwd": (C.c_int, [C.POINTER(TransitionBwdArgs), _vp]),
+    "mf_cast_batch": (C.c_int, [C.POINTER(CastItem), _i32, _vp]),
     "mf_last_error_string": (C.c_char_p, []),
     "mf_version": (C.c_int, []),
     "mf_kernel_launch_count": (C.c_uint64, []),
@@ -100,7 +108,8 @@ SYMBOLS = {
 }
 
 _lib = None
-_lock = threading.Lock()
+_native = None
+_lock = threading.RLock()
 
 
 def lib() -> C.CDLL:
@@ -121,6 +130,25 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def native():
+    """The torch functions over the library (csrc/torch_ops.cpp): allocation, autograd and autocast in native code."""
+    global _native
+    if _native is not None:
+        return _native
+    with _lock:
+        if _native is None:
+            if not os.path.exists(NATIVE_PATH):
+                from . import build as _build
+                _build.build()
+            lib()
+            spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            module.load(LIB_PATH)
+            _native = module
+    return _native
+
+
 def dtype_code(dt: torch.dtype) -> int:
     try:
         return _DTYPES[dt]
@@ -134,19 +162,8 @@ def check(status: int, what: str) -> None:
         raise RuntimeError(f"megafold_b200 {what} failed (status {status}): {msg}")
 
 
-def ptr(t):
-    return None if t is None else t.data_ptr()
-
-
 def stream_ptr(device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
-
-
-def require_cuda(*tensors) -> None:
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise RuntimeError("megafold_b200 operators run on CUDA tensors only (there is no CPU path); "
-                               f"got a tensor on {t.device}")
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:

@@ -3,7 +3,8 @@
     python -m megafold_b200.build [--force] [--verbose]
 
 The library is plain CUDA C++ behind a C ABI (include/megafold_b200.h); it links the static CUDA
-runtime only, so it loads on hosts without a GPU driver (entry points then fail with MF_ERR_CUDA).
+runtime only, so it loads on hosts without a GPU driver (entry points then fail with MF_ERR_CUDA).  The torch functions over it
+are a second shared object (_native.so), which needs the torch it was built against.
 """
 from __future__ import annotations
 
@@ -20,9 +21,10 @@ ROOT = os.path.dirname(PKG)
 # regular library; megafold_b200._lib loads it when MF_TRACE=1 is set there too.
 TRACE = os.environ.get("MF_TRACE") == "1"
 LIB = os.path.join(PKG, "libmegafold_b200_trace.so" if TRACE else "libmegafold_b200.so")
+NATIVE = os.path.join(PKG, "_native.so")          # torch functions over the library (csrc/torch_ops.cpp)
 OBJ_DIR = os.path.join(PKG, "build_trace" if TRACE else "build")
 
-SOURCES = ["api.cu", "evo_simt.cu", "evo_tc.cu", "evo_tc_fwd.cu", "evo_fwd_ws.cu", "evo_bwd_ws.cu", "lnl_ops.cu", "lnl_tc.cu", "transition_tc.cu", "gemm_tc.cu", "transition_bwd_tc.cu"]
+SOURCES = ["api.cu", "evo_simt.cu", "evo_tc.cu", "evo_tc_fwd.cu", "evo_fwd_ws.cu", "evo_bwd_ws.cu", "lnl_ops.cu", "lnl_tc.cu", "transition_tc.cu", "gemm_tc.cu", "transition_bwd_tc.cu", "cast.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",
@@ -52,6 +54,20 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _native_command(src: str):
+    """g++ of one translation unit against the installed torch; the result is imported by file name."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    inc = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    # the C++ runtime has to be the one torch uses: a second, static copy crashes when it formats an error message
+    return ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), src, "-o", NATIVE,
+            f"-L{lib}", f"-Wl,-rpath,{lib}", "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-lstdc++", "-ldl"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ_DIR, exist_ok=True)
     nvcc = _nvcc()
@@ -67,13 +83,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
     def run(cmd):
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
-            raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + p.stdout + p.stderr)
+            raise RuntimeError("compilation failed:\n" + " ".join(cmd) + "\n" + p.stdout + p.stderr)
         return p.stdout + p.stderr
 
-    with ThreadPoolExecutor(max_workers=4) as ex:
+    native_src = os.path.join(CSRC, "torch_ops.cpp")
+    if force or _stale(NATIVE, [native_src, os.path.join(ROOT, "include", "megafold_b200.h"), os.path.abspath(__file__)]):
+        jobs.insert(0, _native_command(native_src))
+    with ThreadPoolExecutor(max_workers=5) as ex:
         for out in ex.map(run, jobs):
             if verbose and out.strip():
                 print(out)
+    jobs = [c for c in jobs if NATIVE not in c]
     objs = [os.path.join(OBJ_DIR, s.replace(".cu", ".o")) for s in SOURCES]
     if force or jobs or _stale(LIB, objs):
         run([nvcc, "-shared", "-o", LIB, *objs, "-Xcompiler", "-fPIC", "-cudart", "static", "-ldl"])

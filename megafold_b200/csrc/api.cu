@@ -252,6 +252,17 @@ int mf_transition_bwd(const mf_transition_bwd_args* args, void* stream) {
   return r;
 }
 
+int mf_cast_batch(const mf_cast_item* items, int32_t n_items, void* stream) {
+  Range nvtx_range("mf_cast_batch");
+  MF_REQUIRE(items && n_items > 0 && n_items <= MF_CAST_MAX, MF_ERR_BAD_ARG, "between 1 and %d arrays are converted at once, got %d", MF_CAST_MAX, n_items);
+  for (int i = 0; i < n_items; ++i) {
+    MF_REQUIRE(items[i].n >= 0 && (items[i].n == 0 || (items[i].src && items[i].dst)), MF_ERR_BAD_ARG, "array %d: bad size or NULL", i);
+    MF_REQUIRE(float_dtype(items[i].src_dtype) && float_dtype(items[i].dst_dtype), MF_ERR_BAD_ARG, "array %d: not a floating type", i);
+  }
+  int r = check_device(); if (r) return r;
+  return cast_batch(items, n_items, static_cast<cudaStream_t>(stream));
+}
+
 const char* mf_last_error_string(void) { return last_error_buf(); }
 int mf_version(void) { return MF_ABI_VERSION; }
 uint64_t mf_kernel_launch_count(void) { return g_launches.load(); }

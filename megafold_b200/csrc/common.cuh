@@ -152,6 +152,8 @@ int transition_bwd(const mf_transition_bwd_args& a, cudaStream_t st);
 size_t transition_fwd_simt_workspace(const mf_transition_fwd_args& a);
 size_t transition_bwd_workspace(const mf_transition_bwd_args& a);
 
+int cast_batch(const mf_cast_item* items, int n_items, cudaStream_t st);
+
 int swiglu_fwd(const void* x, void* y, int64_t M, int inner, int dtype, cudaStream_t st);
 int swiglu_bwd(const void* x, const void* dy, void* dx, int64_t M, int inner, int dtype, cudaStream_t st);
 

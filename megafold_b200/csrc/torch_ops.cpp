@@ -1,0 +1,511 @@
+// The operators as torch functions: allocation, autograd and autocast in native code over the C ABI of the library.
+//
+// A small call is bound by the host: with the argument structures filled through ctypes and the autograd functions in
+// Python, a forward + backward pair of one operator kept one core busy for 180 to 330 us (attention to LayernormLinear
+// under autocast) while the kernels of the single track take 60 to 70 us.  Here the same pair costs a few microseconds
+// per call plus the launches, and the backward runs on the autograd thread without the interpreter lock.
+//
+// The library is opened by path at import (load()), so this module carries no link-time dependency on it and the
+// library itself stays free of torch.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <dlfcn.h>
+#include <torch/extension.h>
+#include <ATen/autocast_mode.h>
+
+#include <array>
+#include <optional>
+#include <tuple>
+#include <vector>
+
+#include "../../include/megafold_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::tensor_list;
+using torch::autograd::Variable;
+using OptTensor = std::optional<Tensor>;
+
+#define MF_ENTRY(name) decltype(&::name) name = nullptr
+struct Api {
+  MF_ENTRY(mf_evo_fwd);
+  MF_ENTRY(mf_evo_bwd_workspace_bytes);
+  MF_ENTRY(mf_evo_bwd);
+  MF_ENTRY(mf_lnl_fwd);
+  MF_ENTRY(mf_lnl_bwd_workspace_bytes);
+  MF_ENTRY(mf_lnl_bwd);
+  MF_ENTRY(mf_swiglu_fwd);
+  MF_ENTRY(mf_swiglu_bwd);
+  MF_ENTRY(mf_transition_fwd_workspace_bytes);
+  MF_ENTRY(mf_transition_fwd);
+  MF_ENTRY(mf_transition_bwd_workspace_bytes);
+  MF_ENTRY(mf_transition_bwd);
+  MF_ENTRY(mf_cast_batch);
+  MF_ENTRY(mf_last_error_string);
+} api;
+#undef MF_ENTRY
+
+void load(const std::string& path) {
+  void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  TORCH_CHECK(h, "megafold_b200: cannot open ", path, ": ", dlerror());
+  auto get = [&](const char* name) {
+    void* p = dlsym(h, name);
+    TORCH_CHECK(p, "megafold_b200: ", path, " does not export ", name);
+    return p;
+  };
+#define MF_LOAD(name) api.name = reinterpret_cast<decltype(api.name)>(get(#name))
+  MF_LOAD(mf_evo_fwd); MF_LOAD(mf_evo_bwd_workspace_bytes); MF_LOAD(mf_evo_bwd);
+  MF_LOAD(mf_lnl_fwd); MF_LOAD(mf_lnl_bwd_workspace_bytes); MF_LOAD(mf_lnl_bwd);
+  MF_LOAD(mf_swiglu_fwd); MF_LOAD(mf_swiglu_bwd);
+  MF_LOAD(mf_transition_fwd_workspace_bytes); MF_LOAD(mf_transition_fwd);
+  MF_LOAD(mf_transition_bwd_workspace_bytes); MF_LOAD(mf_transition_bwd);
+  MF_LOAD(mf_cast_batch); MF_LOAD(mf_last_error_string);
+#undef MF_LOAD
+}
+
+void check(int status, const char* what) {
+  TORCH_CHECK(status == MF_OK, "megafold_b200 ", what, " failed (status ", status, "): ", api.mf_last_error_string());
+}
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return MF_F32;
+    case at::kBFloat16: return MF_BF16;
+    case at::kHalf: return MF_F16;
+    case at::kBool: case at::kByte: return MF_U8;
+    default: TORCH_CHECK_TYPE(false, "megafold_b200: unsupported dtype ", t);
+  }
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+std::string shape(const Tensor& t) {
+  std::string s = "(";
+  for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+  return s + ")";
+}
+
+void require_cuda(std::initializer_list<const Tensor*> ts) {
+  for (const Tensor* t : ts)
+    TORCH_CHECK(!t->defined() || t->is_cuda(),
+                "megafold_b200 operators run on CUDA tensors only (there is no CPU path); got a tensor on ", t->device());
+}
+
+Tensor workspace(size_t bytes, const Tensor& like) {
+  return at::empty({(int64_t)(bytes < 256 ? 256 : bytes)}, like.options().dtype(at::kByte));
+}
+Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+Tensor or_none(const OptTensor& t) { return t ? *t : Tensor(); }
+
+// ---- conversions -------------------------------------------------------------------------------------------------
+// Brings each tensor to its wanted type (and to contiguous memory), all of them in one launch: mixed-precision calls
+// convert four to six small parameters at once, where a launch each costs more than the conversion.
+struct Cast { Tensor* t; at::ScalarType to; };
+void cast_batch(std::initializer_list<Cast> list) {
+  mf_cast_item items[MF_CAST_MAX];
+  Tensor keep[MF_CAST_MAX];
+  int n = 0;
+  Tensor any;
+  for (const Cast& c : list) {
+    if (!c.t->defined()) continue;
+    if (!c.t->is_contiguous()) *c.t = c.t->contiguous();
+    if (c.t->scalar_type() == c.to) continue;
+    const auto from = c.t->scalar_type();
+    const bool plain = from == at::kFloat || from == at::kBFloat16 || from == at::kHalf;
+    if (!plain || n == MF_CAST_MAX) { *c.t = c.t->to(c.to); continue; }
+    if (c.t->numel() == 0) { *c.t = at::empty(c.t->sizes(), c.t->options().dtype(c.to)); continue; }
+    Tensor out = at::empty(c.t->sizes(), c.t->options().dtype(c.to));
+    items[n] = mf_cast_item{c.t->data_ptr(), out.data_ptr(), c.t->numel(), dtype_code(from), dtype_code(c.to)};
+    keep[n++] = *c.t;          // the source must outlive the launch
+    any = out;
+    *c.t = out;
+  }
+  if (n) check(api.mf_cast_batch(items, n, stream_of(any)), "mf_cast_batch");
+}
+
+// What torch.amp.custom_fwd(cast_inputs=torch.bfloat16) does to one argument while autocast is on.
+bool autocast_on() { return at::autocast::is_autocast_enabled(at::kCUDA); }
+at::ScalarType amp_type(const Tensor& t, bool on) {
+  return on && t.defined() && t.is_cuda() && t.is_floating_point() && t.scalar_type() != at::kDouble ? at::kBFloat16 : t.scalar_type();
+}
+
+// ---- attention -----------------------------------------------------------------------------------------------------
+std::array<int64_t, 5> check_shapes(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask, const OptTensor& bias) {
+  TORCH_CHECK_VALUE(q.dim() == 5, "Q must be [B, N_seq, N_res, Head, Dim], got ", shape(q));
+  TORCH_CHECK_VALUE(k.sizes() == q.sizes() && v.sizes() == q.sizes(), "Q, K, V shapes differ: ", shape(q), " ", shape(k), " ", shape(v));
+  TORCH_CHECK_TYPE(q.scalar_type() == k.scalar_type() && q.scalar_type() == v.scalar_type(), "Q, K, V must share a dtype");
+  TORCH_CHECK_VALUE(mask && mask->defined() && bias && bias->defined(), "res_mask and pair_bias are mandatory");
+  const int64_t B = q.size(0), N = q.size(1), L = q.size(2), H = q.size(3), D = q.size(4);
+  TORCH_CHECK_VALUE(bias->dim() == 5 && bias->size(1) == 1 && bias->size(2) == H && bias->size(3) == L && bias->size(4) == L &&
+                        (bias->size(0) == 1 || bias->size(0) == B),
+                    "pair_bias must be [B, 1, Head, N_res, N_res], got ", shape(*bias));
+  TORCH_CHECK_VALUE(mask->dim() == 5 && mask->size(2) == 1 && mask->size(3) == 1 && mask->size(4) == L &&
+                        (mask->size(0) == 1 || mask->size(0) == B) && (mask->size(1) == 1 || mask->size(1) == N),
+                    "res_mask must be [B, N_seq, 1, 1, N_res], got ", shape(*mask));
+  return {B, N, L, H, D};
+}
+
+template <typename A>
+void fill_common(A& a, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& mask, const Tensor& bias, int64_t flags) {
+  a.B = (int32_t)q.size(0); a.N = (int32_t)q.size(1); a.L = (int32_t)q.size(2); a.H = (int32_t)q.size(3); a.D = (int32_t)q.size(4);
+  a.dtype = dtype_code(q.scalar_type()); a.bias_dtype = dtype_code(bias.scalar_type()); a.mask_dtype = dtype_code(mask.scalar_type());
+  a.flags = (uint32_t)flags;
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr();
+  for (int i = 0; i < 5; ++i) { a.q_strides[i] = q.stride(i); a.k_strides[i] = k.stride(i); a.v_strides[i] = v.stride(i); }
+  // an extent of one that stands for B or N is read again for each of them
+  auto step = [](const Tensor& t, int dim, int64_t want) { return t.size(dim) == 1 && want != 1 ? (int64_t)0 : t.stride(dim); };
+  a.mask = mask.data_ptr();
+  a.mask_strides[0] = step(mask, 0, a.B); a.mask_strides[1] = step(mask, 1, a.N); a.mask_strides[2] = mask.stride(4);
+  a.bias = bias.data_ptr();
+  a.bias_strides[0] = step(bias, 0, a.B); a.bias_strides[1] = bias.stride(2); a.bias_strides[2] = bias.stride(3); a.bias_strides[3] = bias.stride(4);
+}
+
+std::tuple<Tensor, Tensor> evo_forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask_, const OptTensor& bias_, int64_t flags) {
+  const Tensor mask = or_none(mask_), bias = or_none(bias_);
+  require_cuda({&q, &k, &v, &mask, &bias});
+  const auto s = check_shapes(q, k, v, mask_, bias_);
+  const c10::cuda::CUDAGuard guard(q.device());
+  Tensor o = at::empty({s[0], s[1], s[2], s[3], s[4]}, q.options());
+  Tensor lse = empty_f32({s[0], s[1], s[3], s[2]}, q);
+  mf_evo_fwd_args a{};
+  fill_common(a, q, k, v, mask, bias, flags);
+  a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
+  check(api.mf_evo_fwd(&a, stream_of(q)), "mf_evo_fwd");
+  return {o, lse};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> evo_backward(const Tensor& d_o_, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask_,
+                                                        const OptTensor& bias_, const Tensor& o_, const Tensor& lse, int64_t flags, int64_t event) {
+  const Tensor mask = or_none(mask_), bias = or_none(bias_);
+  require_cuda({&d_o_, &q, &k, &v, &mask, &bias, &o_, &lse});
+  const auto s = check_shapes(q, k, v, mask_, bias_);
+  const c10::cuda::CUDAGuard guard(q.device());
+  const Tensor d_o = d_o_.contiguous(), o = o_.contiguous();
+  Tensor dq = at::empty({s[0], s[1], s[2], s[3], s[4]}, q.options()), dk = at::empty_like(dq), dv = at::empty_like(dq);
+  const auto bt = bias.scalar_type();
+  Tensor d_bias = at::empty({s[0], 1, s[3], s[2], s[2]}, q.options().dtype(bt == q.scalar_type() ? bt : at::kFloat));
+  mf_evo_bwd_args a{};
+  fill_common(a, q, k, v, mask, bias, flags);
+  a.dbias_dtype = dtype_code(d_bias.scalar_type());
+  a.o = o.data_ptr(); a.d_o = d_o.data_ptr(); a.lse = lse.data_ptr<float>();
+  a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr(); a.d_bias = d_bias.data_ptr();
+  a.dbias_ready_event = reinterpret_cast<void*>(event);
+  Tensor ws = workspace(api.mf_evo_bwd_workspace_bytes(&a), q);
+  a.workspace = ws.data_ptr(); a.workspace_bytes = (size_t)ws.numel();
+  check(api.mf_evo_bwd(&a, stream_of(q)), "mf_evo_bwd");
+  if (bias.size(0) != s[0]) d_bias = d_bias.sum(0, /*keepdim=*/true);      // bias broadcast over the batch
+  if (d_bias.scalar_type() != bt) d_bias = d_bias.to(bt);
+  return {dq, dk, dv, d_bias};
+}
+
+struct EvoFn : torch::autograd::Function<EvoFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& mask, const Tensor& bias) {
+    auto [o, lse] = evo_forward(q, k, v, mask, bias, 0);
+    ctx->save_for_backward({q, k, v, mask, bias, o, lse});
+    return o;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const auto s = ctx->get_saved_variables();
+    auto [dq, dk, dv, db] = evo_backward(g[0], s[0], s[1], s[2], s[3], s[4], s[5], s[6], 0, 0);
+    return {dq, dk, dv, Tensor(), db};
+  }
+};
+
+Tensor evo_attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask, const OptTensor& bias) {
+  if (!at::GradMode::is_enabled()) return std::get<0>(evo_forward(q, k, v, mask, bias, 0));
+  const Tensor m = or_none(mask), b = or_none(bias);
+  require_cuda({&q, &k, &v, &m, &b});
+  check_shapes(q, k, v, mask, bias);
+  return EvoFn::apply(q, k, v, m, b);
+}
+
+// ---- LayernormLinear --------------------------------------------------------------------------------------------------
+int64_t rows_of(const Tensor& x) { return x.size(-1) ? x.numel() / x.size(-1) : 0; }
+
+// x, w and the vectors share one type and are contiguous
+std::tuple<Tensor, Tensor, Tensor> lnl_fwd_raw(const Tensor& x, const Tensor& w, const Tensor& b, const Tensor& lw, const Tensor& lb, double eps, int64_t flags) {
+  const int64_t K = x.size(-1), M = rows_of(x), N = w.size(1);
+  auto sizes = x.sizes().vec();
+  sizes.back() = N;
+  Tensor y = at::empty(sizes, x.options()), mean = empty_f32({M}, x), rstd = empty_f32({M}, x);
+  mf_lnl_fwd_args a{};
+  a.M = M; a.K = (int32_t)K; a.N = (int32_t)N; a.dtype = dtype_code(x.scalar_type()); a.flags = (uint32_t)flags; a.eps = (float)eps;
+  a.x = x.data_ptr(); a.ln_w = lw.data_ptr(); a.ln_b = ptr(lb); a.w = w.data_ptr(); a.b = ptr(b);
+  a.y = y.data_ptr(); a.mean = mean.data_ptr<float>(); a.rstd = rstd.data_ptr<float>();
+  check(api.mf_lnl_fwd(&a, stream_of(x)), "mf_lnl_fwd");
+  return {y, mean, rstd};
+}
+
+// (dx, dw, db, d_ln_w, d_ln_b), parameter gradients fp32
+std::array<Tensor, 5> lnl_bwd_raw(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& lw, const Tensor& lb, const Tensor& mean,
+                                  const Tensor& rstd, bool has_linear_bias, int64_t flags) {
+  const int64_t K = x.size(-1), M = rows_of(x), N = w.size(1);
+  Tensor dx = at::empty(x.sizes(), x.options());
+  Tensor dw = empty_f32({K, N}, x), dlw = empty_f32({K}, x), dlb, db;
+  if (lb.defined()) dlb = empty_f32({K}, x);
+  if (has_linear_bias) db = empty_f32({N}, x);
+  mf_lnl_bwd_args a{};
+  a.M = M; a.K = (int32_t)K; a.N = (int32_t)N; a.dtype = dtype_code(x.scalar_type()); a.flags = (uint32_t)flags;
+  a.x = x.data_ptr(); a.ln_w = lw.data_ptr(); a.ln_b = ptr(lb); a.w = w.data_ptr(); a.dy = dy.data_ptr();
+  a.mean = mean.data_ptr<float>(); a.rstd = rstd.data_ptr<float>();
+  a.dx = dx.data_ptr(); a.dw = dw.data_ptr<float>(); a.db = static_cast<float*>(ptr(db)); a.d_ln_w = dlw.data_ptr<float>();
+  a.d_ln_b = static_cast<float*>(ptr(dlb));
+  Tensor ws = workspace(api.mf_lnl_bwd_workspace_bytes(&a), x);
+  a.workspace = ws.data_ptr(); a.workspace_bytes = (size_t)ws.numel();
+  check(api.mf_lnl_bwd(&a, stream_of(x)), "mf_lnl_bwd");
+  return {dx, dw, db, dlw, dlb};
+}
+
+std::tuple<Tensor, Tensor, Tensor> lnl_forward(const Tensor& x_, const Tensor& w_, const OptTensor& b_, const Tensor& lw_, const OptTensor& lb_, double eps,
+                                               int64_t flags) {
+  Tensor x = x_, w = w_, b = or_none(b_), lw = lw_, lb = or_none(lb_);
+  require_cuda({&x, &w, &b, &lw, &lb});
+  TORCH_CHECK_VALUE(w.dim() == 2 && x.dim() >= 1 && w.size(0) == x.size(-1), "Incompatible dimensions");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto dt = x.scalar_type();
+  cast_batch({{&x, dt}, {&w, dt}, {&b, dt}, {&lw, dt}, {&lb, dt}});
+  return lnl_fwd_raw(x, w, b, lw, lb, eps, flags);
+}
+
+std::array<Tensor, 5> lnl_backward(const Tensor& dy_, const Tensor& x_, const Tensor& w_, const Tensor& lw_, const OptTensor& lb_, const Tensor& mean,
+                                   const Tensor& rstd, bool has_linear_bias, int64_t flags) {
+  Tensor dy = dy_, x = x_, w = w_, lw = lw_, lb = or_none(lb_);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto dt = x.scalar_type();
+  cast_batch({{&x, dt}, {&dy, dt}, {&w, dt}, {&lw, dt}, {&lb, dt}});
+  return lnl_bwd_raw(dy, x, w, lw, lb, mean, rstd, has_linear_bias, flags);
+}
+
+// types of the arguments before autocast converted them: the gradients go back in those
+template <size_t N>
+void save_types(AutogradContext* ctx, const std::array<at::ScalarType, N>& t) {
+  std::vector<int64_t> v;
+  for (auto x : t) v.push_back((int64_t)x);
+  ctx->saved_data["types"] = v;
+}
+std::vector<at::ScalarType> saved_types(AutogradContext* ctx) {
+  std::vector<at::ScalarType> out;
+  for (int64_t x : ctx->saved_data["types"].toIntVector()) out.push_back((at::ScalarType)x);
+  return out;
+}
+at::ScalarType type_of(const Tensor& t) { return t.defined() ? t.scalar_type() : at::kFloat; }
+
+struct LnlFn : torch::autograd::Function<LnlFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& w_, const OptTensor& b_, const Tensor& lw_, const OptTensor& lb_) {
+    Tensor x = x_, w = w_, b = or_none(b_), lw = lw_, lb = or_none(lb_);
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto dt = amp_type(x, autocast_on());
+    save_types<5>(ctx, {type_of(x), type_of(w), type_of(b), type_of(lw), type_of(lb)});
+    cast_batch({{&x, dt}, {&w, dt}, {&b, dt}, {&lw, dt}, {&lb, dt}});
+    auto [y, mean, rstd] = lnl_fwd_raw(x, w, b, lw, lb, 1e-5, 0);
+    ctx->save_for_backward({x, w, lw, lb, mean, rstd});
+    ctx->saved_data["bias"] = b.defined();
+    return y;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const auto s = ctx->get_saved_variables();
+    const auto t = saved_types(ctx);
+    const c10::cuda::CUDAGuard guard(s[0].device());
+    Tensor dy = g[0];
+    cast_batch({{&dy, s[0].scalar_type()}});
+    auto r = lnl_bwd_raw(dy, s[0], s[1], s[2], s[3], s[4], s[5], ctx->saved_data["bias"].toBool(), 0);
+    cast_batch({{&r[0], t[0]}, {&r[1], t[1]}, {&r[2], t[2]}, {&r[3], t[3]}, {&r[4], t[4]}});
+    return {r[0], r[1], r[2], r[3], r[4]};
+  }
+};
+
+Tensor lnl(const Tensor& x, const Tensor& w, const OptTensor& b, const Tensor& lw, const OptTensor& lb) {
+  const Tensor bt = or_none(b), lbt = or_none(lb);
+  require_cuda({&x, &w, &bt, &lw, &lbt});
+  TORCH_CHECK_VALUE(w.dim() == 2 && x.dim() >= 1 && w.size(0) == x.size(-1), "Incompatible dimensions");
+  if (!at::GradMode::is_enabled()) {
+    const bool on = autocast_on();
+    Tensor xc = x, wc = w, bc = bt, lwc = lw, lbc = lbt;
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto dt = amp_type(x, on);
+    cast_batch({{&xc, dt}, {&wc, dt}, {&bc, dt}, {&lwc, dt}, {&lbc, dt}});
+    return std::get<0>(lnl_fwd_raw(xc, wc, bc, lwc, lbc, 1e-5, 0));
+  }
+  return LnlFn::apply(x, w, b, lw, lb);
+}
+
+// ---- SwiGLU ---------------------------------------------------------------------------------------------------------
+Tensor swiglu_fwd_raw(const Tensor& x) {
+  const int64_t inner = x.size(-1) / 2;
+  auto sizes = x.sizes().vec();
+  sizes.back() = inner;
+  Tensor y = at::empty(sizes, x.options());
+  check(api.mf_swiglu_fwd(x.data_ptr(), y.data_ptr(), rows_of(x), (int32_t)inner, dtype_code(x.scalar_type()), stream_of(x)), "mf_swiglu_fwd");
+  return y;
+}
+
+struct SwigluFn : torch::autograd::Function<SwigluFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_) {
+    Tensor x = x_;
+    const c10::cuda::CUDAGuard guard(x.device());
+    save_types<1>(ctx, {type_of(x)});
+    cast_batch({{&x, amp_type(x, autocast_on())}});
+    Tensor y = swiglu_fwd_raw(x);
+    ctx->save_for_backward({x});
+    return y;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const Tensor x = ctx->get_saved_variables()[0];
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor dy = g[0], dx = at::empty_like(x);
+    cast_batch({{&dy, x.scalar_type()}});
+    check(api.mf_swiglu_bwd(x.data_ptr(), dy.data_ptr(), dx.data_ptr(), rows_of(x), (int32_t)(x.size(-1) / 2), dtype_code(x.scalar_type()), stream_of(x)),
+          "mf_swiglu_bwd");
+    cast_batch({{&dx, saved_types(ctx)[0]}});
+    return {dx};
+  }
+};
+
+Tensor swiglu(const Tensor& x) {
+  require_cuda({&x});
+  TORCH_CHECK_VALUE(x.dim() >= 1 && x.size(-1) % 2 == 0, "SwiGLU needs an even last dimension");
+  return SwigluFn::apply(x);
+}
+
+// ---- Transition -------------------------------------------------------------------------------------------------------
+void check_transition(const Tensor& x, const Tensor& w1, const Tensor& w2) {
+  const int64_t dim = x.size(-1), inner = w2.dim() == 2 ? w2.size(1) : -1;
+  TORCH_CHECK_VALUE(w1.dim() == 2 && w2.dim() == 2 && w1.size(0) == dim && w1.size(1) == 2 * inner && w2.size(0) == dim, "weight shapes ", shape(w1),
+                    " / ", shape(w2), " do not fit dim=", dim);
+}
+
+std::tuple<Tensor, Tensor, Tensor> transition_fwd_raw(const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w1, const Tensor& w2, double eps,
+                                                      int64_t flags) {
+  const int64_t M = rows_of(x);
+  Tensor y = at::empty(x.sizes(), x.options()), mean = empty_f32({M}, x), rstd = empty_f32({M}, x);
+  mf_transition_fwd_args a{};
+  a.M = M; a.dim = (int32_t)x.size(-1); a.inner = (int32_t)w2.size(1); a.dtype = dtype_code(x.scalar_type()); a.flags = (uint32_t)flags; a.eps = (float)eps;
+  a.x = x.data_ptr(); a.ln_w = ptr(lw); a.ln_b = ptr(lb); a.w1 = w1.data_ptr(); a.w2 = w2.data_ptr();
+  a.y = y.data_ptr(); a.mean = mean.data_ptr<float>(); a.rstd = rstd.data_ptr<float>();
+  Tensor ws;
+  if (const size_t need = api.mf_transition_fwd_workspace_bytes(&a)) {
+    ws = workspace(need, x);
+    a.workspace = ws.data_ptr(); a.workspace_bytes = (size_t)ws.numel();
+  }
+  check(api.mf_transition_fwd(&a, stream_of(x)), "mf_transition_fwd");
+  return {y, mean, rstd};
+}
+
+// (dx, d_ln_w, d_ln_b, dw1, dw2), parameter gradients fp32
+std::array<Tensor, 5> transition_bwd_raw(const Tensor& dy, const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w1, const Tensor& w2,
+                                         const Tensor& mean, const Tensor& rstd, int64_t flags) {
+  const int64_t dim = x.size(-1), inner = w2.size(1);
+  Tensor dx = at::empty(x.sizes(), x.options());
+  Tensor dw1 = empty_f32({dim, 2 * inner}, x), dw2 = empty_f32({dim, inner}, x), dlw, dlb;
+  if (lw.defined()) dlw = empty_f32({dim}, x);
+  if (lb.defined()) dlb = empty_f32({dim}, x);
+  mf_transition_bwd_args a{};
+  a.M = rows_of(x); a.dim = (int32_t)dim; a.inner = (int32_t)inner; a.dtype = dtype_code(x.scalar_type()); a.flags = (uint32_t)flags;
+  a.x = x.data_ptr(); a.ln_w = ptr(lw); a.ln_b = ptr(lb); a.w1 = w1.data_ptr(); a.w2 = w2.data_ptr(); a.dy = dy.data_ptr();
+  a.mean = mean.data_ptr<float>(); a.rstd = rstd.data_ptr<float>();
+  a.dx = dx.data_ptr(); a.dw1 = dw1.data_ptr<float>(); a.dw2 = dw2.data_ptr<float>();
+  a.d_ln_w = static_cast<float*>(ptr(dlw)); a.d_ln_b = static_cast<float*>(ptr(dlb));
+  Tensor ws = workspace(api.mf_transition_bwd_workspace_bytes(&a), x);
+  a.workspace = ws.data_ptr(); a.workspace_bytes = (size_t)ws.numel();
+  check(api.mf_transition_bwd(&a, stream_of(x)), "mf_transition_bwd");
+  return {dx, dlw, dlb, dw1, dw2};
+}
+
+std::tuple<Tensor, Tensor, Tensor> transition_forward(const Tensor& x_, const OptTensor& lw_, const OptTensor& lb_, const Tensor& w1_, const Tensor& w2_,
+                                                      double eps, int64_t flags) {
+  Tensor x = x_, lw = or_none(lw_), lb = or_none(lb_), w1 = w1_, w2 = w2_;
+  require_cuda({&x, &lw, &lb, &w1, &w2});
+  check_transition(x, w1, w2);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto dt = x.scalar_type();
+  cast_batch({{&x, dt}, {&lw, dt}, {&lb, dt}, {&w1, dt}, {&w2, dt}});
+  return transition_fwd_raw(x, lw, lb, w1, w2, eps, flags);
+}
+
+std::array<Tensor, 5> transition_backward(const Tensor& dy_, const Tensor& x_, const OptTensor& lw_, const OptTensor& lb_, const Tensor& w1_,
+                                          const Tensor& w2_, const Tensor& mean, const Tensor& rstd, int64_t flags) {
+  Tensor dy = dy_, x = x_, lw = or_none(lw_), lb = or_none(lb_), w1 = w1_, w2 = w2_;
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto dt = x.scalar_type();
+  cast_batch({{&x, dt}, {&dy, dt}, {&lw, dt}, {&lb, dt}, {&w1, dt}, {&w2, dt}});
+  return transition_bwd_raw(dy, x, lw, lb, w1, w2, mean, rstd, flags);
+}
+
+struct TransitionFn : torch::autograd::Function<TransitionFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_, const OptTensor& lw_, const OptTensor& lb_, const Tensor& w1_, const Tensor& w2_) {
+    Tensor x = x_, lw = or_none(lw_), lb = or_none(lb_), w1 = w1_, w2 = w2_;
+    const c10::cuda::CUDAGuard guard(x.device());
+    const auto dt = amp_type(x, autocast_on());
+    save_types<5>(ctx, {type_of(x), type_of(lw), type_of(lb), type_of(w1), type_of(w2)});
+    cast_batch({{&x, dt}, {&lw, dt}, {&lb, dt}, {&w1, dt}, {&w2, dt}});
+    auto [y, mean, rstd] = transition_fwd_raw(x, lw, lb, w1, w2, 1e-5, 0);
+    ctx->save_for_backward({x, lw, lb, w1, w2, mean, rstd});
+    return y;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const auto s = ctx->get_saved_variables();
+    const auto t = saved_types(ctx);
+    const c10::cuda::CUDAGuard guard(s[0].device());
+    Tensor dy = g[0];
+    cast_batch({{&dy, s[0].scalar_type()}});
+    auto r = transition_bwd_raw(dy, s[0], s[1], s[2], s[3], s[4], s[5], s[6], 0);
+    cast_batch({{&r[0], t[0]}, {&r[1], t[1]}, {&r[2], t[2]}, {&r[3], t[3]}, {&r[4], t[4]}});
+    return {r[0], r[1], r[2], r[3], r[4]};
+  }
+};
+
+Tensor transition(const Tensor& x, const OptTensor& lw, const OptTensor& lb, const Tensor& w1, const Tensor& w2) {
+  const Tensor lwt = or_none(lw), lbt = or_none(lb);
+  require_cuda({&x, &lwt, &lbt, &w1, &w2});
+  check_transition(x, w1, w2);
+  if (!at::GradMode::is_enabled()) {
+    const auto dt = amp_type(x, autocast_on());
+    Tensor xc = x, lwc = lwt, lbc = lbt, w1c = w1, w2c = w2;
+    const c10::cuda::CUDAGuard guard(x.device());
+    cast_batch({{&xc, dt}, {&lwc, dt}, {&lbc, dt}, {&w1c, dt}, {&w2c, dt}});
+    return std::get<0>(transition_fwd_raw(xc, lwc, lbc, w1c, w2c, 1e-5, 0));
+  }
+  return TransitionFn::apply(x, lw, lb, w1, w2);
+}
+
+// std::array of tensors, undefined ones as None
+template <size_t N>
+std::array<OptTensor, N> optional(std::array<Tensor, N> r) {
+  std::array<OptTensor, N> o;
+  for (size_t i = 0; i < N; ++i)
+    if (r[i].defined()) o[i] = std::move(r[i]);
+  return o;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_native, m) {
+  using release = pybind11::call_guard<pybind11::gil_scoped_release>;
+  m.def("load", &load);
+  m.def("check_shapes", [](const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask, const OptTensor& bias) {
+    const auto s = check_shapes(q, k, v, mask, bias);
+    return std::make_tuple(s[0], s[1], s[2], s[3], s[4]);
+  });
+  m.def("evo_forward", &evo_forward, release());
+  m.def("evo_backward", &evo_backward, release());
+  m.def("evo_attention", &evo_attention, release());
+  m.def("lnl_forward", &lnl_forward, release());
+  m.def("lnl_backward", [](const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& lw, const OptTensor& lb, const Tensor& mean, const Tensor& rstd,
+                           bool has_linear_bias, int64_t flags) { return optional(lnl_backward(dy, x, w, lw, lb, mean, rstd, has_linear_bias, flags)); },
+        release());
+  m.def("lnl", &lnl, release());
+  m.def("swiglu", &swiglu, release());
+  m.def("transition_forward", &transition_forward, release());
+  m.def("transition_backward", [](const Tensor& dy, const Tensor& x, const OptTensor& lw, const OptTensor& lb, const Tensor& w1, const Tensor& w2,
+                                  const Tensor& mean, const Tensor& rstd, int64_t flags) {
+    return optional(transition_backward(dy, x, lw, lb, w1, w2, mean, rstd, flags));
+  }, release());
+  m.def("transition", &transition, release());
+}
