@@ -6,10 +6,11 @@ sum that forms d_pair_bias, so the rows are cut into chunks that flow through th
 chunk i+1, kernels of chunk i, download of chunk i-1 - and PCIe runs in both directions while the GPU computes.
 The results land in pinned host tensors; d_pair_bias is accumulated on the device over the chunks.
 
-A step issues a few hundred copies and launches, which costs the CPU more than the GPU work takes once the chunks
-are small.  So the second call with the same host buffers records the whole three-stream schedule into a CUDA
-graph and every later call replays it (one launch); a call with other buffers, or a failed capture, runs the
-schedule directly.
+A step issues about 150 copies and launches: 1 to 2 ms of host time, which the copies of a large step hide and those of
+a small one do not.  So a second call in a row with the same host buffers records the whole three-stream schedule into a
+CUDA graph and every later call replays it (one launch).  A graph is tied to its buffers and takes 10 to 40 ms to record,
+so a caller whose buffers change from call to call (a data loader with several pinned sets) gets the schedule issued
+directly each time, as does a failed capture.
 """
 from __future__ import annotations
 
@@ -59,7 +60,7 @@ class HostPipeline:
         self.out = dict(o=pin(shape, dtype), dq=pin(shape, dtype), dk=pin(shape, dtype), dv=pin(shape, dtype),
                         d_bias=pin(bias_shape, bias_dtype))
         self.keep = []
-        self.graph, self.graph_key, self.calls, self.use_graph, self.group = None, None, 0, True, None
+        self.graph, self.graph_key, self.last_key, self.use_graph, self.group = None, None, None, True, None
         self.s_cap = torch.cuda.Stream(dev)
 
     def run(self, q, k, v, res_mask, pair_bias, d_out, group=None):
@@ -76,8 +77,8 @@ class HostPipeline:
             self.graph.replay()                      # on the current stream
             cur.synchronize()
             return self.out
-        self.calls += 1
-        if self.use_graph and self.calls >= 2 and all(t.is_pinned() for t in host.values()):
+        again, self.last_key = key == self.last_key, key
+        if self.use_graph and again and all(t.is_pinned() for t in host.values()):
             try:
                 self.s_cap.wait_stream(cur)
                 g = torch.cuda.CUDAGraph()
