@@ -85,6 +85,12 @@ typedef struct mf_evo_fwd_args {
 
 MF_API int mf_evo_fwd(const mf_evo_fwd_args* args, void* stream);
 
+/* The same with scratch: a 16-bit pair bias whose rows are not multiples of 16 bytes (an odd L) or a permuted view of one
+ * is brought to a pitch that TMA can address, which the faster kernel needs.  mf_evo_fwd_workspace_bytes() is 0 where
+ * no scratch helps; with less than that (or NULL) the call runs as mf_evo_fwd does.  256-byte aligned. */
+MF_API size_t mf_evo_fwd_workspace_bytes(const mf_evo_fwd_args* args);
+MF_API int mf_evo_fwd_with_workspace(const mf_evo_fwd_args* args, void* workspace, size_t workspace_bytes, void* stream);
+
 /*
  * Backward of the above.  d_o, o: contiguous [B,N,L,H,D].  dq,dk,dv: contiguous [B,N,L,H,D] in
  * `dtype`.  d_bias: contiguous [B,1,H,L,L] in `dbias_dtype` (MF_F32 or `dtype`), the sum of dS over

@@ -85,6 +85,8 @@ class CastItem(C.Structure):
 # every symbol include/megafold_b200.h declares: name -> (restype, argtypes)
 SYMBOLS = {
     "mf_evo_fwd": (C.c_int, [C.POINTER(EvoFwdArgs), _vp]),
+    "mf_evo_fwd_workspace_bytes": (_sz, [C.POINTER(EvoFwdArgs)]),
+    "mf_evo_fwd_with_workspace": (C.c_int, [C.POINTER(EvoFwdArgs), _vp, _sz, _vp]),
     "mf_evo_bwd_workspace_bytes": (_sz, [C.POINTER(EvoBwdArgs)]),
     "mf_evo_bwd": (C.c_int, [C.POINTER(EvoBwdArgs), _vp]),
     "mf_evo_bwd_noalloc": (C.c_int, [C.POINTER(EvoBwdArgs), _vp]),

@@ -61,18 +61,29 @@ using namespace mf;
 
 extern "C" {
 
-int mf_evo_fwd(const mf_evo_fwd_args* args, void* stream) {
+static bool evo_fwd_use_tc(const mf_evo_fwd_args& a) {
+  // the tensor-core kernels write o with 16-byte stores
+  return !(a.flags & MF_FLAG_FORCE_SIMT) && ((uintptr_t)a.o & 15) == 0 &&
+         evo_tc_supported(a.B, a.N, a.L, a.H, a.D, a.dtype, a.q_strides, a.k_strides, a.v_strides, a.q, a.k, a.v);
+}
+
+size_t mf_evo_fwd_workspace_bytes(const mf_evo_fwd_args* args) {
+  if (!args) return 0;
+  return evo_fwd_use_tc(*args) ? evo_fwd_ws_workspace(*args) : 0;
+}
+
+int mf_evo_fwd_with_workspace(const mf_evo_fwd_args* args, void* workspace, size_t workspace_bytes, void* stream) {
   Range nvtx_range("mf_evo_fwd");
   MF_REQUIRE(args, MF_ERR_BAD_ARG, "args is NULL");
   const mf_evo_fwd_args& a = *args;
   int r = check_evo_common(a); if (r) return r;
   MF_REQUIRE(a.o && a.lse, MF_ERR_BAD_ARG, "o and lse must not be NULL");
+  if (!workspace) workspace_bytes = 0;
+  MF_REQUIRE(((uintptr_t)workspace & 255) == 0, MF_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   r = check_device(); if (r) return r;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // the tensor-core kernels write o with 16-byte stores
-  if (!(a.flags & MF_FLAG_FORCE_SIMT) && ((uintptr_t)a.o & 15) == 0 &&
-      evo_tc_supported(a.B, a.N, a.L, a.H, a.D, a.dtype, a.q_strides, a.k_strides, a.v_strides, a.q, a.k, a.v)) {
-    r = evo_fwd_ws_supported(a) ? evo_fwd_ws(a, st) : evo_fwd_tc(a, st);
+  if (evo_fwd_use_tc(a)) {
+    r = evo_fwd_ws_supported(a, workspace_bytes) ? evo_fwd_ws(a, workspace, st) : evo_fwd_tc(a, st);
     if (r == MF_OK) set_last_path("tcgen05");
     return r;
   }
@@ -80,6 +91,8 @@ int mf_evo_fwd(const mf_evo_fwd_args* args, void* stream) {
   if (r == MF_OK) set_last_path("simt");
   return r;
 }
+
+int mf_evo_fwd(const mf_evo_fwd_args* args, void* stream) { return mf_evo_fwd_with_workspace(args, nullptr, 0, stream); }
 
 static bool evo_bwd_use_tc(const mf_evo_bwd_args& a) {
   // the tensor-core kernels read o / d_o and write dq / dk / dv with 16-byte accesses

@@ -128,8 +128,9 @@ bool evo_tc_supported(int B, int N, int L, int H, int D, int dtype, const int64_
 int tc_async_status();
 int bounded_wait_selftest(cudaStream_t st);
 int evo_fwd_tc(const mf_evo_fwd_args& a, cudaStream_t st);
-bool evo_fwd_ws_supported(const mf_evo_fwd_args& a);
-int evo_fwd_ws(const mf_evo_fwd_args& a, cudaStream_t st);
+size_t evo_fwd_ws_workspace(const mf_evo_fwd_args& a);
+bool evo_fwd_ws_supported(const mf_evo_fwd_args& a, size_t workspace_bytes);
+int evo_fwd_ws(const mf_evo_fwd_args& a, void* workspace, cudaStream_t st);
 bool evo_bwd_ws_shape_ok(int L, int D);
 int evo_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st);
 size_t evo_bwd_ws_workspace(const mf_evo_bwd_args& a);

@@ -24,7 +24,8 @@
 //
 // delta_i = rowsum(dO_i * O_i) and the term tiles come from a small pre-kernel.  The bias tile of a half block is the A
 // operand [128 keys x 16 queries] of the products that add it: the caller's bias ([queries][keys]) is exactly that in
-// MN-major form and is loaded in place when TMA can address it; otherwise a transposed 16-bit copy is made first.  All waits are bounded
+// MN-major form and is loaded in place when TMA can address it; otherwise a 16-bit copy with a 16-byte pitch is made
+// first (copy_bias_rows: [4, 32, 384, 384] fp32 in 20 us, where the transposed copy made before took 38).  All waits are bounded
 // (tc.cuh); on expiry the CTA runs dry without touching global memory and the host sees mf_async_status() != 0.
 #include <type_traits>
 
@@ -39,7 +40,7 @@ constexpr int kHalf = 64;           // queries per half block
 constexpr int kComputeWarps = 16;
 constexpr int kThreads = (kComputeWarps + 4) * 32;
 constexpr int kTileB = 128 * 64;    // [128 x 32] 16-bit operand tile, 64-byte rows, 64B swizzle
-constexpr int kAtomB = 128 * 128;   // [128 x 64] 16-bit tile, 128-byte rows, 128B swizzle (bias^T atoms, dS^T atoms)
+constexpr int kAtomB = 128 * 128;   // [128 x 64] 16-bit tile, 128-byte rows, 128B swizzle (bias atoms, dS^T atoms)
 constexpr int kDP = 32;             // padded head size
 // Head sizes up to 64 are handled as NH = 1 or 2 halves of 32 columns: every operand is loaded as NH tiles of [128 x 32]
 // (the same layout whatever the head size), the score products run over 2 * NH slices of 16, and each half has its own
@@ -49,7 +50,7 @@ template <int NH> struct Geo {
   static constexpr int kDbStageB = 4 * NH * kTileB + 2 * 4096;      // dBias kernel: one row's Q, dO, K, V tiles and its two term tiles
   static constexpr int NQ = NH == 1 ? 3 : 2;       // (Q, dO, XQ) stages
   static constexpr int NKV = NH == 1 ? 2 : 1;      // (K, V, XK) stages
-  static constexpr int NB = NH == 1 ? 3 : 2;       // bias^T atoms
+  static constexpr int NB = NH == 1 ? 3 : 2;       // bias atoms
   static constexpr int NS = NH == 1 ? 3 : 2;       // dBias kernel: operand stages
   static constexpr size_t kMainSmem = 1024 + 4 * (size_t)kAtomB + NB * (size_t)kAtomB + (NQ + NKV) * (size_t)kStageB + 2048 + kXTileB;
   static constexpr size_t kDbSmem = 1024 + 2 * (size_t)kAtomB + NS * (size_t)kDbStageB + 2048 + kXTileB;
@@ -72,7 +73,6 @@ struct BwdWsP {
   uint32_t fmt, bfmt;
   int n_alpha; float alpha[2];
   int bias_b_mul;
-  int bias_mn;           // the bias atoms hold the caller's bias as it is ([queries][keys]) and are read MN-major
   const uint8_t* xq; const uint8_t* xk;     // rank-one term tiles (evo_extras_ws_kernel)
   const int* flags;                         // per (b, n, h): every key of the row is masked
   void* dbias_direct;                       // N == 1 and a 16-bit d_pair_bias: dS is the answer, written by this kernel
@@ -154,49 +154,6 @@ __global__ void evo_extras_ws_kernel(const T* __restrict__ o, const T* __restric
   }
 }
 
-// biasT[b][h][j][i] = bias[b][h][i][j] in the 16-bit type TO, rows padded to `lpad` entries (the padding is zeroed by
-// the caller).  The kernels work with keys on the TMEM lanes, so the tile they need has the queries contiguous.
-template <typename TB, typename TO>
-__global__ void transpose_bias_ws_kernel(const TB* __restrict__ bias, TO* __restrict__ biasT, int H, int L, int lpad,
-                                         int64_t sb, int64_t sh, int64_t si, int64_t sj) {
-  // 64 x 64 tiles; a thread moves two neighbouring entries at a time, on the way in (two keys of one query) and on the
-  // way out (two queries of one key), so that a warp reads and writes 128 or more contiguous bytes
-  __shared__ float tile[64][65];
-  const int bh = blockIdx.z, b = bh / H, h = bh % H;
-  const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
-  const TB* src = bias + b * sb + h * sh;
-  const bool pair_in = sj == 1 && sizeof(TB) == 2 && (si & 1) == 0 && (((sb | sh) & 1) == 0) && (reinterpret_cast<uintptr_t>(bias) & 3) == 0;
-  for (int k = threadIdx.y; k < 64; k += blockDim.y) {
-    const int i = i0 + k, j = j0 + 2 * threadIdx.x;
-    if (i >= L) continue;
-    bool done = false;
-    if constexpr (sizeof(TB) == 2) {
-      if (pair_in && j + 1 < L) {
-        const uint32_t v = *reinterpret_cast<const uint32_t*>(src + (int64_t)i * si + j);
-        TB lo, hi;
-        *reinterpret_cast<unsigned short*>(&lo) = (unsigned short)(v & 0xffffu);
-        *reinterpret_cast<unsigned short*>(&hi) = (unsigned short)(v >> 16);
-        tile[k][2 * threadIdx.x] = to_f(lo); tile[k][2 * threadIdx.x + 1] = to_f(hi);
-        done = true;
-      }
-    }
-    if (!done) {
-      if (j < L) tile[k][2 * threadIdx.x] = to_f(src[(int64_t)i * si + (int64_t)j * sj]);
-      if (j + 1 < L) tile[k][2 * threadIdx.x + 1] = to_f(src[(int64_t)i * si + (int64_t)(j + 1) * sj]);
-    }
-  }
-  __syncthreads();
-  for (int k = threadIdx.y; k < 64; k += blockDim.y) {
-    const int j = j0 + k, i = i0 + 2 * threadIdx.x;
-    if (j >= L || i >= L) continue;
-    TO* dst = biasT + ((int64_t)bh * L + j) * lpad + i;         // lpad is a multiple of 128 and i is even: 4-byte aligned
-    const TO a = from_f<TO>(tile[2 * threadIdx.x][k]);
-    const TO c = i + 1 < L ? from_f<TO>(tile[2 * threadIdx.x + 1][k]) : from_f<TO>(0.f);
-    uint32_t v = (uint32_t)*reinterpret_cast<const unsigned short*>(&a) | ((uint32_t)*reinterpret_cast<const unsigned short*>(&c) << 16);
-    *reinterpret_cast<uint32_t*>(dst) = v;
-  }
-}
-
 // P^T and dS^T of one thread for 16 query columns.  sr: scores S''^T with the bias, mask and log-sum-exp terms already
 // inside (see the rank-one terms above), dr: dP^T - delta.  Results packed two queries per word.  `careful`: the row (b, n)
 // has every key masked - P is uniform over the keys of the row and no gradient passes through the (masked) logits.
@@ -229,7 +186,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   constexpr int kStageB = Geo<NH>::kStageB, NQ = Geo<NH>::NQ, NKV = Geo<NH>::NKV, NB = Geo<NH>::NB;
   uint8_t* sDS = smem;                          // [2 blocks][2 atoms]: dS^T tiles for the dQ product
-  uint8_t* sBT = sDS + 4 * kAtomB;              // bias^T atoms, ring of NB
+  uint8_t* sBT = sDS + 4 * kAtomB;              // bias atoms, ring of NB
   uint8_t* sKV = sBT + NB * kAtomB;             // [NKV stages][K halves, V halves, XK]
   uint8_t* sQD = sKV + NKV * kStageB;           // [NQ stages][Q halves, dO halves, XQ]
   uint8_t* sI = sQD + NQ * kStageB;             // alpha * I, two terms
@@ -566,14 +523,13 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       // ========================================================================== score issuer: per half block
       //   S''^T = K_j Q_i^T + alpha * bias^T,  dP^T = V_j dO_i^T
       const uint32_t id_s = idesc_f16(128, kHalf, p.fmt, 0, 0);
-      // The bias atom of a half block is the A operand [128 keys x 64 queries] of four K = 16 products.  Either it holds
-      // rows of a transposed copy of the bias (keys as rows, K-major A), or - when TMA can address the caller's bias - the
-      // bias as it is: two [64 queries x 64 keys] pieces read MN-major (keys contiguous), and no copy is made.
-      const uint32_t id_b = idesc_f16(128, 16, p.bfmt, p.bias_mn ? 1u : 0u, 0);
+      // The bias atom of a half block is the A operand [128 keys x 64 queries] of four K = 16 products: two pieces
+      // [64 queries x 64 keys] of the bias as it is, read MN-major (keys contiguous).
+      const uint32_t id_b = idesc_f16(128, 16, p.bfmt, 1, 0);
       const uint32_t id_x = idesc_f16(128, kHalf, 1u, 0, 0);        // the rank-one term tiles are bf16 whatever q/k/v are
       const uint32_t xc_lo = desc_lo(smem_u32(sXC), 16);
-      const uint32_t bt_base = desc_lo(smem_u32(sBT), p.bias_mn ? 8192 : 16);
-      const uint32_t bstep = p.bias_mn ? 2048 / 16 : 2;            // 16 queries further: 16 rows of 128 bytes, or 32 bytes
+      const uint32_t bt_base = desc_lo(smem_u32(sBT), 8192);
+      constexpr uint32_t bstep = 2048 / 16;                        // 16 queries further: 16 rows of 128 bytes
       const uint32_t i_lo0 = desc_lo(smem_u32(sI), 16), i_lo1 = i_lo0 + 1024 / 16;
       const bool two_terms = p.n_alpha > 1;
       MF_TRACE_DECL(tr, 3, blockIdx.x == 0 && lane == 0);
@@ -665,12 +621,9 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
               if (dead()) break;
               if (elect_one()) {
                 mbar_expect_tx(&bar.bt_full[bslot], kAtomB);
-                if (p.bias_mn) {       // [64 queries x 64 keys] pieces of the bias itself: keys 0-63 | 64-127 of the tile
-                  tma_load_4d(sBT + bslot * kAtomB, &mbt, &bar.bt_full[bslot], jt * kT, it * kT + half * kHalf, h, b * p.bias_b_mul);
-                  tma_load_4d(sBT + bslot * kAtomB + 8192, &mbt, &bar.bt_full[bslot], jt * kT + 64, it * kT + half * kHalf, h, b * p.bias_b_mul);
-                } else {
-                  tma_load_4d(sBT + bslot * kAtomB, &mbt, &bar.bt_full[bslot], it * kT + half * kHalf, jt * kT, h, b * p.bias_b_mul);
-                }
+                // [64 queries x 64 keys] pieces of the bias: keys 0-63 | 64-127 of the tile
+                tma_load_4d(sBT + bslot * kAtomB, &mbt, &bar.bt_full[bslot], jt * kT, it * kT + half * kHalf, h, b * p.bias_b_mul);
+                tma_load_4d(sBT + bslot * kAtomB + 8192, &mbt, &bar.bt_full[bslot], jt * kT + 64, it * kT + half * kHalf, h, b * p.bias_b_mul);
               }
               ++nbt;
               if (++bslot == NB) { bslot = 0; ++buse; }
@@ -700,7 +653,6 @@ struct DbP {
   uint32_t fmt, bfmt;
   int n_alpha; float alpha[2];
   int bias_b_mul;
-  int bias_mn;            // as in BwdWsP
   const uint8_t* xq; const uint8_t* xk;      // rank-one term tiles (evo_extras_ws_kernel)
   float* part;            // fp32 [nsplit][B][H][L][L] partial sums
   void* out16;            // with a single row range and a 16-bit d_bias: the result itself, [B][H][L][L] in the q/k/v type
@@ -709,7 +661,7 @@ struct DbP {
 
 struct DbBars {
   uint64_t op_full[3], op_empty[3];          // Q, dO, K, V, XQ, XK of one row n
-  uint64_t bt_full, bt_free;                 // the unit's two bias^T atoms
+  uint64_t bt_full, bt_free;                 // the unit's two bias atoms
   uint64_t sd_ready[2], loaded[2];
 };
 
@@ -720,7 +672,7 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
                     const __grid_constant__ CUtensorMap mbt, const DbP p MF_TRACE_PARAM) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sBT = smem;                          // two bias^T atoms (queries 0-63 | 64-127 of the tile)
+  uint8_t* sBT = smem;                          // two bias atoms (queries 0-63 | 64-127 of the tile)
   constexpr int kDbStageB = Geo<NH>::kDbStageB, NS = Geo<NH>::NS;
   uint8_t* sOP = sBT + 2 * kAtomB;              // [NS stages][Q halves, dO halves, K halves, V halves, XQ, XK]
   uint8_t* sI = sOP + NS * kDbStageB;
@@ -838,9 +790,9 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
     const uint32_t id_x = idesc_f16(128, 128, 1u, 0, 0);          // the rank-one term tiles are bf16 whatever q/k/v are
     if (warp == kComputeWarps) {
       // ========================================================================== score issuer: S''^T = K Q^T + alpha * bias^T
-      const uint32_t id_b = idesc_f16(128, 16, p.bfmt, p.bias_mn ? 1u : 0u, 0);      // see the main kernel's score issuer
-      const uint32_t bt_lo = desc_lo(smem_u32(sBT), p.bias_mn ? 8192 : 16);
-      const uint32_t bstep = p.bias_mn ? 2048 / 16 : 2;
+      const uint32_t id_b = idesc_f16(128, 16, p.bfmt, 1, 0);      // see the main kernel's score issuer
+      const uint32_t bt_lo = desc_lo(smem_u32(sBT), 8192);
+      constexpr uint32_t bstep = 2048 / 16;
       const uint32_t i_lo0 = desc_lo(smem_u32(sI), 16), i_lo1 = i_lo0 + 1024 / 16;
       const bool two_terms = p.n_alpha > 1;
       MF_TRACE_DECL(tr, 2, blockIdx.x == 0 && lane == 0);
@@ -908,15 +860,10 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
         if (dead()) break;
         if (elect_one()) {
           mbar_expect_tx(&bar.bt_full, 2 * kAtomB);
-          if (p.bias_mn) {
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4)       // (query half, key half) pieces of [64 x 64]
-              tma_load_4d(sBT + (q4 >> 1) * kAtomB + (q4 & 1) * 8192, &mbt, &bar.bt_full, x.jt * kT + (q4 & 1) * 64,
-                          x.it * kT + (q4 >> 1) * kHalf, x.h, x.b * p.bias_b_mul);
-          } else {
-            tma_load_4d(sBT, &mbt, &bar.bt_full, x.it * kT, x.jt * kT, x.h, x.b * p.bias_b_mul);
-            tma_load_4d(sBT + kAtomB, &mbt, &bar.bt_full, x.it * kT + kHalf, x.jt * kT, x.h, x.b * p.bias_b_mul);
-          }
+          for (int q4 = 0; q4 < 4; ++q4)       // (query half, key half) pieces of [64 x 64]
+            tma_load_4d(sBT + (q4 >> 1) * kAtomB + (q4 & 1) * 8192, &mbt, &bar.bt_full, x.jt * kT + (q4 & 1) * 64,
+                        x.it * kT + (q4 >> 1) * kHalf, x.h, x.b * p.bias_b_mul);
         }
         for (int n = x.n0; n < x.n1; ++n, ++g) {
           if (suse >= 1) wait_or_flag(&bar.op_empty[stage], (suse - 1) & 1, abort_flag);
@@ -987,22 +934,10 @@ int bwd_ksplit(int64_t bnh, int nt, int sms) {
   return k < 1 ? 1 : (int)k;
 }
 
-// Can TMA address the caller's bias ([.., queries, keys], 16-bit, keys contiguous, 16-byte multiples elsewhere)?  Then its
-// tiles are loaded as they are and read MN-major; otherwise a transposed 16-bit copy is made first.
-bool bias_tma_ok(const mf_evo_bwd_args& a) {
-  if (a.bias_dtype != MF_BF16 && a.bias_dtype != MF_F16) return false;
-  const int64_t* s = a.bias_strides;
-  if (s[3] != 1 || (reinterpret_cast<uintptr_t>(a.bias) & 15) != 0) return false;
-  if ((s[2] * 2) % 16 != 0 || s[2] <= 0) return false;
-  if (a.H > 1 && ((s[1] * 2) % 16 != 0 || s[1] <= 0)) return false;
-  if (a.B > 1 && s[0] != 0 && ((s[0] * 2) % 16 != 0 || s[0] < 0)) return false;
-  return true;
-}
-
 struct BwdPlan {
   int nt, lpad, ksplit, dq_stream, dbuf, nsplit;
   bool dq_fp32, part_direct, bias_direct;
-  size_t off_flags, off_xq, off_xk, off_part, off_dq, off_biasT, total;
+  size_t off_flags, off_xq, off_xk, off_part, off_dq, off_bias, total;
 };
 
 BwdPlan plan_bwd(const mf_evo_bwd_args& a) {
@@ -1034,8 +969,8 @@ BwdPlan plan_bwd(const mf_evo_bwd_args& a) {
   pl.off_xk = off; off += (size_t)a.B * a.N * pl.nt * kXTileB;
   pl.off_part = off; if (!pl.part_direct) off += align_up(sizeof(float) * (size_t)pl.nsplit * a.B * a.H * a.L * a.L, 256);
   pl.off_dq = off; if (pl.dq_fp32) off += align_up(sizeof(float) * (size_t)a.B * a.N * a.L * a.H * a.D, 256);
-  pl.bias_direct = bias_tma_ok(a);
-  pl.off_biasT = off; if (!pl.bias_direct) off += align_up(2 * (size_t)a.B * a.H * a.L * pl.lpad, 256);
+  pl.bias_direct = bias_tma_ok(a.bias, a.bias_dtype, a.bias_strides, a.B, a.H);
+  pl.off_bias = off; if (!pl.bias_direct) off += bias_copy_bytes(a.bias_strides, a.B, a.H, a.L);
   pl.total = off;
   return pl;
 }
@@ -1059,27 +994,23 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
   uint8_t* xk = reinterpret_cast<uint8_t*>(ws + pl.off_xk);
   float* part = !pl.part_direct ? reinterpret_cast<float*>(ws + pl.off_part) : (a.dbias_dtype == MF_F32 ? static_cast<float*>(a.d_bias) : nullptr);
   float* dq_acc = reinterpret_cast<float*>(ws + pl.off_dq);
-  // the transposed bias copy is kept in a 16-bit type: the bias dtype when that is one, else the q/k/v dtype
+  // a bias that TMA cannot address is copied in a 16-bit type: the bias dtype when that is one, else the q/k/v dtype
   using TT = typename std::conditional<sizeof(TB) == 2, TB, T>::type;
   const int bt_dtype = sizeof(TB) == 2 ? a.bias_dtype : a.dtype;
-  TT* biasT = reinterpret_cast<TT*>(ws + pl.off_biasT);
   const int lpad = pl.lpad;
-  const int bias_b_mul = pl.bias_direct ? (a.bias_strides[0] == 0 ? 0 : 1) : 1;
-  if (pl.bias_direct) {
+  const int bias_b_mul = a.bias_strides[0] == 0 ? 0 : 1;
+  {
+    const void* bias = a.bias;
+    int64_t str[4] = {1, a.bias_strides[2], a.bias_strides[1], a.bias_strides[0]};
+    if (!pl.bias_direct) {
+      void* copy = ws + pl.off_bias;
+      if ((r = copy_bias_rows(a.bias, a.bias_dtype, a.bias_strides, copy, bt_dtype, a.B, a.H, a.L, st))) return r;
+      bias = copy;
+      str[1] = bias_pitch(a.L); str[2] = str[1] * a.L; str[3] = str[2] * a.H;
+    }
     const int64_t dims[4] = {a.L, a.L, a.H, bias_b_mul ? a.B : 1};
-    const int64_t str[4] = {1, a.bias_strides[2], a.bias_strides[1], a.bias_strides[0]};
     const int box[4] = {64, 64, 1, 1};
-    if ((r = make_tiled_map(&mbt, a.bias, a.bias_dtype, 4, dims, str, box, 128))) return r;
-  } else {
-    if (lpad != a.L) MF_CUDA(cudaMemsetAsync(biasT, 0, 2 * (size_t)a.B * a.H * a.L * lpad, st));      // the row padding
-    dim3 grid((a.L + 63) / 64, (a.L + 63) / 64, a.B * a.H), block(32, 8);
-    transpose_bias_ws_kernel<TB, TT><<<grid, block, 0, st>>>(static_cast<const TB*>(a.bias), biasT, a.H, a.L, lpad, a.bias_strides[0],
-                                                             a.bias_strides[1], a.bias_strides[2], a.bias_strides[3]);
-    MF_LAUNCHED("transpose_bias_ws_kernel");
-    const int64_t dims[4] = {lpad, a.L, a.H, a.B};
-    const int64_t str[4] = {1, lpad, (int64_t)a.L * lpad, (int64_t)a.H * a.L * lpad};
-    const int box[4] = {kHalf, 128, 1, 1};
-    if ((r = make_tiled_map(&mbt, biasT, bt_dtype, 4, dims, str, box, 128))) return r;
+    if ((r = make_tiled_map(&mbt, bias, bt_dtype, 4, dims, str, box, 128))) return r;
   }
   MF_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)a.B * a.N * a.H, st));
   {
@@ -1106,7 +1037,7 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     p.c1 = kLog2e / sqrtf((float)a.D);
     p.fmt = a.dtype == MF_BF16 ? 1u : 0u; p.bfmt = bt_dtype == MF_BF16 ? 1u : 0u;
     p.n_alpha = n_alpha; p.alpha[0] = alpha[0]; p.alpha[1] = alpha[1];
-    p.bias_b_mul = bias_b_mul; p.bias_mn = pl.bias_direct ? 1 : 0;
+    p.bias_b_mul = bias_b_mul;
     p.xq = xq; p.xk = xk;
     p.part = part;
     p.out16 = pl.part_direct && a.dbias_dtype != MF_F32 ? a.d_bias : nullptr;
@@ -1138,7 +1069,7 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     p.scale = 1.0f / sqrtf((float)a.D); p.c1 = kLog2e * p.scale; p.inv_L = 1.0f / a.L;
     p.fmt = a.dtype == MF_BF16 ? 1u : 0u; p.bfmt = bt_dtype == MF_BF16 ? 1u : 0u;
     p.n_alpha = n_alpha; p.alpha[0] = alpha[0]; p.alpha[1] = alpha[1];
-    p.bias_b_mul = bias_b_mul; p.bias_mn = pl.bias_direct ? 1 : 0;
+    p.bias_b_mul = bias_b_mul;
     p.xq = xq; p.xk = xk; p.flags = flags;
     p.dbias_direct = dbias_direct ? a.d_bias : nullptr;
     p.dq = a.dq; p.dk = a.dk; p.dv = a.dv;

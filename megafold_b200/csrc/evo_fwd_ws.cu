@@ -500,20 +500,31 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, cudaStream_t st) {
 
 }  // namespace
 
-// The warp-specialised kernel covers head sizes up to 32, rows up to 2048 tokens and a 16-bit pair bias whose rows
-// TMA can address (unit stride on keys, 16-byte multiples elsewhere); other calls use the general kernel.
-bool evo_fwd_ws_supported(const mf_evo_fwd_args& a) {
-  if (a.D > 32 || a.L > 2048) return false;
-  if (a.bias_dtype != MF_BF16 && a.bias_dtype != MF_F16) return false;
-  const int64_t* s = a.bias_strides;
-  if (s[3] != 1 || (reinterpret_cast<uintptr_t>(a.bias) & 15) != 0) return false;
-  if ((s[2] * 2) % 16 != 0 || s[2] <= 0) return false;
-  if (a.H > 1 && ((s[1] * 2) % 16 != 0 || s[1] <= 0)) return false;
-  if (a.B > 1 && s[0] != 0 && ((s[0] * 2) % 16 != 0 || s[0] < 0)) return false;
-  return true;
+// The warp-specialised kernel covers head sizes up to 32, rows up to 2048 tokens and a 16-bit pair bias; other calls use
+// the general kernel.
+static bool shape_ok(const mf_evo_fwd_args& a) { return a.D <= 32 && a.L <= 2048 && (a.bias_dtype == MF_BF16 || a.bias_dtype == MF_F16); }
+
+// A bias whose rows TMA cannot address (a chain of odd length) is copied to a 16-byte pitch when the caller gives the
+// scratch for it: an exact copy, and 3 us against the 1000 us that the general kernel's reads of such a bias in place cost
+// at [467, 467, 4, 32].
+size_t evo_fwd_ws_workspace(const mf_evo_fwd_args& a) {
+  if (!shape_ok(a) || bias_tma_ok(a.bias, a.bias_dtype, a.bias_strides, a.B, a.H)) return 0;
+  return bias_copy_bytes(a.bias_strides, a.B, a.H, a.L);
+}
+bool evo_fwd_ws_supported(const mf_evo_fwd_args& a, size_t workspace_bytes) {
+  return shape_ok(a) && workspace_bytes >= evo_fwd_ws_workspace(a);
 }
 
-int evo_fwd_ws(const mf_evo_fwd_args& a, cudaStream_t st) {
+int evo_fwd_ws(const mf_evo_fwd_args& args, void* workspace, cudaStream_t st) {
+  mf_evo_fwd_args a = args;
+  if (evo_fwd_ws_workspace(args)) {
+    int r = copy_bias_rows(a.bias, a.bias_dtype, a.bias_strides, workspace, a.bias_dtype, a.B, a.H, a.L, st);
+    if (r) return r;
+    const int64_t row = bias_pitch(a.L);
+    a.bias = workspace;
+    a.bias_strides[3] = 1; a.bias_strides[2] = row; a.bias_strides[1] = row * a.L;
+    a.bias_strides[0] = args.bias_strides[0] == 0 ? 0 : row * a.L * a.H;
+  }
   if (a.dtype == MF_BF16)
     return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16>(a, st) : launch_fwd_ws<__nv_bfloat16, __half>(a, st);
   return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16>(a, st) : launch_fwd_ws<__half, __half>(a, st);

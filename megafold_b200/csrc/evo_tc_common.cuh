@@ -298,6 +298,25 @@ inline bool qkv_strides_ok(const void* p, const int64_t* s, int B, int N, int L,
   return true;
 }
 
+// Can TMA address a pair bias with these strides (element strides b, h, query, key): a 16-bit type, keys contiguous,
+// 16-byte multiples elsewhere?
+inline bool bias_tma_ok(const void* bias, int dtype, const int64_t* s, int B, int H) {
+  if (dtype != MF_BF16 && dtype != MF_F16) return false;
+  if (s[3] != 1 || (reinterpret_cast<uintptr_t>(bias) & 15) != 0) return false;
+  if ((s[2] * 2) % 16 != 0 || s[2] <= 0) return false;
+  if (H > 1 && ((s[1] * 2) % 16 != 0 || s[1] <= 0)) return false;
+  if (B > 1 && s[0] != 0 && ((s[0] * 2) % 16 != 0 || s[0] < 0)) return false;
+  return true;
+}
+// A pair bias that TMA cannot address (rows of an odd length, fp32, a permuted view) is first copied to
+// [B, H, L, bias_pitch(L)] in a 16-bit type; a bias shared by the batch elements is copied once.
+inline int bias_pitch(int L) { return (L + 7) / 8 * 8; }
+inline int bias_copies(const int64_t* s, int B) { return s[0] == 0 ? 1 : B; }
+inline size_t bias_copy_bytes(const int64_t* s, int B, int H, int L) {
+  return align_up(2 * (size_t)bias_copies(s, B) * H * L * bias_pitch(L), 256);
+}
+int copy_bias_rows(const void* bias, int dtype, const int64_t* s, void* dst, int dst_dtype, int B, int H, int L, cudaStream_t st);
+
 // Status word of the calling thread's device: pinned host memory mapped into the device, so that a
 // kernel that gave up on a bounded wait can say so and the host can read it without a device sync.
 struct StatusWord { int* host = nullptr; int* dev = nullptr; };

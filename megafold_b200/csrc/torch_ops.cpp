@@ -30,7 +30,8 @@ using OptTensor = std::optional<Tensor>;
 
 #define MF_ENTRY(name) decltype(&::name) name = nullptr
 struct Api {
-  MF_ENTRY(mf_evo_fwd);
+  MF_ENTRY(mf_evo_fwd_workspace_bytes);
+  MF_ENTRY(mf_evo_fwd_with_workspace);
   MF_ENTRY(mf_evo_bwd_workspace_bytes);
   MF_ENTRY(mf_evo_bwd);
   MF_ENTRY(mf_lnl_fwd);
@@ -56,7 +57,7 @@ void load(const std::string& path) {
     return p;
   };
 #define MF_LOAD(name) api.name = reinterpret_cast<decltype(api.name)>(get(#name))
-  MF_LOAD(mf_evo_fwd); MF_LOAD(mf_evo_bwd_workspace_bytes); MF_LOAD(mf_evo_bwd);
+  MF_LOAD(mf_evo_fwd_workspace_bytes); MF_LOAD(mf_evo_fwd_with_workspace); MF_LOAD(mf_evo_bwd_workspace_bytes); MF_LOAD(mf_evo_bwd);
   MF_LOAD(mf_lnl_fwd); MF_LOAD(mf_lnl_bwd_workspace_bytes); MF_LOAD(mf_lnl_bwd);
   MF_LOAD(mf_swiglu_fwd); MF_LOAD(mf_swiglu_bwd);
   MF_LOAD(mf_transition_fwd_workspace_bytes); MF_LOAD(mf_transition_fwd);
@@ -173,7 +174,10 @@ std::tuple<Tensor, Tensor> evo_forward(const Tensor& q, const Tensor& k, const T
   mf_evo_fwd_args a{};
   fill_common(a, q, k, v, mask, bias, flags);
   a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
-  check(api.mf_evo_fwd(&a, stream_of(q)), "mf_evo_fwd");
+  Tensor ws;
+  const size_t need = api.mf_evo_fwd_workspace_bytes(&a);
+  if (need) ws = workspace(need, q);
+  check(api.mf_evo_fwd_with_workspace(&a, ptr(ws), need, stream_of(q)), "mf_evo_fwd");
   return {o, lse};
 }
 
