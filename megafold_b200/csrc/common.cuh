@@ -11,6 +11,7 @@
 #include <stdio.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/megafold_b200.h"
 
@@ -49,6 +50,22 @@ inline int after_launch(const char* name) {
 }
 #define MF_LAUNCHED(name) \
   do { int r__ = ::mf::after_launch(name); if (r__ != MF_OK) return r__; } while (0)
+
+// Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device; the call costs the host about as much
+// as a launch, so what has been granted is remembered.
+template <auto Kernel>
+int opt_in_smem(size_t bytes) {
+  static std::atomic<int> granted[64];
+  static std::mutex mu;
+  int dev = 0;
+  MF_CUDA(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < 64 && granted[dev].load(std::memory_order_acquire) >= (int)bytes) return MF_OK;
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev >= 0 && dev < 64 && granted[dev].load(std::memory_order_relaxed) >= (int)bytes) return MF_OK;
+  MF_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  if (dev >= 0 && dev < 64) granted[dev].store((int)bytes, std::memory_order_release);
+  return MF_OK;
+}
 
 inline size_t dtype_size(int dt) {
   switch (dt) {

@@ -99,12 +99,14 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
 // and, for h == 0, the XK row of key i.  Consecutive threads take the heads of one token, then the next token: a warp
 // reads one contiguous piece of o and dO.  (Measured against a thread per token walking all heads, and against
 // consecutive threads taking consecutive tokens of one head: 22.8 us against 27.3 and 28.5 at the benchmark size.)
-// flags[bnh] is raised when the row (b, n) has every key masked (lse = -FLT_MAX).
+// flags[bnh]: the row (b, n) has every key masked (lse = -FLT_MAX, for all of its queries alike).  The fp32 accumulator of
+// dQ, where one is used, is cleared here as well: each memset in front of the kernels cost 2 us of GPU time and as much of
+// the host's.
 template <typename T>
 __global__ void evo_extras_ws_kernel(const T* __restrict__ o, const T* __restrict__ d_o, const float* __restrict__ lse,
                                      const void* __restrict__ mask, int64_t ms_b, int64_t ms_n, int64_t ms_l, int mask_dtype,
                                      uint8_t* __restrict__ xq, uint8_t* __restrict__ xk, int* __restrict__ flags,
-                                     int64_t n_threads, int N, int L, int lpad, int H, int D) {
+                                     float* __restrict__ dq_acc, int64_t n_threads, int N, int L, int lpad, int H, int D) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_threads) return;
   const int hg = (int)(idx % H); const int64_t t = idx / H; const int i = (int)(t % lpad); const int64_t bn = t / lpad;
@@ -131,7 +133,11 @@ __global__ void evo_extras_ws_kernel(const T* __restrict__ o, const T* __restric
       }
       nd = -dl;
       const float lv = lse[bnh * L + i];
-      if (lv <= -3e38f) flags[bnh] = 1; else nl = -lv * sqrt_d;
+      const bool masked = lv <= -3e38f;
+      if (!masked) nl = -lv * sqrt_d;
+      if (i == 0) flags[bnh] = masked;
+      if (dq_acc)
+        for (int c = 0; c < D / 4; ++c) reinterpret_cast<float4*>(dq_acc + row * D)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __nv_bfloat16 a[3], b[3];
     split3(nl, a); split3(nd, b);
@@ -1012,16 +1018,14 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     const int box[4] = {64, 64, 1, 1};
     if ((r = make_tiled_map(&mbt, bias, bt_dtype, 4, dims, str, box, 128))) return r;
   }
-  MF_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)a.B * a.N * a.H, st));
   {
     const int64_t n_threads = (int64_t)a.B * a.N * lpad * a.H;
     evo_extras_ws_kernel<T><<<(unsigned)((n_threads + 255) / 256), 256, 0, st>>>(static_cast<const T*>(a.o), static_cast<const T*>(a.d_o), a.lse,
                                                                              a.mask, a.mask_strides[0], a.mask_strides[1], a.mask_strides[2], a.mask_dtype,
-                                                                             xq, xk, flags, n_threads, a.N, a.L, lpad, a.H, a.D);
+                                                                             xq, xk, flags, pl.dq_fp32 ? dq_acc : nullptr, n_threads, a.N, a.L, lpad, a.H, a.D);
   }
   MF_LAUNCHED("evo_extras_ws_kernel");
   const int64_t n_dq = (int64_t)a.B * a.N * a.L * a.H * a.D;
-  if (pl.dq_fp32) MF_CUDA(cudaMemsetAsync(dq_acc, 0, sizeof(float) * (size_t)n_dq, st));
 
   float alpha[2];
   const int n_alpha = split_alpha(a.D, bt_dtype, alpha);
@@ -1045,8 +1049,8 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     const size_t smem = Geo<NH>::kDbSmem;
     int grid = sm_count();
     if (grid > p.n_units) grid = p.n_units;
-    auto kern = evo_dbias_ws_kernel<T, TT, NH>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = evo_dbias_ws_kernel<T, TT, NH>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     MF_LAUNCHED("evo_dbias_ws_kernel");
     if (!pl.part_direct) {
@@ -1078,12 +1082,12 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     int grid = sm_count();
     if (grid > p.n_items) grid = p.n_items;
     if (pl.dq_stream) {
-      auto kern = evo_bwd_ws_kernel<T, TT, true, NH>;
-      MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      constexpr auto kern = evo_bwd_ws_kernel<T, TT, true, NH>;
+      if (int e = opt_in_smem<kern>(smem)) return e;
       kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     } else {
-      auto kern = evo_bwd_ws_kernel<T, TT, false, NH>;
-      MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      constexpr auto kern = evo_bwd_ws_kernel<T, TT, false, NH>;
+      if (int e = opt_in_smem<kern>(smem)) return e;
       kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     }
     MF_LAUNCHED("evo_bwd_ws_kernel");

@@ -488,11 +488,13 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, cudaStream_t st) {
   if (grid > pairs) grid = pairs;
   p.items_per_stream = (p.n_items + 2 * grid - 1) / (2 * grid);
   const size_t smem = 1024 + 2 * (size_t)kStreamBytes + 2048 + kXTileB;
-  auto kern = evo_fwd_ws_kernel<T, TB>;
-  cudaFuncAttributes fa;
-  MF_CUDA(cudaFuncGetAttributes(&fa, kern));
-  MF_REQUIRE(fa.numRegs == kLaunchRegs, MF_ERR_CUDA, "evo_fwd_ws_kernel was built with %d registers per thread, %d expected", fa.numRegs, kLaunchRegs);
-  MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr auto kern = evo_fwd_ws_kernel<T, TB>;
+  static const int regs = [] {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : -1;
+  }();
+  MF_REQUIRE(regs == kLaunchRegs, MF_ERR_CUDA, "evo_fwd_ws_kernel was built with %d registers per thread, %d expected", regs, kLaunchRegs);
+  if (int e = opt_in_smem<kern>(smem)) return e;
   kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p MF_TRACE_ARG);
   MF_LAUNCHED("evo_fwd_ws_kernel");
   return MF_OK;

@@ -447,12 +447,12 @@ int launch_fwd(const mf_evo_fwd_args& a, cudaStream_t st) {
   p.items_per_stream = (p.n_items + 2 * grid - 1) / (2 * grid);
   const size_t smem = 1024 + 2 * (size_t)C::STREAM_BYTES(btma) + 2 * sizeof(float) * p.lpad;
   if (btma) {
-    auto kern = evo_fwd_tc_kernel<DP, T, TB, true>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = evo_fwd_tc_kernel<DP, T, TB, true>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p);
   } else {
-    auto kern = evo_fwd_tc_kernel<DP, T, TB, false>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = evo_fwd_tc_kernel<DP, T, TB, false>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p);
   }
   MF_LAUNCHED("evo_fwd_tc_kernel");

@@ -257,12 +257,12 @@ int gemm_tc(const GemmTcArgs& g, cudaStream_t st) {
   const int n_items = p.m_tiles * p.n_tiles * p.k_splits;
   int grid = sms < n_items ? sms : n_items;
   if (g.dtype == MF_BF16) {
-    auto kern = gemm_tc_kernel<__nv_bfloat16>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = gemm_tc_kernel<__nv_bfloat16>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(ma, mb, mc, p);
   } else {
-    auto kern = gemm_tc_kernel<__half>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = gemm_tc_kernel<__half>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(ma, mb, mc, p);
   }
   MF_LAUNCHED("gemm_tc_kernel");

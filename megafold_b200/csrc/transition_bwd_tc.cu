@@ -418,12 +418,12 @@ int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, flo
   int grid = sm_count();
   if (grid > p.n_mt) grid = p.n_mt;
   if (a.dtype == MF_BF16) {
-    auto kern = transition_bwd_tc_kernel<__nv_bfloat16>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = transition_bwd_tc_kernel<__nv_bfloat16>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, p);
   } else {
-    auto kern = transition_bwd_tc_kernel<__half>;
-    MF_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = transition_bwd_tc_kernel<__half>;
+    if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, p);
   }
   MF_LAUNCHED("transition_bwd_tc_kernel");
