@@ -1,6 +1,7 @@
 // C ABI of the library: argument validation and dispatch to the kernel families.
 #include "common.cuh"
 
+#include <cuda.h>
 #include <nvtx3/nvToolsExt.h>
 
 namespace mf {
@@ -26,11 +27,35 @@ struct Range {
 
 bool float_dtype(int dt) { return dt == MF_F32 || dt == MF_BF16 || dt == MF_F16; }
 
+// A thread that has made no runtime call yet (an autograd worker) has no current context, which the tensor-map encoding,
+// a driver call, needs; cudaSetDevice of the device that is current already does not make one.  The calls used here are
+// legal while any stream is being captured.
+int bind_context(int dev) {
+  static std::mutex mu;
+  static CUcontext primary[64] = {};
+  auto entry = [](const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    return cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) == cudaSuccess ? f : nullptr;
+  };
+  static const auto get = reinterpret_cast<CUresult (*)(CUcontext*)>(entry("cuCtxGetCurrent"));
+  static const auto set = reinterpret_cast<CUresult (*)(CUcontext)>(entry("cuCtxSetCurrent"));
+  static const auto retain = reinterpret_cast<CUresult (*)(CUcontext*, CUdevice)>(entry("cuDevicePrimaryCtxRetain"));
+  CUcontext cur = nullptr;
+  MF_REQUIRE(get && set && retain && dev >= 0 && dev < 64, MF_ERR_CUDA, "the driver's context calls are not available");
+  if (get(&cur) == CUDA_SUCCESS && cur) return MF_OK;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!primary[dev]) MF_REQUIRE(retain(&primary[dev], dev) == CUDA_SUCCESS, MF_ERR_CUDA, "no primary context on device %d", dev);
+  MF_REQUIRE(set(primary[dev]) == CUDA_SUCCESS, MF_ERR_CUDA, "the primary context of device %d cannot be made current", dev);
+  return MF_OK;
+}
+
 int check_device() {
   static thread_local int checked_dev = -1;
   int dev = 0;
   MF_CUDA(cudaGetDevice(&dev));
   if (dev == checked_dev) return MF_OK;
+  { int r = bind_context(dev); if (r) return r; }
   int major = 0;
   MF_CUDA(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
   MF_REQUIRE(major == 10, MF_ERR_ARCH, "device %d has compute capability %d.x; this library is built for sm_100a only", dev, major);

@@ -1,4 +1,4 @@
-// Interface of the general tensor-core GEMM (gemm_tc.cu).
+// Interfaces of the tensor-core pieces that backward passes are composed of.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -15,8 +15,25 @@ struct GemmTcArgs {
   int64_t M, N, R;
   int dtype, a_mn, b_mn, out_kind;
   int accumulate = 0;
+  // A = LayerNorm of the array given (a_mn = 1: its rows are the reduction index), from saved row statistics; the normalised
+  // matrix is formed in shared memory, rounded to the operand dtype, and never stored.
+  const float *ln_mean = nullptr, *ln_rstd = nullptr;
+  const void *ln_gain = nullptr, *ln_shift = nullptr;
 };
 bool gemm_tc_ok(const GemmTcArgs& g);
 int gemm_tc(const GemmTcArgs& g, cudaStream_t st);
+
+// One pass over dy of the LayernormLinear backward (lnl_bwd_tc.cu): dx, and per block the column sums
+// part [blocks][K] (gain gradient) and, with db_part, [blocks][N] (bias gradient).
+struct LnlBwdRowsArgs {
+  int64_t M; int K, N, dtype;
+  const void *x, *gamma, *w, *dy;
+  const float *mean, *rstd;
+  void* dx;
+  float *part, *db_part;
+};
+bool lnl_bwd_rows_tc_ok(int64_t M, int K, int N);
+int lnl_bwd_rows_tc_blocks(int64_t M);
+int lnl_bwd_rows_tc(const LnlBwdRowsArgs& a, cudaStream_t st);
 
 }  // namespace mf

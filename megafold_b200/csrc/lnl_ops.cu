@@ -324,6 +324,35 @@ int colsum_small(const char* name, const float* p, int rows, int ncols, float* o
   return after_launch(name);
 }
 
+// The same of two such matrices that share their rows, in one launch: the first blocks take a's columns.
+__global__ void __launch_bounds__(1024)
+colsum_pair_kernel(const float* __restrict__ a, int na, float* __restrict__ out_a, const float* __restrict__ b, int nb, float* __restrict__ out_b, int rows) {
+  __shared__ float red[32][33];
+  const int a_blocks = (na + 31) / 32;
+  const bool first = (int)blockIdx.x < a_blocks;
+  const float* p = first ? a : b;
+  const int n = first ? na : nb, c = (first ? blockIdx.x : blockIdx.x - a_blocks) * 32 + threadIdx.x;
+  float s = 0.f;
+  if (c < n)
+    for (int m = threadIdx.y; m < rows; m += 32) s += p[(int64_t)m * n + c];
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  s = warp_sum(red[threadIdx.x][threadIdx.y]);
+  const int cc = (first ? blockIdx.x : blockIdx.x - a_blocks) * 32 + threadIdx.y;
+  if (threadIdx.x == 0 && cc < n) (first ? out_a : out_b)[cc] = s;
+}
+
+// out[k] = sum_n w[k, n] v[n]: a warp per row
+template <typename T>
+__global__ void __launch_bounds__(256) rows_dot_kernel(const T* __restrict__ w, const float* __restrict__ v, float* __restrict__ out, int K, int N) {
+  const int k = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= K) return;
+  float s = 0.f;
+  for (int n = threadIdx.x & 31; n < N; n += 32) s = fmaf(to_f(w[(int64_t)k * N + n]), v[n], s);
+  s = warp_sum(s);
+  if ((threadIdx.x & 31) == 0) out[k] = s;
+}
+
 int sum_slices(const float* part, float* out, int64_t n, int slices, cudaStream_t st) {
   sum_slices_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(part, out, n, slices);
   return after_launch("sum_slices_kernel");
@@ -473,6 +502,22 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
   int r;
   float* col_scratch = ws.take<float>((size_t)kColSlices * (K > N ? K : N));
   if constexpr (sizeof(T) == 2) {
+    if (tc && !xln_ready && lnl_bwd_rows_tc_ok(M, K, N)) {
+      const int blocks = lnl_bwd_rows_tc_blocks(M);
+      float* part = ws.take<float>((size_t)blocks * K);
+      float* dpart = db || d_ln_b ? ws.take<float>((size_t)blocks * N) : nullptr;
+      r = lnl_bwd_rows_tc(LnlBwdRowsArgs{M, K, N, dtype, x, gain, w, dy, mean, rstd, dx, part, dpart}, st);
+      if (r) return r;
+      float* db_sum = db || !d_ln_b ? db : ws.take<float>(N);
+      colsum_pair_kernel<<<(K + 31) / 32 + (db_sum ? (N + 31) / 32 : 0), dim3(32, 32), 0, st>>>(part, K, d_ln_w, dpart, N, db_sum, blocks);
+      MF_LAUNCHED("colsum_pair_kernel");
+      if (d_ln_b) {
+        // the shift gradient: sum over the rows of dy W^T
+        rows_dot_kernel<T><<<(K + 7) / 8, 256, 0, st>>>(w, db_sum, d_ln_b, K, N);
+        MF_LAUNCHED("rows_dot_kernel");
+      }
+      return gemm_tc(GemmTcArgs{x, dy, dw, K, N, M, dtype, 1, 1, 2, 0, mean, rstd, gain, shift}, st);
+    }
     if (tc) {
       float* dyln = dyln_ready ? const_cast<float*>(dyln_ready) : ws.take<float>((size_t)M * K);
       T* xln = xln_ready ? nullptr : ws.take<T>((size_t)M * K);
@@ -532,8 +577,13 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
   return MF_OK;
 }
 
-size_t lnl_bwd_core_bytes(int64_t M, int K, int N, bool has_ln, bool tc, int dtype) {
+size_t lnl_bwd_core_bytes(int64_t M, int K, int N, bool has_ln, bool tc, int dtype, bool xln_ready = false) {
   size_t b = align_up(sizeof(float) * (size_t)kColSlices * (K > N ? K : N), 256);
+  if (tc && !xln_ready && lnl_bwd_rows_tc_ok(M, K, N)) {
+    const size_t blocks = lnl_bwd_rows_tc_blocks(M);
+    return b + align_up(sizeof(float) * blocks * K, 256) + align_up(sizeof(float) * blocks * N, 256) +
+           align_up(sizeof(float) * N, 256);
+  }
   if (tc) {
     b += align_up(sizeof(float) * (size_t)M * K, 256) + align_up(dtype_size(dtype) * (size_t)M * K, 256) +
          align_up(sizeof(float) * (size_t)kRowBlocks * 2 * K, 256) + align_up(sizeof(float) * (size_t)kRowBlocks * N, 256);
@@ -676,7 +726,7 @@ size_t transition_bwd_workspace(const mf_transition_bwd_args& a) {
     const size_t es = dtype_size(a.dtype);
     return align_up((size_t)a.M * 2 * a.inner * es, 256) + 2 * align_up((size_t)a.M * a.inner * es, 256) +   // h/dh, g, dg
            align_up((size_t)a.M * a.dim * es, 256) +                                                          // LN(x)
-           lnl_bwd_core_bytes(a.M, a.dim, 2 * a.inner, true, true, a.dtype);
+           lnl_bwd_core_bytes(a.M, a.dim, 2 * a.inner, true, true, a.dtype, true);
   }
   size_t simt = align_up((size_t)a.M * 2 * a.inner * dtype_size(a.dtype), 256);     // h, then dh in place
   int S = dw_splits(a.dim, a.inner, a.M);
