@@ -185,8 +185,8 @@ int mf_lnl_fwd(const mf_lnl_fwd_args* args, void* stream) {
   MF_REQUIRE(a.x && a.ln_w && a.w && a.y && a.mean && a.rstd, MF_ERR_BAD_ARG, "x, ln_w, w, y, mean, rstd must not be NULL");
   if (a.M == 0) return MF_OK;
   int r = check_device(); if (r) return r;
-  if (!(a.flags & MF_FLAG_FORCE_SIMT) && lnl_fwd_tc_supported(a)) {
-    r = lnl_fwd_tc(a, static_cast<cudaStream_t>(stream));
+  if (!(a.flags & MF_FLAG_FORCE_SIMT) && (lnl_fwd_tc_supported(a) || lnl_fwd_wide_supported(a))) {
+    r = lnl_fwd_tc_supported(a) ? lnl_fwd_tc(a, static_cast<cudaStream_t>(stream)) : lnl_fwd_wide(a, static_cast<cudaStream_t>(stream));
     if (r == MF_OK) set_last_path("tcgen05");
     return r;
   }
@@ -237,11 +237,14 @@ int mf_swiglu_bwd(const void* x, const void* dy, void* dx, int64_t M, int32_t in
 static bool transition_fwd_use_tc(const mf_transition_fwd_args& a) {
   return !(a.flags & MF_FLAG_FORCE_SIMT) && transition_fwd_tc_supported(a);
 }
+static bool transition_fwd_use_wide(const mf_transition_fwd_args& a) {
+  return !(a.flags & MF_FLAG_FORCE_SIMT) && transition_fwd_wide_supported(a);
+}
 
 size_t mf_transition_fwd_workspace_bytes(const mf_transition_fwd_args* args) {
   if (!args) return 0;
   if (transition_fwd_use_tc(*args)) return 0;      // the fused kernel keeps the hidden activation on chip
-  return transition_fwd_simt_workspace(*args);
+  return transition_fwd_use_wide(*args) ? transition_fwd_wide_workspace(*args) : transition_fwd_simt_workspace(*args);
 }
 
 int mf_transition_fwd(const mf_transition_fwd_args* args, void* stream) {
@@ -256,8 +259,8 @@ int mf_transition_fwd(const mf_transition_fwd_args* args, void* stream) {
   MF_REQUIRE(need == 0 || (a.workspace && a.workspace_bytes >= need), MF_ERR_WORKSPACE,
              "workspace of %zu bytes needed, %zu given", need, a.workspace ? a.workspace_bytes : (size_t)0);
   int r = check_device(); if (r) return r;
-  if (transition_fwd_use_tc(a)) {
-    r = transition_fwd_tc(a, static_cast<cudaStream_t>(stream));
+  if (transition_fwd_use_tc(a) || transition_fwd_use_wide(a)) {
+    r = transition_fwd_use_tc(a) ? transition_fwd_tc(a, static_cast<cudaStream_t>(stream)) : transition_fwd_wide(a, static_cast<cudaStream_t>(stream));
     if (r == MF_OK) set_last_path("tcgen05");
     return r;
   }

@@ -155,6 +155,8 @@ size_t evo_bwd_ws_workspace(const mf_evo_bwd_args& a);
 int lnl_fwd_simt(const mf_lnl_fwd_args& a, cudaStream_t st);
 bool lnl_fwd_tc_supported(const mf_lnl_fwd_args& a);
 int lnl_fwd_tc(const mf_lnl_fwd_args& a, cudaStream_t st);
+bool lnl_fwd_wide_supported(const mf_lnl_fwd_args& a);
+int lnl_fwd_wide(const mf_lnl_fwd_args& a, cudaStream_t st);
 int lnl_bwd(const mf_lnl_bwd_args& a, cudaStream_t st);   // picks tensor-core GEMMs when lnl_bwd_runs_on_tc
 bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a);
 bool transition_bwd_runs_on_tc(const mf_transition_bwd_args& a);
@@ -166,6 +168,9 @@ size_t lnl_bwd_workspace(const mf_lnl_bwd_args& a);
 int transition_fwd_simt(const mf_transition_fwd_args& a, cudaStream_t st);
 bool transition_fwd_tc_supported(const mf_transition_fwd_args& a);
 int transition_fwd_tc(const mf_transition_fwd_args& a, cudaStream_t st);
+bool transition_fwd_wide_supported(const mf_transition_fwd_args& a);
+size_t transition_fwd_wide_workspace(const mf_transition_fwd_args& a);
+int transition_fwd_wide(const mf_transition_fwd_args& a, cudaStream_t st);
 int transition_bwd(const mf_transition_bwd_args& a, cudaStream_t st);
 size_t transition_fwd_simt_workspace(const mf_transition_fwd_args& a);
 size_t transition_bwd_workspace(const mf_transition_bwd_args& a);

@@ -300,46 +300,32 @@ int colsum(const char* name, F f, float* out, float* scratch, int64_t M, int nco
   return after_launch("sum_slices_kernel");
 }
 
-// Column sums of a small fp32 matrix [rows, ncols] (the per-block partial sums of a row pass) in one launch and in a fixed
-// order: columns [0, split) go to out_a, the others to out_b (which may be NULL).
+// Column sums of one or two small fp32 matrices that share their rows (the per-block partial sums of a row pass), in one
+// launch and in a fixed order: a's columns [0, split) go to out_a, its others to out_a2 (which may be NULL), b's to out_b.
 __global__ void __launch_bounds__(1024)
-colsum_small_kernel(const float* __restrict__ p, int rows, int ncols, float* __restrict__ out_a, float* __restrict__ out_b, int split) {
-  __shared__ float red[32][33];
-  const int c = blockIdx.x * 32 + threadIdx.x;
-  float s = 0.f;
-  if (c < ncols)
-    for (int m = threadIdx.y; m < rows; m += 32) s += p[(int64_t)m * ncols + c];
-  red[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.y == 0 && c < ncols) {
-    float t = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) t += red[i][threadIdx.x];
-    if (c < split) out_a[c] = t;
-    else if (out_b) out_b[c - split] = t;
-  }
-}
-int colsum_small(const char* name, const float* p, int rows, int ncols, float* out_a, float* out_b, int split, cudaStream_t st) {
-  colsum_small_kernel<<<(ncols + 31) / 32, dim3(32, 32), 0, st>>>(p, rows, ncols, out_a, out_b, split);
-  return after_launch(name);
-}
-
-// The same of two such matrices that share their rows, in one launch: the first blocks take a's columns.
-__global__ void __launch_bounds__(1024)
-colsum_pair_kernel(const float* __restrict__ a, int na, float* __restrict__ out_a, const float* __restrict__ b, int nb, float* __restrict__ out_b, int rows) {
+colsum_pair_kernel(const float* __restrict__ a, int na, int split, float* __restrict__ out_a, float* __restrict__ out_a2, const float* __restrict__ b, int nb,
+                   float* __restrict__ out_b, int rows) {
   __shared__ float red[32][33];
   const int a_blocks = (na + 31) / 32;
   const bool first = (int)blockIdx.x < a_blocks;
   const float* p = first ? a : b;
-  const int n = first ? na : nb, c = (first ? blockIdx.x : blockIdx.x - a_blocks) * 32 + threadIdx.x;
+  const int n = first ? na : nb, c0 = (first ? blockIdx.x : blockIdx.x - a_blocks) * 32, c = c0 + threadIdx.x;
   float s = 0.f;
   if (c < n)
     for (int m = threadIdx.y; m < rows; m += 32) s += p[(int64_t)m * n + c];
   red[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
   s = warp_sum(red[threadIdx.x][threadIdx.y]);
-  const int cc = (first ? blockIdx.x : blockIdx.x - a_blocks) * 32 + threadIdx.y;
-  if (threadIdx.x == 0 && cc < n) (first ? out_a : out_b)[cc] = s;
+  const int cc = c0 + threadIdx.y;
+  if (threadIdx.x == 0 && cc < n) {
+    if (!first) out_b[cc] = s;
+    else if (cc < split) out_a[cc] = s;
+    else if (out_a2) out_a2[cc - split] = s;
+  }
+}
+int colsum_pair(const char* name, const float* a, int na, int split, float* out_a, float* out_a2, const float* b, int nb, float* out_b, int rows, cudaStream_t st) {
+  colsum_pair_kernel<<<(na + 31) / 32 + (nb + 31) / 32, dim3(32, 32), 0, st>>>(a, na, split, out_a, out_a2, b, nb, out_b, rows);
+  return after_launch(name);
 }
 
 // out[k] = sum_n w[k, n] v[n]: a warp per row
@@ -479,7 +465,7 @@ bool lnl_bwd_core_tc_ok(int64_t M, int K, int N, int dtype, bool has_ln, const v
 template <typename T>
 int launch_ln_bwd_rows(const float* dyln, const T* x, const T* gain, const T* shift, const float* mean, const float* rstd,
                        T* dx, T* xln, float* part, int64_t M, int K, cudaStream_t st) {
-  int blocks = (int)((M + 63) / 64); if (blocks > kRowBlocks) blocks = kRowBlocks;
+  int blocks = (int)((M + 7) / 8 < kRowBlocks ? (M + 7) / 8 : kRowBlocks);      // one row per warp where rows are few
   const int64_t rpb = (M + blocks - 1) / blocks;
   blocks = (int)((M + rpb - 1) / rpb);
   const size_t sm = sizeof(float) * 8 * 2 * K;
@@ -509,8 +495,8 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
       r = lnl_bwd_rows_tc(LnlBwdRowsArgs{M, K, N, dtype, x, gain, w, dy, mean, rstd, dx, part, dpart}, st);
       if (r) return r;
       float* db_sum = db || !d_ln_b ? db : ws.take<float>(N);
-      colsum_pair_kernel<<<(K + 31) / 32 + (db_sum ? (N + 31) / 32 : 0), dim3(32, 32), 0, st>>>(part, K, d_ln_w, dpart, N, db_sum, blocks);
-      MF_LAUNCHED("colsum_pair_kernel");
+      r = colsum_pair("lnl_bwd_column_sums", part, K, K, d_ln_w, nullptr, dpart, db_sum ? N : 0, db_sum, blocks, st);
+      if (r) return r;
       if (d_ln_b) {
         // the shift gradient: sum over the rows of dy W^T
         rows_dot_kernel<T><<<(K + 7) / 8, 256, 0, st>>>(w, db_sum, d_ln_b, K, N);
@@ -528,23 +514,18 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
         if (r) return r;
       }
       const int blocks = launch_ln_bwd_rows<T>(dyln, x, gain, shift, mean, rstd, dx, xln, part, M, K, st);
-      r = colsum_small("lnl_bwd_dgain_dshift", part, blocks, 2 * K, d_ln_w, d_ln_b, K, st);
-      if (r) return r;
-      if (db) {
-        if (N <= 2048) {
-          int cb = (int)((M + 63) / 64); if (cb > kRowBlocks) cb = kRowBlocks;
-          const int64_t rows = (M + cb - 1) / cb;
-          cb = (int)((M + rows - 1) / rows);
-          float* dpart = ws.take<float>((size_t)kRowBlocks * N);
-          const int lanes = 256 / (N / 8);
-          colsum16_partial_kernel<T><<<cb, 256, sizeof(float) * lanes * N, st>>>(dy, dpart, M, N, rows);
-          MF_LAUNCHED("colsum16_partial_kernel");
-          r = colsum_small("lnl_bwd_dbias", dpart, cb, N, db, nullptr, N, st);
-        } else {
-          r = colsum("lnl_bwd_dbias", ColT<T>{dy, N}, db, col_scratch, M, N, st);
-        }
-        if (r) return r;
+      if (db && N <= 2048) {
+        const int64_t rows = (M + blocks - 1) / blocks;           // the same blocks of rows as the pass above
+        float* dpart = ws.take<float>((size_t)kRowBlocks * N);
+        const int lanes = 256 / (N / 8);
+        colsum16_partial_kernel<T><<<blocks, 256, sizeof(float) * lanes * N, st>>>(dy, dpart, M, N, rows);
+        MF_LAUNCHED("colsum16_partial_kernel");
+        r = colsum_pair("lnl_bwd_column_sums", part, 2 * K, K, d_ln_w, d_ln_b, dpart, N, db, blocks, st);
+      } else {
+        r = colsum_pair("lnl_bwd_column_sums", part, 2 * K, K, d_ln_w, d_ln_b, nullptr, 0, nullptr, blocks, st);
+        if (!r && db) r = colsum("lnl_bwd_dbias", ColT<T>{dy, N}, db, col_scratch, M, N, st);
       }
+      if (r) return r;
       // dw[K,N] = LN(x)^T @ dy: both operands are given with the reduction index (rows) outermost
       return gemm_tc(GemmTcArgs{xln_ready ? xln_ready : xln, dy, dw, K, N, M, dtype, 1, 1, 2}, st);
     }
@@ -828,7 +809,7 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
     r = gemm_tc(g1, st);
     if (r) return r;
   }
-  int r = colsum_small("transition_bwd_dgain_dshift", part, part_rows, 2 * K, a.d_ln_w, a.d_ln_b, K, st);
+  int r = colsum_pair("transition_bwd_dgain_dshift", part, 2 * K, K, a.d_ln_w, a.d_ln_b, nullptr, 0, nullptr, part_rows, st);
   if (r) return r;
   return unpermute_dw1(dw1p, a.dw1, K, I, st);
 }
