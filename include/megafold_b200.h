@@ -128,6 +128,15 @@ typedef struct mf_evo_bwd_args {
 MF_API size_t mf_evo_bwd_workspace_bytes(const mf_evo_bwd_args* args);
 MF_API int mf_evo_bwd(const mf_evo_bwd_args* args, void* stream);
 
+/* Both directions with o, d_o and dq / dk / dv (one layout for the three) in places of the caller's choosing: element
+ * strides of the batch, row and token index; heads are D apart and a head's elements adjacent.  So the gradients of a merged
+ * q/k/v projection can be written where its backward reads them, and attention along the other axis of a pair
+ * representation needs no transposed copy.  layout == NULL: contiguous.  On the forward only `o` is read.  The workspace
+ * sizes are those of the contiguous calls when all strides are multiples of 8 elements, else ask with MF_FLAG_FORCE_SIMT set. */
+typedef struct mf_evo_layout { int64_t o[3], d_o[3], d_qkv[3]; } mf_evo_layout;
+MF_API int mf_evo_fwd_laid_out(const mf_evo_fwd_args* args, const mf_evo_layout* layout, void* workspace, size_t workspace_bytes, void* stream);
+MF_API int mf_evo_bwd_laid_out(const mf_evo_bwd_args* args, const mf_evo_layout* layout, void* stream);
+
 /*
  * mf_evo_bwd without a workspace and without any allocation.  (No counterpart in the reference; added for
  * hosts that cannot allocate.)
@@ -190,6 +199,10 @@ typedef struct mf_lnl_bwd_args {
 
 MF_API size_t mf_lnl_bwd_workspace_bytes(const mf_lnl_bwd_args* args);
 MF_API int mf_lnl_bwd(const mf_lnl_bwd_args* args, void* stream);
+/* The same with gradients that reach x beside the operator (a second projection of x, a residual connection) added where dx
+ * is produced: dx = add2 + (add1 + dx), each [M,K] contiguous in `dtype` or NULL, and each sum rounded to `dtype` as if the
+ * tensors were added one after the other.  (No counterpart in the reference, where autograd adds them.) */
+MF_API int mf_lnl_bwd_add(const mf_lnl_bwd_args* args, const void* add1, const void* add2, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * SwiGLU:  y[M,I] = silu(x[M, I:2I]) * x[M, 0:I]   (gate = right half)
@@ -236,6 +249,22 @@ typedef struct mf_transition_bwd_args {
  * ask with the structure filled in as it will be passed to mf_transition_bwd. */
 MF_API size_t mf_transition_bwd_workspace_bytes(const mf_transition_bwd_args* args);
 MF_API int mf_transition_bwd(const mf_transition_bwd_args* args, void* stream);
+
+/* ------------------------------------------------------------------------------------------
+ * Pieces between the operators of a block (the reference leaves them to torch: attention.py:203-210, megafold.py:635).
+ *
+ * Output gate:  out[r,c] = o[r,c] * s, s = sigmoid(g[r * g_stride + c]);  backward from d = d_out:  d_o = d * s,
+ * d_g[r * dg_stride + c] = (d * o) * (1 - s) * s;  every step is rounded to `dtype`, as it is where each is an operation
+ * of its own, so that the values are those of the composed form.  Contiguous [rows, cols] unless a stride (in elements) is
+ * given; cols and strides multiples of 8, pointers 16-byte aligned.
+ *
+ * Pair-bias rows [L * L, np] (a projection padded to np columns) <-> planes [H, L, L]; swap != 0: plane element (i, j)
+ * belongs to row j * L + i (attention along the other axis).  to_rows != 0 writes the rows, columns H.. as zeros.
+ * ------------------------------------------------------------------------------------------ */
+MF_API int mf_gate_fwd(const void* o, const void* g, int64_t g_stride, void* out, int64_t rows, int32_t cols, int32_t dtype, void* stream);
+MF_API int mf_gate_bwd(const void* d, const void* o, const void* g, int64_t g_stride, void* d_o, void* d_g, int64_t dg_stride, int64_t rows, int32_t cols,
+                       int32_t dtype, void* stream);
+MF_API int mf_bias_layout(void* rows, void* planes, int32_t L, int32_t np, int32_t H, int32_t swap, int32_t to_rows, int32_t dtype, void* stream);
 
 /* ------------------------------------------------------------------------------------------
  * Type conversion of several contiguous arrays (fp32, bf16, fp16 in any combination) in one launch, for hosts that

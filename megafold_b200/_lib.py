@@ -49,6 +49,10 @@ class EvoBwdArgs(C.Structure):
                 ("dbias_ready_event", _vp)]
 
 
+class EvoLayout(C.Structure):
+    _fields_ = [("o", _i64 * 3), ("d_o", _i64 * 3), ("d_qkv", _i64 * 3)]
+
+
 class LnlFwdArgs(C.Structure):
     _fields_ = [("M", _i64), ("K", _i32), ("N", _i32), ("dtype", _i32), ("flags", _u32), ("eps", _f32),
                 ("x", _vp), ("ln_w", _vp), ("ln_b", _vp), ("w", _vp), ("b", _vp),
@@ -87,6 +91,8 @@ SYMBOLS = {
     "mf_evo_fwd": (C.c_int, [C.POINTER(EvoFwdArgs), _vp]),
     "mf_evo_fwd_workspace_bytes": (_sz, [C.POINTER(EvoFwdArgs)]),
     "mf_evo_fwd_with_workspace": (C.c_int, [C.POINTER(EvoFwdArgs), _vp, _sz, _vp]),
+    "mf_evo_fwd_laid_out": (C.c_int, [C.POINTER(EvoFwdArgs), C.POINTER(EvoLayout), _vp, _sz, _vp]),
+    "mf_evo_bwd_laid_out": (C.c_int, [C.POINTER(EvoBwdArgs), C.POINTER(EvoLayout), _vp]),
     "mf_evo_bwd_workspace_bytes": (_sz, [C.POINTER(EvoBwdArgs)]),
     "mf_evo_bwd": (C.c_int, [C.POINTER(EvoBwdArgs), _vp]),
     "mf_evo_bwd_noalloc": (C.c_int, [C.POINTER(EvoBwdArgs), _vp]),
@@ -94,6 +100,10 @@ SYMBOLS = {
     "mf_lnl_fwd": (C.c_int, [C.POINTER(LnlFwdArgs), _vp]),
     "mf_lnl_bwd_workspace_bytes": (_sz, [C.POINTER(LnlBwdArgs)]),
     "mf_lnl_bwd": (C.c_int, [C.POINTER(LnlBwdArgs), _vp]),
+    "mf_lnl_bwd_add": (C.c_int, [C.POINTER(LnlBwdArgs), _vp, _vp, _vp]),
+    "mf_gate_fwd": (C.c_int, [_vp, _vp, _i64, _vp, _i64, _i32, _i32, _vp]),
+    "mf_gate_bwd": (C.c_int, [_vp, _vp, _vp, _i64, _vp, _vp, _i64, _i64, _i32, _i32, _vp]),
+    "mf_bias_layout": (C.c_int, [_vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp]),
     "mf_swiglu_fwd": (C.c_int, [_vp, _vp, _i64, _i32, _i32, _vp]),
     "mf_swiglu_bwd": (C.c_int, [_vp, _vp, _vp, _i64, _i32, _i32, _vp]),
     "mf_transition_fwd_workspace_bytes": (_sz, [C.POINTER(TransitionFwdArgs)]),

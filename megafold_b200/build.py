@@ -24,7 +24,7 @@ LIB = os.path.join(PKG, "libmegafold_b200_trace.so" if TRACE else "libmegafold_b
 NATIVE = os.path.join(PKG, "_native.so")          # torch functions over the library (csrc/torch_ops.cpp)
 OBJ_DIR = os.path.join(PKG, "build_trace" if TRACE else "build")
 
-SOURCES = ["api.cu", "evo_simt.cu", "evo_tc.cu", "evo_tc_fwd.cu", "evo_fwd_ws.cu", "evo_bwd_ws.cu", "lnl_ops.cu", "lnl_tc.cu", "transition_tc.cu", "gemm_tc.cu", "transition_bwd_tc.cu", "cast.cu", "lnl_bwd_tc.cu", "ln_wide_tc.cu"]
+SOURCES = ["api.cu", "evo_simt.cu", "evo_tc.cu", "evo_tc_fwd.cu", "evo_fwd_ws.cu", "evo_bwd_ws.cu", "lnl_ops.cu", "lnl_tc.cu", "transition_tc.cu", "gemm_tc.cu", "transition_bwd_tc.cu", "cast.cu", "lnl_bwd_tc.cu", "ln_wide_tc.cu", "block_ops.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr",

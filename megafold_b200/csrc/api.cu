@@ -86,18 +86,51 @@ using namespace mf;
 
 extern "C" {
 
-static bool evo_fwd_use_tc(const mf_evo_fwd_args& a) {
-  // the tensor-core kernels write o with 16-byte stores
-  return !(a.flags & MF_FLAG_FORCE_SIMT) && ((uintptr_t)a.o & 15) == 0 &&
+}  // extern "C"
+
+namespace mf {
+namespace {
+
+template <typename A>
+mf_evo_layout contiguous_layout(const A& a) {
+  mf_evo_layout l;
+  const int64_t tok = (int64_t)a.H * a.D;
+  for (int64_t* s : {l.o, l.d_o, l.d_qkv}) { s[0] = tok * a.L * a.N; s[1] = tok * a.L; s[2] = tok; }
+  return l;
+}
+// the tensor-core kernels use 16-byte accesses on these arrays
+bool rows16(const int64_t (&s)[3]) { return (s[0] % 8 | s[1] % 8 | s[2] % 8) == 0; }
+
+bool evo_fwd_use_tc(const mf_evo_fwd_args& a, const mf_evo_layout& lay) {
+  return !(a.flags & MF_FLAG_FORCE_SIMT) && ((uintptr_t)a.o & 15) == 0 && rows16(lay.o) &&
+         evo_tc_supported(a.B, a.N, a.L, a.H, a.D, a.dtype, a.q_strides, a.k_strides, a.v_strides, a.q, a.k, a.v);
+}
+bool evo_bwd_use_tc(const mf_evo_bwd_args& a, const mf_evo_layout& lay) {
+  const uintptr_t align = (uintptr_t)a.o | (uintptr_t)a.d_o | (uintptr_t)a.dq | (uintptr_t)a.dk | (uintptr_t)a.dv;
+  return !(a.flags & MF_FLAG_FORCE_SIMT) && (align & 15) == 0 && rows16(lay.o) && rows16(lay.d_o) && rows16(lay.d_qkv) && evo_bwd_ws_shape_ok(a.L, a.D) &&
          evo_tc_supported(a.B, a.N, a.L, a.H, a.D, a.dtype, a.q_strides, a.k_strides, a.v_strides, a.q, a.k, a.v);
 }
 
-size_t mf_evo_fwd_workspace_bytes(const mf_evo_fwd_args* args) {
-  if (!args) return 0;
-  return evo_fwd_use_tc(*args) ? evo_fwd_ws_workspace(*args) : 0;
+int check_evo_bwd(const mf_evo_bwd_args& a) {
+  int r = check_evo_common(a); if (r) return r;
+  MF_REQUIRE(a.o && a.d_o && a.lse, MF_ERR_BAD_ARG, "o, d_o and lse must not be NULL");
+  MF_REQUIRE(a.dq && a.dk && a.dv && a.d_bias, MF_ERR_BAD_ARG, "dq, dk, dv and d_bias must not be NULL");
+  MF_REQUIRE(a.dbias_dtype == MF_F32 || a.dbias_dtype == a.dtype, MF_ERR_BAD_ARG,
+             "d_bias dtype must be fp32 or the q/k/v dtype");
+  return MF_OK;
 }
 
-int mf_evo_fwd_with_workspace(const mf_evo_fwd_args* args, void* workspace, size_t workspace_bytes, void* stream) {
+}  // namespace
+}  // namespace mf
+
+extern "C" {
+
+size_t mf_evo_fwd_workspace_bytes(const mf_evo_fwd_args* args) {
+  if (!args) return 0;
+  return evo_fwd_use_tc(*args, contiguous_layout(*args)) ? evo_fwd_ws_workspace(*args) : 0;
+}
+
+int mf_evo_fwd_laid_out(const mf_evo_fwd_args* args, const mf_evo_layout* layout, void* workspace, size_t workspace_bytes, void* stream) {
   Range nvtx_range("mf_evo_fwd");
   MF_REQUIRE(args, MF_ERR_BAD_ARG, "args is NULL");
   const mf_evo_fwd_args& a = *args;
@@ -106,68 +139,60 @@ int mf_evo_fwd_with_workspace(const mf_evo_fwd_args* args, void* workspace, size
   if (!workspace) workspace_bytes = 0;
   MF_REQUIRE(((uintptr_t)workspace & 255) == 0, MF_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   r = check_device(); if (r) return r;
+  const mf_evo_layout lay = layout ? *layout : contiguous_layout(a);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (evo_fwd_use_tc(a)) {
-    r = evo_fwd_ws_supported(a, workspace_bytes) ? evo_fwd_ws(a, workspace, st) : evo_fwd_tc(a, st);
+  if (evo_fwd_use_tc(a, lay)) {
+    r = evo_fwd_ws_supported(a, workspace_bytes) ? evo_fwd_ws(a, lay, workspace, st) : evo_fwd_tc(a, lay, st);
     if (r == MF_OK) set_last_path("tcgen05");
     return r;
   }
-  r = evo_fwd_simt(a, st);
+  r = evo_fwd_simt(a, lay, st);
   if (r == MF_OK) set_last_path("simt");
   return r;
 }
 
-int mf_evo_fwd(const mf_evo_fwd_args* args, void* stream) { return mf_evo_fwd_with_workspace(args, nullptr, 0, stream); }
-
-static bool evo_bwd_use_tc(const mf_evo_bwd_args& a) {
-  // the tensor-core kernels read o / d_o and write dq / dk / dv with 16-byte accesses
-  const uintptr_t align = (uintptr_t)a.o | (uintptr_t)a.d_o | (uintptr_t)a.dq | (uintptr_t)a.dk | (uintptr_t)a.dv;
-  return !(a.flags & MF_FLAG_FORCE_SIMT) && (align & 15) == 0 && evo_bwd_ws_shape_ok(a.L, a.D) &&
-         evo_tc_supported(a.B, a.N, a.L, a.H, a.D, a.dtype, a.q_strides, a.k_strides, a.v_strides, a.q, a.k, a.v);
+int mf_evo_fwd_with_workspace(const mf_evo_fwd_args* args, void* workspace, size_t workspace_bytes, void* stream) {
+  return mf_evo_fwd_laid_out(args, nullptr, workspace, workspace_bytes, stream);
 }
+int mf_evo_fwd(const mf_evo_fwd_args* args, void* stream) { return mf_evo_fwd_laid_out(args, nullptr, nullptr, 0, stream); }
 
 size_t mf_evo_bwd_workspace_bytes(const mf_evo_bwd_args* args) {
   if (!args) return 0;
-  return evo_bwd_use_tc(*args) ? evo_bwd_ws_workspace(*args) : evo_bwd_simt_workspace(*args);
+  return evo_bwd_use_tc(*args, contiguous_layout(*args)) ? evo_bwd_ws_workspace(*args) : evo_bwd_simt_workspace(*args);
 }
 
-int mf_evo_bwd(const mf_evo_bwd_args* args, void* stream) {
+int mf_evo_bwd_laid_out(const mf_evo_bwd_args* args, const mf_evo_layout* layout, void* stream) {
   Range nvtx_range("mf_evo_bwd");
   MF_REQUIRE(args, MF_ERR_BAD_ARG, "args is NULL");
   const mf_evo_bwd_args& a = *args;
-  int r = check_evo_common(a); if (r) return r;
-  MF_REQUIRE(a.o && a.d_o && a.lse, MF_ERR_BAD_ARG, "o, d_o and lse must not be NULL");
-  MF_REQUIRE(a.dq && a.dk && a.dv && a.d_bias, MF_ERR_BAD_ARG, "dq, dk, dv and d_bias must not be NULL");
-  MF_REQUIRE(a.dbias_dtype == MF_F32 || a.dbias_dtype == a.dtype, MF_ERR_BAD_ARG,
-             "d_bias dtype must be fp32 or the q/k/v dtype");
-  const size_t need = mf_evo_bwd_workspace_bytes(args);
+  int r = check_evo_bwd(a); if (r) return r;
+  const mf_evo_layout lay = layout ? *layout : contiguous_layout(a);
+  const bool tc = evo_bwd_use_tc(a, lay);
+  const size_t need = tc ? evo_bwd_ws_workspace(a) : evo_bwd_simt_workspace(a);
   MF_REQUIRE(a.workspace && a.workspace_bytes >= need, MF_ERR_WORKSPACE, "workspace of %zu bytes needed, %zu given", need,
              a.workspace ? a.workspace_bytes : (size_t)0);
   MF_REQUIRE(((uintptr_t)a.workspace & 255) == 0, MF_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   r = check_device(); if (r) return r;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (evo_bwd_use_tc(a)) {
-    r = evo_bwd_ws(a, st);
+  if (tc) {
+    r = evo_bwd_ws(a, lay, st);
     if (r == MF_OK) set_last_path("tcgen05");
     return r;
   }
-  r = evo_bwd_simt(a, st);
+  r = evo_bwd_simt(a, lay, st);
   if (r == MF_OK && a.dbias_ready_event) MF_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(a.dbias_ready_event), st));
   if (r == MF_OK) set_last_path("simt");
   return r;
 }
+int mf_evo_bwd(const mf_evo_bwd_args* args, void* stream) { return mf_evo_bwd_laid_out(args, nullptr, stream); }
 
 int mf_evo_bwd_noalloc(const mf_evo_bwd_args* args, void* stream) {
   Range nvtx_range("mf_evo_bwd_noalloc");
   MF_REQUIRE(args, MF_ERR_BAD_ARG, "args is NULL");
   const mf_evo_bwd_args& a = *args;
-  int r = check_evo_common(a); if (r) return r;
-  MF_REQUIRE(a.o && a.d_o && a.lse, MF_ERR_BAD_ARG, "o, d_o and lse must not be NULL");
-  MF_REQUIRE(a.dq && a.dk && a.dv && a.d_bias, MF_ERR_BAD_ARG, "dq, dk, dv and d_bias must not be NULL");
-  MF_REQUIRE(a.dbias_dtype == MF_F32 || a.dbias_dtype == a.dtype, MF_ERR_BAD_ARG,
-             "d_bias dtype must be fp32 or the q/k/v dtype");
+  int r = check_evo_bwd(a); if (r) return r;
   r = check_device(); if (r) return r;
-  r = evo_bwd_simt_noalloc(a, static_cast<cudaStream_t>(stream));
+  r = evo_bwd_simt_noalloc(a, contiguous_layout(a), static_cast<cudaStream_t>(stream));
   if (r == MF_OK && a.dbias_ready_event)
     MF_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(a.dbias_ready_event), static_cast<cudaStream_t>(stream)));
   if (r == MF_OK) set_last_path("simt");
@@ -200,7 +225,9 @@ size_t mf_lnl_bwd_workspace_bytes(const mf_lnl_bwd_args* args) {
   return lnl_bwd_workspace(*args);
 }
 
-int mf_lnl_bwd(const mf_lnl_bwd_args* args, void* stream) {
+int mf_lnl_bwd(const mf_lnl_bwd_args* args, void* stream) { return mf_lnl_bwd_add(args, nullptr, nullptr, stream); }
+
+int mf_lnl_bwd_add(const mf_lnl_bwd_args* args, const void* add1, const void* add2, void* stream) {
   Range nvtx_range("mf_lnl_bwd");
   MF_REQUIRE(args, MF_ERR_BAD_ARG, "args is NULL");
   const mf_lnl_bwd_args& a = *args;
@@ -213,7 +240,7 @@ int mf_lnl_bwd(const mf_lnl_bwd_args* args, void* stream) {
              a.workspace ? a.workspace_bytes : (size_t)0);
   MF_REQUIRE(((uintptr_t)a.workspace & 255) == 0, MF_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   int r = check_device(); if (r) return r;
-  r = lnl_bwd(a, static_cast<cudaStream_t>(stream));
+  r = lnl_bwd(a, add1, add2, static_cast<cudaStream_t>(stream));
   if (r == MF_OK) set_last_path(lnl_bwd_runs_on_tc(a) ? "tcgen05" : "simt");
   return r;
 }
@@ -291,6 +318,28 @@ int mf_transition_bwd(const mf_transition_bwd_args* args, void* stream) {
   r = transition_bwd(a, static_cast<cudaStream_t>(stream));
   if (r == MF_OK) set_last_path(transition_bwd_runs_on_tc(a) ? "tcgen05" : "simt");
   return r;
+}
+
+int mf_gate_fwd(const void* o, const void* g, int64_t g_stride, void* out, int64_t rows, int32_t cols, int32_t dtype, void* stream) {
+  Range nvtx_range("mf_gate_fwd");
+  MF_REQUIRE(o && g && out && rows >= 0 && cols > 0 && float_dtype(dtype), MF_ERR_BAD_ARG, "bad gate arguments");
+  int r = check_device(); if (r) return r;
+  return gate_fwd(o, g, g_stride, out, rows, cols, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int mf_gate_bwd(const void* d, const void* o, const void* g, int64_t g_stride, void* d_o, void* d_g, int64_t dg_stride, int64_t rows, int32_t cols,
+                int32_t dtype, void* stream) {
+  Range nvtx_range("mf_gate_bwd");
+  MF_REQUIRE(d && o && g && d_o && d_g && rows >= 0 && cols > 0 && float_dtype(dtype), MF_ERR_BAD_ARG, "bad gate arguments");
+  int r = check_device(); if (r) return r;
+  return gate_bwd(d, o, g, g_stride, d_o, d_g, dg_stride, rows, cols, dtype, static_cast<cudaStream_t>(stream));
+}
+
+int mf_bias_layout(void* rows, void* planes, int32_t L, int32_t np, int32_t H, int32_t swap, int32_t to_rows, int32_t dtype, void* stream) {
+  Range nvtx_range("mf_bias_layout");
+  MF_REQUIRE(rows && planes && L > 0 && np > 0 && H > 0 && float_dtype(dtype), MF_ERR_BAD_ARG, "bad pair-bias layout arguments");
+  int r = check_device(); if (r) return r;
+  return bias_layout(rows, planes, L, np, H, swap != 0, to_rows != 0, dtype, static_cast<cudaStream_t>(stream));
 }
 
 int mf_cast_batch(const mf_cast_item* items, int32_t n_items, void* stream) {

@@ -11,6 +11,7 @@
 #include <stdio.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <mutex>
 
 #include "../../include/megafold_b200.h"
@@ -133,23 +134,30 @@ __device__ __forceinline__ float warp_sum(float v) {
     default: return ::mf::fail(MF_ERR_BAD_ARG, "unknown dtype %d", (int)(dt)); \
   }
 
+// Element offset of token (b, n, l) in an array laid out by mf_evo_layout's three strides.
+struct TokenStrides {
+  int64_t b, n, l;
+  __host__ __device__ __forceinline__ int64_t at(int bb, int nn, int ll) const { return bb * b + nn * n + (int64_t)ll * l; }
+};
+inline TokenStrides token_strides(const int64_t (&s)[3]) { return TokenStrides{s[0], s[1], s[2]}; }
+
 // ---- internal entry points of the kernel families ---------------------------------------------
-int evo_fwd_simt(const mf_evo_fwd_args& a, cudaStream_t st);
-int evo_bwd_simt(const mf_evo_bwd_args& a, cudaStream_t st);
+int evo_fwd_simt(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st);
+int evo_bwd_simt(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st);
 size_t evo_bwd_simt_workspace(const mf_evo_bwd_args& a);
-int evo_bwd_simt_noalloc(const mf_evo_bwd_args& a, cudaStream_t st);
+int evo_bwd_simt_noalloc(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st);
 size_t evo_bwd_noalloc_max_rows();
 
 bool evo_tc_supported(int B, int N, int L, int H, int D, int dtype, const int64_t* qs, const int64_t* ks,
                       const int64_t* vs, const void* q, const void* k, const void* v);
 int tc_async_status();
 int bounded_wait_selftest(cudaStream_t st);
-int evo_fwd_tc(const mf_evo_fwd_args& a, cudaStream_t st);
+int evo_fwd_tc(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st);
 size_t evo_fwd_ws_workspace(const mf_evo_fwd_args& a);
 bool evo_fwd_ws_supported(const mf_evo_fwd_args& a, size_t workspace_bytes);
-int evo_fwd_ws(const mf_evo_fwd_args& a, void* workspace, cudaStream_t st);
+int evo_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, void* workspace, cudaStream_t st);
 bool evo_bwd_ws_shape_ok(int L, int D);
-int evo_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st);
+int evo_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st);
 size_t evo_bwd_ws_workspace(const mf_evo_bwd_args& a);
 
 int lnl_fwd_simt(const mf_lnl_fwd_args& a, cudaStream_t st);
@@ -157,7 +165,7 @@ bool lnl_fwd_tc_supported(const mf_lnl_fwd_args& a);
 int lnl_fwd_tc(const mf_lnl_fwd_args& a, cudaStream_t st);
 bool lnl_fwd_wide_supported(const mf_lnl_fwd_args& a);
 int lnl_fwd_wide(const mf_lnl_fwd_args& a, cudaStream_t st);
-int lnl_bwd(const mf_lnl_bwd_args& a, cudaStream_t st);   // picks tensor-core GEMMs when lnl_bwd_runs_on_tc
+int lnl_bwd(const mf_lnl_bwd_args& a, const void* add1, const void* add2, cudaStream_t st);   // picks tensor-core GEMMs when lnl_bwd_runs_on_tc
 bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a);
 bool transition_bwd_runs_on_tc(const mf_transition_bwd_args& a);
 bool transition_bwd_fused_ok(const mf_transition_bwd_args& a);
@@ -175,6 +183,9 @@ int transition_bwd(const mf_transition_bwd_args& a, cudaStream_t st);
 size_t transition_fwd_simt_workspace(const mf_transition_fwd_args& a);
 size_t transition_bwd_workspace(const mf_transition_bwd_args& a);
 
+int gate_fwd(const void* o, const void* g, int64_t gs, void* out, int64_t rows, int cols, int dtype, cudaStream_t st);
+int gate_bwd(const void* d, const void* o, const void* g, int64_t gs, void* d_o, void* d_g, int64_t dgs, int64_t rows, int cols, int dtype, cudaStream_t st);
+int bias_layout(void* rows, void* planes, int L, int np, int H, bool swap, bool to_rows, int dtype, cudaStream_t st);
 int cast_batch(const mf_cast_item* items, int n_items, cudaStream_t st);
 
 int swiglu_fwd(const void* x, void* y, int64_t M, int inner, int dtype, cudaStream_t st);

@@ -76,7 +76,7 @@ struct BwdWsP {
   const uint8_t* xq; const uint8_t* xk;     // rank-one term tiles (evo_extras_ws_kernel)
   const int* flags;                         // per (b, n, h): every key of the row is masked
   void* dbias_direct;                       // N == 1 and a 16-bit d_pair_bias: dS is the answer, written by this kernel
-  void *dq, *dk, *dv;
+  void *dq, *dk, *dv; TokenStrides gs;
   int* status;
 };
 
@@ -103,7 +103,7 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
 // dQ, where one is used, is cleared here as well: each memset in front of the kernels cost 2 us of GPU time and as much of
 // the host's.
 template <typename T>
-__global__ void evo_extras_ws_kernel(const T* __restrict__ o, const T* __restrict__ d_o, const float* __restrict__ lse,
+__global__ void evo_extras_ws_kernel(const T* __restrict__ o, TokenStrides os, const T* __restrict__ d_o, TokenStrides ds, const float* __restrict__ lse,
                                      const void* __restrict__ mask, int64_t ms_b, int64_t ms_n, int64_t ms_l, int mask_dtype,
                                      uint8_t* __restrict__ xq, uint8_t* __restrict__ xk, int* __restrict__ flags,
                                      float* __restrict__ dq_acc, int64_t n_threads, int N, int L, int lpad, int H, int D) {
@@ -119,8 +119,9 @@ __global__ void evo_extras_ws_kernel(const T* __restrict__ o, const T* __restric
     float nl = kMinusBig, nd = 0.f;
     if (i < L) {
       const int64_t row = (bn * L + i) * H + h;
-      const uint4* po = reinterpret_cast<const uint4*>(o + row * D);
-      const uint4* pg = reinterpret_cast<const uint4*>(d_o + row * D);
+      const int b = (int)(bn / N), n = (int)(bn % N);
+      const uint4* po = reinterpret_cast<const uint4*>(o + os.at(b, n, i) + h * D);
+      const uint4* pg = reinterpret_cast<const uint4*>(d_o + ds.at(b, n, i) + h * D);
       float dl = 0.f;
       for (int c = 0; c < D / 8; ++c) {
         const uint4 a = __ldg(po + c), g = __ldg(pg + c);
@@ -266,7 +267,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       tc_fence_before();
       if (j < p.L && !*abort_flag) {
         const float sc = kv_which == 0 ? p.scale : 1.f;
-        T* orow = static_cast<T*>(kv_which == 0 ? p.dk : p.dv) + ((((int64_t)b * p.N + n) * p.L + j) * p.H + h) * p.D + kv_hh * 32;
+        T* orow = static_cast<T*>(kv_which == 0 ? p.dk : p.dv) + p.gs.at(b, n, j) + h * p.D + kv_hh * 32;
 #pragma unroll
         for (int d8 = 0; d8 < 4; ++d8) {
           if (kv_hh * 32 + d8 * 8 < p.D) {
@@ -419,7 +420,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             tc_fence_before();
             const int i = it * kT + r;
             if (i < p.L && !*abort_flag) {
-              T* orow = static_cast<T*>(p.dq) + ((((int64_t)b * p.N + n) * p.L + i) * p.H + h) * p.D + hh * 32;
+              T* orow = static_cast<T*>(p.dq) + p.gs.at(b, n, i) + h * p.D + hh * 32;
 #pragma unroll
               for (int d8 = 0; d8 < 4; ++d8) {
                 if (hh * 32 + d8 * 8 < p.D) {
@@ -925,10 +926,18 @@ __global__ void dbias_finish_kernel(const float* __restrict__ part, TO* __restri
   }
 }
 
+// the fp32 accumulator of dQ ([B, N, L, H, D], D a multiple of 8) to its 16-bit place, eight elements per thread
 template <typename T>
-__global__ void cast_rows_ws_kernel(const float* __restrict__ src, T* __restrict__ dst, int64_t n) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = from_f<T>(src[i]);
+__global__ void __launch_bounds__(256) cast_dq_kernel(const float* __restrict__ src, T* __restrict__ dst, TokenStrides gs, int64_t n8, int HD, int L, int N) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n8) return;
+  const int64_t tok = i * 8 / HD;
+  const int e = (int)(i * 8 - tok * HD);
+  const int l = (int)(tok % L); const int64_t bn = tok / L;
+  const float4 x = reinterpret_cast<const float4*>(src)[2 * i], y = reinterpret_cast<const float4*>(src)[2 * i + 1];
+  uint4 v;
+  v.x = Pack2<T>::pack(x.x, x.y); v.y = Pack2<T>::pack(x.z, x.w); v.z = Pack2<T>::pack(y.x, y.y); v.w = Pack2<T>::pack(y.z, y.w);
+  *reinterpret_cast<uint4*>(dst + gs.at((int)(bn / N), (int)(bn % N), l) + e) = v;
 }
 
 // With few (b, n, h) triples (single-representation attention: N = 1) the key tiles of each are spread over several
@@ -982,11 +991,11 @@ BwdPlan plan_bwd(const mf_evo_bwd_args& a) {
 }
 
 template <typename T, typename TB, int NH>
-int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
+int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   const BwdPlan pl = plan_bwd(a);
   CUtensorMap mq, mk, mv, mg, mbt;
   int r;
-  const int64_t cs[5] = {(int64_t)a.N * a.L * a.H * a.D, (int64_t)a.L * a.H * a.D, (int64_t)a.H * a.D, a.D, 1};
+  const int64_t cs[5] = {lay.d_o[0], lay.d_o[1], lay.d_o[2], a.D, 1};
   if ((r = make_qkv_map(&mq, a.q, a.dtype, a.B, a.N, a.L, a.H, a.D, a.q_strides, kDP, kT))) return r;
   if ((r = make_qkv_map(&mk, a.k, a.dtype, a.B, a.N, a.L, a.H, a.D, a.k_strides, kDP, kT))) return r;
   if ((r = make_qkv_map(&mv, a.v, a.dtype, a.B, a.N, a.L, a.H, a.D, a.v_strides, kDP, kT))) return r;
@@ -1020,7 +1029,7 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
   }
   {
     const int64_t n_threads = (int64_t)a.B * a.N * lpad * a.H;
-    evo_extras_ws_kernel<T><<<(unsigned)((n_threads + 255) / 256), 256, 0, st>>>(static_cast<const T*>(a.o), static_cast<const T*>(a.d_o), a.lse,
+    evo_extras_ws_kernel<T><<<(unsigned)((n_threads + 255) / 256), 256, 0, st>>>(static_cast<const T*>(a.o), token_strides(lay.o), static_cast<const T*>(a.d_o), token_strides(lay.d_o), a.lse,
                                                                              a.mask, a.mask_strides[0], a.mask_strides[1], a.mask_strides[2], a.mask_dtype,
                                                                              xq, xk, flags, pl.dq_fp32 ? dq_acc : nullptr, n_threads, a.N, a.L, lpad, a.H, a.D);
   }
@@ -1076,7 +1085,7 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     p.bias_b_mul = bias_b_mul;
     p.xq = xq; p.xk = xk; p.flags = flags;
     p.dbias_direct = dbias_direct ? a.d_bias : nullptr;
-    p.dq = a.dq; p.dk = a.dk; p.dv = a.dv;
+    p.dq = a.dq; p.dk = a.dk; p.dv = a.dv; p.gs = token_strides(lay.d_qkv);
     p.status = status;
     const size_t smem = Geo<NH>::kMainSmem;
     int grid = sm_count();
@@ -1094,8 +1103,9 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
     if (a.dbias_ready_event && dbias_direct) MF_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(a.dbias_ready_event), st));
   }
   if (pl.dq_fp32) {
-    cast_rows_ws_kernel<T><<<(unsigned)((n_dq + 255) / 256), 256, 0, st>>>(dq_acc, static_cast<T*>(a.dq), n_dq);
-    MF_LAUNCHED("cast_rows_ws_kernel");
+    const int64_t n8 = n_dq / 8;
+    cast_dq_kernel<T><<<(unsigned)((n8 + 255) / 256), 256, 0, st>>>(dq_acc, static_cast<T*>(a.dq), token_strides(lay.d_qkv), n8, a.H * a.D, a.L, a.N);
+    MF_LAUNCHED("cast_dq_kernel");
   }
   return MF_OK;
 }
@@ -1118,12 +1128,12 @@ size_t evo_bwd_ws_workspace(const mf_evo_bwd_args& a) { return plan_bwd(a).total
     default: return fail(MF_ERR_BAD_ARG, "unknown bias dtype %d", (int)(dt)); \
   }
 
-int evo_bwd_ws(const mf_evo_bwd_args& a, cudaStream_t st) {
+int evo_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   int r = MF_OK;
   if (a.dtype == MF_BF16) {
-    MF_DISPATCH_BIAS(a.bias_dtype, TB, { r = a.D <= kDP ? launch_bwd_ws<__nv_bfloat16, TB, 1>(a, st) : launch_bwd_ws<__nv_bfloat16, TB, 2>(a, st); });
+    MF_DISPATCH_BIAS(a.bias_dtype, TB, { r = a.D <= kDP ? launch_bwd_ws<__nv_bfloat16, TB, 1>(a, lay, st) : launch_bwd_ws<__nv_bfloat16, TB, 2>(a, lay, st); });
   } else {
-    MF_DISPATCH_BIAS(a.bias_dtype, TB, { r = a.D <= kDP ? launch_bwd_ws<__half, TB, 1>(a, st) : launch_bwd_ws<__half, TB, 2>(a, st); });
+    MF_DISPATCH_BIAS(a.bias_dtype, TB, { r = a.D <= kDP ? launch_bwd_ws<__half, TB, 1>(a, lay, st) : launch_bwd_ws<__half, TB, 2>(a, lay, st); });
   }
   return r;
 }

@@ -41,7 +41,7 @@ struct FwdWsP {
   uint32_t fmt, bfmt;     // tcgen05 operand formats of q/k/v and of the bias (1 = bf16, 0 = f16)
   int n_alpha; float alpha[2];
   const void* mask; int64_t ms[3]; int mask_dtype;
-  void* o; float* lse; int* status;
+  void* o; TokenStrides os; float* lse; int* status;
 };
 
 struct StreamBars {
@@ -225,7 +225,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       tr(8);
       if (i < p.L && !*abort_flag) {
         const float inv = 1.f / l;
-        T* orow = static_cast<T*>(p.o) + ((((int64_t)ip.b * p.N + ip.n) * p.L + i) * p.H + ip.h) * p.D;
+        T* orow = static_cast<T*>(p.o) + p.os.at(ip.b, ip.n, i) + ip.h * p.D;
 #pragma unroll
         for (int d8 = 0; d8 < 4; ++d8) {
           if (d8 * 8 < p.D) {
@@ -454,7 +454,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
 }
 
 template <typename T, typename TB>
-int launch_fwd_ws(const mf_evo_fwd_args& a, cudaStream_t st) {
+int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   CUtensorMap mq, mk, mv, mb;
   int r;
   if ((r = make_qkv_map(&mq, a.q, a.dtype, a.B, a.N, a.L, a.H, a.D, a.q_strides, 32, kT))) return r;
@@ -471,7 +471,7 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, cudaStream_t st) {
   p.n_alpha = split_alpha(a.D, a.bias_dtype, p.alpha);
   p.mask = a.mask; for (int i = 0; i < 3; ++i) p.ms[i] = a.mask_strides[i];
   p.mask_dtype = a.mask_dtype;
-  p.o = a.o; p.lse = a.lse;
+  p.o = a.o; p.os = token_strides(lay.o); p.lse = a.lse;
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
@@ -517,7 +517,7 @@ bool evo_fwd_ws_supported(const mf_evo_fwd_args& a, size_t workspace_bytes) {
   return shape_ok(a) && workspace_bytes >= evo_fwd_ws_workspace(a);
 }
 
-int evo_fwd_ws(const mf_evo_fwd_args& args, void* workspace, cudaStream_t st) {
+int evo_fwd_ws(const mf_evo_fwd_args& args, const mf_evo_layout& lay, void* workspace, cudaStream_t st) {
   mf_evo_fwd_args a = args;
   if (evo_fwd_ws_workspace(args)) {
     int r = copy_bias_rows(a.bias, a.bias_dtype, a.bias_strides, workspace, a.bias_dtype, a.B, a.H, a.L, st);
@@ -528,8 +528,8 @@ int evo_fwd_ws(const mf_evo_fwd_args& args, void* workspace, cudaStream_t st) {
     a.bias_strides[0] = args.bias_strides[0] == 0 ? 0 : row * a.L * a.H;
   }
   if (a.dtype == MF_BF16)
-    return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16>(a, st) : launch_fwd_ws<__nv_bfloat16, __half>(a, st);
-  return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16>(a, st) : launch_fwd_ws<__half, __half>(a, st);
+    return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16>(a, lay, st) : launch_fwd_ws<__nv_bfloat16, __half>(a, lay, st);
+  return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16>(a, lay, st) : launch_fwd_ws<__half, __half>(a, lay, st);
 }
 
 }  // namespace mf

@@ -36,6 +36,8 @@ struct EvoP {
   // backward
   const void *d_o; const float* delta;
   void *dq, *dk, *dv; void* d_bias;
+  TokenStrides os, gs;                   // of o / of dq, dk, dv
+  int64_t ds[5];                         // of d_o
   int nt, nsplit;                        // tiles per sequence; ranges of the N rows that d_pair_bias is summed in
   float* part;                           // [nsplit][B][H][L][L] sums of the ranges, or NULL: one block sums all of them
 };
@@ -136,13 +138,13 @@ __device__ __forceinline__ float row_sum(float v) {
 }
 
 template <typename T, int DP>
-__device__ __forceinline__ void store_rows(void* out, const float (&acc)[4][DP / 16], const float (&f)[4], int b, int n, int h, int row0, int ty, int tx,
+__device__ __forceinline__ void store_rows(void* out, const TokenStrides& s, const float (&acc)[4][DP / 16], const float (&f)[4], int b, int n, int h, int row0, int ty, int tx,
                                            const EvoP& p) {
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
     const int l = row0 + ty + 16 * a;
     if (l >= p.L) continue;
-    T* row = static_cast<T*>(out) + ((((int64_t)b * p.N + n) * p.L + l) * p.H + h) * p.D;
+    T* row = static_cast<T*>(out) + s.at(b, n, l) + h * p.D;
 #pragma unroll
     for (int e = 0; e < DP / 16; ++e) {
       const int d = tx * (DP / 16) + e;
@@ -219,7 +221,7 @@ __global__ void __launch_bounds__(kThreads) evo_fwd_simt_kernel(const __grid_con
   float inv[4];
 #pragma unroll
   for (int a = 0; a < 4; ++a) inv[a] = 1.f / l[a];
-  store_rows<T, DP>(p.o, acc, inv, b, n, h, i0, ty, tx, p);
+  store_rows<T, DP>(p.o, p.os, acc, inv, b, n, h, i0, ty, tx, p);
   if (tx == 0)
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
@@ -232,19 +234,19 @@ __global__ void __launch_bounds__(kThreads) evo_fwd_simt_kernel(const __grid_con
 // backward, step 0: delta[b,n,h,i] = sum_d dO * O      (eight threads per (b,n,i,h))
 // ------------------------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(kThreads) evo_delta_kernel(const T* __restrict__ o, const T* __restrict__ d_o, float* __restrict__ delta, int64_t rows,
-                                                             int L, int H, int D) {
+__global__ void __launch_bounds__(kThreads) evo_delta_kernel(const T* __restrict__ o, TokenStrides os, const T* __restrict__ d_o, TokenStrides ds,
+                                                             float* __restrict__ delta, int64_t rows, int N, int L, int H, int D) {
   const int64_t row = (int64_t)blockIdx.x * (kThreads / 8) + (threadIdx.x >> 3);
+  // row = ((b*N+n)*L + i)*H + h  ->  delta index ((b*N+n)*H + h)*L + i
+  const int h = row % H; const int64_t t = row / H; const int i = t % L; const int64_t bn = t / L;
   float s = 0.f;
-  if (row < rows)
-    for (int d = threadIdx.x & 7; d < D; d += 8) s = fmaf(to_f(o[row * D + d]), to_f(d_o[row * D + d]), s);
+  if (row < rows) {
+    const T *po = o + os.at((int)(bn / N), (int)(bn % N), i) + h * D, *pg = d_o + ds.at((int)(bn / N), (int)(bn % N), i) + h * D;
+    for (int d = threadIdx.x & 7; d < D; d += 8) s = fmaf(to_f(po[d]), to_f(pg[d]), s);
+  }
 #pragma unroll
   for (int k = 4; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
-  if (row < rows && (threadIdx.x & 7) == 0) {
-    // row = ((b*N+n)*L + i)*H + h  ->  delta index ((b*N+n)*H + h)*L + i
-    const int h = row % H; const int64_t t = row / H; const int i = t % L; const int64_t bn = t / L;
-    delta[(bn * H + h) * L + i] = s;
-  }
+  if (row < rows && (threadIdx.x & 7) == 0) delta[(bn * H + h) * L + i] = s;
 }
 
 // P and dS of one logit from its product sums
@@ -262,7 +264,6 @@ __device__ __forceinline__ void bwd_dkv(const EvoP& p, float* smem, int b, int n
   constexpr int kOp = kTile * (DP + 4);
   float *Ks = smem, *Vs = Ks + kOp, *Qs = Vs + kOp, *Gs = Qs + kOp, *Ps = Gs + kOp, *Ds = Ps + kTile * kPPitch;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t gs[5] = {(int64_t)p.N * p.L * p.H * p.D, (int64_t)p.L * p.H * p.D, (int64_t)p.H * p.D, p.D, 1};
   load_tile<T, DP>(Ks, p.k, p.ks, p.k_vec, b, n, h, j0, p.L, p.D);
   load_tile<T, DP>(Vs, p.v, p.vs, p.v_vec, b, n, h, j0, p.L, p.D);
   float dk[4][DP / 16] = {}, dv[4][DP / 16] = {}, mt[4];
@@ -271,7 +272,7 @@ __device__ __forceinline__ void bwd_dkv(const EvoP& p, float* smem, int b, int n
   for (int i0 = 0; i0 < p.L; i0 += kTile) {
     __syncthreads();
     load_tile<T, DP>(Qs, p.q, p.qs, p.q_vec, b, n, h, i0, p.L, p.D);
-    load_tile<T, DP>(Gs, p.d_o, gs, p.g_vec, b, n, h, i0, p.L, p.D);
+    load_tile<T, DP>(Gs, p.d_o, p.ds, p.g_vec, b, n, h, i0, p.L, p.D);
     float bias[4][4], lse[4], dl[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -299,8 +300,8 @@ __device__ __forceinline__ void bwd_dkv(const EvoP& p, float* smem, int b, int n
     sum_tile<DP>(Ds, Qs, ty, tx, dk);
   }
   const float one[4] = {1.f, 1.f, 1.f, 1.f}, sc[4] = {p.scale, p.scale, p.scale, p.scale};
-  store_rows<T, DP>(p.dk, dk, sc, b, n, h, j0, ty, tx, p);
-  store_rows<T, DP>(p.dv, dv, one, b, n, h, j0, ty, tx, p);
+  store_rows<T, DP>(p.dk, p.gs, dk, sc, b, n, h, j0, ty, tx, p);
+  store_rows<T, DP>(p.dv, p.gs, dv, one, b, n, h, j0, ty, tx, p);
 }
 
 // S and dP of a (query tile, key tile) pair of row n turned into dS; rows are queries, columns keys
@@ -342,9 +343,8 @@ __device__ __forceinline__ void bwd_dq(const EvoP& p, float* smem, int b, int n,
   constexpr int kOp = kTile * (DP + 4);
   float *Ks = smem, *Vs = Ks + kOp, *Qs = Vs + kOp, *Gs = Qs + kOp, *Ds = Gs + kOp;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t gs[5] = {(int64_t)p.N * p.L * p.H * p.D, (int64_t)p.L * p.H * p.D, (int64_t)p.H * p.D, p.D, 1};
   load_tile<T, DP>(Qs, p.q, p.qs, p.q_vec, b, n, h, i0, p.L, p.D);
-  load_tile<T, DP>(Gs, p.d_o, gs, p.g_vec, b, n, h, i0, p.L, p.D);
+  load_tile<T, DP>(Gs, p.d_o, p.ds, p.g_vec, b, n, h, i0, p.L, p.D);
   float dq[4][DP / 16] = {};
   for (int j0 = 0; j0 < p.L; j0 += kTile) {
     __syncthreads();
@@ -362,7 +362,7 @@ __device__ __forceinline__ void bwd_dq(const EvoP& p, float* smem, int b, int n,
     sum_tile<DP>(Ds, Ks, ty, tx, dq);
   }
   const float sc[4] = {p.scale, p.scale, p.scale, p.scale};
-  store_rows<T, DP>(p.dq, dq, sc, b, n, h, i0, ty, tx, p);
+  store_rows<T, DP>(p.dq, p.gs, dq, sc, b, n, h, i0, ty, tx, p);
 }
 
 // dBias of a 64 x 64 tile: the sum of dS over range `sp` of the N rows (or, without room for partial sums, over all ranges
@@ -372,7 +372,6 @@ __device__ __forceinline__ void bwd_dbias(const EvoP& p, float* smem, int b, int
   constexpr int kOp = kTile * (DP + 4);
   float *Ks = smem, *Vs = Ks + kOp, *Qs = Vs + kOp, *Gs = Qs + kOp;
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int64_t gs[5] = {(int64_t)p.N * p.L * p.H * p.D, (int64_t)p.L * p.H * p.D, (int64_t)p.H * p.D, p.D, 1};
   float bias[4][4], total[4][4];
   bias_tile(p, b, h, i0, j0, ty, tx, bias);
   const int sp_end = p.part ? sp + 1 : p.nsplit;
@@ -382,7 +381,7 @@ __device__ __forceinline__ void bwd_dbias(const EvoP& p, float* smem, int b, int
     for (int n = n0; n < n1; ++n) {
       __syncthreads();
       load_tile<T, DP>(Qs, p.q, p.qs, p.q_vec, b, n, h, i0, p.L, p.D);
-      load_tile<T, DP>(Gs, p.d_o, gs, p.g_vec, b, n, h, i0, p.L, p.D);
+      load_tile<T, DP>(Gs, p.d_o, p.ds, p.g_vec, b, n, h, i0, p.L, p.D);
       load_tile<T, DP>(Ks, p.k, p.ks, p.k_vec, b, n, h, j0, p.L, p.D);
       load_tile<T, DP>(Vs, p.v, p.vs, p.v_vec, b, n, h, j0, p.L, p.D);
       __syncthreads();
@@ -477,10 +476,10 @@ size_t delta_bytes(const mf_evo_bwd_args& a) { return align_up(sizeof(float) * (
   else if ((D) <= 128) { constexpr int DP = 128; __VA_ARGS__; } \
   else return fail(MF_ERR_UNSUPPORTED, "head size %d > 128 is not supported", (D));
 
-int evo_fwd_simt(const mf_evo_fwd_args& a, cudaStream_t st) {
+int evo_fwd_simt(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   EvoP p{};
   fill_common(p, a);
-  p.o = a.o; p.lse = a.lse;
+  p.o = a.o; p.os = token_strides(lay.o); p.lse = a.lse;
   MF_DISPATCH_FLOAT(a.dtype, T, MF_DISPATCH_DP(a.D, DP, {
     constexpr size_t smem = sizeof(float) * (3 * kTile * (DP + 4) + kTile * kPPitch);
     constexpr auto kern = evo_fwd_simt_kernel<T, DP>;
@@ -497,20 +496,22 @@ size_t evo_bwd_simt_workspace(const mf_evo_bwd_args& a) {
 }
 
 // partials: the workspace has room for the sums of the row ranges behind delta
-static int bwd_simt(const mf_evo_bwd_args& a, bool partials, cudaStream_t st) {
+static int bwd_simt(const mf_evo_bwd_args& a, const mf_evo_layout& lay, bool partials, cudaStream_t st) {
   EvoP p{};
   fill_common(p, a);
   p.lse = const_cast<float*>(a.lse);
   float* delta = static_cast<float*>(a.workspace);
   p.d_o = a.d_o; p.delta = delta;
   p.dq = a.dq; p.dk = a.dk; p.dv = a.dv; p.d_bias = a.d_bias; p.dbias_dtype = a.dbias_dtype;
-  p.g_vec = a.D % 4 == 0 && reinterpret_cast<uintptr_t>(a.d_o) % (4 * dtype_size(a.dtype)) == 0;
+  p.gs = token_strides(lay.d_qkv);
+  p.ds[0] = lay.d_o[0]; p.ds[1] = lay.d_o[1]; p.ds[2] = lay.d_o[2]; p.ds[3] = a.D; p.ds[4] = 1;
+  p.g_vec = rows_vec(a.d_o, p.ds, a.D, dtype_size(a.dtype));
   p.nsplit = bias_ranges(a.B, a.N, a.L, a.H);
   p.part = partials ? delta + delta_bytes(a) / sizeof(float) : nullptr;
   MF_DISPATCH_FLOAT(a.dtype, T, {
     const int64_t rows = (int64_t)a.B * a.N * a.L * a.H;
-    evo_delta_kernel<T><<<(unsigned)((rows + kThreads / 8 - 1) / (kThreads / 8)), kThreads, 0, st>>>(static_cast<const T*>(a.o), static_cast<const T*>(a.d_o),
-                                                                                                     delta, rows, a.L, a.H, a.D);
+    evo_delta_kernel<T><<<(unsigned)((rows + kThreads / 8 - 1) / (kThreads / 8)), kThreads, 0, st>>>(
+        static_cast<const T*>(a.o), token_strides(lay.o), static_cast<const T*>(a.d_o), token_strides(lay.d_o), delta, rows, a.N, a.L, a.H, a.D);
     MF_LAUNCHED("evo_delta_kernel");
     MF_DISPATCH_DP(a.D, DP, {
       constexpr size_t smem = sizeof(float) * (4 * kTile * (DP + 4) + 2 * kTile * kPPitch);
@@ -531,7 +532,7 @@ static int bwd_simt(const mf_evo_bwd_args& a, bool partials, cudaStream_t st) {
   return MF_OK;
 }
 
-int evo_bwd_simt(const mf_evo_bwd_args& a, cudaStream_t st) { return bwd_simt(a, true, st); }
+int evo_bwd_simt(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st) { return bwd_simt(a, lay, true, st); }
 
 // ---- backward without any allocation ------------------------------------------------------------------
 // Scratch for the variant below: the per-query delta = rowsum(dO * O) values, B*N*H*L floats.  The array is part
@@ -541,7 +542,7 @@ static __device__ __align__(256) float g_noalloc_delta[kNoAllocDeltaFloats];
 
 size_t evo_bwd_noalloc_max_rows() { return kNoAllocDeltaFloats; }
 
-int evo_bwd_simt_noalloc(const mf_evo_bwd_args& a, cudaStream_t st) {
+int evo_bwd_simt_noalloc(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   const size_t need = (size_t)a.B * a.N * a.H * a.L;
   MF_REQUIRE(need <= kNoAllocDeltaFloats, MF_ERR_UNSUPPORTED,
              "mf_evo_bwd_noalloc: B*N*H*L = %zu query rows exceed the built-in scratch of %zu rows; use mf_evo_bwd with a workspace",
@@ -561,7 +562,7 @@ int evo_bwd_simt_noalloc(const mf_evo_bwd_args& a, cudaStream_t st) {
   mf_evo_bwd_args b = a;
   b.workspace = scratch;
   b.workspace_bytes = kNoAllocDeltaFloats * sizeof(float);
-  return bwd_simt(b, false, st);     // delta is fully rewritten for the B*N*H*L rows in use: nothing to clear
+  return bwd_simt(b, lay, false, st);     // delta is fully rewritten for the B*N*H*L rows in use: nothing to clear
 }
 
 }  // namespace mf

@@ -51,7 +51,7 @@ struct FwdP {
   uint32_t ab_fmt;        // 1 = bf16, 0 = f16
   const void* bias; int64_t bs[4]; int bias_fast;
   const void* mask; int64_t ms[3]; int mask_dtype;
-  void* o; float* lse; int* status;
+  void* o; TokenStrides os; float* lse; int* status;
 };
 
 struct StreamBars {
@@ -378,7 +378,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       fold();
       if (row_ok && !*abort_flag) {
         const float inv = 1.f / l;
-        T* orow = static_cast<T*>(p.o) + ((((int64_t)b * p.N + n) * p.L + i) * p.H + h) * p.D;
+        T* orow = static_cast<T*>(p.o) + p.os.at(b, n, i) + h * p.D;
 #pragma unroll
         for (int d8 = 0; d8 < DP / 8; ++d8) {
           if (d8 * 8 < p.D) {
@@ -406,7 +406,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
 }
 
 template <int DP, typename T, typename TB>
-int launch_fwd(const mf_evo_fwd_args& a, cudaStream_t st) {
+int launch_fwd(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   using C = Cfg<DP>;
   CUtensorMap mq, mk, mv, mb;
   int r;
@@ -426,7 +426,7 @@ int launch_fwd(const mf_evo_fwd_args& a, cudaStream_t st) {
                 (a.bias_strides[0] * bes) % 16 == 0 && (a.bias_strides[1] * bes) % 16 == 0 && (a.bias_strides[2] * bes) % 16 == 0;
   p.mask = a.mask; for (int i = 0; i < 3; ++i) p.ms[i] = a.mask_strides[i];
   p.mask_dtype = a.mask_dtype;
-  p.o = a.o; p.lse = a.lse;
+  p.o = a.o; p.os = token_strides(lay.o); p.lse = a.lse;
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
@@ -469,15 +469,15 @@ int launch_fwd(const mf_evo_fwd_args& a, cudaStream_t st) {
     default: return fail(MF_ERR_BAD_ARG, "unknown bias dtype %d", (int)(dt)); \
   }
 
-int evo_fwd_tc(const mf_evo_fwd_args& a, cudaStream_t st) {
+int evo_fwd_tc(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   int r = MF_OK;
   if (a.dtype == MF_BF16) {
     MF_DISPATCH_BIAS(a.bias_dtype, TB, {
-      r = a.D <= 32 ? launch_fwd<32, __nv_bfloat16, TB>(a, st) : launch_fwd<64, __nv_bfloat16, TB>(a, st);
+      r = a.D <= 32 ? launch_fwd<32, __nv_bfloat16, TB>(a, lay, st) : launch_fwd<64, __nv_bfloat16, TB>(a, lay, st);
     });
   } else {
     MF_DISPATCH_BIAS(a.bias_dtype, TB, {
-      r = a.D <= 32 ? launch_fwd<32, __half, TB>(a, st) : launch_fwd<64, __half, TB>(a, st);
+      r = a.D <= 32 ? launch_fwd<32, __half, TB>(a, lay, st) : launch_fwd<64, __half, TB>(a, lay, st);
     });
   }
   return r;

@@ -29,6 +29,7 @@ struct LnlBwdRowsArgs {
   int64_t M; int K, N, dtype;
   const void *x, *gamma, *w, *dy;
   const float *mean, *rstd;
+  const void *add1, *add2;   // NULL, or added to dx in this order, each sum rounded
   void* dx;
   float *part, *db_part;
 };

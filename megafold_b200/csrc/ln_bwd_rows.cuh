@@ -1,9 +1,13 @@
 // LayerNorm backward of a 128-row tile whose gradient behind the normalisation sits in TMEM: shared by the kernels that
-// produce that gradient (lnl_bwd_tc.cu, transition_bwd_tc.cu), so that it never goes through memory.
+// produce that gradient, so that it never goes through memory.
 //
 // P * 128 threads, thread (row, part): CW = K / P columns of its row.  With w = dyln * gain, xh = (x - mean) * rstd:
-//     dx = (w - (mean_k(xh w) * xh + mean_k(w))) * rstd        d_gain += dyln xh        d_shift += dyln   (sums over rows)
-// The parts of a row exchange their partial means through shared memory.
+//     dx = (w - (mean_k(xh w) * xh + mean_k(w))) * rstd        d_gain += dyln xh   (a sum over rows)
+// The parts of a row exchange sums of four neighbouring columns through shared memory, and every part adds them up in the
+// order of the row-pass kernel (lnl_ops.cu: four columns per lane, then a butterfly over the lanes), each step with that
+// kernel's rounding.  dx is thereby the same bit for bit whichever kernel a size takes.  Where it matters: the gradient of
+// the shift of a pair-bias projection is 0 up to the rounding of d_pair_bias (the logit gradients of a softmax sum to 0), so
+// one flipped bit of dx makes it another number.
 #pragma once
 #include "evo_tc_common.cuh"
 
@@ -28,22 +32,13 @@ __device__ __forceinline__ float column_sum(float (&v)[CW], int lane) {
   return t;
 }
 
-// Sums over the rows, formed tile by tile by a transposing butterfly: two registers per 32 columns.
-template <int CW> struct ColumnSums {
-  float gain[CW / 32], shift[CW / 32];
-  __device__ __forceinline__ ColumnSums() {
-#pragma unroll
-    for (int i = 0; i < CW / 32; ++i) gain[i] = shift[i] = 0.f;
-  }
-};
-
 // dy: the thread's CW columns of dyln (fp32 bits); raw: the same columns of x; gam: the gain of them (shared memory,
-// 16-byte aligned); red: [P][128] float2 of shared memory; `barrier`: a named barrier of the P * 128 threads.
-// Rows beyond the last one come with dy = raw = 0 and mu = rs = 0 and contribute nothing.  Results leave NC columns at a
-// time, packed: emit(first column / NC, dx); grad(k, d, xh) sees each pair of columns once.
-template <typename T, int CW, int P, int NC, typename Emit, typename Grad>
+// 16-byte aligned); red: [P][CW / 8][128] float4 of shared memory; `barrier`: a named barrier of the P * 128 threads.
+// Rows beyond the last one come with dy = raw = 0 and mu = rs = 0 and contribute nothing.  The result leaves packed through
+// emit(dx); grad(k, d, xh) sees each pair of columns once.
+template <typename T, int CW, int P, typename Emit, typename Grad>
 __device__ __forceinline__ void ln_bwd_row(const uint32_t (&dy)[CW], const uint4 (&raw)[CW / 8], float mu, float rs, const float* gam,
-                                           float2 (*red)[128], int part, int row, int barrier, Emit emit, Grad grad) {
+                                           float4 (*red)[CW / 8][128], int part, int row, int barrier, Emit emit, Grad grad) {
   const float2 mm = make_float2(mu, mu), rr = make_float2(rs, rs);
   auto xhat = [&](int k) {             // columns k, k + 1 (k a compile-time constant after unrolling)
     const uint4& q = raw[k / 8];
@@ -51,39 +46,55 @@ __device__ __forceinline__ void ln_bwd_row(const uint32_t (&dy)[CW], const uint4
     return mul2(sub2(Pack2<T>::unpack(u), mm), rr);
   };
   auto grad_of = [&](int k) { return make_float2(__uint_as_float(dy[k]), __uint_as_float(dy[k + 1])); };
-  float2 c1p = make_float2(0.f, 0.f), c2p = c1p;
+  constexpr int G = CW / 4;                  // groups of four columns
+  float s1[G], s2[G];
 #pragma unroll
-  for (int k = 0; k < CW; k += 4) {
+  for (int i = 0; i < G; ++i) {
+    const int k = i * 4;
     const float4 g = *reinterpret_cast<const float4*>(gam + k);
-    const float2 w0 = mul2(grad_of(k), make_float2(g.x, g.y)), w1 = mul2(grad_of(k + 2), make_float2(g.z, g.w));
-    c1p = fma2(xhat(k), w0, c1p); c1p = fma2(xhat(k + 2), w1, c1p);
-    c2p = add2(c2p, add2(w0, w1));
+    const float2 w0 = mul2(grad_of(k), make_float2(g.x, g.y)), w1 = mul2(grad_of(k + 2), make_float2(g.z, g.w)), h0 = xhat(k), h1 = xhat(k + 2);
+    s1[i] = __fmaf_rn(h1.y, w1.y, __fmaf_rn(h1.x, w1.x, __fmaf_rn(h0.y, w0.y, __fmul_rn(h0.x, w0.x))));
+    s2[i] = __fadd_rn(__fadd_rn(__fadd_rn(w0.x, w0.y), w1.x), w1.y);
   }
-  red[part][row] = make_float2(c1p.x + c1p.y, c2p.x + c2p.y);
+#pragma unroll
+  for (int i = 0; i < G / 4; ++i) {
+    red[part][i][row] = make_float4(s1[4 * i], s1[4 * i + 1], s1[4 * i + 2], s1[4 * i + 3]);
+    red[part][G / 4 + i][row] = make_float4(s2[4 * i], s2[4 * i + 1], s2[4 * i + 2], s2[4 * i + 3]);
+  }
   named_sync(barrier, P * 128);
-  float c1 = 0.f, c2 = 0.f;
+  auto total = [&](int at) {                 // the butterfly: parts 0 + 2 and 1 + 3, then these, then the halves of a part's groups
+    static_assert(P == 4, "four parts");
+    float u[G];
 #pragma unroll
-  for (int i = 0; i < P; ++i) { const float2 o = red[i][row]; c1 += o.x; c2 += o.y; }
-  named_sync(barrier, P * 128);              // everybody has read before the next tile writes
-  constexpr float inv_k = 1.f / (CW * P);
-  const float2 cc1 = make_float2(-c1 * inv_k, -c1 * inv_k), cc2 = make_float2(-c2 * inv_k, -c2 * inv_k);
-#pragma unroll
-  for (int n = 0; n < CW; n += NC) {
-    uint32_t o[NC / 2];
-#pragma unroll
-    for (int i = 0; i < NC; i += 4) {
-      const float4 g = *reinterpret_cast<const float4*>(gam + n + i);
-#pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const int k = n + i + e;
-        const float2 h = xhat(k), d = grad_of(k), gg = e ? make_float2(g.z, g.w) : make_float2(g.x, g.y);
-        const float2 z = mul2(fma2(d, gg, fma2(cc1, h, cc2)), rr);
-        o[(i + e) / 2] = Pack2<T>::pack(z.x, z.y);
-        grad(k, d, h);
-      }
+    for (int i = 0; i < G / 4; ++i) {
+      const float4 a = red[0][at + i][row], b = red[1][at + i][row], c = red[2][at + i][row], d = red[3][at + i][row];
+      u[4 * i] = __fadd_rn(__fadd_rn(a.x, c.x), __fadd_rn(b.x, d.x)); u[4 * i + 1] = __fadd_rn(__fadd_rn(a.y, c.y), __fadd_rn(b.y, d.y));
+      u[4 * i + 2] = __fadd_rn(__fadd_rn(a.z, c.z), __fadd_rn(b.z, d.z)); u[4 * i + 3] = __fadd_rn(__fadd_rn(a.w, c.w), __fadd_rn(b.w, d.w));
     }
-    emit(n / NC, o);
+#pragma unroll
+    for (int h = G / 2; h > 0; h >>= 1)
+#pragma unroll
+      for (int i = 0; i < h; ++i) u[i] = __fadd_rn(u[i], u[i + h]);
+    return u[0];
+  };
+  constexpr float inv_k = 1.f / (CW * P);
+  const float c1 = __fmul_rn(total(0), inv_k), c2 = __fmul_rn(total(G / 4), inv_k);
+  named_sync(barrier, P * 128);              // everybody has read before the next tile writes
+  uint32_t o[CW / 2];
+#pragma unroll
+  for (int i = 0; i < CW; i += 4) {
+    const float4 g = *reinterpret_cast<const float4*>(gam + i);
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+      const int k = i + e;
+      const float2 h = xhat(k), d = grad_of(k);
+      const float2 t = make_float2(__fadd_rn(__fmul_rn(c1, h.x), c2), __fadd_rn(__fmul_rn(c1, h.y), c2));      // (packed, the two would be fused)
+      const float2 z = mul2(fma2(d, e ? make_float2(g.z, g.w) : make_float2(g.x, g.y), make_float2(-t.x, -t.y)), rr);
+      o[k / 2] = Pack2<T>::pack(z.x, z.y);
+      grad(k, d, h);
+    }
   }
+  emit(o);
 }
 
 // TMA stores of staged tiles and their bulk groups

@@ -8,7 +8,7 @@
 //
 // Bound: HBM.  dy and x are read once, dx is written once: 2 (N + 2 K) bytes a row, 35 us at 147456 x 128 -> 512 at the
 // measured copy rate.  Before, dyln went through memory in fp32 and dy was read a second time for the bias
-// gradient: a GEMM, a row pass and a column-sum pass of 121 us together, now 58.  The copies alone take 45 us of those (with the
+// gradient: a GEMM, a row pass and a column-sum pass of 121 us together, now 60.  The copies alone take 45 us of those (with the
 // arithmetic taken out): eight tiles per CTA leave a fill and a drain that a longer run would hide.
 //
 // Persistent CTA per SM, 128-row tiles, 640 threads:
@@ -18,8 +18,8 @@
 //   warp 16     tcgen05.mma: dyln (+)= dy slab x W slab (4 products, N = K) into one of two accumulators; for the bias
 //               gradient, per pair of slabs, eight N = 16 products dy^T x ones: the slabs as they are, read MN-major, give
 //               the sums over the rows of 128 columns of dy, and stay in TMEM until the CTA is done.
-//   warp 17     TMA: 64-column slabs of dy (ring of four).  W is fetched once and stays in shared memory when it fits
-//               (N <= 512 at K = 128); otherwise its slabs travel in the ring beside those of dy, from L2.
+//   warp 17     TMA: 64-column slabs of dy and of W (ring of four; W comes from L2: keeping it in shared memory where it
+//               fits, up to N = 512, changed nothing).
 // Every wait is bounded; on expiry the CTA raises a flag, drains and reports through mf_async_status().
 #include "gemm_tc.cuh"
 #include "ln_bwd_rows.cuh"
@@ -30,23 +30,22 @@ using namespace tcx;
 
 constexpr int kRows = 128, kRowWarps = 16, kThreads = (kRowWarps + 4) * 32, kStages = 4;
 // registers per thread: at launch / row warps / helper warps after setmaxnreg (the raise draws on what the drop releases)
-constexpr int kLaunchRegs = 96, kRowRegs = 104, kHelperRegs = 64;
+constexpr int kLaunchRegs = 96, kRowRegs = 112, kHelperRegs = 32;
 static_assert(kRowWarps * 32 * kRowRegs + 128 * kHelperRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 constexpr int kSlabB = kRows * 128;                  // [128 rows][64 columns] of dy
-constexpr int kResidentCap = 128 * 1024;             // bytes of W that stay in shared memory
 constexpr int kMaxN = 2048;                          // 16 TMEM columns per 128 columns of dy: 256 beside the accumulators
 constexpr int kBarrier = 1;
 
 struct LbP {
-  int64_t M; int N, n_mt, n_slabs, w_resident, has_db;
+  int64_t M; int N, n_mt, n_slabs, has_db;
   uint32_t ab_fmt;
-  const void *x, *gamma;
+  const void *x, *gamma, *add1, *add2;
   const float *mean, *rstd;
   float *part, *db_part;
   int* status;
 };
 
-struct Bars { uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2], w_full, db_full; };
+struct Bars { uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2], db_full; };
 
 __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {       // 16-byte multiples
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(p)), "r"(bytes) : "memory");
@@ -58,16 +57,15 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
                   const LbP p) {
   constexpr int CW = K / 4;                          // columns per thread of the LayerNorm backward
   constexpr int kWSlabB = K * 128;                   // [K rows][64 columns] of W
-  constexpr int kOutB = 32 * 32;                     // a warp's staging slab: [32 rows][16 columns]
+  constexpr int kOutB = 32 * CW * 2;                 // a warp's staging slab: [32 rows][CW columns]
+  constexpr int stage_b = kSlabB + kWSlabB;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int stage_b = kSlabB + (p.w_resident ? 0 : kWSlabB);
   uint8_t* sOut = smem;                              // [kRowWarps]
   uint8_t* sRing = sOut + kRowWarps * kOutB;
-  uint8_t* sW = sRing + kStages * stage_b;           // resident slabs of W
+  float4 (*red)[CW / 8][128] = reinterpret_cast<float4 (*)[CW / 8][128]>(sRing + kStages * stage_b);      // [4 parts]
   __shared__ Bars bar;
   __shared__ __align__(16) float gam_s[K];
-  __shared__ float2 red_s[4][128];
   __shared__ __align__(128) uint8_t ones_s[16 * 32];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
@@ -76,7 +74,7 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
     abort_s = 0;
     for (int i = 0; i < kStages; ++i) { mbar_init(&bar.full[i], 1); mbar_init(&bar.empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&bar.acc_full[i], 1); mbar_init(&bar.acc_empty[i], kRowWarps); }
-    mbar_init(&bar.w_full, 1); mbar_init(&bar.db_full, 1);
+    mbar_init(&bar.db_full, 1);
     mbar_fence_init();
     prefetch_tmap(&mdy); prefetch_tmap(&mw); prefetch_tmap(&mdx);
   }
@@ -125,17 +123,32 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
       if (lane == 0) mbar_arrive(&bar.acc_empty[ab]);
       if (named_sync_or(kBarrier, kRowWarps * 32, *abort_flag)) break;
       const bool any = row0 + quarter * 32 < p.M;                    // a store must not start past the last row
-      ln_bwd_row<T, CW, 4, 16>(dy, raw, mu, rs, gam, red_s, part, row_l, kBarrier,
-                               [&](int g, const uint32_t (&out)[8]) {
+      ln_bwd_row<T, CW, 4>(dy, raw, mu, rs, gam, red, part, row_l, kBarrier,
+                               [&](uint32_t (&out)[CW / 2]) {
+                                 auto add = [&](const void* from) {       // a gradient that reaches x beside the operator
+                                   const uint4* ar = reinterpret_cast<const uint4*>(static_cast<const T*>(from) + row * K + part * CW);
+#pragma unroll
+                                   for (int c = 0; c < CW / 8; ++c) {
+                                     const uint4 v = ok ? __ldg(ar + c) : make_uint4(0u, 0u, 0u, 0u);
+                                     const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                                     for (int e = 0; e < 4; ++e) {
+                                       const float2 y = add2(Pack2<T>::unpack(u[e]), Pack2<T>::unpack(out[c * 4 + e]));
+                                       out[c * 4 + e] = Pack2<T>::pack(y.x, y.y);
+                                     }
+                                   }
+                                 };
+                                 if (p.add1) add(p.add1);
+                                 if (p.add2) add(p.add2);
                                  if (lane == 0) bulk_wait_group_read<0>();  // the previous store has read the slab
                                  __syncwarp();
 #pragma unroll
-                                 for (int c = 0; c < 2; ++c)
-                                   *reinterpret_cast<uint4*>(slab + swz_offset(lane, c, 32)) = make_uint4(out[c * 4], out[c * 4 + 1], out[c * 4 + 2], out[c * 4 + 3]);
+                                 for (int c = 0; c < CW / 8; ++c)
+                                   *reinterpret_cast<uint4*>(slab + swz_offset(lane, c, CW * 2)) = make_uint4(out[c * 4], out[c * 4 + 1], out[c * 4 + 2], out[c * 4 + 3]);
                                  fence_async_smem();
                                  __syncwarp();
                                  if (lane == 0) {
-                                   if (any) tma_store_2d(&mdx, slab, part * CW + g * 16, row0 + quarter * 32);
+                                   if (any) tma_store_2d(&mdx, slab, part * CW, row0 + quarter * 32);
                                    bulk_commit_group();
                                  }
                                },
@@ -146,7 +159,7 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
 #pragma unroll
     for (int i = 0; i < CW / 2; ++i) { v[2 * i] = gain[i].x; v[2 * i + 1] = gain[i].y; }
     const float mine = column_sum(v, lane);
-    float* scratch = reinterpret_cast<float*>(red_s);                // [4][K]
+    float* scratch = reinterpret_cast<float*>(red);                  // [4][K]
     named_sync(kBarrier, kRowWarps * 32);
     if (lane < CW) scratch[quarter * K + part * CW + lane] = mine;
     named_sync(kBarrier, kRowWarps * 32);
@@ -167,10 +180,6 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kHelperRegs));
     if (warp == kRowWarps + 1 && lane == 0) {
     // ---------------------------------------------------------------------------------------- TMA producer
-    if (p.w_resident) {
-      mbar_expect_tx(&bar.w_full, ns * kWSlabB);
-      for (int s = 0; s < ns; ++s) tma_load_2d(sW + s * kWSlabB, &mw, &bar.w_full, s * 64, 0);
-    }
     uint32_t cnt = 0;
     for (int t = 0; t < my_tiles && !*abort_flag; ++t) {
       const int row0 = ((int)blockIdx.x + t * (int)gridDim.x) * kRows;
@@ -179,11 +188,16 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
         if (cnt >= kStages) wait_or_flag(&bar.empty[st], ((cnt / kStages) - 1) & 1, abort_flag);
         if (*abort_flag) break;
         // the next tile of x, which the row warps read with plain loads once its products are done
-        if (s == 0 && row0 + (int)gridDim.x * kRows + kRows <= p.M) prefetch_l2(static_cast<const T*>(p.x) + (int64_t)(row0 + (int)gridDim.x * kRows) * K, kRows * K * 2);
+        if (s == 0 && row0 + (int)gridDim.x * kRows + kRows <= p.M) {
+          const int64_t next = (int64_t)(row0 + (int)gridDim.x * kRows) * K;
+          prefetch_l2(static_cast<const T*>(p.x) + next, kRows * K * 2);
+          if (p.add1) prefetch_l2(static_cast<const T*>(p.add1) + next, kRows * K * 2);
+          if (p.add2) prefetch_l2(static_cast<const T*>(p.add2) + next, kRows * K * 2);
+        }
         uint8_t* a = sRing + st * stage_b;
         mbar_expect_tx(&bar.full[st], stage_b);
         tma_load_2d(a, &mdy, &bar.full[st], s * 64, row0);           // columns beyond N and rows beyond M arrive as zeros
-        if (!p.w_resident) tma_load_2d(a + kSlabB, &mw, &bar.full[st], s * 64, 0);
+        tma_load_2d(a + kSlabB, &mw, &bar.full[st], s * 64, 0);
       }
     }
     } else if (warp == kRowWarps) {
@@ -193,7 +207,6 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
     auto dead = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };
     const uint32_t id = idesc_f16(128, K, p.ab_fmt, 0, 0), id_db = idesc_f16(128, 16, p.ab_fmt, 1, 0);
     const uint32_t ones_lo = desc_lo(smem_u32(ones_s), 16);
-    if (p.w_resident) wait_or_flag(&bar.w_full, 0, abort_flag);
     uint32_t cnt = 0;
     for (int t = 0; t < my_tiles && !dead(); ++t) {
       const int ab = t & 1;
@@ -204,7 +217,7 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
         tc_fence_after();
         if (dead()) break;
         const uint32_t a = smem_u32(sRing + st * stage_b);
-        const uint32_t a_lo = desc_lo(a, 16), w_lo = desc_lo(p.w_resident ? smem_u32(sW + s * kWSlabB) : a + kSlabB, 16);
+        const uint32_t a_lo = desc_lo(a, 16), w_lo = desc_lo(a + kSlabB, 16);
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           mma_ss_el(tAcc + ab * K, a_lo + ks * 2, desc_hi(1024, kSw128), w_lo + ks * 2, desc_hi(1024, kSw128), id, s > 0 || ks > 0);
@@ -244,23 +257,21 @@ int launch(const LnlBwdRowsArgs& a, int grid, cudaStream_t st) {
   }
   {
     const int64_t dims[2] = {K, a.M}, str[2] = {1, K};
-    const int box[2] = {16, 32};
-    if ((r = make_tiled_map(&mdx, a.dx, a.dtype, 2, dims, str, box, 32))) return r;
+    const int box[2] = {K / 4, 32};
+    if ((r = make_tiled_map(&mdx, a.dx, a.dtype, 2, dims, str, box, K / 2))) return r;
   }
   LbP p{};
   p.M = a.M; p.N = a.N;
   p.n_mt = (int)((a.M + kRows - 1) / kRows);
   p.n_slabs = (a.N + 127) / 128 * 2;
-  p.w_resident = p.n_slabs * K * 128 <= kResidentCap;
   p.has_db = a.db_part != nullptr;
   p.ab_fmt = a.dtype == MF_BF16 ? 1u : 0u;
-  p.x = a.x; p.gamma = a.gamma; p.mean = a.mean; p.rstd = a.rstd;
+  p.x = a.x; p.gamma = a.gamma; p.add1 = a.add1; p.add2 = a.add2; p.mean = a.mean; p.rstd = a.rstd;
   p.part = a.part; p.db_part = a.db_part;
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
-  const size_t out = kRowWarps * 32 * 32;
-  const size_t smem = 1024 + out + kStages * (size_t)(kSlabB + (p.w_resident ? 0 : K * 128)) + (p.w_resident ? (size_t)p.n_slabs * K * 128 : 0);
+  constexpr size_t smem = 1024 + kRowWarps * 32 * (size_t)K / 2 + kStages * (size_t)(kSlabB + K * 128) + 128 * (size_t)K * 2;
   constexpr auto kern = lnl_bwd_tc_kernel<K, T>;
   if (int e = opt_in_smem<kern>(smem)) return e;
   kern<<<grid, kThreads, smem, st>>>(mdy, mw, mdx, p);

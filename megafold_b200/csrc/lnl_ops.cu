@@ -116,11 +116,21 @@ __global__ void ln_stats_kernel(const T* __restrict__ x, float* __restrict__ mea
   if (lane == 0) { mean[m] = mu; rstd[m] = rsqrtf(v + eps); }
 }
 
+// Gradients that reach x beside the operator, added to dx one after the other, each sum rounded to T (a == NULL: none).
+template <typename T> struct DxAdd {
+  const T *a = nullptr, *b = nullptr;
+  __device__ T operator()(T v, int64_t at) const {
+    T r = from_f<T>(to_f(a[at]) + to_f(v));
+    if (b) r = from_f<T>(to_f(b[at]) + to_f(r));
+    return r;
+  }
+};
+
 // dx = (wdy - (c1*xhat + c2)) * rstd with wdy = dyln*gain, c1 = mean_k(xhat*wdy), c2 = mean_k(wdy)
 template <typename T>
 __global__ void ln_bwd_rows_kernel(const float* __restrict__ dyln, const T* __restrict__ x, const T* __restrict__ gain,
                                    const float* __restrict__ mean, const float* __restrict__ rstd,
-                                   T* __restrict__ dx, int64_t M, int K) {
+                                   T* __restrict__ dx, DxAdd<T> add, int64_t M, int K) {
   const int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (m >= M) return;
   const int lane = threadIdx.x & 31;
@@ -135,7 +145,8 @@ __global__ void ln_bwd_rows_kernel(const float* __restrict__ dyln, const T* __re
   for (int k = lane; k < K; k += 32) {
     float xh = (to_f(x[m * K + k]) - mu) * rs;
     float w = dyln[m * K + k] * to_f(gain[k]);
-    dx[m * K + k] = from_f<T>((w - (c1 * xh + c2)) * rs);
+    const T v = from_f<T>((w - (c1 * xh + c2)) * rs);
+    dx[m * K + k] = add.a ? add(v, m * K + k) : v;
   }
 }
 
@@ -146,7 +157,7 @@ template <typename T, int KJ>
 __global__ void __launch_bounds__(256)
 ln_bwd_rows_fused_kernel(const float* __restrict__ dyln, const T* __restrict__ x, const T* __restrict__ gain,
                          const T* __restrict__ shift, const float* __restrict__ mean, const float* __restrict__ rstd,
-                         T* __restrict__ dx, T* __restrict__ xln, float* __restrict__ part, int64_t M, int K,
+                         T* __restrict__ dx, DxAdd<T> add, T* __restrict__ xln, float* __restrict__ part, int64_t M, int K,
                          int64_t rows_per_block) {
   extern __shared__ float red[];   // [8][2 * K]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -200,6 +211,10 @@ ln_bwd_rows_fused_kernel(const float* __restrict__ dyln, const T* __restrict__ x
           l[e] = from_f<T>(fmaf(xh[j][e], gn[j][e], sh[j][e]));
           dgn[j][e] = fmaf(d[j][e], xh[j][e], dgn[j][e]);
           dsh[j][e] += d[j][e];
+        }
+        if (add.a) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[e] = add(o[e], m * K + k + e);
         }
         *reinterpret_cast<uint2*>(dx + m * K + k) = *reinterpret_cast<const uint2*>(o);
         if (xln) *reinterpret_cast<uint2*>(xln + m * K + k) = *reinterpret_cast<const uint2*>(l);
@@ -464,13 +479,13 @@ bool lnl_bwd_core_tc_ok(int64_t M, int K, int N, int dtype, bool has_ln, const v
 // The fused LayerNorm-backward row pass over M rows; returns the number of blocks (= rows of `part`, [blocks][2 K]).
 template <typename T>
 int launch_ln_bwd_rows(const float* dyln, const T* x, const T* gain, const T* shift, const float* mean, const float* rstd,
-                       T* dx, T* xln, float* part, int64_t M, int K, cudaStream_t st) {
+                       T* dx, DxAdd<T> add, T* xln, float* part, int64_t M, int K, cudaStream_t st) {
   int blocks = (int)((M + 7) / 8 < kRowBlocks ? (M + 7) / 8 : kRowBlocks);      // one row per warp where rows are few
   const int64_t rpb = (M + blocks - 1) / blocks;
   blocks = (int)((M + rpb - 1) / rpb);
   const size_t sm = sizeof(float) * 8 * 2 * K;
   const int kj = (K + 127) / 128;
-#define MF_ROWS(KJ) ln_bwd_rows_fused_kernel<T, KJ><<<blocks, 256, sm, st>>>(dyln, x, gain, shift, mean, rstd, dx, xln, part, M, K, rpb)
+#define MF_ROWS(KJ) ln_bwd_rows_fused_kernel<T, KJ><<<blocks, 256, sm, st>>>(dyln, x, gain, shift, mean, rstd, dx, add, xln, part, M, K, rpb)
   if (kj == 1) MF_ROWS(1); else if (kj == 2) MF_ROWS(2); else if (kj == 3) MF_ROWS(3); else MF_ROWS(4);
 #undef MF_ROWS
   MF_LAUNCHED("ln_bwd_rows_fused_kernel");
@@ -482,7 +497,7 @@ int launch_ln_bwd_rows(const float* dyln, const T* x, const T* gain, const T* sh
 // tc: both GEMMs on the tensor cores (gemm_tc), with one fused row pass between them.
 template <typename T>
 int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* shift, const T* w, const T* dy,
-                 const float* mean, const float* rstd, T* dx, float* dw, float* db, float* d_ln_w, float* d_ln_b,
+                 const float* mean, const float* rstd, T* dx, DxAdd<T> add, float* dw, float* db, float* d_ln_w, float* d_ln_b,
                  Carver& ws, bool tc, int dtype, cudaStream_t st, const T* xln_ready = nullptr,
                  const float* dyln_ready = nullptr) {
   int r;
@@ -492,7 +507,7 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
       const int blocks = lnl_bwd_rows_tc_blocks(M);
       float* part = ws.take<float>((size_t)blocks * K);
       float* dpart = db || d_ln_b ? ws.take<float>((size_t)blocks * N) : nullptr;
-      r = lnl_bwd_rows_tc(LnlBwdRowsArgs{M, K, N, dtype, x, gain, w, dy, mean, rstd, dx, part, dpart}, st);
+      r = lnl_bwd_rows_tc(LnlBwdRowsArgs{M, K, N, dtype, x, gain, w, dy, mean, rstd, add.a, add.b, dx, part, dpart}, st);
       if (r) return r;
       float* db_sum = db || !d_ln_b ? db : ws.take<float>(N);
       r = colsum_pair("lnl_bwd_column_sums", part, K, K, d_ln_w, nullptr, dpart, db_sum ? N : 0, db_sum, blocks, st);
@@ -513,7 +528,7 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
         r = gemm_tc(GemmTcArgs{dy, w, dyln, M, K, N, dtype, 0, 0, 1}, st);
         if (r) return r;
       }
-      const int blocks = launch_ln_bwd_rows<T>(dyln, x, gain, shift, mean, rstd, dx, xln, part, M, K, st);
+      const int blocks = launch_ln_bwd_rows<T>(dyln, x, gain, shift, mean, rstd, dx, add, xln, part, M, K, st);
       if (db && N <= 2048) {
         const int64_t rows = (M + blocks - 1) / blocks;           // the same blocks of rows as the pass above
         float* dpart = ws.take<float>((size_t)kRowBlocks * N);
@@ -537,12 +552,12 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
     r = launch_gemm_simt<false, true>("lnl_bwd_dyln", M, K, N, 1, LoadRM<T>{dy, N}, LoadTr<T>{w, N},
                                       EpiPartial{dyln, 0, K, K}, st);
     if (r) return r;
-    ln_bwd_rows_kernel<T><<<(unsigned)((M + 7) / 8), 256, 0, st>>>(dyln, x, gain, mean, rstd, dx, M, K);
+    ln_bwd_rows_kernel<T><<<(unsigned)((M + 7) / 8), 256, 0, st>>>(dyln, x, gain, mean, rstd, dx, add, M, K);
     MF_LAUNCHED("ln_bwd_rows_kernel");
     r = colsum("lnl_bwd_dgain", ColDyXhat<T>{dyln, x, mean, rstd, K}, d_ln_w, col_scratch, M, K, st);
     if (r) return r;
     if (d_ln_b) { r = colsum("lnl_bwd_dshift", ColF32{dyln, K}, d_ln_b, col_scratch, M, K, st); if (r) return r; }
-  } else {
+  } else {       // without LayerNorm: only the Transition comes here, which adds nothing
     r = launch_gemm_simt<false, true>("lin_bwd_dx", M, K, N, 1, LoadRM<T>{dy, N}, LoadTr<T>{w, N},
                                       EpiStore<T>{dx, K, K, nullptr}, st);
     if (r) return r;
@@ -616,13 +631,14 @@ size_t lnl_bwd_workspace(const mf_lnl_bwd_args& a) {
 bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a) { return lnl_bwd_use_tc(a); }
 bool transition_bwd_runs_on_tc(const mf_transition_bwd_args& a) { return transition_bwd_use_tc(a); }
 
-int lnl_bwd(const mf_lnl_bwd_args& a, cudaStream_t st) {
+int lnl_bwd(const mf_lnl_bwd_args& a, const void* add1, const void* add2, cudaStream_t st) {
   Carver ws(a.workspace);
-  const bool tc = lnl_bwd_use_tc(a);
+  const bool tc = lnl_bwd_use_tc(a) && ((reinterpret_cast<uintptr_t>(add1) | reinterpret_cast<uintptr_t>(add2)) & 15) == 0;
+  if (!add1) { add1 = add2; add2 = nullptr; }
   MF_DISPATCH_FLOAT(a.dtype, T, {
     int r = lnl_bwd_core<T>(a.M, a.K, a.N, static_cast<const T*>(a.x), static_cast<const T*>(a.ln_w),
                             static_cast<const T*>(a.ln_b), static_cast<const T*>(a.w), static_cast<const T*>(a.dy),
-                            a.mean, a.rstd, static_cast<T*>(a.dx), a.dw, a.db, a.d_ln_w, a.d_ln_b, ws, tc, a.dtype, st);
+                            a.mean, a.rstd, static_cast<T*>(a.dx), DxAdd<T>{static_cast<const T*>(add1), static_cast<const T*>(add2)}, a.dw, a.db, a.d_ln_w, a.d_ln_b, ws, tc, a.dtype, st);
     if (r) return r;
   });
   return MF_OK;
@@ -746,7 +762,7 @@ int transition_bwd_tc(const mf_transition_bwd_args& a, cudaStream_t st) {
   if (r) return r;
   return lnl_bwd_core<T>(M, a.dim, 2 * I, static_cast<const T*>(a.x), static_cast<const T*>(a.ln_w),
                          static_cast<const T*>(a.ln_b), static_cast<const T*>(a.w1), h, a.mean, a.rstd,
-                         static_cast<T*>(a.dx), a.dw1, nullptr, a.d_ln_w, a.d_ln_b, ws, true, a.dtype, st, xln);
+                         static_cast<T*>(a.dx), DxAdd<T>{}, a.dw1, nullptr, a.d_ln_w, a.d_ln_b, ws, true, a.dtype, st, xln);
 }
 
 // Fused composition (dim = 128): one kernel recomputes h on chip and leaves g, dh (chunk-ordered columns) and dyln in
@@ -802,7 +818,7 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
     r = gemm_tc(g2, st);
     if (r) return r;
     part_rows += launch_ln_bwd_rows<T>(dyln, static_cast<const T*>(ac.x), static_cast<const T*>(a.ln_w), static_cast<const T*>(a.ln_b),
-                                       ac.mean, ac.rstd, static_cast<T*>(ac.dx), xln, part + (size_t)part_rows * 2 * K, rows, K, st);
+                                       ac.mean, ac.rstd, static_cast<T*>(ac.dx), DxAdd<T>{}, xln, part + (size_t)part_rows * 2 * K, rows, K, st);
     // dw1 (chunk-ordered columns) += LN(x)^T dh
     GemmTcArgs g1{xln, dh, dw1p, K, 2 * I, rows, a.dtype, 1, 1, 2};
     g1.accumulate = c > 0;
@@ -846,7 +862,7 @@ int transition_bwd(const mf_transition_bwd_args& a, cudaStream_t st) {
     if (r) return r;
     // 4. LayernormLinear backward with dy := dh
     r = lnl_bwd_core<T>(a.M, a.dim, 2 * I, x, static_cast<const T*>(a.ln_w), static_cast<const T*>(a.ln_b), w1, h,
-                        a.mean, a.rstd, static_cast<T*>(a.dx), a.dw1, nullptr, a.d_ln_w, a.d_ln_b, ws, false, a.dtype, st);
+                        a.mean, a.rstd, static_cast<T*>(a.dx), DxAdd<T>{}, a.dw1, nullptr, a.d_ln_w, a.d_ln_b, ws, false, a.dtype, st);
     if (r) return r;
   });
   return MF_OK;

@@ -36,7 +36,12 @@ struct Api {
   MF_ENTRY(mf_evo_bwd);
   MF_ENTRY(mf_lnl_fwd);
   MF_ENTRY(mf_lnl_bwd_workspace_bytes);
-  MF_ENTRY(mf_lnl_bwd);
+  MF_ENTRY(mf_lnl_bwd_add);
+  MF_ENTRY(mf_gate_fwd);
+  MF_ENTRY(mf_gate_bwd);
+  MF_ENTRY(mf_bias_layout);
+  MF_ENTRY(mf_evo_fwd_laid_out);
+  MF_ENTRY(mf_evo_bwd_laid_out);
   MF_ENTRY(mf_swiglu_fwd);
   MF_ENTRY(mf_swiglu_bwd);
   MF_ENTRY(mf_transition_fwd_workspace_bytes);
@@ -58,7 +63,8 @@ void load(const std::string& path) {
   };
 #define MF_LOAD(name) api.name = reinterpret_cast<decltype(api.name)>(get(#name))
   MF_LOAD(mf_evo_fwd_workspace_bytes); MF_LOAD(mf_evo_fwd_with_workspace); MF_LOAD(mf_evo_bwd_workspace_bytes); MF_LOAD(mf_evo_bwd);
-  MF_LOAD(mf_lnl_fwd); MF_LOAD(mf_lnl_bwd_workspace_bytes); MF_LOAD(mf_lnl_bwd);
+  MF_LOAD(mf_lnl_fwd); MF_LOAD(mf_lnl_bwd_workspace_bytes); MF_LOAD(mf_lnl_bwd_add);
+  MF_LOAD(mf_gate_fwd); MF_LOAD(mf_gate_bwd); MF_LOAD(mf_bias_layout); MF_LOAD(mf_evo_fwd_laid_out); MF_LOAD(mf_evo_bwd_laid_out);
   MF_LOAD(mf_swiglu_fwd); MF_LOAD(mf_swiglu_bwd);
   MF_LOAD(mf_transition_fwd_workspace_bytes); MF_LOAD(mf_transition_fwd);
   MF_LOAD(mf_transition_bwd_workspace_bytes); MF_LOAD(mf_transition_bwd);
@@ -246,7 +252,7 @@ std::tuple<Tensor, Tensor, Tensor> lnl_fwd_raw(const Tensor& x, const Tensor& w,
 
 // (dx, dw, db, d_ln_w, d_ln_b), parameter gradients fp32
 std::array<Tensor, 5> lnl_bwd_raw(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& lw, const Tensor& lb, const Tensor& mean,
-                                  const Tensor& rstd, bool has_linear_bias, int64_t flags) {
+                                  const Tensor& rstd, bool has_linear_bias, int64_t flags, const Tensor* add1 = nullptr, const Tensor* add2 = nullptr) {
   const int64_t K = x.size(-1), M = rows_of(x), N = w.size(1);
   Tensor dx = at::empty(x.sizes(), x.options());
   Tensor dw = empty_f32({K, N}, x), dlw = empty_f32({K}, x), dlb, db;
@@ -260,7 +266,7 @@ std::array<Tensor, 5> lnl_bwd_raw(const Tensor& dy, const Tensor& x, const Tenso
   a.d_ln_b = static_cast<float*>(ptr(dlb));
   Tensor ws = workspace(api.mf_lnl_bwd_workspace_bytes(&a), x);
   a.workspace = ws.data_ptr(); a.workspace_bytes = (size_t)ws.numel();
-  check(api.mf_lnl_bwd(&a, stream_of(x)), "mf_lnl_bwd");
+  check(api.mf_lnl_bwd_add(&a, add1 ? add1->data_ptr() : nullptr, add2 ? add2->data_ptr() : nullptr, stream_of(x)), "mf_lnl_bwd");
   return {dx, dw, db, dlw, dlb};
 }
 
@@ -479,6 +485,212 @@ Tensor transition(const Tensor& x, const OptTensor& lw, const OptTensor& lb, con
   return TransitionFn::apply(x, lw, lb, w1, w2);
 }
 
+// ---- pieces of a Pairformer block -----------------------------------------------------------------------------------
+// Attention with a merged q/k/v/gate projection, its output gate, output projection and residual connection as one
+// function: q, k and v are strided views of the projection, their gradients are written straight into the projection's
+// gradient, attention along the other axis of a square x (`swap`) works on strides, and the gradients of the residual
+// connection and of the bias projection are added where the merged projection's backward produces dx.  Composed from
+// separate autograd functions, the copies and additions between them took a quarter of the block's time.
+//
+// Every value is that of the composed form, rounding for rounding: the gradient of a bias projection's shift is 0 up to the
+// rounding of d_pair_bias (a softmax's logit gradients sum to 0), so it is another number as soon as one bit before it is.
+struct Attn { Tensor lw, lb, w, b, w_out; };
+
+mf_evo_layout token_layout(int64_t n, int64_t L, int64_t tok_o, int64_t tok_q, bool swap) {
+  mf_evo_layout l{};
+  for (int64_t* s : {l.o, l.d_o}) { s[0] = n * L * tok_o; s[1] = swap ? tok_o : L * tok_o; s[2] = swap ? L * tok_o : tok_o; }
+  l.d_qkv[0] = n * L * tok_q; l.d_qkv[1] = swap ? tok_q : L * tok_q; l.d_qkv[2] = swap ? L * tok_q : tok_q;
+  return l;
+}
+template <typename A>
+void fill_attn(A& a, const Tensor& y, const Tensor& mask, const Tensor& bias, int64_t n, int64_t L, int64_t H, int64_t D, bool swap) {
+  const int64_t inner = H * D, tok = 4 * inner, es = y.element_size();
+  a.B = 1; a.N = (int32_t)(swap ? L : n); a.L = (int32_t)(swap ? n : L); a.H = (int32_t)H; a.D = (int32_t)D;
+  a.dtype = dtype_code(y.scalar_type()); a.bias_dtype = dtype_code(bias.scalar_type()); a.mask_dtype = dtype_code(mask.scalar_type());
+  const char* p = static_cast<const char*>(y.data_ptr());
+  a.q = p; a.k = p + inner * es; a.v = p + 2 * inner * es;
+  for (int64_t* s : {a.q_strides, a.k_strides, a.v_strides}) {
+    s[0] = n * L * tok; s[1] = swap ? tok : L * tok; s[2] = swap ? L * tok : tok; s[3] = D; s[4] = 1;
+  }
+  a.mask = mask.data_ptr();
+  a.mask_strides[0] = a.mask_strides[1] = 0; a.mask_strides[2] = mask.stride(0);
+  a.bias = bias.data_ptr();
+  a.bias_strides[0] = bias.stride(0); a.bias_strides[1] = bias.stride(2); a.bias_strides[2] = bias.stride(3); a.bias_strides[3] = bias.stride(4);
+}
+
+struct AttnSaved { Tensor y, mean, rstd, o, lse, og; };
+// x [n, L, C] contiguous -> x + attention(x)
+Tensor attn_fwd(const Tensor& x, const Attn& p, const Tensor& mask, const Tensor& bias, int64_t H, bool swap, AttnSaved& s, int64_t lnl_flags) {
+  const int64_t n = x.size(0), L = x.size(1), inner = p.w.size(1) / 4, D = inner / H;
+  std::tie(s.y, s.mean, s.rstd) = lnl_fwd_raw(x, p.w, p.b, p.lw, p.lb, 1e-5, lnl_flags);
+  s.o = at::empty({n, L, inner}, x.options());
+  s.lse = empty_f32({swap ? L : n, H, swap ? n : L}, x);
+  mf_evo_fwd_args a{};
+  fill_attn(a, s.y, mask, bias, n, L, H, D, swap);
+  a.o = s.o.data_ptr(); a.lse = s.lse.data_ptr<float>();
+  const mf_evo_layout lay = token_layout(n, L, inner, 4 * inner, swap);
+  // no scratch: a bias that TMA cannot address (L not a multiple of 8) takes the general kernel, whose values the composed
+  // form had
+  check(api.mf_evo_fwd_laid_out(&a, &lay, nullptr, 0, stream_of(x)), "mf_evo_fwd");
+  s.og = at::empty_like(s.o);
+  check(api.mf_gate_fwd(s.o.data_ptr(), static_cast<char*>(s.y.data_ptr()) + 3 * inner * x.element_size(), 4 * inner, s.og.data_ptr(), n * L, (int32_t)inner,
+                        a.dtype, stream_of(x)), "mf_gate_fwd");
+  Tensor out = at::mm(s.og.view({n * L, inner}), p.w_out.t());
+  return out.add_(x.view({n * L, x.size(2)})).view(x.sizes());
+}
+
+struct AttnGrads { Tensor dx, dw, db, dlw, dlb, d_w_out, d_bias; };
+// bias_dx turns d_bias into the gradient that x receives through the bias (undefined: none); dx comes with it and with
+// d_out, the residual connection's, added in the order of the composed form
+template <typename BiasDx>
+AttnGrads attn_bwd(const Tensor& d_out, const Tensor& x, const Attn& p, const Tensor& mask, const Tensor& bias, int64_t H, bool swap, const AttnSaved& s,
+                   BiasDx bias_dx) {
+  const int64_t n = x.size(0), L = x.size(1), C = x.size(2), inner = p.w.size(1) / 4, D = inner / H, P = n * L, es = x.element_size();
+  AttnGrads g;
+  const Tensor d2 = d_out.view({P, C});
+  g.d_w_out = at::mm(d2.t(), s.og.view({P, inner}));
+  Tensor d_og = at::mm(d2, p.w_out), d_o = at::empty({n, L, inner}, x.options()), dy = at::empty({P, 4 * inner}, x.options());
+  const char* y = static_cast<const char*>(s.y.data_ptr());
+  char* dyp = static_cast<char*>(dy.data_ptr());
+  const int dt = dtype_code(x.scalar_type());
+  check(api.mf_gate_bwd(d_og.data_ptr(), s.o.data_ptr(), y + 3 * inner * es, 4 * inner, d_o.data_ptr(), dyp + 3 * inner * es, 4 * inner, P, (int32_t)inner, dt,
+                        stream_of(x)), "mf_gate_bwd");
+  d_og.reset();
+  g.d_bias = at::empty(bias.sizes(), bias.options());
+  mf_evo_bwd_args a{};
+  fill_attn(a, s.y, mask, bias, n, L, H, D, swap);
+  a.dbias_dtype = dtype_code(g.d_bias.scalar_type());
+  a.o = s.o.data_ptr(); a.d_o = d_o.data_ptr(); a.lse = s.lse.data_ptr<float>();
+  a.dq = dyp; a.dk = dyp + inner * es; a.dv = dyp + 2 * inner * es; a.d_bias = g.d_bias.data_ptr();
+  const mf_evo_layout lay = token_layout(n, L, inner, 4 * inner, swap);
+  Tensor ws = workspace(api.mf_evo_bwd_workspace_bytes(&a), x);
+  a.workspace = ws.data_ptr(); a.workspace_bytes = (size_t)ws.numel();
+  check(api.mf_evo_bwd_laid_out(&a, &lay, stream_of(x)), "mf_evo_bwd");
+  ws.reset(); d_o.reset();
+  const Tensor through_bias = bias_dx(g.d_bias);
+  const Tensor *add1 = through_bias.defined() ? &through_bias : nullptr, *add2 = &d_out;
+  if (!swap) std::swap(add1, add2);
+  auto r = lnl_bwd_raw(dy, x, p.w, p.lw, p.lb, s.mean, s.rstd, true, 0, add1, add2);
+  cast_batch({{&r[1], p.w.scalar_type()}, {&r[2], p.b.scalar_type()}, {&r[3], p.lw.scalar_type()}, {&r[4], p.lb.scalar_type()}});
+  g.dx = r[0]; g.dw = r[1]; g.db = r[2]; g.dlw = r[3]; g.dlb = r[4];
+  return g;
+}
+
+// Pair bias [1, 1, H, L, L] projected from x [L, L, C]: element (i, j) from x[i, j], or from x[j, i] with `swap`.
+struct BiasSaved { Tensor mean, rstd; };
+Tensor bias_fwd(const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w, int64_t H, bool swap, BiasSaved& s) {
+  const int64_t L = x.size(0);
+  Tensor rows;
+  std::tie(rows, s.mean, s.rstd) = lnl_fwd_raw(x, w, Tensor(), lw, lb, 1e-5, 0);
+  Tensor bias = at::empty({1, 1, H, L, L}, x.options());
+  check(api.mf_bias_layout(rows.data_ptr(), bias.data_ptr(), (int32_t)L, (int32_t)w.size(1), (int32_t)H, swap, 0, dtype_code(x.scalar_type()), stream_of(x)),
+        "mf_bias_layout");
+  return bias;
+}
+// (dx, dw, dlw, dlb)
+std::array<Tensor, 4> bias_bwd(const Tensor& d_bias, const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w, bool swap, const BiasSaved& s) {
+  const int64_t L = x.size(0), np = w.size(1);
+  Tensor rows = at::empty({L * L, np}, x.options());
+  check(api.mf_bias_layout(rows.data_ptr(), d_bias.data_ptr(), (int32_t)L, (int32_t)np, (int32_t)d_bias.size(2), swap, 1, dtype_code(x.scalar_type()),
+                           stream_of(x)), "mf_bias_layout");
+  auto r = lnl_bwd_raw(rows, x, w, lw, lb, s.mean, s.rstd, false, 0);
+  cast_batch({{&r[1], w.scalar_type()}, {&r[3], lw.scalar_type()}, {&r[4], lb.scalar_type()}});
+  return {r[0], r[1], r[3], r[4]};
+}
+
+// x [L, L, C] + attention over its rows (or, with `swap`, its columns) with a pair bias projected from x itself
+struct TriangleFn : torch::autograd::Function<TriangleFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out,
+                          const Tensor& plw, const Tensor& plb, const Tensor& pw, const Tensor& mask, int64_t H, bool swap) {
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = x_.contiguous();
+    AttnSaved s; BiasSaved bs;
+    const Tensor bias = bias_fwd(x, plw, plb, pw, H, swap, bs);
+    Tensor out = attn_fwd(x, {lw, lb, w, b, w_out}, mask, bias, H, swap, s, 0);
+    ctx->save_for_backward({x, lw, lb, w, b, w_out, plw, plb, pw, mask, bias, s.y, s.mean, s.rstd, s.o, s.lse, s.og, bs.mean, bs.rstd});
+    ctx->saved_data["H"] = H; ctx->saved_data["swap"] = swap;
+    return out;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const auto v = ctx->get_saved_variables();
+    const c10::cuda::CUDAGuard guard(v[0].device());
+    const int64_t H = ctx->saved_data["H"].toInt();
+    const bool swap = ctx->saved_data["swap"].toBool();
+    const AttnSaved s{v[11], v[12], v[13], v[14], v[15], v[16]};
+    std::array<Tensor, 4> p;
+    AttnGrads a = attn_bwd(g[0].contiguous(), v[0], {v[1], v[2], v[3], v[4], v[5]}, v[9], v[10], H, swap, s, [&](const Tensor& d_bias) {
+      p = bias_bwd(d_bias, v[0], v[6], v[7], v[8], swap, BiasSaved{v[17], v[18]});
+      return p[0];
+    });
+    return {a.dx, a.dlw, a.dlb, a.dw, a.db, a.d_w_out, p[2], p[3], p[1], Tensor(), Tensor(), Tensor()};
+  }
+};
+
+// x [n, L, C] + attention over its rows with a given pair bias
+struct GatedAttnFn : torch::autograd::Function<GatedAttnFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out,
+                          const Tensor& mask, const Tensor& bias, int64_t H) {
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = x_.contiguous();
+    AttnSaved s;
+    // the projection of these few wide rows keeps fp32 operands and sums (0.4 % of a block at 768 tokens): its values too
+    // are those of the composed form
+    Tensor out = attn_fwd(x, {lw, lb, w, b, w_out}, mask, bias, H, false, s, MF_FLAG_FORCE_SIMT);
+    ctx->save_for_backward({x, lw, lb, w, b, w_out, mask, bias, s.y, s.mean, s.rstd, s.o, s.lse, s.og});
+    ctx->saved_data["H"] = H;
+    return out;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const auto v = ctx->get_saved_variables();
+    const c10::cuda::CUDAGuard guard(v[0].device());
+    const AttnSaved s{v[8], v[9], v[10], v[11], v[12], v[13]};
+    AttnGrads a = attn_bwd(g[0].contiguous(), v[0], {v[1], v[2], v[3], v[4], v[5]}, v[6], v[7], ctx->saved_data["H"].toInt(), false, s,
+                           [](const Tensor&) { return Tensor(); });
+    return {a.dx, a.dlw, a.dlb, a.dw, a.db, a.d_w_out, Tensor(), a.d_bias, Tensor()};
+  }
+};
+
+struct PairBiasFn : torch::autograd::Function<PairBiasFn> {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, int64_t H) {
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const Tensor x = x_.contiguous();
+    BiasSaved s;
+    Tensor bias = bias_fwd(x, lw, lb, w, H, false, s);
+    ctx->save_for_backward({x, lw, lb, w, s.mean, s.rstd});
+    return bias;
+  }
+  static tensor_list backward(AutogradContext* ctx, tensor_list g) {
+    at::NoGradGuard no_grad;
+    const auto v = ctx->get_saved_variables();
+    const c10::cuda::CUDAGuard guard(v[0].device());
+    auto p = bias_bwd(g[0].contiguous(), v[0], v[1], v[2], v[3], false, BiasSaved{v[4], v[5]});
+    return {p[0], p[2], p[3], p[1], Tensor()};
+  }
+};
+
+Tensor triangle(const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out, const Tensor& plw, const Tensor& plb,
+                const Tensor& pw, const Tensor& mask, int64_t H, bool swap) {
+  require_cuda({&x, &lw, &lb, &w, &b, &w_out, &plw, &plb, &pw, &mask});
+  TORCH_CHECK_VALUE(x.dim() == 3 && x.size(0) == x.size(1) && mask.dim() == 1 && mask.size(0) == x.size(1) && w.size(0) == x.size(2) && pw.size(0) == x.size(2) &&
+                        w.size(1) % (4 * H) == 0 && pw.size(1) >= H, "x must be [L, L, C] with a mask [L], got ", shape(x), " and ", shape(mask));
+  return TriangleFn::apply(x, lw, lb, w, b, w_out, plw, plb, pw, mask, H, swap);
+}
+Tensor gated_attention(const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out, const Tensor& mask,
+                       const Tensor& bias, int64_t H) {
+  require_cuda({&x, &lw, &lb, &w, &b, &w_out, &mask, &bias});
+  TORCH_CHECK_VALUE(x.dim() == 3 && mask.dim() == 1 && mask.size(0) == x.size(1) && w.size(0) == x.size(2) && w.size(1) % (4 * H) == 0 && bias.dim() == 5 &&
+                        bias.size(2) == H && bias.size(3) == x.size(1) && bias.size(4) == x.size(1), "x must be [n, L, C] with a mask [L] and a bias [1, 1, H, L, L], got ",
+                    shape(x), ", ", shape(mask), " and ", shape(bias));
+  return GatedAttnFn::apply(x, lw, lb, w, b, w_out, mask, bias, H);
+}
+Tensor pair_bias(const Tensor& x, const Tensor& lw, const Tensor& lb, const Tensor& w, int64_t H) {
+  require_cuda({&x, &lw, &lb, &w});
+  TORCH_CHECK_VALUE(x.dim() == 3 && x.size(0) == x.size(1) && w.size(0) == x.size(2) && w.size(1) >= H, "x must be [L, L, C], got ", shape(x));
+  return PairBiasFn::apply(x, lw, lb, w, H);
+}
+
 // std::array of tensors, undefined ones as None
 template <size_t N>
 std::array<OptTensor, N> optional(std::array<Tensor, N> r) {
@@ -512,4 +724,7 @@ PYBIND11_MODULE(_native, m) {
     return optional(transition_backward(dy, x, lw, lb, w1, w2, mean, rstd, flags));
   }, release());
   m.def("transition", &transition, release());
+  m.def("triangle", &triangle, release());
+  m.def("gated_attention", &gated_attention, release());
+  m.def("pair_bias", &pair_bias, release());
 }

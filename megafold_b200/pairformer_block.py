@@ -162,7 +162,7 @@ class PairformerBlock(nn.Module):
                  expansion=4, group=None, ops=None, device=None, dtype=None):
         super().__init__()
         kw = dict(device=device, dtype=dtype)
-        self.group, self.ops = group, ops
+        self.group, self.ops, self.native_ok = group, ops, ops is None
         self.tri_start = _Attn(dim_pair, tri_heads, tri_dim_head, dim_pair, **kw)
         self.tri_end = _Attn(dim_pair, tri_heads, tri_dim_head, dim_pair, **kw)
         self.single_attn = _Attn(dim_single, single_heads, single_dim_head, dim_pair, **kw)
@@ -191,11 +191,32 @@ class PairformerBlock(nn.Module):
         o = (o * torch.sigmoid(g)).reshape(n, L, a.inner)            # the gate is read through its strided view: no packing copy
         return F.linear(o, a.w_out)
 
+    def _whole(self, x, single):
+        """One GPU holds all rows and everything has one type: the attentions run as single native functions (projection,
+        attention, gate, output projection, residual; csrc/torch_ops.cpp), the ending-node one on strides instead of a
+        transposed copy.  Otherwise, and with injected operators, they are composed from the pieces above."""
+        return (self.native_ok and _world(self.group) == 1 and x.is_cuda and x.shape[0] == x.shape[1] and not torch.is_autocast_enabled("cuda")
+                and all(t.dtype == x.dtype for t in (single, *self.parameters()))
+                and all(a.inner % 8 == 0 for a in (self.tri_start, self.tri_end, self.single_attn)))
+
+    def _forward_whole(self, x, single, mask):
+        from . import _lib
+        native = _lib.native()
+        mask = mask.contiguous()
+        for a, swap in ((self.tri_start, False), (self.tri_end, True)):
+            x = native.triangle(x, a.ln_w, a.ln_b, a.w_qkvg, a.b_qkvg, a.w_out, a.pair_ln_w, a.pair_ln_b, a.w_pair_bias, mask, a.heads, swap)
+        x = x + native.transition(x, self.tr_ln_w, self.tr_ln_b, self.tr_w1, self.tr_w2)
+        a = self.single_attn
+        bias = native.pair_bias(x, a.pair_ln_w, a.pair_ln_b, a.w_pair_bias, a.heads)
+        return x, native.gated_attention(single[None], a.ln_w, a.ln_b, a.w_qkvg, a.b_qkvg, a.w_out, mask, bias, a.heads)[0]
+
     # ---- block -------------------------------------------------------------------------------------
     def forward(self, pair_rows, single, mask):
         """pair_rows [n_local, L, dim_pair] (this rank's rows), single [L, dim_single] (replicated), mask bool [L]."""
         if self.ops is None:
             self.ops = cuda_ops()
+        if self._whole(pair_rows, single):
+            return self._forward_whole(pair_rows, single, mask)
         L = pair_rows.shape[1]
         x = pair_rows
         x = x + self._attention(self.tri_start, x, mask, self._pair_bias(self.tri_start, x, L, True))
