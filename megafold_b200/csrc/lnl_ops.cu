@@ -765,9 +765,9 @@ int transition_bwd_tc(const mf_transition_bwd_args& a, cudaStream_t st) {
                          static_cast<T*>(a.dx), DxAdd<T>{}, a.dw1, nullptr, a.d_ln_w, a.d_ln_b, ws, true, a.dtype, st, xln);
 }
 
-// Fused composition (dim = 128): one kernel recomputes h on chip and leaves g, dh (chunk-ordered columns) and dyln in
-// HBM; then the LayerNorm row pass and the two weight-gradient GEMMs.  The rows are processed in ranges of at most
-// kTransitionChunkRows so that the scratch (g, dh, dyln, LN(x): 3.8 KB per row at inner = 512) stays below what the
+// Fused composition (dim = 128): one kernel recomputes h on chip, leaves g and dh (chunk-ordered columns) in HBM and writes
+// dx; then the two weight-gradient GEMMs.  The rows are processed in ranges of at most kTransitionChunkRows so that the
+// scratch (g and dh: 3 KB per row at inner = 512) stays below what the
 // reference's forward keeps as saved activations; the weight gradients accumulate over the ranges, the partial column
 // sums of every range are reduced together at the end.
 constexpr int64_t kTransitionChunkRows = 131072;
@@ -783,9 +783,8 @@ size_t transition_bwd_fused_bytes(const mf_transition_bwd_args& a) {
   const size_t es = dtype_size(a.dtype);
   const TransitionChunks ch = transition_chunks(a.M);
   const size_t rows = (size_t)(ch.rows < a.M ? ch.rows : a.M);
-  return align_up(rows * a.inner * es, 256) + align_up(rows * 2 * a.inner * es, 256) + align_up(sizeof(float) * rows * a.dim, 256) +
-         align_up(rows * a.dim * es, 256) + align_up(sizeof(float) * (size_t)a.dim * 2 * a.inner, 256) +
-         align_up(sizeof(float) * (size_t)ch.n * kRowBlocks * 2 * a.dim, 256);
+  return align_up(rows * a.inner * es, 256) + align_up(rows * 2 * a.inner * es, 256) + align_up(sizeof(float) * (size_t)a.dim * 2 * a.inner, 256) +
+         align_up(sizeof(float) * (size_t)ch.n * transition_bwd_fused_blocks(rows) * 2 * a.dim, 256);
 }
 
 template <typename T>
@@ -797,10 +796,8 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
   const size_t rows_max = (size_t)(ch.rows < M ? ch.rows : M);
   T* g = ws.take<T>(rows_max * I);
   T* dh = ws.take<T>(rows_max * 2 * I);
-  float* dyln = ws.take<float>(rows_max * K);
-  T* xln = ws.take<T>(rows_max * K);
   float* dw1p = ws.take<float>((size_t)K * 2 * I);
-  float* part = ws.take<float>((size_t)ch.n * kRowBlocks * 2 * K);
+  float* part = ws.take<float>((size_t)ch.n * transition_bwd_fused_blocks(rows_max) * 2 * K);
   int part_rows = 0;
   for (int c = 0; c < ch.n; ++c) {
     const int64_t m0 = (int64_t)c * ch.rows, rows = (m0 + ch.rows < M ? ch.rows : M - m0);
@@ -811,16 +808,15 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
     ac.dy = static_cast<const T*>(a.dy) + m0 * K;
     ac.dx = static_cast<T*>(a.dx) + m0 * K;
     ac.mean = a.mean + m0; ac.rstd = a.rstd + m0;
-    int r = transition_bwd_fused(ac, g, dh, dyln, st);
+    int r = transition_bwd_fused(ac, g, dh, part + (size_t)part_rows * 2 * K, st);
     if (r) return r;
+    part_rows += transition_bwd_fused_blocks(rows);
     GemmTcArgs g2{ac.dy, g, a.dw2, K, I, rows, a.dtype, 1, 1, 2};
     g2.accumulate = c > 0;
     r = gemm_tc(g2, st);
     if (r) return r;
-    part_rows += launch_ln_bwd_rows<T>(dyln, static_cast<const T*>(ac.x), static_cast<const T*>(a.ln_w), static_cast<const T*>(a.ln_b),
-                                       ac.mean, ac.rstd, static_cast<T*>(ac.dx), DxAdd<T>{}, xln, part + (size_t)part_rows * 2 * K, rows, K, st);
     // dw1 (chunk-ordered columns) += LN(x)^T dh
-    GemmTcArgs g1{xln, dh, dw1p, K, 2 * I, rows, a.dtype, 1, 1, 2};
+    GemmTcArgs g1{ac.x, dh, dw1p, K, 2 * I, rows, a.dtype, 1, 1, 2, 0, ac.mean, ac.rstd, a.ln_w, a.ln_b};
     g1.accumulate = c > 0;
     r = gemm_tc(g1, st);
     if (r) return r;
