@@ -97,6 +97,87 @@ __device__ __forceinline__ void ln_bwd_row(const uint32_t (&dy)[CW], const uint4
   emit(o);
 }
 
+// The same for a thread that has all 128 columns of its row in registers.  at(c): where the raw columns 8 c .. 8 c + 7 of the
+// row lie in shared memory; dx replaces them.  sums: the gain and shift sums of the warp's rows so far, [2][128].
+template <typename T, typename At>
+__device__ __forceinline__ void ln_bwd_whole_row(uint32_t (&dy)[128], float mu, float rs, const float* gam, float* sums, int lane, At at) {
+  const float2 mm = make_float2(mu, mu), rr = make_float2(rs, rs);
+  auto xhat = [&](uint32_t u) { return mul2(sub2(Pack2<T>::unpack(u), mm), rr); };
+  auto grad_of = [&](int k) { return make_float2(__uint_as_float(dy[k]), __uint_as_float(dy[k + 1])); };
+  // sums of four neighbouring columns, of groups i, i + 16 and i + 8, i + 24, then a tree over i: the butterfly's order
+  float a1[8], a2[8];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {              // groups 2 j and 2 j + 1 of each quarter
+    float q1[4][2], q2[4][2];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 raw = *at(q * 4 + j);
+      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = q * 32 + j * 8 + h * 4;
+        const float4 g = *reinterpret_cast<const float4*>(gam + k);
+        const float2 w0 = mul2(grad_of(k), make_float2(g.x, g.y)), w1 = mul2(grad_of(k + 2), make_float2(g.z, g.w)), h0 = xhat(u[2 * h]), h1 = xhat(u[2 * h + 1]);
+        q1[q][h] = __fmaf_rn(h1.y, w1.y, __fmaf_rn(h1.x, w1.x, __fmaf_rn(h0.y, w0.y, __fmul_rn(h0.x, w0.x))));
+        q2[q][h] = __fadd_rn(__fadd_rn(__fadd_rn(w0.x, w0.y), w1.x), w1.y);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      a1[2 * j + h] = __fadd_rn(__fadd_rn(q1[0][h], q1[2][h]), __fadd_rn(q1[1][h], q1[3][h]));
+      a2[2 * j + h] = __fadd_rn(__fadd_rn(q2[0][h], q2[2][h]), __fadd_rn(q2[1][h], q2[3][h]));
+    }
+  }
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int i = 0; i < h; ++i) { a1[i] = __fadd_rn(a1[i], a1[i + h]); a2[i] = __fadd_rn(a2[i], a2[i + h]); }
+  constexpr float inv_k = 1.f / 128;
+  const float c1 = __fmul_rn(a1[0], inv_k), c2 = __fmul_rn(a2[0], inv_k);
+  // 32 columns at a time: dx, and the first step of both column sums (columns k and k + 16 of the block) while they are at hand
+  auto fold = [&](float a, float b, int s) {
+    const bool up = lane & s;
+    return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, s);
+  };
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float vg[16], vs[16];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float p[2][8];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint4* slot = at(q * 4 + half * 2 + j);
+        const uint4 raw = *slot;
+        const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int k = q * 32 + half * 16 + j * 8 + e * 2;
+          const float2 g = *reinterpret_cast<const float2*>(gam + k), h = xhat(u[e]), d = grad_of(k);
+          const float2 t = make_float2(__fadd_rn(__fmul_rn(c1, h.x), c2), __fadd_rn(__fmul_rn(c1, h.y), c2));      // (packed, the two would be fused)
+          const float2 z = mul2(fma2(d, g, make_float2(-t.x, -t.y)), rr);
+          o[e] = Pack2<T>::pack(z.x, z.y);
+          const float2 dh = mul2(d, h);
+          p[half][e * 2] = dh.x; p[half][e * 2 + 1] = dh.y;
+        }
+        *slot = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        vg[j * 8 + e] = fold(p[0][e], p[1][e], 16);
+        vs[j * 8 + e] = fold(__uint_as_float(dy[q * 32 + j * 8 + e]), __uint_as_float(dy[q * 32 + 16 + j * 8 + e]), 16);
+      }
+    }
+#pragma unroll
+    for (int s = 8; s > 0; s >>= 1)
+#pragma unroll
+      for (int i = 0; i < s; ++i) { vg[i] = fold(vg[i], vg[i + s], s); vs[i] = fold(vs[i], vs[i + s], s); }
+    sums[q * 32 + lane] += vg[0];
+    sums[128 + q * 32 + lane] += vs[0];
+  }
+}
+
 // TMA stores of staged tiles and their bulk groups
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* src, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"

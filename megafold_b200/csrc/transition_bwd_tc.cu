@@ -16,9 +16,10 @@
 //   warps 0-15   workers, two teams that take alternate chunks, thread (row, half): 16 value, 16 gate, 16 dg columns from
 //                TMEM; g, dh in registers with one MUFU op per element; dh packed to TMEM (A operand of the dyln product,
 //                column order inside a chunk: [value 0-15 | gate 0-15 | value 16-31 | gate 16-31]), dh and g to shared-memory
-//                tiles that are TMA-stored.  One chunk into the next tile all sixteen write out dx of this one: the
-//                LayerNorm backward from TMEM (ln_bwd_rows.cuh).
-//   warps 16-19  LayerNorm of the X tile (thread per row, saved statistics) to TMEM, dY beside it.
+//                tiles that are TMA-stored.
+//   warps 16-19  rows: LayerNorm of the next X tile (thread per row, saved statistics) to TMEM, dY beside it; then this
+//                tile's dyln row into registers, which frees the accumulator at once, and the LayerNorm backward of it while
+//                the workers are in the next tile.  dx replaces the raw row of x in shared memory and is TMA-stored.
 //   warp 20      MMAs of H(c) = A W1blocks (8 x N=64, the two blocks as the two swizzle atoms of one MN-major B operand)
 //                and DG(c) = dY W2block (8 x N=32) into one of two TMEM buffers.
 //   warp 21      TMA loads: X and dY tiles, per chunk the W1 value / gate blocks and the W2 block ([128 rows][32 columns],
@@ -26,9 +27,11 @@
 //   warp 22      MMAs of dyln += dh(c) [W1 value block; W1 gate block]^T (4 x N=128; the same shared-memory blocks read
 //                K-major) once the workers have written dh(c).
 //   warp 23      TMA stores of the dh and g tiles of every chunk.
+// (The workers doing the LayerNorm backward between two tiles, four threads a row, held up the dyln products, and with them
+// the weight stages, for 14000 cycles a tile: 341 us.)
 // dh is stored chunk by chunk in that column order ([M][inner/32][64]); dW1 computed from it has its columns in the same
 // order and is put back by a small kernel.
-// [262144, 128], inner 512: XX us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
+// [262144, 128], inner 512: 331 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
 // Every wait is bounded; on expiry the CTA raises a flag, drains and reports through mf_async_status().
 #include "ln_bwd_rows.cuh"
 
@@ -41,18 +44,16 @@ constexpr int K = 128;               // dim
 constexpr int kHC = 32;              // hidden (value) columns per chunk
 constexpr int kWorkWarps = 16;       // two teams of eight
 constexpr int kThreads = (kWorkWarps + 8) * 32;
-// registers per thread: at launch / workers / normalising warps / issuers after setmaxnreg (the raises draw on the drop)
-constexpr int kLaunchRegs = 80, kWorkRegs = 80, kNormRegs = 128, kIssueRegs = 32;
-static_assert(kWorkWarps * 32 * kWorkRegs + 128 * kNormRegs + 128 * kIssueRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
+// registers per thread: at launch / workers / row warps / issuers after setmaxnreg (the raises draw on the drop)
+constexpr int kLaunchRegs = 80, kWorkRegs = 72, kRowRegs = 160, kIssueRegs = 32;
+static_assert(kWorkWarps * 32 * kWorkRegs + 128 * kRowRegs + 128 * kIssueRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 constexpr int A_BYTES = kRows * K * 2;          // 32 KB: X or dY tile, two 64-column atoms
 constexpr int WB = K * 64;                       // 8 KB: one [128 rows][32 columns] weight block
 constexpr int W_BYTES = 3 * WB;                  // W1 value | W1 gate | W2
 constexpr int DH_BYTES = kRows * 128;            // [128 rows][64 columns] 16 bit
 constexpr int G_BYTES = kRows * 64;              // [128 rows][32 columns] 16 bit
-constexpr int RED_BYTES = 4 * 4 * 128 * 16;      // partial sums of the row pass, then the slabs of dx on their way out
 constexpr int kWS = 3;                           // weight stages: a stage is released only by the dyln GEMM of its chunk,
                                                  // one chunk after its H / DG GEMMs, so two stages would stall the TMA refill
-constexpr int kBarrier = 1;                      // named barrier of the workers
 
 struct TbP {
   int64_t M; int inner, n_mt, n_ch;
@@ -66,7 +67,7 @@ struct TbP {
 struct Bars {
   uint64_t x_full, x_empty, dy_full, dy_empty, a_full, a_empty;
   uint64_t w_full[kWS], w_empty[kWS];
-  uint64_t hd_full[2], hd_empty[2], dh_full[2], dh_empty[2], st_done[2], acc_full, acc_empty;
+  uint64_t xr_full[4], hd_full[2], hd_empty[2], dh_full[2], dh_empty[2], st_done[2], acc_full, acc_empty;
 };
 
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mdy,
                          const __grid_constant__ CUtensorMap mw1, const __grid_constant__ CUtensorMap mw2,
                          const __grid_constant__ CUtensorMap mdh, const __grid_constant__ CUtensorMap mg,
-                         const __grid_constant__ CUtensorMap mdx, const TbP p) {
+                         const __grid_constant__ CUtensorMap mxr, const __grid_constant__ CUtensorMap mdx, const TbP p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sX = smem;                          // raw rows of X
@@ -88,10 +89,11 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
   uint8_t* sW = sDY + A_BYTES;                 // [kWS] weight stages
   uint8_t* sDH = sW + kWS * W_BYTES;           // [2] dh tiles
   uint8_t* sG = sDH + 2 * DH_BYTES;            // [2] g tiles
-  uint8_t* sRed = sG + 2 * G_BYTES;
+  uint8_t* sXR = sG + 2 * G_BYTES;             // rows of X once more, then rows of dx
 
   __shared__ Bars bar;
   __shared__ __align__(16) float gam_s[K], bet_s[K];
+  __shared__ float sum_s[4][2 * K];            // gain and shift sums over the rows of each row warp
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -104,14 +106,16 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       mbar_init(&bar.dh_full[i], 8); mbar_init(&bar.dh_empty[i], 1); mbar_init(&bar.st_done[i], 1);
     }
     for (int i = 0; i < kWS; ++i) { mbar_init(&bar.w_full[i], 1); mbar_init(&bar.w_empty[i], 1); }
-    mbar_init(&bar.acc_full, 1); mbar_init(&bar.acc_empty, kWorkWarps);
+    mbar_init(&bar.acc_full, 1); mbar_init(&bar.acc_empty, 4);
+    for (int i = 0; i < 4; ++i) mbar_init(&bar.xr_full[i], 1);
     mbar_fence_init();
-    prefetch_tmap(&mx); prefetch_tmap(&mdy); prefetch_tmap(&mw1); prefetch_tmap(&mw2); prefetch_tmap(&mdh); prefetch_tmap(&mg); prefetch_tmap(&mdx);
+    prefetch_tmap(&mx); prefetch_tmap(&mdy); prefetch_tmap(&mw1); prefetch_tmap(&mw2); prefetch_tmap(&mdh); prefetch_tmap(&mg); prefetch_tmap(&mxr); prefetch_tmap(&mdx);
   }
   for (int k = tid; k < K; k += kThreads) {
     gam_s[k] = to_f(static_cast<const T*>(p.gamma)[k]);
     bet_s[k] = p.beta ? to_f(static_cast<const T*>(p.beta)[k]) : 0.f;
   }
+  for (int k = tid; k < 4 * 2 * K; k += kThreads) (&sum_s[0][0])[k] = 0.f;
   if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
@@ -127,134 +131,77 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
 
   if (warp < kWorkWarps) {
     // ---------------------------------------------------------------------------------- workers
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kWorkRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kWorkRegs));
     const int team = warp >> 3, half = (warp >> 2) & 1;
-    const int quarter = warp & 3, part = warp >> 2;       // rows and columns of mine in the write-out of dx
-    constexpr int CW = K / 4;
-    float4 (*red)[CW / 8][128] = reinterpret_cast<float4 (*)[CW / 8][128]>(sRed);
-    uint8_t* slab = sRed + warp * (32 * CW * 2);          // [32 rows][32 columns] of dx, once the sums have been read
     const uint32_t tMine = tHD + team * 96 + half * 16 + lane_addr, tOut = tDH + team * 32 + half * 16 + lane_addr;
     uint8_t* dh = sDH + team * DH_BYTES;
     uint8_t* g = sG + team * G_BYTES;
-    float gain = 0.f, shift = 0.f;                        // sums over my rows of column part * 32 + lane
-
-    // dx of tile t, one chunk into the next tile; false once anybody has given up.  All sixteen warps come here for every
-    // tile in order, whatever happened: its barriers are not bounded.
-    auto write_out = [&](int t) -> bool {
-      const int row0 = (int)(((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows);
-      const int64_t row = (int64_t)row0 + row_l;
-      const bool ok = row < p.M;
-      uint4 raw[CW / 8];
-      const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + row * K + part * CW);
-#pragma unroll
-      for (int c = 0; c < CW / 8; ++c) raw[c] = ok ? __ldg(xr + c) : make_uint4(0u, 0u, 0u, 0u);
-      const float mu = ok ? p.mean[row] : 0.f, rs = ok ? p.rstd[row] : 0.f;
-      wait_or_flag(&bar.acc_full, t & 1, abort_flag);
+    int t = 0, c = team;                                  // my next chunk: c of tile t, once c is brought below nch
+    for (uint32_t n = 0;; ++n, c += 2) {                  // n: my chunks so far
+      while (t < my_tiles && c >= nch) { c -= nch; ++t; }
+      if (t >= my_tiles || __any_sync(0xffffffffu, *abort_flag)) break;
+      wait_or_flag(&bar.hd_full[team], n & 1, abort_flag);
       tc_fence_after();
-      uint32_t dy[CW];
-      tmem_ld32(tACC + part * CW + lane_addr, dy);
-      tmem_ld_wait();
+      uint32_t gp[8], dv[8], db[8];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {                     // 8 columns at a time: registers
+        uint32_t hv[8], hg[8], dg[8];
+        tmem_ld8(tMine + s * 8, hv);
+        tmem_ld8(tMine + 32 + s * 8, hg);
+        tmem_ld8(tMine + 64 + s * 8, dg);
+        tmem_ld_wait();
+        if (s == 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar.hd_empty[team]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = make_float2(__uint_as_float(hv[2 * e]), __uint_as_float(hv[2 * e + 1]));
+          const float2 b = make_float2(__uint_as_float(hg[2 * e]), __uint_as_float(hg[2 * e + 1]));
+          const float2 d = make_float2(__uint_as_float(dg[2 * e]), __uint_as_float(dg[2 * e + 1]));
+          const float2 h = make_float2(0.5f, 0.5f), b2 = mul2(b, h);
+          const float2 sg = fma2(h, make_float2(tanh_approx(b2.x), tanh_approx(b2.y)), h);      // sigmoid(b)
+          const float2 sl = mul2(b, sg);                                                         // silu(b)
+          const float2 ds = fma2(sl, sub2(make_float2(1.f, 1.f), sg), sg);                       // d/db silu(b) = sg + sl * (1 - sg)
+          const float2 go = mul2(sl, v), dvo = mul2(d, sl), dbo = mul2(mul2(d, v), ds);
+          gp[s * 4 + e] = Pack2<T>::pack(go.x, go.y); dv[s * 4 + e] = Pack2<T>::pack(dvo.x, dvo.y); db[s * 4 + e] = Pack2<T>::pack(dbo.x, dbo.y);
+        }
+      }
+      // dh to TMEM, once the dyln product of two chunks ago has read it; dh and g to the tiles, once the TMA stores have
+      if (n > 0) wait_or_flag(&bar.dh_empty[team], (n - 1) & 1, abort_flag);
+      tc_fence_after();
+      tmem_st8(tOut, dv);
+      tmem_st8(tOut + 8, db);
+      if (n > 0) wait_or_flag(&bar.st_done[team], (n - 1) & 1, abort_flag);
+      // dh row (128 B): [value 0-15 | gate 0-15 | value 16-31 | gate 16-31]; my 16 + 16 columns are chunks half*4 .. +3
+      *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 0, 128)) = make_uint4(dv[0], dv[1], dv[2], dv[3]);
+      *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 1, 128)) = make_uint4(dv[4], dv[5], dv[6], dv[7]);
+      *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 2, 128)) = make_uint4(db[0], db[1], db[2], db[3]);
+      *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 3, 128)) = make_uint4(db[4], db[5], db[6], db[7]);
+      // g row (64 B): columns in natural order, mine are chunks half*2, half*2 + 1
+      *reinterpret_cast<uint4*>(g + swz_offset(row_l, half * 2 + 0, 64)) = make_uint4(gp[0], gp[1], gp[2], gp[3]);
+      *reinterpret_cast<uint4*>(g + swz_offset(row_l, half * 2 + 1, 64)) = make_uint4(gp[4], gp[5], gp[6], gp[7]);
+      fence_async_smem();
+      tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&bar.acc_empty); bulk_wait_group_read<0>(); }      // my store of the previous tile has read its slab
-      __syncwarp();
-      if (named_sync_or(kBarrier, kWorkWarps * 32, *abort_flag)) return false;            // ... and so have everybody's
-      float v[CW];
-      ln_bwd_row<T, CW, 4>(dy, raw, mu, rs, gam_s + part * CW, red, part, row_l, kBarrier,
-                           [&](uint32_t (&out)[CW / 2]) {
-#pragma unroll
-                             for (int c = 0; c < CW / 8; ++c)
-                               *reinterpret_cast<uint4*>(slab + swz_offset(lane, c, CW * 2)) = make_uint4(out[c * 4], out[c * 4 + 1], out[c * 4 + 2], out[c * 4 + 3]);
-                             fence_async_smem();
-                             __syncwarp();
-                             if (lane == 0) {
-                               if (row0 + quarter * 32 < p.M) tma_store_2d(&mdx, slab, part * CW, row0 + quarter * 32);      // never past the last row
-                               bulk_commit_group();
-                             }
-                           },
-                           [&](int k, float2 d, float2 h) { v[k] = d.x * h.x; v[k + 1] = d.y * h.y; });
-      gain += column_sum(v, lane);
-#pragma unroll
-      for (int k = 0; k < CW; ++k) v[k] = __uint_as_float(dy[k]);
-      shift += column_sum(v, lane);
-      return true;
-    };
-
-    uint32_t ch_cnt = 0;                                  // chunks seen (buffer = team = ch_cnt & 1)
-    int pending = -1;                                     // tile whose dx has not been written out
-    bool alive = true;
-    for (int t = 0; t < my_tiles && alive; ++t) {
-      for (int c = 0; c < nch && alive; ++c, ++ch_cnt) {
-        if ((int)(ch_cnt & 1) != team) continue;
-        wait_or_flag(&bar.hd_full[team], (ch_cnt >> 1) & 1, abort_flag);
-        tc_fence_after();
-        uint32_t gp[8], dv[8], db[8];
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {                     // 8 columns at a time keeps the live registers down
-          uint32_t hv[8], hg[8], dg[8];
-          tmem_ld8(tMine + s * 8, hv);
-          tmem_ld8(tMine + 32 + s * 8, hg);
-          tmem_ld8(tMine + 64 + s * 8, dg);
-          tmem_ld_wait();
-          if (s == 1) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bar.hd_empty[team]);
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float go[2], dvo[2], dbo[2];
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const float v = __uint_as_float(hv[2 * e + q]), b = __uint_as_float(hg[2 * e + q]), d = __uint_as_float(dg[2 * e + q]);
-              const float sg = fmaf(0.5f, tanh_approx(0.5f * b), 0.5f);      // sigmoid(b)
-              const float sl = b * sg;                                        // silu(b)
-              go[q] = sl * v;
-              dvo[q] = d * sl;
-              dbo[q] = d * v * fmaf(sl, 1.f - sg, sg);                        // d/db silu(b) = sg + sl * (1 - sg)
-            }
-            gp[s * 4 + e] = Pack2<T>::pack(go[0], go[1]); dv[s * 4 + e] = Pack2<T>::pack(dvo[0], dvo[1]); db[s * 4 + e] = Pack2<T>::pack(dbo[0], dbo[1]);
-          }
-        }
-        // dh to TMEM, once the dyln product of two chunks ago has read it; dh and g to the tiles, once the TMA stores have
-        if (ch_cnt >= 2) wait_or_flag(&bar.dh_empty[team], ((ch_cnt >> 1) - 1) & 1, abort_flag);
-        tc_fence_after();
-        tmem_st8(tOut, dv);
-        tmem_st8(tOut + 8, db);
-        if (ch_cnt >= 2) wait_or_flag(&bar.st_done[team], ((ch_cnt >> 1) - 1) & 1, abort_flag);
-        // dh row (128 B): [value 0-15 | gate 0-15 | value 16-31 | gate 16-31]; my 16 + 16 columns are chunks half*4 .. +3
-        *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 0, 128)) = make_uint4(dv[0], dv[1], dv[2], dv[3]);
-        *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 1, 128)) = make_uint4(dv[4], dv[5], dv[6], dv[7]);
-        *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 2, 128)) = make_uint4(db[0], db[1], db[2], db[3]);
-        *reinterpret_cast<uint4*>(dh + swz_offset(row_l, half * 4 + 3, 128)) = make_uint4(db[4], db[5], db[6], db[7]);
-        // g row (64 B): columns in natural order, mine are chunks half*2, half*2 + 1
-        *reinterpret_cast<uint4*>(g + swz_offset(row_l, half * 2 + 0, 64)) = make_uint4(gp[0], gp[1], gp[2], gp[3]);
-        *reinterpret_cast<uint4*>(g + swz_offset(row_l, half * 2 + 1, 64)) = make_uint4(gp[4], gp[5], gp[6], gp[7]);
-        fence_async_smem();
-        tmem_st_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.dh_full[team]);
-        if (pending >= 0) { alive = write_out(pending); pending = -1; }
-      }
-      if (alive && pending >= 0) alive = write_out(pending);     // a tile without a chunk of mine
-      pending = t;
+      if (lane == 0) mbar_arrive(&bar.dh_full[team]);
     }
-    if (alive && pending >= 0) write_out(pending);
-    // the CTA's sums over its rows: the four row quarters of each column through shared memory
-    if (lane == 0) bulk_wait_group<0>();
-    __syncwarp();
-    float* scratch = reinterpret_cast<float*>(sRed);      // [4][2 K]
-    named_sync(kBarrier, kWorkWarps * 32);
-    scratch[quarter * 2 * K + part * CW + lane] = gain;
-    scratch[quarter * 2 * K + K + part * CW + lane] = shift;
-    named_sync(kBarrier, kWorkWarps * 32);
-    if (tid < 2 * K) p.part[(int64_t)blockIdx.x * 2 * K + tid] = (scratch[tid] + scratch[2 * K + tid]) + (scratch[4 * K + tid] + scratch[6 * K + tid]);
   } else if (warp < kWorkWarps + 4) {
-    // ---------------------------------------------------------------------------------- normalising warps
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kNormRegs));
-    for (int t = 0; t < my_tiles && !*abort_flag; ++t) {
-      const int64_t row = ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows + row_l;
+    // ---------------------------------------------------------------------------------- row warps
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
+    const int quarter = warp & 3;
+    uint64_t* xr_full = &bar.xr_full[quarter];
+    uint8_t* xr = sXR + quarter * 32 * 128;                // my 32 rows of the first 64 columns; the others are kRows * 128 further
+    auto row_of = [&](int t) { return ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows; };
+    auto load_raw = [&](int t) {                           // (lane 0) my rows of tile t for the write-out
+      mbar_expect_tx(xr_full, 2 * 32 * 128);
+      for (int q = 0; q < K / 64; ++q) tma_load_2d(xr + q * (kRows * 128), &mxr, xr_full, q * 64, (int)row_of(t) + quarter * 32);
+    };
+    // LN(X) and dY of tile t to TMEM
+    auto normalise = [&](int t) {
+      const int64_t row = row_of(t) + row_l;
       const bool ok = row < p.M;
       const float mu = ok ? p.mean[row] : 0.f, rs = ok ? p.rstd[row] : 0.f;     // saved by the forward pass
       const float2 mm = make_float2(mu, mu), rr = make_float2(rs, rs);
@@ -272,7 +219,6 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           const float2 y1 = fma2(mul2(sub2(Pack2<T>::unpack(u[e + 1]), mm), rr), make_float2(ga.z, ga.w), make_float2(be.z, be.w));
           o[c * 4 + e] = ok ? Pack2<T>::pack(y0.x, y0.y) : 0u; o[c * 4 + e + 1] = ok ? Pack2<T>::pack(y1.x, y1.y) : 0u;
         }
-        if (c % 4 == 3) asm volatile("" ::: "memory");     // loads no further ahead than this: registers
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.x_empty);
@@ -294,7 +240,41 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.a_full);
+    };
+    if (my_tiles > 0) {
+      if (lane == 0) load_raw(0);
+      normalise(0);
     }
+    for (int t = 0; t < my_tiles; ++t) {
+      if (t + 1 < my_tiles) normalise(t + 1);
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      const int64_t row = row_of(t) + row_l;
+      const bool ok = row < p.M;
+      const float mu = ok ? p.mean[row] : 0.f, rs = ok ? p.rstd[row] : 0.f;
+      wait_or_flag(xr_full, t & 1, abort_flag);
+      wait_or_flag(&bar.acc_full, t & 1, abort_flag);
+      tc_fence_after();
+      uint32_t dy[K];
+#pragma unroll
+      for (int q = 0; q < K / 32; ++q) tmem_ld32(tACC + q * 32 + lane_addr, *reinterpret_cast<uint32_t (*)[32]>(dy + q * 32));
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.acc_empty);
+      ln_bwd_whole_row<T>(dy, mu, rs, gam_s, sum_s[quarter], lane,
+                          [&](int c) { return reinterpret_cast<uint4*>(xr + (c >> 3) * (kRows * 128) + swz_offset(lane, c & 7, 128)); });
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (row_of(t) + quarter * 32 < p.M)                 // never past the last row
+          for (int q = 0; q < K / 64; ++q) tma_store_2d(&mdx, xr + q * (kRows * 128), q * 64, (int)row_of(t) + quarter * 32);
+        bulk_commit_group();
+        bulk_wait_group_read<0>();
+        if (t + 1 < my_tiles) load_raw(t + 1);
+      }
+      __syncwarp();
+    }
+    if (lane == 0) bulk_wait_group<0>();
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     auto dead = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };      // the MMA roles are run by whole warps
@@ -303,9 +283,9 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       const uint32_t id_h = idesc_f16(128, 64, p.ab_fmt, 0, 1);     // B = W1 value|gate blocks MN-major, N = 64
       const uint32_t id_g = idesc_f16(128, 32, p.ab_fmt, 0, 1);     // A = dY, B = W2 block MN-major, N = 32
       uint32_t ch_cnt = 0;
-      for (int t = 0; t < my_tiles && !dead(); ++t) {
+      for (int t = 0; t < my_tiles; ++t) {
         wait_or_flag(&bar.a_full, t & 1, abort_flag);
-        for (int c = 0; c < nch && !dead(); ++c, ++ch_cnt) {
+        for (int c = 0; c < nch; ++c, ++ch_cnt) {
           const int hb = ch_cnt & 1, ws = ch_cnt % kWS;
           wait_or_flag(&bar.w_full[ws], (ch_cnt / kWS) & 1, abort_flag);
           if (ch_cnt >= 2) wait_or_flag(&bar.hd_empty[hb], ((ch_cnt >> 1) - 1) & 1, abort_flag);
@@ -329,8 +309,8 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       // (one warp issuing both would wait for the workers' dh of one chunk before it could start the next chunk's H)
       const uint32_t id_a = idesc_f16(128, 128, p.ab_fmt, 0, 0);    // B = W1 blocks K-major, N = dim
       uint32_t ch_cnt = 0;
-      for (int t = 0; t < my_tiles && !dead(); ++t) {
-        for (int c = 0; c < nch && !dead(); ++c, ++ch_cnt) {        // dyln (+)= dh(c) [W1v; W1g](c)^T
+      for (int t = 0; t < my_tiles; ++t) {
+        for (int c = 0; c < nch; ++c, ++ch_cnt) {                   // dyln (+)= dh(c) [W1v; W1g](c)^T
           const int hb = ch_cnt & 1;
           wait_or_flag(&bar.dh_full[hb], (ch_cnt >> 1) & 1, abort_flag);
           if (c == 0 && t > 0) wait_or_flag(&bar.acc_empty, (t - 1) & 1, abort_flag);
@@ -359,8 +339,8 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           tma_store_2d(&mdh, sDH + hb * DH_BYTES, c * 64, row0);               // rows >= M are clipped
           tma_store_2d(&mg, sG + hb * G_BYTES, c * kHC, row0);
           bulk_commit_group();
-          bulk_wait_group_read<0>();
-          mbar_arrive(&bar.st_done[hb]);
+          bulk_wait_group_read<1>();
+          if (ch_cnt > 0) mbar_arrive(&bar.st_done[hb ^ 1]);                   // the chunk before this one has been read
         }
       }
       bulk_wait_group<0>();
@@ -399,6 +379,7 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
 
   tc_fence_before();
   __syncthreads();
+  if (tid < 2 * K) p.part[(int64_t)blockIdx.x * 2 * K + tid] = (sum_s[0][tid] + sum_s[1][tid]) + (sum_s[2][tid] + sum_s[3][tid]);
   if (tid == 0 && abort_s) *reinterpret_cast<volatile int*>(p.status) = 1;
   if (warp == 0) tmem_dealloc(tmem_base_s, 512);
 }
@@ -432,15 +413,16 @@ int transition_bwd_fused_blocks(int64_t M) {
 
 // g [M, inner], dh [M, inner/32, 64] (chunk-ordered columns), dx, and per block the column sums part [blocks][2 * 128]
 int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, float* part, cudaStream_t st) {
-  CUtensorMap mx, mdy, mw1, mw2, mdh, mg, mdx;
+  CUtensorMap mx, mdy, mw1, mw2, mdh, mg, mxr, mdx;
   int r;
   {
     const int64_t dims[2] = {K, a.M}, str[2] = {1, K};
     const int box[2] = {64, kRows};
     if ((r = make_tiled_map(&mx, a.x, a.dtype, 2, dims, str, box, 128))) return r;
     if ((r = make_tiled_map(&mdy, a.dy, a.dtype, 2, dims, str, box, 128))) return r;
-    const int slab[2] = {K / 4, 32};             // one worker warp's part of dx
-    if ((r = make_tiled_map(&mdx, a.dx, a.dtype, 2, dims, str, slab, K / 2))) return r;
+    const int slab[2] = {64, 32};                // half of a row warp's rows
+    if ((r = make_tiled_map(&mxr, a.x, a.dtype, 2, dims, str, slab, 128))) return r;
+    if ((r = make_tiled_map(&mdx, a.dx, a.dtype, 2, dims, str, slab, 128))) return r;
   }
   {
     const int64_t dims[2] = {2 * (int64_t)a.inner, K}, str[2] = {1, 2 * (int64_t)a.inner};
@@ -472,16 +454,16 @@ int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, flo
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
-  constexpr size_t smem = 1024 + 2 * (size_t)A_BYTES + kWS * (size_t)W_BYTES + 2 * (size_t)DH_BYTES + 2 * (size_t)G_BYTES + RED_BYTES;
+  constexpr size_t smem = 1024 + 3 * (size_t)A_BYTES + kWS * (size_t)W_BYTES + 2 * (size_t)DH_BYTES + 2 * (size_t)G_BYTES;
   const int grid = transition_bwd_fused_blocks(a.M);
   if (a.dtype == MF_BF16) {
     constexpr auto kern = transition_bwd_tc_kernel<__nv_bfloat16>;
     if (int e = opt_in_smem<kern>(smem)) return e;
-    kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, mdx, p);
+    kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, mxr, mdx, p);
   } else {
     constexpr auto kern = transition_bwd_tc_kernel<__half>;
     if (int e = opt_in_smem<kern>(smem)) return e;
-    kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, mdx, p);
+    kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, mxr, mdx, p);
   }
   MF_LAUNCHED("transition_bwd_tc_kernel");
   return MF_OK;
