@@ -37,7 +37,7 @@ template <int BN> struct Geo {
 struct GemmP {
   int m_tiles, n_tiles, k_splits, slabs_total, slabs_per_split;
   int n_cols; int64_t n_rows;
-  int a_mn, b_mn, out_kind;     // out_kind: 0 = 16-bit store, 1 = fp32 store, 2 = fp32 add-reduction
+  int a_mn, b_mn, b_panels, out_kind;     // out_kind: 0 = 16-bit store, 1 = fp32 store, 2 = fp32 add-reduction
   uint32_t ab_fmt;
   const float *mean, *rstd; const void *gain, *shift; int m_total; int64_t r_total;      // LN only
   int* status;
@@ -113,7 +113,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
         } else {        // stored [M, R]: one [128 m][64 r] box
           tma_load_2d(a, &ma, &bar.full[st], s * kBK, mt * kBM);
         }
-        if (p.b_mn) {
+        if (p.b_panels) {
+#pragma unroll
+          for (int at = 0; at < kBN / 64; ++at) tma_load_3d(b + at * 8192, &mb, &bar.full[st], 0, s * kBK, nt * (kBN / 64) + at);
+        } else if (p.b_mn) {
 #pragma unroll
           for (int at = 0; at < kBN / 64; ++at) tma_load_2d(b + at * 8192, &mb, &bar.full[st], nt * kBN + at * 64, s * kBK);
         } else {
@@ -309,7 +312,11 @@ int gemm_tc(const GemmTcArgs& g, cudaStream_t st) {
   if (g.out_kind == 2 && g.N > 128 && (int64_t)p.m_tiles * ((g.N + 255) / 256) * (p.slabs_total / 16) >= sms) bn = 256;
   else if ((int64_t)p.m_tiles * ((g.N + 127) / 128) * (g.out_kind == 2 ? (p.slabs_total + 3) / 4 : 1) <= sms / 2) bn = 64;
   p.n_tiles = (int)((g.N + bn - 1) / bn);
-  {
+  if (g.b_panels) {
+    const int64_t dims[3] = {64, g.R, (g.N + 63) / 64}, str[3] = {1, 64, 64 * g.R};
+    const int box[3] = {64, 64, 1};
+    if ((r = make_tiled_map(&mb, g.b, g.dtype, 3, dims, str, box, 128))) return r;
+  } else {
     const int64_t dims[2] = {g.b_mn ? g.N : g.R, g.b_mn ? g.R : g.N}, str[2] = {1, dims[0]};
     const int box[2] = {64, g.b_mn ? 64 : bn};
     if ((r = make_tiled_map(&mb, g.b, g.dtype, 2, dims, str, box, 128))) return r;
@@ -326,7 +333,7 @@ int gemm_tc(const GemmTcArgs& g, cudaStream_t st) {
   p.slabs_per_split = (p.slabs_total + splits - 1) / splits;
   p.k_splits = (p.slabs_total + p.slabs_per_split - 1) / p.slabs_per_split;
   p.n_cols = (int)g.N; p.n_rows = g.M;
-  p.a_mn = g.a_mn; p.b_mn = g.b_mn; p.out_kind = g.out_kind;
+  p.a_mn = g.a_mn; p.b_mn = g.b_mn; p.b_panels = g.b_panels; p.out_kind = g.out_kind;
   p.ab_fmt = g.dtype == MF_BF16 ? 1u : 0u;
   p.mean = g.ln_mean; p.rstd = g.ln_rstd; p.gain = g.ln_gain; p.shift = g.ln_shift; p.m_total = (int)g.M; p.r_total = g.R;
   MF_REQUIRE(!g.ln_gain || g.a_mn, MF_ERR_UNSUPPORTED, "gemm_tc: LayerNorm is applied along the rows of an MN-major A");

@@ -19,6 +19,8 @@ struct GemmTcArgs {
   // matrix is formed in shared memory, rounded to the operand dtype, and never stored.
   const float *ln_mean = nullptr, *ln_rstd = nullptr;
   const void *ln_gain = nullptr, *ln_shift = nullptr;
+  // b_mn = 1: B is stored in panels of 64 columns, [panel][R][64], so that every box of 64 rows is one run of 8 KB
+  int b_panels = 0;
 };
 bool gemm_tc_ok(const GemmTcArgs& g);
 int gemm_tc(const GemmTcArgs& g, cudaStream_t st);

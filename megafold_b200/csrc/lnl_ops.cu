@@ -783,7 +783,7 @@ size_t transition_bwd_fused_bytes(const mf_transition_bwd_args& a) {
   const size_t es = dtype_size(a.dtype);
   const TransitionChunks ch = transition_chunks(a.M);
   const size_t rows = (size_t)(ch.rows < a.M ? ch.rows : a.M);
-  return align_up(rows * a.inner * es, 256) + align_up(rows * 2 * a.inner * es, 256) + align_up(sizeof(float) * (size_t)a.dim * 2 * a.inner, 256) +
+  return align_up(rows * (size_t)((a.inner + 63) / 64 * 64) * es, 256) + align_up(rows * 2 * a.inner * es, 256) + align_up(sizeof(float) * (size_t)a.dim * 2 * a.inner, 256) +
          align_up(sizeof(float) * (size_t)ch.n * transition_bwd_fused_blocks(rows) * 2 * a.dim, 256);
 }
 
@@ -794,7 +794,7 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
   const int64_t M = a.M;
   const TransitionChunks ch = transition_chunks(M);
   const size_t rows_max = (size_t)(ch.rows < M ? ch.rows : M);
-  T* g = ws.take<T>(rows_max * I);
+  T* g = ws.take<T>(rows_max * ((I + 63) / 64 * 64));      // whole panels
   T* dh = ws.take<T>(rows_max * 2 * I);
   float* dw1p = ws.take<float>((size_t)K * 2 * I);
   float* part = ws.take<float>((size_t)ch.n * transition_bwd_fused_blocks(rows_max) * 2 * K);
@@ -812,12 +812,12 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
     if (r) return r;
     part_rows += transition_bwd_fused_blocks(rows);
     GemmTcArgs g2{ac.dy, g, a.dw2, K, I, rows, a.dtype, 1, 1, 2};
-    g2.accumulate = c > 0;
+    g2.accumulate = c > 0; g2.b_panels = 1;
     r = gemm_tc(g2, st);
     if (r) return r;
     // dw1 (chunk-ordered columns) += LN(x)^T dh
     GemmTcArgs g1{ac.x, dh, dw1p, K, 2 * I, rows, a.dtype, 1, 1, 2, 0, ac.mean, ac.rstd, a.ln_w, a.ln_b};
-    g1.accumulate = c > 0;
+    g1.accumulate = c > 0; g1.b_panels = 1;
     r = gemm_tc(g1, st);
     if (r) return r;
   }

@@ -29,9 +29,10 @@
 //   warp 23      TMA stores of the dh and g tiles of every chunk.
 // (The workers doing the LayerNorm backward between two tiles, four threads a row, held up the dyln products, and with them
 // the weight stages, for 14000 cycles a tile: 341 us.)
-// dh is stored chunk by chunk in that column order ([M][inner/32][64]); dW1 computed from it has its columns in the same
-// order and is put back by a small kernel.
-// [262144, 128], inner 512: 331 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
+// dh is stored in that column order, a panel [M][64] per chunk; dW1 computed from it has its columns in the same order and is
+// put back by a small kernel.  (Panels, of g too: a chunk of a tile is one run of 16 KB.  128-byte pieces at the pitch of a
+// whole row took 25 us more.)
+// [262144, 128], inner 512: 303 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
 // Every wait is bounded; on expiry the CTA raises a flag, drains and reports through mf_async_status().
 #include "ln_bwd_rows.cuh"
 
@@ -336,8 +337,8 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           const int hb = ch_cnt & 1;
           wait_or_flag(&bar.dh_full[hb], (ch_cnt >> 1) & 1, abort_flag);      // written and fenced by the team's eight warps
           if (*abort_flag) break;
-          tma_store_2d(&mdh, sDH + hb * DH_BYTES, c * 64, row0);               // rows >= M are clipped
-          tma_store_2d(&mg, sG + hb * G_BYTES, c * kHC, row0);
+          tma_store_3d(&mdh, sDH + hb * DH_BYTES, 0, row0, c);               // rows >= M are clipped
+          tma_store_3d(&mg, sG + hb * G_BYTES, (c & 1) * kHC, row0, c >> 1);
           bulk_commit_group();
           bulk_wait_group_read<1>();
           if (ch_cnt > 0) mbar_arrive(&bar.st_done[hb ^ 1]);                   // the chunk before this one has been read
@@ -411,7 +412,7 @@ int transition_bwd_fused_blocks(int64_t M) {
   return (int)(tiles < sm_count() ? tiles : sm_count());
 }
 
-// g [M, inner], dh [M, inner/32, 64] (chunk-ordered columns), dx, and per block the column sums part [blocks][2 * 128]
+// g [panels of 64 columns][M][64], dh [inner/32][M][64] (chunk-ordered columns), dx, and per block the column sums part [blocks][2 * 128]
 int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, float* part, cudaStream_t st) {
   CUtensorMap mx, mdy, mw1, mw2, mdh, mg, mxr, mdx;
   int r;
@@ -435,14 +436,14 @@ int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, flo
     if ((r = make_tiled_map(&mw2, a.w2, a.dtype, 2, dims, str, box, 64))) return r;
   }
   {
-    const int64_t dims[2] = {2 * (int64_t)a.inner, a.M}, str[2] = {1, 2 * (int64_t)a.inner};
-    const int box[2] = {64, kRows};
-    if ((r = make_tiled_map(&mdh, dh, a.dtype, 2, dims, str, box, 128))) return r;
+    const int64_t dims[3] = {64, a.M, a.inner / kHC}, str[3] = {1, 64, 64 * a.M};
+    const int box[3] = {64, kRows, 1};
+    if ((r = make_tiled_map(&mdh, dh, a.dtype, 3, dims, str, box, 128))) return r;
   }
   {
-    const int64_t dims[2] = {a.inner, a.M}, str[2] = {1, a.inner};
-    const int box[2] = {kHC, kRows};
-    if ((r = make_tiled_map(&mg, g, a.dtype, 2, dims, str, box, 64))) return r;
+    const int64_t dims[3] = {64, a.M, (a.inner + 63) / 64}, str[3] = {1, 64, 64 * a.M};
+    const int box[3] = {kHC, kRows, 1};
+    if ((r = make_tiled_map(&mg, g, a.dtype, 3, dims, str, box, 64))) return r;
   }
   TbP p{};
   p.M = a.M; p.inner = a.inner;
