@@ -170,6 +170,7 @@ bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a);
 bool transition_bwd_runs_on_tc(const mf_transition_bwd_args& a);
 bool transition_bwd_fused_ok(const mf_transition_bwd_args& a);
 int transition_bwd_fused_blocks(int64_t M);
+namespace tcx { int sm_count(); }
 int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, float* part, cudaStream_t st);
 int unpermute_dw1(const float* src, float* dst, int dim, int inner, cudaStream_t st);
 size_t lnl_bwd_workspace(const mf_lnl_bwd_args& a);

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("M,inner,dtype,shift", [(1, 32, torch.bfloat16, True), (128, 96, torch.float16, False), (33, 64, torch.bfloat16, True),
                                                  (3 * 148 * 128 + 77, 32, torch.bfloat16, True), (2 * 148 * 128 + 1, 160, torch.float16, True),
-                                                 (131072 + 129, 64, torch.bfloat16, True)])
+                                                 (262144 + 129, 64, torch.bfloat16, True)])
 def test_transition_bwd_chunks(M, inner, dtype, shift):
     g = torch.Generator(device="cuda").manual_seed(M + inner)
     r = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
