@@ -3,11 +3,11 @@
 // rows longer than 2048 tokens.
 //
 // A persistent CTA (one per SM, 256 threads) runs TWO independent streams, one per warpgroup.  A stream walks a
-// contiguous range of work items (b, n, h, 128-query tile) and, per item, the key tiles of 128.  Inside a stream every
+// contiguous range of work items (b, n, h, 128-query tile) and, per item, the key tiles (128 keys, 64 for DP = 64).  Inside a stream every
 // thread owns one query row (= one TMEM lane); three "officer" threads of the warpgroup also issue the stream's
 // tcgen05.mma instructions (thread 0), its Q/K/V TMA loads (thread 32) and its bias TMA loads (thread 64):
 //
-//   wait S(t) in TMEM -> tcgen05.ld the whole 128-column row into registers -> group barrier ->
+//   wait S(t) in TMEM -> tcgen05.ld the whole row of the tile into registers -> group barrier ->
 //   S(t+1) = Q K(t+1)^T is issued at once (the S buffer is free again: registers double-buffer it)
 //   -> row thread: logits in base 2 (scale, bias from shared memory, key mask), running max, exp2,
 //   row sum, packed 16-bit P -> fold O_tile(t-1) from TMEM into the register accumulator ->
@@ -17,7 +17,11 @@
 // Operand tiles are [128 rows x DP] (DP = 32: 64-byte rows, 64B swizzle; DP = 64: 128-byte rows) fetched
 // from the strided [B, N, L, H, D] tensors by 5-D tensor maps; smaller head sizes are zero-filled by TMA.
 // A 16-bit pair bias with TMA-addressable rows is staged as [128 rows x 64 columns] chunks (128-byte rows, 128B
-// swizzle, DP = 32 only); otherwise the row thread reads it from global memory.
+// swizzle, DP = 32 only).  Other aligned biases (fp32, or DP = 64 whose operand tiles leave less room) go through a ring per
+// warp of [32 rows x 64 bytes] chunks, filled by cp.async six chunks ahead: the row threads' own loads from global memory,
+// 128 bytes of a row at a time with their latency in the open, made the fp32 bias of [4, 1, 384, 32, 64] cost 72 us where
+// this takes XX.  Unaligned or strided biases, and DP = 64 beyond 2176 keys (the mask rows need the room), are still read
+// by the row thread.
 //
 // Every wait is bounded; on expiry the CTA raises a flag that all threads honour at their next group
 // barrier, TMEM is freed and the host sees mf_async_status() != 0.
@@ -27,21 +31,28 @@ namespace mf {
 namespace {
 using namespace tcx;
 
-constexpr int kQT = 128, kKT = 128;
+constexpr int kQT = 128;
 constexpr int kThreads = 256;
 constexpr int kVS = 2;        // V ring stages per stream
 constexpr int kBC = 3;        // bias chunk ring per stream (2 chunks per key tile: every TMA issue costs the
                               // issuing thread, a lane of a compute warp, some hundreds of cycles)
 constexpr int kBCW = 64;      // columns per bias chunk (128-byte rows)
 constexpr int kBChunkBytes = 128 * kBCW * 2;
+constexpr size_t kSmemLimit = 232448 - 1024;       // of a block, less the static arrays
+constexpr int kWC = 6, kWChunkBytes = 32 * 64;      // staged bias: ring per warp
+enum BiasMode { kDirect, kTma, kStaged };
 
 template <int DP> struct Cfg {
   static constexpr int ROWB = DP * 2;
-  static constexpr int TILEB = 128 * ROWB;
-  static constexpr int KS = DP == 32 ? 3 : 2;     // K ring stages per stream
+  // keys per tile: a row thread holds its scores and its DP outputs in registers; 128 + 64 spilled 100 registers to L2
+  static constexpr int KT = DP == 32 ? 128 : 64;
+  static constexpr int QB = kQT * ROWB, TILEB = KT * ROWB;
+  static constexpr int KS = 3;                    // K ring stages per stream
   static constexpr Swizzle SW = DP == 32 ? kSw64 : kSw128;
   static constexpr int SBO = 8 * ROWB;
-  static constexpr int STREAM_BYTES(bool btma) { return TILEB * (1 + KS + kVS) + (btma ? kBC * kBChunkBytes : 0); }
+  static constexpr int STREAM_BYTES(int mode) {
+    return QB + TILEB * (KS + kVS) + (mode == kTma ? kBC * kBChunkBytes : mode == kStaged ? 4 * kWC * kWChunkBytes : 0);
+  }
 };
 
 struct FwdP {
@@ -57,6 +68,12 @@ struct FwdP {
 struct StreamBars {
   uint64_t q_full, k_full[3], v_full[kVS], b_full[kBC], b_empty[kBC], s_ready, pv_done;
 };
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, int bytes) {      // the rest of the 16 is zero
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // 32 consecutive bias values of one row as fp32 from global memory; `p` 16-byte aligned, in bounds.
 template <typename TB>
@@ -85,14 +102,14 @@ __device__ __forceinline__ void load_bias32_slow(const TB* row, int64_t sj, int 
   for (int i = 0; i < 32; ++i) out[i] = (j0 + i < L) ? to_f(row[(int64_t)(j0 + i) * sj]) : 0.f;
 }
 
-template <int DP, typename T, typename TB, bool BTMA>
+template <int DP, typename T, typename TB, int BM>
 __global__ void __launch_bounds__(kThreads, 1)
 evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                   const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mb, const FwdP p) {
   using C = Cfg<DP>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  constexpr int kStreamBytes = C::STREAM_BYTES(BTMA);
+  constexpr int kKT = C::KT, kStreamBytes = C::STREAM_BYTES(BM);
 
   __shared__ StreamBars bars[2];
   __shared__ uint32_t tmem_base_s;
@@ -115,7 +132,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     }
     mbar_fence_init();
     prefetch_tmap(&mq); prefetch_tmap(&mk); prefetch_tmap(&mv);
-    if (BTMA) prefetch_tmap(&mb);
+    if (BM == kTma) prefetch_tmap(&mb);
   }
   if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
   tc_fence_before();
@@ -125,7 +142,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   StreamBars& bar = bars[s];
   uint8_t* sb = smem + s * kStreamBytes;
   uint8_t* sQ = sb;
-  uint8_t* sK = sQ + C::TILEB;
+  uint8_t* sK = sQ + C::QB;
   uint8_t* sV = sK + C::KS * C::TILEB;
   uint8_t* sB = sV + kVS * C::TILEB;
   float* mask2 = reinterpret_cast<float*>(smem + 2 * kStreamBytes) + s * p.lpad;
@@ -168,7 +185,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   int gk = 0, gv = 0, cb_next = 0, cb_quarter = 0;
   uint32_t kslot = 0, vslot = 0, pslot = 0, puse = 0;
   auto issue_q = [&]() {      // Q of the cursor's item, then advance to the next item
-    mbar_expect_tx(&bar.q_full, C::TILEB);
+    mbar_expect_tx(&bar.q_full, C::QB);
     tma_load_5d(sQ, &mq, &bar.q_full, 0, cq.h, cq.qt * kQT, cq.n, cq.b);
     cursor_next_item(cq);
   };
@@ -190,7 +207,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     }
   };
   auto pump_b = [&]() {
-    if (!BTMA) return;
+    if (BM != kTma) return;
     while (cb_next < g_total * (kKT / kBCW)) {
       if (puse > 0 && !mbar_test(&bar.b_empty[pslot], (puse - 1) & 1)) break;
       mbar_expect_tx(&bar.b_full[pslot], kBChunkBytes);
@@ -200,6 +217,26 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       if (++cb_quarter == kKT / kBCW) { cb_quarter = 0; cursor_next_tile(cbias); }
       if (++pslot == kBC) { pslot = 0; ++puse; }
     }
+  };
+  // staged bias: my warp's next chunk, four lanes a row; always one cp.async group
+  constexpr int kWCols = 64 / sizeof(TB), kWChunks = kKT / kWCols;      // per chunk / chunks per key tile
+  uint8_t* const ring = sB + (warp & 3) * (kWC * kWChunkBytes);
+  auto stage_bias = [&]() {
+    if (cb_next < g_total * kWChunks) {
+      const int col = cbias.t * kKT + cb_quarter * kWCols + (lane & 3) * (16 / (int)sizeof(TB));
+      int bytes = (p.L - col) * (int)sizeof(TB);
+      bytes = bytes < 0 ? 0 : bytes > 16 ? 16 : bytes;                  // zeros beyond the last key
+      const TB* base = static_cast<const TB*>(p.bias) + cbias.b * p.bs[0] + cbias.h * p.bs[1] + (bytes > 0 ? col : 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int rl = k * 8 + (lane >> 2), row = cbias.qt * kQT + (warp & 3) * 32 + rl;
+        cp_async16(ring + pslot * kWChunkBytes + swz_offset(rl, lane & 3, 64), base + (int64_t)(row < p.L ? row : p.L - 1) * p.bs[2], bytes);
+      }
+      ++cb_next;
+      if (++cb_quarter == kWChunks) { cb_quarter = 0; cursor_next_tile(cbias); }
+      if (++pslot == kWC) pslot = 0;
+    }
+    cp_async_commit();
   };
   auto issue_s = [&](int g) {     // S(g) = Q K(g)^T
     const uint32_t q_lo = desc_lo(smem_u32(sQ), 16), k_lo = desc_lo(smem_u32(sK + (g % C::KS) * C::TILEB), 16);
@@ -219,6 +256,8 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   if (g_total > 0) {
     if (officer_kv) { issue_q(); pump_k(0); pump_v(0); }
     if (officer_b) pump_b();
+    if (BM == kStaged)
+      for (int i = 0; i < kWC; ++i) stage_bias();
   }
 
   const TB* bias = static_cast<const TB*>(p.bias);
@@ -283,7 +322,8 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     uint32_t sr[kKT];
     {
       uint32_t (*s4)[32] = reinterpret_cast<uint32_t (*)[32]>(sr);
-      tmem_ld32(tS, s4[0]); tmem_ld32(tS + 32, s4[1]); tmem_ld32(tS + 64, s4[2]); tmem_ld32(tS + 96, s4[3]);
+#pragma unroll
+      for (int c = 0; c < kKT / 32; ++c) tmem_ld32(tS + c * 32, s4[c]);
       tmem_ld_wait();
     }
     tc_fence_before();
@@ -305,9 +345,9 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     const int j0 = t * kKT;
     float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-    for (int cb = 0; cb < 4; ++cb) {
+    for (int cb = 0; cb < kKT / 32; ++cb) {
       float bv[32];
-      if (BTMA) {
+      if constexpr (BM == kTma) {
         // a chunk holds 64 columns: two passes of this loop read its two halves
         if ((cb & 1) == 0) wait_or_flag(&bar.b_full[bslot], bphase, abort_flag);
         const uint8_t* chunk = sB + bslot * kBChunkBytes;
@@ -321,6 +361,29 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         if (cb & 1) {
           mbar_arrive(&bar.b_empty[bslot]);
           if (++bslot == kBC) { bslot = 0; bphase ^= 1; }
+        }
+      } else if constexpr (BM == kStaged) {
+#pragma unroll
+        for (int c = 0; c < 32 / kWCols; ++c) {
+          cp_async_wait<kWC - 1>();
+          __syncwarp();
+#pragma unroll
+          for (int pc = 0; pc < 4; ++pc) {
+            const uint4 x = *reinterpret_cast<const uint4*>(ring + bslot * kWChunkBytes + swz_offset(lane, pc, 64));
+            const uint32_t u[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if constexpr (sizeof(TB) == 4) {
+                bv[c * 16 + pc * 4 + e] = __uint_as_float(u[e]);
+              } else {
+                const float2 v = Pack2<TB>::unpack(u[e]);
+                bv[pc * 8 + e * 2] = v.x; bv[pc * 8 + e * 2 + 1] = v.y;
+              }
+            }
+          }
+          __syncwarp();                       // everybody has read: the slot may be filled again
+          if (++bslot == kWC) bslot = 0;
+          stage_bias();
         }
       } else {
         if (p.bias_fast && (j0 + kKT <= p.L)) load_bias32_fast<TB>(brow + j0 + cb * 32, bv);
@@ -348,7 +411,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     }
     float rs4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int cb = 0; cb < 2; ++cb) {
+    for (int cb = 0; cb < kKT / 64; ++cb) {
       uint32_t pk[32];
 #pragma unroll
       for (int jj = 0; jj < 32; ++jj) {
@@ -408,6 +471,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
 template <int DP, typename T, typename TB>
 int launch_fwd(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   using C = Cfg<DP>;
+  constexpr int kKT = C::KT;
   CUtensorMap mq, mk, mv, mb;
   int r;
   if ((r = make_qkv_map(&mq, a.q, a.dtype, a.B, a.N, a.L, a.H, a.D, a.q_strides, DP, kQT))) return r;
@@ -431,10 +495,12 @@ int launch_fwd(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t 
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
 
-  // bias through TMA: 16-bit dtype, unit inner stride, 16-byte aligned rows, and room in shared memory (DP = 32)
-  const bool btma = DP == 32 && bes == 2 && p.bias_fast;
+  // bias through shared memory: unit inner stride, 16-byte aligned rows, and room; by TMA for a 16-bit dtype and DP = 32
+  constexpr int kModeFast = DP == 32 && sizeof(TB) == 2 ? kTma : kStaged;
+  const auto smem_of = [&](int mode) { return 1024 + 2 * (size_t)C::STREAM_BYTES(mode) + 2 * sizeof(float) * p.lpad; };
+  const bool fast = p.bias_fast && smem_of(kModeFast) <= kSmemLimit;
   mb = mq;
-  if (btma) {
+  if (fast && kModeFast == kTma) {
     p.bias_b_mul = a.bias_strides[0] == 0 ? 0 : 1;
     const int64_t dims[4] = {a.L, a.L, a.H, p.bias_b_mul ? a.B : 1};
     const int64_t str[4] = {1, a.bias_strides[2], a.bias_strides[1], a.bias_strides[0]};
@@ -445,13 +511,13 @@ int launch_fwd(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t 
   const int pairs = (p.n_items + 1) / 2;
   if (grid > pairs) grid = pairs;
   p.items_per_stream = (p.n_items + 2 * grid - 1) / (2 * grid);
-  const size_t smem = 1024 + 2 * (size_t)C::STREAM_BYTES(btma) + 2 * sizeof(float) * p.lpad;
-  if (btma) {
-    constexpr auto kern = evo_fwd_tc_kernel<DP, T, TB, true>;
+  const size_t smem = smem_of(fast ? kModeFast : kDirect);
+  if (fast) {
+    constexpr auto kern = evo_fwd_tc_kernel<DP, T, TB, kModeFast>;
     if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p);
   } else {
-    constexpr auto kern = evo_fwd_tc_kernel<DP, T, TB, false>;
+    constexpr auto kern = evo_fwd_tc_kernel<DP, T, TB, kDirect>;
     if (int e = opt_in_smem<kern>(smem)) return e;
     kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p);
   }
