@@ -95,36 +95,68 @@ __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_
                ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
-// One thread per (b, n, i < lpad, h): delta = sum_d dO * O (16-byte loads; D is a multiple of 8), the XQ row of query i
-// and, for h == 0, the XK row of key i.  Consecutive threads take the heads of one token, then the next token: a warp
-// reads one contiguous piece of o and dO.  (Measured against a thread per token walking all heads, and against
-// consecutive threads taking consecutive tokens of one head: 22.8 us against 27.3 and 28.5 at the benchmark size.)
+// One thread per (b, n, i < lpad, h): delta = sum_d dO * O (D is a multiple of 8), the XQ row of query i and, for h == 0,
+// the XK row of key i.  Consecutive threads take the heads of one token, then the next token: a warp's pieces of o and dO
+// are contiguous, token by token.  A block stays in one row (b, n), so that indexes are taken apart in 32 bits (21.8 -> 20.5 us
+// for [1, 384, 384, 4, 32], 14.4 of them the bytes).  Above 32 columns (DP = 64) a warp fetches its pieces together and hands
+// them out through shared memory: with every thread reading its own 2 D bytes each load instruction touched 32 lines
+// ([4, 1, 384, 32, 64]: 13.7 -> 8.3 us; at 32 columns the detour costs 1 us more than it gives).
 // flags[bnh]: the row (b, n) has every key masked (lse = -FLT_MAX, for all of its queries alike).  The fp32 accumulator of
 // dQ, where one is used, is cleared here as well: each memset in front of the kernels cost 2 us of GPU time and as much of
 // the host's.
-template <typename T>
-__global__ void evo_extras_ws_kernel(const T* __restrict__ o, TokenStrides os, const T* __restrict__ d_o, TokenStrides ds, const float* __restrict__ lse,
+constexpr int kXWarps = 4;
+template <typename T, int DP>
+__global__ void __launch_bounds__(kXWarps * 32) evo_extras_ws_kernel(const T* __restrict__ o, TokenStrides os, const T* __restrict__ d_o, TokenStrides ds, const float* __restrict__ lse,
                                      const void* __restrict__ mask, int64_t ms_b, int64_t ms_n, int64_t ms_l, int mask_dtype,
                                      uint8_t* __restrict__ xq, uint8_t* __restrict__ xk, int* __restrict__ flags,
-                                     float* __restrict__ dq_acc, int64_t n_threads, int N, int L, int lpad, int H, int D) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n_threads) return;
-  const int hg = (int)(idx % H); const int64_t t = idx / H; const int i = (int)(t % lpad); const int64_t bn = t / lpad;
-  constexpr int hpt = 1;
+                                     float* __restrict__ dq_acc, int row_blocks, int N, int L, int lpad, int H, int D) {
+  constexpr bool kShared = DP > 32;
+  __shared__ uint4 piece_s[kShared ? kXWarps : 1][2][32 * (DP / 8 + 1)];
+  const int bn = (int)(blockIdx.x / (unsigned)row_blocks), b = bn / N, n = bn - b * N;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned first = ((blockIdx.x - (unsigned)bn * row_blocks) * kXWarps + warp) * 32, total = (unsigned)lpad * H, real = (unsigned)L * H;
+  const int per_row = D / 8, pitch = per_row | 1;        // 16-byte pieces; odd: no bank conflicts
+#pragma unroll
+  for (int k0 = 0; kShared && k0 < DP / 8; k0 += 4) {
+    uint4 a[4], g[4];
+    int at[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int f = (k0 + k) * 32 + lane, pr = f / per_row, c = f - pr * per_row;
+      const unsigned idx = first + pr;
+      at[k] = pr < 32 && idx < real ? pr * pitch + c : -1;
+      if (at[k] >= 0) {
+        const int i = (int)(idx / (unsigned)H), h = (int)(idx - (unsigned)i * H);
+        a[k] = __ldg(reinterpret_cast<const uint4*>(o + os.at(b, n, i) + h * D) + c);
+        g[k] = __ldg(reinterpret_cast<const uint4*>(d_o + ds.at(b, n, i) + h * D) + c);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (at[k] >= 0) { piece_s[warp][0][at[k]] = a[k]; piece_s[warp][1][at[k]] = g[k]; }
+  }
+  if (dq_acc && first < real) {
+    float4* z = reinterpret_cast<float4*>(dq_acc + ((int64_t)bn * real + first) * D);
+    const int n_z = (int)(real - first < 32u ? real - first : 32u) * (D / 4);
+    for (int f = lane; f < n_z; f += 32) z[f] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  if (kShared) __syncwarp();
+  const unsigned idx = first + lane;
+  if (idx >= total) return;
+  const int i = (int)(idx / (unsigned)H), h = (int)(idx - (unsigned)i * H);
   const float sqrt_d = sqrtf((float)D);
   const __nv_bfloat16 one = __float2bfloat16_rn(1.f), zero = __float2bfloat16_rn(0.f);
   const int nt = lpad / 128, tile = i >> 7, r = i & 127;
-  for (int h = hg * hpt; h < (hg + 1) * hpt; ++h) {
-    const int64_t bnh = bn * H + h;
+  {
+    const int64_t bnh = (int64_t)bn * H + h;
     float nl = kMinusBig, nd = 0.f;
     if (i < L) {
-      const int64_t row = (bn * L + i) * H + h;
-      const int b = (int)(bn / N), n = (int)(bn % N);
+      float dl = 0.f;
       const uint4* po = reinterpret_cast<const uint4*>(o + os.at(b, n, i) + h * D);
       const uint4* pg = reinterpret_cast<const uint4*>(d_o + ds.at(b, n, i) + h * D);
-      float dl = 0.f;
-      for (int c = 0; c < D / 8; ++c) {
-        const uint4 a = __ldg(po + c), g = __ldg(pg + c);
+#pragma unroll 4
+      for (int c = 0; c < per_row; ++c) {
+        const uint4 a = kShared ? piece_s[warp][0][lane * pitch + c] : __ldg(po + c), g = kShared ? piece_s[warp][1][lane * pitch + c] : __ldg(pg + c);
         const uint32_t av[4] = {a.x, a.y, a.z, a.w}, gv[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -137,8 +169,6 @@ __global__ void evo_extras_ws_kernel(const T* __restrict__ o, TokenStrides os, c
       const bool masked = lv <= -3e38f;
       if (!masked) nl = -lv * sqrt_d;
       if (i == 0) flags[bnh] = masked;
-      if (dq_acc)
-        for (int c = 0; c < D / 4; ++c) reinterpret_cast<float4*>(dq_acc + row * D)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     __nv_bfloat16 a[3], b[3];
     split3(nl, a); split3(nd, b);
@@ -146,10 +176,9 @@ __global__ void evo_extras_ws_kernel(const T* __restrict__ o, TokenStrides os, c
     *reinterpret_cast<uint4*>(base + swz_offset(r, 0, 32)) = make_uint4(pack_bf(one, one), pack_bf(one, a[0]), pack_bf(a[1], a[2]), pack_bf(b[0], b[1]));
     *reinterpret_cast<uint4*>(base + swz_offset(r, 1, 32)) = make_uint4(pack_bf(b[2], zero), 0u, 0u, 0u);
   }
-  if (hg == 0) {
+  if (h == 0) {
     float mv = kMinusBig;
     if (i < L) {
-      const int n = (int)(bn % N); const int64_t b = bn / N;
       const int64_t mi = b * ms_b + n * ms_n + (int64_t)i * ms_l;
       mv = mask_dtype == MF_U8 ? (static_cast<const uint8_t*>(mask)[mi] ? 0.f : kMinusBig) : fmaxf(load_rt(mask, mi, mask_dtype) * sqrt_d, kMinusBig);
     }
@@ -1028,10 +1057,11 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
     if ((r = make_tiled_map(&mbt, bias, bt_dtype, 4, dims, str, box, 128))) return r;
   }
   {
-    const int64_t n_threads = (int64_t)a.B * a.N * lpad * a.H;
-    evo_extras_ws_kernel<T><<<(unsigned)((n_threads + 255) / 256), 256, 0, st>>>(static_cast<const T*>(a.o), token_strides(lay.o), static_cast<const T*>(a.d_o), token_strides(lay.d_o), a.lse,
+    const int row_blocks = (int)(((int64_t)lpad * a.H + kXWarps * 32 - 1) / (kXWarps * 32));
+    auto kern = a.D <= 32 ? evo_extras_ws_kernel<T, 32> : evo_extras_ws_kernel<T, 64>;
+    kern<<<(unsigned)((int64_t)a.B * a.N * row_blocks), kXWarps * 32, 0, st>>>(static_cast<const T*>(a.o), token_strides(lay.o), static_cast<const T*>(a.d_o), token_strides(lay.d_o), a.lse,
                                                                              a.mask, a.mask_strides[0], a.mask_strides[1], a.mask_strides[2], a.mask_dtype,
-                                                                             xq, xk, flags, pl.dq_fp32 ? dq_acc : nullptr, n_threads, a.N, a.L, lpad, a.H, a.D);
+                                                                             xq, xk, flags, pl.dq_fp32 ? dq_acc : nullptr, row_blocks, a.N, a.L, lpad, a.H, a.D);
   }
   MF_LAUNCHED("evo_extras_ws_kernel");
   const int64_t n_dq = (int64_t)a.B * a.N * a.L * a.H * a.D;

@@ -20,7 +20,7 @@
 // swizzle, DP = 32 only).  Other aligned biases (fp32, or DP = 64 whose operand tiles leave less room) go through a ring per
 // warp of [32 rows x 64 bytes] chunks, filled by cp.async six chunks ahead: the row threads' own loads from global memory,
 // 128 bytes of a row at a time with their latency in the open, made the fp32 bias of [4, 1, 384, 32, 64] cost 72 us where
-// this takes XX.  Unaligned or strided biases, and DP = 64 beyond 2176 keys (the mask rows need the room), are still read
+// this takes 48.  Unaligned or strided biases, and DP = 64 beyond 2176 keys (the mask rows need the room), are still read
 // by the row thread.
 //
 // Every wait is bounded; on expiry the CTA raises a flag that all threads honour at their next group
@@ -39,7 +39,7 @@ constexpr int kBC = 3;        // bias chunk ring per stream (2 chunks per key ti
 constexpr int kBCW = 64;      // columns per bias chunk (128-byte rows)
 constexpr int kBChunkBytes = 128 * kBCW * 2;
 constexpr size_t kSmemLimit = 232448 - 1024;       // of a block, less the static arrays
-constexpr int kWC = 6, kWChunkBytes = 32 * 64;      // staged bias: ring per warp
+constexpr int kWChunkBytes = 32 * 64;      // staged bias: ring per warp
 enum BiasMode { kDirect, kTma, kStaged };
 
 template <int DP> struct Cfg {
@@ -48,10 +48,11 @@ template <int DP> struct Cfg {
   static constexpr int KT = DP == 32 ? 128 : 64;
   static constexpr int QB = kQT * ROWB, TILEB = KT * ROWB;
   static constexpr int KS = 3;                    // K ring stages per stream
+  static constexpr int WC = 6;                    // staged bias: chunks in the ring of a warp
   static constexpr Swizzle SW = DP == 32 ? kSw64 : kSw128;
   static constexpr int SBO = 8 * ROWB;
   static constexpr int STREAM_BYTES(int mode) {
-    return QB + TILEB * (KS + kVS) + (mode == kTma ? kBC * kBChunkBytes : mode == kStaged ? 4 * kWC * kWChunkBytes : 0);
+    return QB + TILEB * (KS + kVS) + (mode == kTma ? kBC * kBChunkBytes : mode == kStaged ? 4 * WC * kWChunkBytes : 0);
   }
 };
 
@@ -109,7 +110,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   using C = Cfg<DP>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  constexpr int kKT = C::KT, kStreamBytes = C::STREAM_BYTES(BM);
+  constexpr int kKT = C::KT, kWC = C::WC, kStreamBytes = C::STREAM_BYTES(BM);
 
   __shared__ StreamBars bars[2];
   __shared__ uint32_t tmem_base_s;
@@ -150,11 +151,13 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   const int r = (warp & 3) * 32 + lane;                              // TMEM lane = query row in the tile
   const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t tS = tmem_base_s + s * 256 + lane_addr, tP = tS + 128, tO = tS + 192;
-  const uint32_t tS0 = tmem_base_s + s * 256;                        // lane 0 addresses for the MMA issuer
+  const uint32_t tS0 = tmem_base_s + s * 256;                      // lane 0 addresses for the MMA issuer
   const uint32_t id_s = idesc_f16(128, kKT, p.ab_fmt, 0, 0);
   const uint32_t id_o = idesc_f16(128, DP, p.ab_fmt, 0, 1);
 
-  const int stream = blockIdx.x * 2 + s;
+  // first streams of all SMs before the second ones: where there are fewer items than streams, or one and a bit per stream,
+  // most SMs then run one stream undisturbed
+  const int stream = s * gridDim.x + blockIdx.x;
   const int item_begin = stream * p.items_per_stream;
   int item_end = item_begin + p.items_per_stream;
   if (item_end > p.n_items) item_end = p.n_items;
@@ -343,10 +346,11 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     if (officer_b) pump_b();
     // ------------------------------------------------------------------ pass 1: base-2 logits, row max
     const int j0 = t * kKT;
+    constexpr int kW = BM == kStaged ? kWCols : 32;      // columns at a time
     float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-    for (int cb = 0; cb < kKT / 32; ++cb) {
-      float bv[32];
+    for (int cb = 0; cb < kKT / kW; ++cb) {
+      float bv[kW];
       if constexpr (BM == kTma) {
         // a chunk holds 64 columns: two passes of this loop read its two halves
         if ((cb & 1) == 0) wait_or_flag(&bar.b_full[bslot], bphase, abort_flag);
@@ -363,39 +367,36 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           if (++bslot == kBC) { bslot = 0; bphase ^= 1; }
         }
       } else if constexpr (BM == kStaged) {
+        cp_async_wait<kWC - 1>();
+        __syncwarp();
 #pragma unroll
-        for (int c = 0; c < 32 / kWCols; ++c) {
-          cp_async_wait<kWC - 1>();
-          __syncwarp();
+        for (int pc = 0; pc < 4; ++pc) {
+          const uint4 x = *reinterpret_cast<const uint4*>(ring + bslot * kWChunkBytes + swz_offset(lane, pc, 64));
+          const uint32_t u[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-          for (int pc = 0; pc < 4; ++pc) {
-            const uint4 x = *reinterpret_cast<const uint4*>(ring + bslot * kWChunkBytes + swz_offset(lane, pc, 64));
-            const uint32_t u[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if constexpr (sizeof(TB) == 4) {
-                bv[c * 16 + pc * 4 + e] = __uint_as_float(u[e]);
-              } else {
-                const float2 v = Pack2<TB>::unpack(u[e]);
-                bv[pc * 8 + e * 2] = v.x; bv[pc * 8 + e * 2 + 1] = v.y;
-              }
+          for (int e = 0; e < 4; ++e) {
+            if constexpr (sizeof(TB) == 4) {
+              bv[pc * 4 + e] = __uint_as_float(u[e]);
+            } else {
+              const float2 v = Pack2<TB>::unpack(u[e]);
+              bv[pc * 8 + e * 2] = v.x; bv[pc * 8 + e * 2 + 1] = v.y;
             }
           }
-          __syncwarp();                       // everybody has read: the slot may be filled again
-          if (++bslot == kWC) bslot = 0;
-          stage_bias();
         }
+        __syncwarp();                         // everybody has read: the slot may be filled again
+        if (++bslot == kWC) bslot = 0;
+        stage_bias();
       } else {
         if (p.bias_fast && (j0 + kKT <= p.L)) load_bias32_fast<TB>(brow + j0 + cb * 32, bv);
         else load_bias32_slow<TB>(brow, p.bs[3], j0 + cb * 32, p.L, bv);
       }
 #pragma unroll
-      for (int q4 = 0; q4 < 8; ++q4) {
-        const float4 mk4 = *reinterpret_cast<const float4*>(mask2 + j0 + cb * 32 + q4 * 4);
+      for (int q4 = 0; q4 < kW / 4; ++q4) {
+        const float4 mk4 = *reinterpret_cast<const float4*>(mask2 + j0 + cb * kW + q4 * 4);
         const float mk[4] = {mk4.x, mk4.y, mk4.z, mk4.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int jj = cb * 32 + q4 * 4 + e;
+          const int jj = cb * kW + q4 * 4 + e;
           const float v = fmaf(__uint_as_float(sr[jj]), p.c1, fmaf(bv[q4 * 4 + e], kLog2e, mk[e]));
           sr[jj] = __float_as_uint(v);
           mx4[e] = fmaxf(mx4[e], v);
@@ -497,7 +498,7 @@ int launch_fwd(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t 
 
   // bias through shared memory: unit inner stride, 16-byte aligned rows, and room; by TMA for a 16-bit dtype and DP = 32
   constexpr int kModeFast = DP == 32 && sizeof(TB) == 2 ? kTma : kStaged;
-  const auto smem_of = [&](int mode) { return 1024 + 2 * (size_t)C::STREAM_BYTES(mode) + 2 * sizeof(float) * p.lpad; };
+  const auto smem_of = [&](int mode) { return 1024 + 2 * ((size_t)C::STREAM_BYTES(mode) + sizeof(float) * p.lpad); };
   const bool fast = p.bias_fast && smem_of(kModeFast) <= kSmemLimit;
   mb = mq;
   if (fast && kModeFast == kTma) {
@@ -508,8 +509,7 @@ int launch_fwd(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t 
     if ((r = make_tiled_map(&mb, a.bias, a.bias_dtype, 4, dims, str, box, kBCW * 2))) return r;
   }
   int grid = sm_count();
-  const int pairs = (p.n_items + 1) / 2;
-  if (grid > pairs) grid = pairs;
+  if (grid > p.n_items) grid = p.n_items;
   p.items_per_stream = (p.n_items + 2 * grid - 1) / (2 * grid);
   const size_t smem = smem_of(fast ? kModeFast : kDirect);
   if (fast) {
