@@ -134,9 +134,51 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     const float2 c1c1 = make_float2(p.c1, p.c1);
     uint32_t g = 0;
     MF_TRACE_DECL(tr, 0, blockIdx.x == 0 && tid == 0);
+    ItemPos pos = item_pos(item_begin, p);        // stepped from item to item: four divisions took 600 cycles each time
+    float l_done = 1.f, m_done = 0.f;
+    int i_done = 0;
+    T* o_done = nullptr;
+    float* lse_done = nullptr;
+    // O / l and the log-sum-exp of the item before, whose last product is complete.  Four lanes exchange their 16-byte pieces,
+    // so that a store instruction writes whole rows of eight tokens instead of a piece of 32.
+    auto write_out = [&]() {
+      tc_fence_after();
+      uint32_t o32[32];
+      tmem_ld32(tO, o32);
+      tmem_ld_wait();
+      tc_fence_before();
+      const float inv = 1.f / l_done;
+      uint32_t w[4][4];                            // [piece of eight columns][word]
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[c][e] = Pack2<T>::pack(__uint_as_float(o32[c * 8 + 2 * e]) * inv, __uint_as_float(o32[c * 8 + 2 * e + 1]) * inv);
+      const int q = lane & 3;
+#pragma unroll
+      for (int s2 = 2; s2 > 0; s2 >>= 1) {         // 4 x 4 transposition over lanes q
+        const bool up = q & s2;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          if (c & s2) continue;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[c][e] : w[c + s2][e], s2);
+            if (up) w[c][e] = got; else w[c + s2][e] = got;
+          }
+        }
+      }
+      if (*abort_flag) return;
+      T* piece = o_done + q * 8;
+#pragma unroll
+      for (int c = 0; c < 4; ++c)                  // w[c]: piece q of row i_done - q + c
+        if (i_done - q + c < p.L && q * 8 < p.D)
+          *reinterpret_cast<uint4*>(piece + (c - q) * p.os.l) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+      // a row whose keys are all masked has every logit at the mask term (about -1e30): uniform attention over its L
+      // keys; its log-sum-exp is stored as -FLT_MAX, the value the backward kernels recognise
+      if (i_done < p.L) *lse_done = m_done <= -1e28f ? -FLT_MAX : (m_done * p.c1 + lg2f(l_done)) * kLn2;
+    };
     for (int il = 0; il < n_my; ++il) {
-      const ItemPos ip = item_pos(item_begin + il, p);
-      const int i = ip.qt * kT + r;
+      const int i = pos.qt * kT + r;
       float m_used = 0.f;
       float2 lsum0 = make_float2(0.f, 0.f), lsum1 = lsum0;        // row sum of P relative to m_used (four partial sums)
       for (int t = 0; t < n_kt; ++t, ++g) {
@@ -190,6 +232,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         }
         // ---------------------------------------------------------------- pass 2: P = 2^(x - m) as packed 16-bit
         if (g > 0) wait_or_flag(&bar.pv_done, (g - 1) & 1, abort_flag);      // the previous product has read P
+        if (t == 0 && il > 0) write_out();
         tr(5);
         // x = c1 * (s - m): the difference first, so that logits equal to the maximum give exactly 0 whatever their size
         // (a fully masked row sits at about -1e30, where a fused c1 * s - c1 * m would leave a huge rounding residue)
@@ -213,35 +256,15 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         if (lane == 0) mbar_arrive(&bar.p_ready);
         tr(6);
       }
-      // ------------------------------------------------------------------ item done: O / l and the log-sum-exp
+      // the item's last product is under way: what its output needs is kept until the next item's first maximum
+      l_done = (lsum0.x + lsum0.y) + (lsum1.x + lsum1.y); m_done = m_used; i_done = i;
+      o_done = static_cast<T*>(p.o) + p.os.at(pos.b, pos.n, i) + pos.h * p.D;
+      lse_done = p.lse + ((int64_t)((int64_t)pos.b * p.N + pos.n) * p.H + pos.h) * p.L + i;
+      if (++pos.qt == p.n_qt) { pos.qt = 0; if (++pos.h == p.H) { pos.h = 0; if (++pos.n == p.N) { pos.n = 0; ++pos.b; } } }
+    }
+    if (n_my > 0) {
       wait_or_flag(&bar.pv_done, (g - 1) & 1, abort_flag);
-      tc_fence_after();
-      tr(7);
-      uint32_t o32[32];
-      tmem_ld32(tO, o32);
-      const float l = (lsum0.x + lsum0.y) + (lsum1.x + lsum1.y);
-      tmem_ld_wait();
-      tc_fence_before();
-      tr(8);
-      if (i < p.L && !*abort_flag) {
-        const float inv = 1.f / l;
-        T* orow = static_cast<T*>(p.o) + p.os.at(ip.b, ip.n, i) + ip.h * p.D;
-#pragma unroll
-        for (int d8 = 0; d8 < 4; ++d8) {
-          if (d8 * 8 < p.D) {
-            uint4 v;
-            v.x = Pack2<T>::pack(__uint_as_float(o32[d8 * 8]) * inv, __uint_as_float(o32[d8 * 8 + 1]) * inv);
-            v.y = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 2]) * inv, __uint_as_float(o32[d8 * 8 + 3]) * inv);
-            v.z = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 4]) * inv, __uint_as_float(o32[d8 * 8 + 5]) * inv);
-            v.w = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 6]) * inv, __uint_as_float(o32[d8 * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(orow + d8 * 8) = v;
-          }
-        }
-        // a row whose keys are all masked has every logit at the mask term (about -1e30): uniform attention over its L
-        // keys; its log-sum-exp is stored as -FLT_MAX, the value the backward kernels recognise
-        p.lse[(((int64_t)ip.b * p.N + ip.n) * p.H + ip.h) * p.L + i] = m_used <= -1e28f ? -FLT_MAX : (m_used * p.c1 + lg2f(l)) * kLn2;
-      }
-      tr(9);
+      write_out();
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kHelperRegs));
