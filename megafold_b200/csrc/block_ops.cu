@@ -3,6 +3,8 @@
 // products, their gradients, packing copies of the strided gate) and three (slice, permute, zero-filled padding).
 //
 // Bound: HBM.  [768 * 768, 128] bf16: gate forward 3 x 151 MB in 89 us, backward 5 x 151 MB in 120 us.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace mf {
@@ -61,12 +63,32 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(const T* __restrict__ d, 
 
 // rows [L * L, np] <-> planes [H, L, L] (H <= np) in 32 x 32 tiles through shared memory, so that both sides are touched in
 // whole lines; `swap`: plane element (i, j) belongs to row j * L + i.  To rows: columns H .. np - 1 become zero.
-template <typename T, bool TO_ROWS>
+// VEC: rows of whole 16-byte pieces of 16-bit values are moved a piece at a time.  (A value at a time, with three divisions
+// each: 28 us for [768, 768, 8] and four heads, 8 to planes and 16 to rows now; the bytes take 2.)
+template <typename T, bool TO_ROWS, bool VEC>
 __global__ void __launch_bounds__(256) bias_layout_kernel(T* __restrict__ rows, T* __restrict__ planes, int L, int np, int H, bool swap) {
   extern __shared__ __align__(16) uint8_t raw[];
   T* tile = reinterpret_cast<T*>(raw);              // [H][32][33], plane order
   const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;      // plane coordinates
   auto move_rows = [&] {
+    if constexpr (VEC) {
+      for (int e = threadIdx.x; e < 32 * 32; e += 256) {
+        const int c = e % 32, r = e / 32, i = swap ? c : r, j = swap ? r : c;
+        if (i0 + i >= L || j0 + j >= L) continue;
+        uint4* p = reinterpret_cast<uint4*>(rows + ((int64_t)(swap ? j0 + j : i0 + i) * L + (swap ? i0 + i : j0 + j)) * np);
+        for (int h0 = 0; h0 < np; h0 += 8) {
+          Vec8<T> v;
+          if (!TO_ROWS) *reinterpret_cast<uint4*>(v.e) = p[h0 / 8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            if (TO_ROWS) v.e[k] = h0 + k < H ? tile[((h0 + k) * 32 + i) * 33 + j] : from_f<T>(0.f);
+            else if (h0 + k < H) tile[((h0 + k) * 32 + i) * 33 + j] = v.e[k];
+          }
+          if (TO_ROWS) p[h0 / 8] = *reinterpret_cast<const uint4*>(v.e);
+        }
+      }
+      return;
+    }
     for (int e = threadIdx.x; e < 32 * 32 * np; e += 256) {
       const int h = e % np, c = e / np % 32, r = e / np / 32;      // row block r, column c of it, in the order of memory
       const int i = swap ? c : r, j = swap ? r : c;
@@ -127,11 +149,17 @@ int bias_layout(void* rows, void* planes, int L, int np, int H, bool swap, bool 
   const dim3 grid((L + 31) / 32, (L + 31) / 32);
   MF_DISPATCH_FLOAT(dtype, T, {
     const size_t smem = sizeof(T) * (size_t)H * 32 * 33;
-    constexpr auto there = bias_layout_kernel<T, true>;
-    constexpr auto back = bias_layout_kernel<T, false>;
-    if (int e = to_rows ? opt_in_smem<there>(smem) : opt_in_smem<back>(smem)) return e;
-    if (to_rows) there<<<grid, 256, smem, st>>>(static_cast<T*>(rows), static_cast<T*>(planes), L, np, H, swap);
-    else back<<<grid, 256, smem, st>>>(static_cast<T*>(rows), static_cast<T*>(planes), L, np, H, swap);
+    auto launch = [&](auto to, auto vec) -> int {
+      constexpr auto kern = bias_layout_kernel<T, decltype(to)::value, decltype(vec)::value>;
+      if (int e = opt_in_smem<kern>(smem)) return e;
+      kern<<<grid, 256, smem, st>>>(static_cast<T*>(rows), static_cast<T*>(planes), L, np, H, swap);
+      return MF_OK;
+    };
+    using Yes = std::true_type; using No = std::false_type;
+    constexpr bool can = sizeof(T) == 2;
+    const bool vec = can && np % 8 == 0 && aligned16({rows});
+    using Vec = std::bool_constant<can>;
+    if (int e = vec ? (to_rows ? launch(Yes{}, Vec{}) : launch(No{}, Vec{})) : (to_rows ? launch(Yes{}, No{}) : launch(No{}, No{}))) return e;
     MF_LAUNCHED("bias_layout_kernel");
   });
   return MF_OK;

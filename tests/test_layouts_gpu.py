@@ -79,7 +79,7 @@ def test_gate(rows, cols, dtype):
     assert float(d_wide[:, :cols].abs().max()) == 0
 
 
-@pytest.mark.parametrize("L,H,np_", [(1, 4, 8), (33, 4, 8), (96, 16, 16), (127, 3, 8)])
+@pytest.mark.parametrize("L,H,np_", [(1, 4, 8), (33, 4, 8), (96, 16, 16), (127, 3, 8), (33, 3, 5)])
 @pytest.mark.parametrize("swap", [0, 1])
 def test_bias_layout(L, H, np_, swap):
     rows = torch.randn(L * L, np_, device="cuda").bfloat16()
