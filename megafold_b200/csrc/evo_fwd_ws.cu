@@ -17,7 +17,7 @@
 // packed 16-bit P = 2^(x - m) back to TMEM while adding up the row sum (packed adds that hide under the
 // exponentials).  P V accumulates into O in TMEM over the key tiles; O and the sum are only multiplied by
 // 2^(m_old - m_new) when the running maximum has grown by more than 8 (rare after the first tile; P then stays
-// below 2^8, far inside the 16-bit range).  Only O and the log-sum-exp reach global memory.
+// below 2^8, far inside the 16-bit range), or at all (kExactStep).  Only O and the log-sum-exp reach global memory.
 //
 // Every wait is bounded; on expiry the CTA raises a flag, all roles run dry without touching global memory, TMEM is
 // freed and the host sees mf_async_status() != 0.
@@ -33,6 +33,13 @@ constexpr int kTileB = 128 * 64;             // [128 x 32] 16-bit tile, 64-byte 
 constexpr int kAtomB = 128 * 128;            // bias atom: [128 rows x 64 columns] 16-bit, 128-byte rows, 128B swizzle
 constexpr int kStreamBytes = 6 * kTileB + 3 * kAtomB + 2 * kXTileB;     // Q x2, K x2, V x2, three bias atoms, mask-term tile x2
 constexpr float kRescaleStep = 8.f;          // O is rescaled only when the running maximum grows by more than this (base-2 logits)
+// A bias that had to be copied belongs to a length whose calls ran the general kernel (evo_tc_fwd.cu), which takes every
+// tile's probabilities relative to the running maximum and the bias as it is.  For them the step is 0 and sqrt(D) keeps its
+// second term, so that they are as close to the exact result as there: the largest probability of a row is then exactly 1.
+// Distance from 64 bits at [1, 200, 467, 4, 32] bf16: 2.25e-3 with the step of 8 (2.04e-3 the general kernel and now),
+// fp16 at 323: 3.02e-4 with it, 2.81e-4 without but with one term, 2.54e-4 now.  It costs 275 -> 295 us at [1, 467, 467, 4, 32];
+// a template parameter, because a step read from the arguments cost the other lengths 1.5 %.
+constexpr float kExactStep = 0.f;
 
 struct FwdWsP {
   int B, N, L, H, D;
@@ -64,7 +71,7 @@ constexpr int kLaunchRegs = 128, kSoftmaxRegs = 208, kHelperRegs = 48;      // r
 static_assert(kLaunchRegs * kThreads <= 65536, "register file");
 static_assert(256 * kSoftmaxRegs + (kThreads - 256) * kHelperRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 
-template <typename T, typename TB>
+template <typename T, typename TB, bool EXACT>      // EXACT: see kExactStep
 __global__ void __maxnreg__(kLaunchRegs)
 evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                   const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mb, const FwdWsP p MF_TRACE_PARAM) {
@@ -210,7 +217,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         if (t == 0) {
           m_used = m_blk;
         } else {
-          const bool grow = (m_blk - m_used) * p.c1 > kRescaleStep;
+          const bool grow = (m_blk - m_used) * p.c1 > (EXACT ? kExactStep : kRescaleStep);
           if (__any_sync(0xffffffffu, grow)) {
             // rare: bring O and the row sum of this warp's rows to the new maximum
             wait_or_flag(&bar.pv_done, (g - 1) & 1, abort_flag);
@@ -476,7 +483,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   if (warp == 0) tmem_dealloc(tmem_base_s, 512);
 }
 
-template <typename T, typename TB>
+template <typename T, typename TB, bool EXACT>
 int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   CUtensorMap mq, mk, mv, mb;
   int r;
@@ -491,7 +498,7 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   p.c1 = kLog2e / sqrtf((float)a.D);
   p.fmt = a.dtype == MF_BF16 ? 1u : 0u;
   p.bfmt = a.bias_dtype == MF_BF16 ? 1u : 0u;
-  p.n_alpha = split_alpha(a.D, a.bias_dtype, p.alpha);
+  p.n_alpha = split_alpha(a.D, a.bias_dtype, p.alpha, EXACT);
   p.mask = a.mask; for (int i = 0; i < 3; ++i) p.ms[i] = a.mask_strides[i];
   p.mask_dtype = a.mask_dtype;
   p.o = a.o; p.os = token_strides(lay.o); p.lse = a.lse;
@@ -511,7 +518,7 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   if (grid > pairs) grid = pairs;
   p.items_per_stream = (p.n_items + 2 * grid - 1) / (2 * grid);
   const size_t smem = 1024 + 2 * (size_t)kStreamBytes + 2048 + kXTileB;
-  constexpr auto kern = evo_fwd_ws_kernel<T, TB>;
+  constexpr auto kern = evo_fwd_ws_kernel<T, TB, EXACT>;
   static const int regs = [] {
     cudaFuncAttributes fa;
     return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : -1;
@@ -523,6 +530,13 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   return MF_OK;
 }
 
+template <bool EXACT>
+int dispatch(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
+  if (a.dtype == MF_BF16)
+    return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16, EXACT>(a, lay, st) : launch_fwd_ws<__nv_bfloat16, __half, EXACT>(a, lay, st);
+  return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16, EXACT>(a, lay, st) : launch_fwd_ws<__half, __half, EXACT>(a, lay, st);
+}
+
 }  // namespace
 
 // The warp-specialised kernel covers head sizes up to 32, rows up to 2048 tokens and a 16-bit pair bias; other calls use
@@ -530,8 +544,8 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
 static bool shape_ok(const mf_evo_fwd_args& a) { return a.D <= 32 && a.L <= 2048 && (a.bias_dtype == MF_BF16 || a.bias_dtype == MF_F16); }
 
 // A bias whose rows TMA cannot address (a chain of odd length) is copied to a 16-byte pitch when the caller gives the
-// scratch for it: an exact copy, and 3 us against the 1000 us that the general kernel's reads of such a bias in place cost
-// at [467, 467, 4, 32].
+// scratch for it: an exact copy in 3 us.  At [1, 467, 467, 4, 32] the call takes 295 us, where the general kernel that reads
+// such a bias in place takes 1263, and the same kernel on the copied bias 457.
 size_t evo_fwd_ws_workspace(const mf_evo_fwd_args& a) {
   if (!shape_ok(a) || bias_tma_ok(a.bias, a.bias_dtype, a.bias_strides, a.B, a.H)) return 0;
   return bias_copy_bytes(a.bias_strides, a.B, a.H, a.L);
@@ -542,7 +556,8 @@ bool evo_fwd_ws_supported(const mf_evo_fwd_args& a, size_t workspace_bytes) {
 
 int evo_fwd_ws(const mf_evo_fwd_args& args, const mf_evo_layout& lay, void* workspace, cudaStream_t st) {
   mf_evo_fwd_args a = args;
-  if (evo_fwd_ws_workspace(args)) {
+  const bool copied = evo_fwd_ws_workspace(args) != 0;
+  if (copied) {
     int r = copy_bias_rows(a.bias, a.bias_dtype, a.bias_strides, workspace, a.bias_dtype, a.B, a.H, a.L, st);
     if (r) return r;
     const int64_t row = bias_pitch(a.L);
@@ -550,9 +565,7 @@ int evo_fwd_ws(const mf_evo_fwd_args& args, const mf_evo_layout& lay, void* work
     a.bias_strides[3] = 1; a.bias_strides[2] = row; a.bias_strides[1] = row * a.L;
     a.bias_strides[0] = args.bias_strides[0] == 0 ? 0 : row * a.L * a.H;
   }
-  if (a.dtype == MF_BF16)
-    return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16>(a, lay, st) : launch_fwd_ws<__nv_bfloat16, __half>(a, lay, st);
-  return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16>(a, lay, st) : launch_fwd_ws<__half, __half>(a, lay, st);
+  return copied ? dispatch<true>(a, lay, st) : dispatch<false>(a, lay, st);
 }
 
 }  // namespace mf

@@ -235,14 +235,14 @@ struct Tracer {
 
 // ---- host side ------------------------------------------------------------------------------------
 // sqrt(D) as a sum of values representable in the 16-bit type `dt`; returns the number of terms (1 when the first
-// one is within 2.5e-4 relative, which is below the rounding of the bias values themselves)
-inline int split_alpha(int D, int dt, float (&alpha)[2]) {
+// one is within 2.5e-4 relative, or, with `exact`, when nothing is left of it)
+inline int split_alpha(int D, int dt, float (&alpha)[2], bool exact) {
   const float a = sqrtf((float)D);
   const float hi = dt == MF_BF16 ? __bfloat162float(__float2bfloat16_rn(a)) : __half2float(__float2half_rn(a));
   const float rest = a - hi;
   const float lo = dt == MF_BF16 ? __bfloat162float(__float2bfloat16_rn(rest)) : __half2float(__float2half_rn(rest));
   alpha[0] = hi; alpha[1] = lo;
-  return fabsf(rest) > 2.5e-4f * a ? 2 : 1;
+  return fabsf(rest) > (exact ? 0.f : 2.5e-4f * a) ? 2 : 1;
 }
 
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
