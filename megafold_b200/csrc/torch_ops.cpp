@@ -495,6 +495,11 @@ Tensor transition(const Tensor& x, const OptTensor& lw, const OptTensor& lb, con
 // Every value is that of the composed form, rounding for rounding: the gradient of a bias projection's shift is 0 up to the
 // rounding of d_pair_bias (a softmax's logit gradients sum to 0), so it is another number as soon as one bit before it is.
 struct Attn { Tensor lw, lb, w, b, w_out; };
+// The kernels take the parameters as contiguous arrays (only w_out is multiplied by torch, on strides): a transposed or
+// otherwise strided parameter is copied.
+Attn contiguous(const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out) {
+  return {lw.contiguous(), lb.contiguous(), w.contiguous(), b.contiguous(), w_out};
+}
 
 mf_evo_layout token_layout(int64_t n, int64_t L, int64_t tok_o, int64_t tok_q, bool swap) {
   mf_evo_layout l{};
@@ -601,13 +606,14 @@ std::array<Tensor, 4> bias_bwd(const Tensor& d_bias, const Tensor& x, const Tens
 // x [L, L, C] + attention over its rows (or, with `swap`, its columns) with a pair bias projected from x itself
 struct TriangleFn : torch::autograd::Function<TriangleFn> {
   static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out,
-                          const Tensor& plw, const Tensor& plb, const Tensor& pw, const Tensor& mask, int64_t H, bool swap) {
+                          const Tensor& plw_, const Tensor& plb_, const Tensor& pw_, const Tensor& mask, int64_t H, bool swap) {
     const c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous();
+    const Tensor x = x_.contiguous(), plw = plw_.contiguous(), plb = plb_.contiguous(), pw = pw_.contiguous();
+    const Attn p = contiguous(lw, lb, w, b, w_out);
     AttnSaved s; BiasSaved bs;
     const Tensor bias = bias_fwd(x, plw, plb, pw, H, swap, bs);
-    Tensor out = attn_fwd(x, {lw, lb, w, b, w_out}, mask, bias, H, swap, s, 0);
-    ctx->save_for_backward({x, lw, lb, w, b, w_out, plw, plb, pw, mask, bias, s.y, s.mean, s.rstd, s.o, s.lse, s.og, bs.mean, bs.rstd});
+    Tensor out = attn_fwd(x, p, mask, bias, H, swap, s, 0);
+    ctx->save_for_backward({x, p.lw, p.lb, p.w, p.b, p.w_out, plw, plb, pw, mask, bias, s.y, s.mean, s.rstd, s.o, s.lse, s.og, bs.mean, bs.rstd});
     ctx->saved_data["H"] = H; ctx->saved_data["swap"] = swap;
     return out;
   }
@@ -633,11 +639,12 @@ struct GatedAttnFn : torch::autograd::Function<GatedAttnFn> {
                           const Tensor& mask, const Tensor& bias, int64_t H) {
     const c10::cuda::CUDAGuard guard(x_.device());
     const Tensor x = x_.contiguous();
+    const Attn p = contiguous(lw, lb, w, b, w_out);
     AttnSaved s;
     // the projection of these few wide rows keeps fp32 operands and sums (0.4 % of a block at 768 tokens): its values too
     // are those of the composed form
-    Tensor out = attn_fwd(x, {lw, lb, w, b, w_out}, mask, bias, H, false, s, MF_FLAG_FORCE_SIMT);
-    ctx->save_for_backward({x, lw, lb, w, b, w_out, mask, bias, s.y, s.mean, s.rstd, s.o, s.lse, s.og});
+    Tensor out = attn_fwd(x, p, mask, bias, H, false, s, MF_FLAG_FORCE_SIMT);
+    ctx->save_for_backward({x, p.lw, p.lb, p.w, p.b, p.w_out, mask, bias, s.y, s.mean, s.rstd, s.o, s.lse, s.og});
     ctx->saved_data["H"] = H;
     return out;
   }
@@ -653,9 +660,9 @@ struct GatedAttnFn : torch::autograd::Function<GatedAttnFn> {
 };
 
 struct PairBiasFn : torch::autograd::Function<PairBiasFn> {
-  static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, int64_t H) {
+  static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw_, const Tensor& lb_, const Tensor& w_, int64_t H) {
     const c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous();
+    const Tensor x = x_.contiguous(), lw = lw_.contiguous(), lb = lb_.contiguous(), w = w_.contiguous();
     BiasSaved s;
     Tensor bias = bias_fwd(x, lw, lb, w, H, false, s);
     ctx->save_for_backward({x, lw, lb, w, s.mean, s.rstd});

@@ -1,0 +1,42 @@
+"""The Pairformer block's native functions in the forms its composed operators take."""
+import pytest
+import torch
+
+import megafold_b200 as mfb
+
+pytestmark = pytest.mark.gpu
+
+
+def make(L, dtype=torch.bfloat16, seed=3, **kw):
+    torch.manual_seed(seed)
+    block = mfb.PairformerBlock(device="cuda", dtype=dtype, **kw)
+    pair, single, d_pair, d_single = (torch.randn(*s, device="cuda").to(dtype) for s in ((L, L, 128), (L, 384)) * 2)
+    mask = torch.arange(L, device="cuda") < L - 2
+    return block, pair.requires_grad_(True), single.requires_grad_(True), mask, [d_pair, d_single]
+
+
+def go(block, pair, single, mask, d):
+    out = block(pair, single, mask)
+    return [*(o.detach() for o in out), *torch.autograd.grad(out, [pair, single, *block.parameters()], d)]
+
+
+def close(got, want, block, tol=1e-2):
+    """2e-3 is what a 16-bit rounding of each result leaves; the block chains about twenty of them."""
+    names = ["x", "s", "d_pair", "d_single", *(n for n, _ in block.named_parameters())]
+    for n, a, b in zip(names, got, want):
+        assert a.shape == b.shape, n
+        if not n.endswith("pair_ln_b"):      # 0 up to rounding errors (a softmax's logit gradients sum to 0): nothing to compare
+            assert float((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)) < tol, n
+
+
+def test_strided_parameters():
+    """Parameters held transposed or as slices of a wider array give what their contiguous copies give."""
+    block, *rest = make(40)
+    with torch.no_grad():
+        for p in block.parameters():      # none of them as the constructor leaves them, so that a wrong order shows
+            p.add_(0.1 * torch.randn_like(p))
+    want = go(block, *rest)
+    for p in block.parameters():
+        p.data = p.data.t().contiguous().t() if p.dim() == 2 else torch.stack([p.data, -p.data], 1)[:, 0]
+    assert not any(p.is_contiguous() for p in block.parameters()) and block._whole(rest[0], rest[1])
+    close(go(block, *rest), want, block)
