@@ -501,6 +501,10 @@ Attn contiguous(const Tensor& lw, const Tensor& lb, const Tensor& w, const Tenso
   return {lw.contiguous(), lb.contiguous(), w.contiguous(), b.contiguous(), w_out};
 }
 
+// The matrix products between the kernels compute in the type of their operands, whose memory the kernels then read: autocast
+// would change it, in a backward pass too that is run inside a region the forward pass was outside of.
+struct NoAutocast { const c10::impl::ExcludeDispatchKeyGuard guard{c10::DispatchKey::AutocastCUDA}; };
+
 mf_evo_layout token_layout(int64_t n, int64_t L, int64_t tok_o, int64_t tok_q, bool swap) {
   mf_evo_layout l{};
   for (int64_t* s : {l.o, l.d_o}) { s[0] = n * L * tok_o; s[1] = swap ? tok_o : L * tok_o; s[2] = swap ? L * tok_o : tok_o; }
@@ -526,6 +530,7 @@ void fill_attn(A& a, const Tensor& y, const Tensor& mask, const Tensor& bias, in
 struct AttnSaved { Tensor y, mean, rstd, o, lse, og; };
 // x [n, L, C] contiguous -> x + attention(x)
 Tensor attn_fwd(const Tensor& x, const Attn& p, const Tensor& mask, const Tensor& bias, int64_t H, bool swap, AttnSaved& s, int64_t lnl_flags) {
+  const NoAutocast no_autocast;
   const int64_t n = x.size(0), L = x.size(1), inner = p.w.size(1) / 4, D = inner / H;
   std::tie(s.y, s.mean, s.rstd) = lnl_fwd_raw(x, p.w, p.b, p.lw, p.lb, 1e-5, lnl_flags);
   s.o = at::empty({n, L, inner}, x.options());
@@ -550,6 +555,7 @@ struct AttnGrads { Tensor dx, dw, db, dlw, dlb, d_w_out, d_bias; };
 template <typename BiasDx>
 AttnGrads attn_bwd(const Tensor& d_out, const Tensor& x, const Attn& p, const Tensor& mask, const Tensor& bias, int64_t H, bool swap, const AttnSaved& s,
                    BiasDx bias_dx) {
+  const NoAutocast no_autocast;
   const int64_t n = x.size(0), L = x.size(1), C = x.size(2), inner = p.w.size(1) / 4, D = inner / H, P = n * L, es = x.element_size();
   AttnGrads g;
   const Tensor d2 = d_out.view({P, C});

@@ -40,3 +40,17 @@ def test_strided_parameters():
         p.data = p.data.t().contiguous().t() if p.dim() == 2 else torch.stack([p.data, -p.data], 1)[:, 0]
     assert not any(p.is_contiguous() for p in block.parameters()) and block._whole(rest[0], rest[1])
     close(go(block, *rest), want, block)
+
+
+@pytest.mark.parametrize("dtype,amp", [(torch.bfloat16, torch.float16), (torch.float32, torch.bfloat16)], ids=["bf16-in-fp16", "fp32-in-bf16"])
+def test_backward_inside_autocast(dtype, amp):
+    """Forward outside, backward inside an autocast region of another type: the values of a backward outside."""
+    block, pair, single, mask, d = make(40, dtype)
+    out = block(pair, single, mask)
+    assert block._whole(pair, single)
+    leaves = [pair, single, *block.parameters()]
+    want = torch.autograd.grad(out, leaves, d, retain_graph=True)
+    with torch.autocast("cuda", amp):
+        got = torch.autograd.grad(out, leaves, d)
+    assert all(a.dtype == b.dtype for a, b in zip(got, want))
+    close([*out, *got], [*out, *want], block, 1e-2 if dtype != torch.float32 else 1e-5)
