@@ -65,9 +65,15 @@ __global__ void __launch_bounds__(256) gate_bwd_kernel(const T* __restrict__ d, 
 // whole lines; `swap`: plane element (i, j) belongs to row j * L + i.  To rows: columns H .. np - 1 become zero.
 // VEC: rows of whole 16-byte pieces of 16-bit values are moved a piece at a time.  (A value at a time, with three divisions
 // each: 28 us for [768, 768, 8] and four heads, 8 to planes and 16 to rows now; the bytes take 2.)
+// A block takes a group of up to 32 columns, all of a projection but the widest: what the tile has room for in fp32.
+constexpr int kHeadGroup = 32;
 template <typename T, bool TO_ROWS, bool VEC>
-__global__ void __launch_bounds__(256) bias_layout_kernel(T* __restrict__ rows, T* __restrict__ planes, int L, int np, int H, bool swap) {
+__global__ void __launch_bounds__(256) bias_layout_kernel(T* __restrict__ rows, T* __restrict__ planes, int L, int np, int all_heads, bool swap) {
   extern __shared__ __align__(16) uint8_t raw[];
+  const int first = blockIdx.z * kHeadGroup;
+  const int cols = min(np - first, kHeadGroup), H = max(min(all_heads - first, kHeadGroup), 0);      // of my group
+  rows += first;
+  planes += (int64_t)first * L * L;
   T* tile = reinterpret_cast<T*>(raw);              // [H][32][33], plane order
   const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;      // plane coordinates
   auto move_rows = [&] {
@@ -76,7 +82,7 @@ __global__ void __launch_bounds__(256) bias_layout_kernel(T* __restrict__ rows, 
         const int c = e % 32, r = e / 32, i = swap ? c : r, j = swap ? r : c;
         if (i0 + i >= L || j0 + j >= L) continue;
         uint4* p = reinterpret_cast<uint4*>(rows + ((int64_t)(swap ? j0 + j : i0 + i) * L + (swap ? i0 + i : j0 + j)) * np);
-        for (int h0 = 0; h0 < np; h0 += 8) {
+        for (int h0 = 0; h0 < cols; h0 += 8) {
           Vec8<T> v;
           if (!TO_ROWS) *reinterpret_cast<uint4*>(v.e) = p[h0 / 8];
 #pragma unroll
@@ -89,8 +95,8 @@ __global__ void __launch_bounds__(256) bias_layout_kernel(T* __restrict__ rows, 
       }
       return;
     }
-    for (int e = threadIdx.x; e < 32 * 32 * np; e += 256) {
-      const int h = e % np, c = e / np % 32, r = e / np / 32;      // row block r, column c of it, in the order of memory
+    for (int e = threadIdx.x; e < 32 * 32 * cols; e += 256) {
+      const int h = e % cols, c = e / cols % 32, r = e / cols / 32;      // row block r, column c of it, in the order of memory
       const int i = swap ? c : r, j = swap ? r : c;
       if (i0 + i >= L || j0 + j >= L) continue;
       T* p = rows + ((int64_t)(swap ? j0 + j : i0 + i) * L + (swap ? i0 + i : j0 + j)) * np + h;
@@ -145,10 +151,10 @@ int gate_bwd(const void* d, const void* o, const void* g, int64_t gs, void* d_o,
 }
 
 int bias_layout(void* rows, void* planes, int L, int np, int H, bool swap, bool to_rows, int dtype, cudaStream_t st) {
-  MF_REQUIRE(np <= 44 && H <= np, MF_ERR_UNSUPPORTED, "pair-bias rows of %d columns for %d heads", np, H);
-  const dim3 grid((L + 31) / 32, (L + 31) / 32);
+  MF_REQUIRE(H <= np, MF_ERR_UNSUPPORTED, "pair-bias rows of %d columns for %d heads", np, H);
+  const dim3 grid((L + 31) / 32, (L + 31) / 32, (np + kHeadGroup - 1) / kHeadGroup);
   MF_DISPATCH_FLOAT(dtype, T, {
-    const size_t smem = sizeof(T) * (size_t)H * 32 * 33;
+    const size_t smem = sizeof(T) * (size_t)(H < kHeadGroup ? H : kHeadGroup) * 32 * 33;
     auto launch = [&](auto to, auto vec) -> int {
       constexpr auto kern = bias_layout_kernel<T, decltype(to)::value, decltype(vec)::value>;
       if (int e = opt_in_smem<kern>(smem)) return e;

@@ -48,9 +48,22 @@ def test_backward_inside_autocast(dtype, amp):
     block, pair, single, mask, d = make(40, dtype)
     out = block(pair, single, mask)
     assert block._whole(pair, single)
+    values = [o.detach() for o in out]
     leaves = [pair, single, *block.parameters()]
     want = torch.autograd.grad(out, leaves, d, retain_graph=True)
     with torch.autocast("cuda", amp):
         got = torch.autograd.grad(out, leaves, d)
     assert all(a.dtype == b.dtype for a, b in zip(got, want))
-    close([*out, *got], [*out, *want], block, 1e-2 if dtype != torch.float32 else 1e-5)
+    close([*values, *got], [*values, *want], block, 1e-2 if dtype != torch.float32 else 1e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,dim_head", [(48, 8), (33, 8), (32, 16)])
+def test_many_heads(heads, dim_head, dtype):
+    """More heads than one group of the pair-bias re-layout takes, against the composed operators."""
+    from megafold_b200.pairformer_block import cuda_ops
+    block, *rest = make(36, dtype, single_heads=heads, single_dim_head=dim_head, tri_heads=heads, tri_dim_head=dim_head)
+    assert block._whole(rest[0], rest[1])
+    got = go(block, *rest)
+    block.native_ok, block.ops = False, cuda_ops()
+    close(got, go(block, *rest), block, 1e-2 if dtype != torch.float32 else 1e-4)
