@@ -404,7 +404,8 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       }
     }
     const float m_new = fmaxf(fmaxf(m, fmaxf(mx4[0], mx4[1])), fmaxf(mx4[2], mx4[3]));
-    const float corr = ex2f(m - m_new);
+    const float m_ref = m_new == -INFINITY ? 0.f : m_new;      // every logit so far is -inf (a mask or bias of -inf): no NaN yet
+    const float corr = ex2f(m - m_ref);
     // ------------------------------------------------------------------ fold O_tile(g-1), then P(g)
     if (t > 0) {
       wait_or_flag(&bar.pv_done, (g - 1) & 1, abort_flag);
@@ -416,8 +417,8 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       uint32_t pk[32];
 #pragma unroll
       for (int jj = 0; jj < 32; ++jj) {
-        const float p0 = ex2f(__uint_as_float(sr[cb * 64 + 2 * jj]) - m_new);
-        const float p1 = ex2f(__uint_as_float(sr[cb * 64 + 2 * jj + 1]) - m_new);
+        const float p0 = ex2f(__uint_as_float(sr[cb * 64 + 2 * jj]) - m_ref);
+        const float p1 = ex2f(__uint_as_float(sr[cb * 64 + 2 * jj + 1]) - m_ref);
         rs4[jj & 3] += p0 + p1;
         pk[jj] = Pack2<T>::pack(p0, p1);
       }
