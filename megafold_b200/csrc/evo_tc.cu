@@ -1,5 +1,7 @@
 // Host-side support shared by the tensor-core attention kernels: status word, device queries and the
 // test that decides whether a call can take the tensor-core path.
+#include <type_traits>
+
 #include "evo_tc_common.cuh"
 
 namespace mf {
@@ -40,6 +42,15 @@ namespace {
 // where the source allows it reads 16-byte pieces too, otherwise element by element (neighbouring threads read
 // neighbouring pieces, so the lines are shared).  Bound: HBM, and at crop sizes latency: [4, 467, 467] bf16 (1.7 MB) takes
 // 3 us, against 1000 us more in the general attention kernel that reads such a bias in place.
+//
+// The kernels that read the copy add it by a product with a multiple of the identity, where an infinite value times 0 would
+// make its neighbours NaN.  So infinities (and fp32 values beyond the range of the copy) become the largest value that stays
+// finite there: probability 0 for -inf, as it should be.
+template <typename TO>
+__device__ __forceinline__ TO bounded(float v) {
+  constexpr float lim = std::is_same_v<TO, __half> ? 65504.f : -tcx::kMinusBig;
+  return from_f<TO>(v < -lim ? -lim : v > lim ? lim : v);      // NaN stays
+}
 template <typename TB, typename TO>
 __global__ void __launch_bounds__(256) copy_bias_rows_kernel(const TB* __restrict__ bias, TO* __restrict__ dst, int64_t pieces, int L, int per_row, int H,
                                                              int64_t sb, int64_t sh, int64_t si, int64_t sj, bool vec) {
@@ -56,10 +67,10 @@ __global__ void __launch_bounds__(256) copy_bias_rows_kernel(const TB* __restric
 #pragma unroll
     for (int k = 0; k < (int)(8 * sizeof(TB) / 16); ++k) reinterpret_cast<uint4*>(in)[k] = __ldg(reinterpret_cast<const uint4*>(src) + k);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) out[k] = from_f<TO>(to_f(in[k]));
+    for (int k = 0; k < 8; ++k) out[k] = bounded<TO>(to_f(in[k]));
   } else {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) out[k] = from_f<TO>(j0 + k < L ? to_f(src[k * sj]) : 0.f);
+    for (int k = 0; k < 8; ++k) out[k] = bounded<TO>(j0 + k < L ? to_f(src[k * sj]) : 0.f);
   }
   *reinterpret_cast<uint4*>(dst + q * 8) = *reinterpret_cast<const uint4*>(out);
 }
