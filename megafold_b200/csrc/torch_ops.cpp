@@ -11,7 +11,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include <torch/extension.h>
+#include <ATen/FuncTorchTLS.h>
 #include <ATen/autocast_mode.h>
+#include <c10/core/AutogradState.h>
 
 #include <array>
 #include <optional>
@@ -98,6 +100,16 @@ void require_cuda(std::initializer_list<const Tensor*> ts) {
   for (const Tensor* t : ts)
     TORCH_CHECK(!t->defined() || t->is_cuda(),
                 "megafold_b200 operators run on CUDA tensors only (there is no CPU path); got a tensor on ", t->device());
+}
+
+// Forward-mode differentiation and torch.func transforms are refused by the autograd functions, which have no rule for them; a
+// call that goes past these because gradients are off must not drop a tangent either.
+void refuse_transforms(std::initializer_list<const Tensor*> ts) {
+  if (const auto& tls = at::functorch::functorchTLSAccessor()) tls->checkSupportsCppAutogradFunction();
+  if (!c10::AutogradState::get_tls_state().get_fw_grad_mode()) return;
+  for (const Tensor* t : ts)
+    TORCH_CHECK_NOT_IMPLEMENTED(!t->defined() || !t->unsafeGetTensorImpl()->_fw_grad(0, *t).defined(),
+                                "megafold_b200 operators do not support forward-mode differentiation");
 }
 
 Tensor workspace(size_t bytes, const Tensor& like) {
@@ -226,8 +238,11 @@ struct EvoFn : torch::autograd::Function<EvoFn> {
 };
 
 Tensor evo_attention(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask, const OptTensor& bias) {
-  if (!at::GradMode::is_enabled()) return std::get<0>(evo_forward(q, k, v, mask, bias, 0));
   const Tensor m = or_none(mask), b = or_none(bias);
+  if (!at::GradMode::is_enabled()) {
+    refuse_transforms({&q, &k, &v, &m, &b});
+    return std::get<0>(evo_forward(q, k, v, mask, bias, 0));
+  }
   require_cuda({&q, &k, &v, &m, &b});
   check_shapes(q, k, v, mask, bias);
   return EvoFn::apply(q, k, v, m, b);
@@ -334,6 +349,7 @@ Tensor lnl(const Tensor& x, const Tensor& w, const OptTensor& b, const Tensor& l
   require_cuda({&x, &w, &bt, &lw, &lbt});
   TORCH_CHECK_VALUE(w.dim() == 2 && x.dim() >= 1 && w.size(0) == x.size(-1), "Incompatible dimensions");
   if (!at::GradMode::is_enabled()) {
+    refuse_transforms({&x, &w, &bt, &lw, &lbt});
     const bool on = autocast_on();
     Tensor xc = x, wc = w, bc = bt, lwc = lw, lbc = lbt;
     const c10::cuda::CUDAGuard guard(x.device());
@@ -476,6 +492,7 @@ Tensor transition(const Tensor& x, const OptTensor& lw, const OptTensor& lb, con
   require_cuda({&x, &lwt, &lbt, &w1, &w2});
   check_transition(x, w1, w2);
   if (!at::GradMode::is_enabled()) {
+    refuse_transforms({&x, &lwt, &lbt, &w1, &w2});
     const auto dt = amp_type(x, autocast_on());
     Tensor xc = x, lwc = lwt, lbc = lbt, w1c = w1, w2c = w2;
     const c10::cuda::CUDAGuard guard(x.device());

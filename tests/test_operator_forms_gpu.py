@@ -1,0 +1,29 @@
+"""The operators under torch's transforms and on unusual forms of their arguments: refused, or the plain call's values."""
+import pytest
+import torch
+import torch.autograd.forward_ad as fwAD
+
+import megafold_b200 as mfb
+
+pytestmark = pytest.mark.gpu
+
+
+def calls():
+    """name -> (function of one tensor, that tensor)"""
+    r = lambda *s: torch.randn(*s, device="cuda")      # noqa: E731
+    k, bias, mask = r(1, 2, 24, 2, 16), r(1, 1, 2, 24, 24), torch.ones(1, 2, 1, 1, 24, dtype=torch.bool, device="cuda")
+    lnl, tr, sw = mfb.LayernormLinear(32, 24, device="cuda"), mfb.FusedTransition(32, device="cuda"), mfb.FusedSwiGLU()
+    return {"attention": (lambda q: mfb.TritonEvoformer(q, k, k, mask, bias), r(1, 2, 24, 2, 16)), "lnl": (lnl, r(6, 32)), "transition": (tr, r(6, 32)),
+            "swiglu": (sw, r(6, 32))}
+
+
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("name", ["attention", "lnl", "transition", "swiglu"])
+def test_transforms_are_refused(name, grad):
+    f, x = calls()[name]
+    with torch.set_grad_enabled(grad):
+        with fwAD.dual_level(), pytest.raises(RuntimeError):
+            f(fwAD.make_dual(x, torch.ones_like(x)))
+        with pytest.raises(RuntimeError):
+            torch.func.vmap(f)(torch.stack([x, x]))
+        f(x)
