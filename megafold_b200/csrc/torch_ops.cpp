@@ -119,6 +119,9 @@ Tensor empty_f32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(s
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 Tensor or_none(const OptTensor& t) { return t ? *t : Tensor(); }
 
+// The values themselves where a negation is still pending (the imaginary part of a conjugate, say): kernels read memory.
+Tensor plain(const Tensor& t) { return t.defined() && t.is_neg() ? t.resolve_neg() : t; }
+
 // ---- conversions -------------------------------------------------------------------------------------------------
 // Brings each tensor to its wanted type (and to contiguous memory), all of them in one launch: mixed-precision calls
 // convert four to six small parameters at once, where a launch each costs more than the conversion.
@@ -130,6 +133,7 @@ void cast_batch(std::initializer_list<Cast> list) {
   Tensor any;
   for (const Cast& c : list) {
     if (!c.t->defined()) continue;
+    *c.t = plain(*c.t);
     if (!c.t->is_contiguous()) *c.t = c.t->contiguous();
     if (c.t->scalar_type() == c.to) continue;
     const auto from = c.t->scalar_type();
@@ -182,8 +186,8 @@ void fill_common(A& a, const Tensor& q, const Tensor& k, const Tensor& v, const 
   a.bias_strides[0] = step(bias, 0, a.B); a.bias_strides[1] = bias.stride(2); a.bias_strides[2] = bias.stride(3); a.bias_strides[3] = bias.stride(4);
 }
 
-std::tuple<Tensor, Tensor> evo_forward(const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask_, const OptTensor& bias_, int64_t flags) {
-  const Tensor mask = or_none(mask_), bias = or_none(bias_);
+std::tuple<Tensor, Tensor> evo_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& mask_, const OptTensor& bias_, int64_t flags) {
+  const Tensor q = plain(q_), k = plain(k_), v = plain(v_), mask = plain(or_none(mask_)), bias = plain(or_none(bias_));
   require_cuda({&q, &k, &v, &mask, &bias});
   const auto s = check_shapes(q, k, v, mask_, bias_);
   const c10::cuda::CUDAGuard guard(q.device());
@@ -199,13 +203,13 @@ std::tuple<Tensor, Tensor> evo_forward(const Tensor& q, const Tensor& k, const T
   return {o, lse};
 }
 
-std::tuple<Tensor, Tensor, Tensor, Tensor> evo_backward(const Tensor& d_o_, const Tensor& q, const Tensor& k, const Tensor& v, const OptTensor& mask_,
+std::tuple<Tensor, Tensor, Tensor, Tensor> evo_backward(const Tensor& d_o_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& mask_,
                                                         const OptTensor& bias_, const Tensor& o_, const Tensor& lse, int64_t flags, int64_t event) {
-  const Tensor mask = or_none(mask_), bias = or_none(bias_);
+  const Tensor q = plain(q_), k = plain(k_), v = plain(v_), mask = plain(or_none(mask_)), bias = plain(or_none(bias_));
   require_cuda({&d_o_, &q, &k, &v, &mask, &bias, &o_, &lse});
   const auto s = check_shapes(q, k, v, mask_, bias_);
   const c10::cuda::CUDAGuard guard(q.device());
-  const Tensor d_o = d_o_.contiguous(), o = o_.contiguous();
+  const Tensor d_o = plain(d_o_).contiguous(), o = plain(o_).contiguous();
   Tensor dq = at::empty({s[0], s[1], s[2], s[3], s[4]}, q.options()), dk = at::empty_like(dq), dv = at::empty_like(dq);
   const auto bt = bias.scalar_type();
   Tensor d_bias = at::empty({s[0], 1, s[3], s[2], s[2]}, q.options().dtype(bt == q.scalar_type() ? bt : at::kFloat));
@@ -515,7 +519,7 @@ struct Attn { Tensor lw, lb, w, b, w_out; };
 // The kernels take the parameters as contiguous arrays (only w_out is multiplied by torch, on strides): a transposed or
 // otherwise strided parameter is copied.
 Attn contiguous(const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out) {
-  return {lw.contiguous(), lb.contiguous(), w.contiguous(), b.contiguous(), w_out};
+  return {plain(lw).contiguous(), plain(lb).contiguous(), plain(w).contiguous(), plain(b).contiguous(), w_out};
 }
 
 // The matrix products between the kernels compute in the type of their operands, whose memory the kernels then read: autocast
@@ -631,7 +635,7 @@ struct TriangleFn : torch::autograd::Function<TriangleFn> {
   static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out,
                           const Tensor& plw_, const Tensor& plb_, const Tensor& pw_, const Tensor& mask, int64_t H, bool swap) {
     const c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous(), plw = plw_.contiguous(), plb = plb_.contiguous(), pw = pw_.contiguous();
+    const Tensor x = plain(x_).contiguous(), plw = plain(plw_).contiguous(), plb = plain(plb_).contiguous(), pw = plain(pw_).contiguous();
     const Attn p = contiguous(lw, lb, w, b, w_out);
     AttnSaved s; BiasSaved bs;
     const Tensor bias = bias_fwd(x, plw, plb, pw, H, swap, bs);
@@ -648,7 +652,7 @@ struct TriangleFn : torch::autograd::Function<TriangleFn> {
     const bool swap = ctx->saved_data["swap"].toBool();
     const AttnSaved s{v[11], v[12], v[13], v[14], v[15], v[16]};
     std::array<Tensor, 4> p;
-    AttnGrads a = attn_bwd(g[0].contiguous(), v[0], {v[1], v[2], v[3], v[4], v[5]}, v[9], v[10], H, swap, s, [&](const Tensor& d_bias) {
+    AttnGrads a = attn_bwd(plain(g[0]).contiguous(), v[0], {v[1], v[2], v[3], v[4], v[5]}, v[9], v[10], H, swap, s, [&](const Tensor& d_bias) {
       p = bias_bwd(d_bias, v[0], v[6], v[7], v[8], swap, BiasSaved{v[17], v[18]});
       return p[0];
     });
@@ -661,7 +665,7 @@ struct GatedAttnFn : torch::autograd::Function<GatedAttnFn> {
   static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw, const Tensor& lb, const Tensor& w, const Tensor& b, const Tensor& w_out,
                           const Tensor& mask, const Tensor& bias, int64_t H) {
     const c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous();
+    const Tensor x = plain(x_).contiguous();
     const Attn p = contiguous(lw, lb, w, b, w_out);
     AttnSaved s;
     // the projection of these few wide rows keeps fp32 operands and sums (0.4 % of a block at 768 tokens): its values too
@@ -676,7 +680,7 @@ struct GatedAttnFn : torch::autograd::Function<GatedAttnFn> {
     const auto v = ctx->get_saved_variables();
     const c10::cuda::CUDAGuard guard(v[0].device());
     const AttnSaved s{v[8], v[9], v[10], v[11], v[12], v[13]};
-    AttnGrads a = attn_bwd(g[0].contiguous(), v[0], {v[1], v[2], v[3], v[4], v[5]}, v[6], v[7], ctx->saved_data["H"].toInt(), false, s,
+    AttnGrads a = attn_bwd(plain(g[0]).contiguous(), v[0], {v[1], v[2], v[3], v[4], v[5]}, v[6], v[7], ctx->saved_data["H"].toInt(), false, s,
                            [](const Tensor&) { return Tensor(); });
     return {a.dx, a.dlw, a.dlb, a.dw, a.db, a.d_w_out, Tensor(), a.d_bias, Tensor()};
   }
@@ -685,7 +689,7 @@ struct GatedAttnFn : torch::autograd::Function<GatedAttnFn> {
 struct PairBiasFn : torch::autograd::Function<PairBiasFn> {
   static Variable forward(AutogradContext* ctx, const Tensor& x_, const Tensor& lw_, const Tensor& lb_, const Tensor& w_, int64_t H) {
     const c10::cuda::CUDAGuard guard(x_.device());
-    const Tensor x = x_.contiguous(), lw = lw_.contiguous(), lb = lb_.contiguous(), w = w_.contiguous();
+    const Tensor x = plain(x_).contiguous(), lw = plain(lw_).contiguous(), lb = plain(lb_).contiguous(), w = plain(w_).contiguous();
     BiasSaved s;
     Tensor bias = bias_fwd(x, lw, lb, w, H, false, s);
     ctx->save_for_backward({x, lw, lb, w, s.mean, s.rstd});
@@ -695,7 +699,7 @@ struct PairBiasFn : torch::autograd::Function<PairBiasFn> {
     at::NoGradGuard no_grad;
     const auto v = ctx->get_saved_variables();
     const c10::cuda::CUDAGuard guard(v[0].device());
-    auto p = bias_bwd(g[0].contiguous(), v[0], v[1], v[2], v[3], false, BiasSaved{v[4], v[5]});
+    auto p = bias_bwd(plain(g[0]).contiguous(), v[0], v[1], v[2], v[3], false, BiasSaved{v[4], v[5]});
     return {p[0], p[2], p[3], p[1], Tensor()};
   }
 };

@@ -27,3 +27,17 @@ def test_transforms_are_refused(name, grad):
         with pytest.raises(RuntimeError):
             torch.func.vmap(f)(torch.stack([x, x]))
         f(x)
+
+
+@pytest.mark.parametrize("amp", [False, True])
+@pytest.mark.parametrize("grad", [True, False])
+@pytest.mark.parametrize("name", ["attention", "lnl", "transition", "swiglu"])
+def test_pending_negation(name, grad, amp):
+    """An argument whose sign has not been written to memory yet, with and without a conversion on the way."""
+    if name == "attention" and amp:
+        pytest.skip("takes its types as they are")
+    f, x = calls()[name]
+    lazy = torch._neg_view(x)
+    assert lazy.is_neg()
+    with torch.set_grad_enabled(grad), torch.autocast("cuda", torch.bfloat16, enabled=amp):
+        assert torch.equal(f(lazy), f(-x))
