@@ -300,9 +300,19 @@ std::tuple<Tensor, Tensor, Tensor> lnl_forward(const Tensor& x_, const Tensor& w
   return lnl_fwd_raw(x, w, b, lw, lb, eps, flags);
 }
 
+// The kernels read M x N values of dy, in whatever shape they come, and M of each row statistic.
+void check_gradient(const Tensor& dy, int64_t M, int64_t N, const Tensor& mean, const Tensor& rstd) {
+  TORCH_CHECK_VALUE(dy.numel() == M * N, "the gradient must hold ", M, " x ", N, " values, got ", shape(dy));
+  TORCH_CHECK_VALUE(mean.numel() == M && rstd.numel() == M && mean.is_contiguous() && rstd.is_contiguous(), "mean and rstd must hold a value for each of the ", M,
+                    " rows, got ", shape(mean), " and ", shape(rstd));
+}
+
 std::array<Tensor, 5> lnl_backward(const Tensor& dy_, const Tensor& x_, const Tensor& w_, const Tensor& lw_, const OptTensor& lb_, const Tensor& mean,
                                    const Tensor& rstd, bool has_linear_bias, int64_t flags) {
   Tensor dy = dy_, x = x_, w = w_, lw = lw_, lb = or_none(lb_);
+  require_cuda({&dy, &x, &w, &lw, &lb, &mean, &rstd});
+  TORCH_CHECK_VALUE(w.dim() == 2 && x.dim() >= 1 && w.size(0) == x.size(-1), "Incompatible dimensions");
+  check_gradient(dy, rows_of(x), w.size(1), mean, rstd);
   const c10::cuda::CUDAGuard guard(x.device());
   const auto dt = x.scalar_type();
   cast_batch({{&x, dt}, {&dy, dt}, {&w, dt}, {&lw, dt}, {&lb, dt}});
@@ -461,6 +471,9 @@ std::tuple<Tensor, Tensor, Tensor> transition_forward(const Tensor& x_, const Op
 std::array<Tensor, 5> transition_backward(const Tensor& dy_, const Tensor& x_, const OptTensor& lw_, const OptTensor& lb_, const Tensor& w1_,
                                           const Tensor& w2_, const Tensor& mean, const Tensor& rstd, int64_t flags) {
   Tensor dy = dy_, x = x_, lw = or_none(lw_), lb = or_none(lb_), w1 = w1_, w2 = w2_;
+  require_cuda({&dy, &x, &lw, &lb, &w1, &w2, &mean, &rstd});
+  check_transition(x, w1, w2);
+  check_gradient(dy, rows_of(x), x.size(-1), mean, rstd);
   const c10::cuda::CUDAGuard guard(x.device());
   const auto dt = x.scalar_type();
   cast_batch({{&x, dt}, {&dy, dt}, {&lw, dt}, {&lb, dt}, {&w1, dt}, {&w2, dt}});

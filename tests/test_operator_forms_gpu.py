@@ -41,3 +41,20 @@ def test_pending_negation(name, grad, amp):
     assert lazy.is_neg()
     with torch.set_grad_enabled(grad), torch.autocast("cuda", torch.bfloat16, enabled=amp):
         assert torch.equal(f(lazy), f(-x))
+
+
+def test_backward_functions_refuse_gradients_of_another_size():
+    """What the reshape of dy to the rows of x refused, and sizes that would be read out of range."""
+    r = lambda *s: torch.randn(*s, device="cuda")      # noqa: E731
+    x, w, lw, w2 = r(2, 3, 32), r(32, 64), r(32), r(32, 32)
+    mean, rstd = r(6), r(6)
+    f = lambda dy, m=mean, w=w: mfb.layernorm_linear_backward(dy, x, w, lw, None, m, rstd, False)      # noqa: E731
+    g = lambda dy, m=mean, w=w: mfb.transition_backward(dy, x, lw, None, w, w2, m, rstd)      # noqa: E731
+    for call, n in ((f, 64), (g, 32)):
+        call(r(6, n))
+        call(r(2, 3, n))
+        for bad in (dict(dy=r(5, n)), dict(dy=r(6, n - 1)), dict(dy=r(6, n), m=r(5)), dict(dy=r(6, n), w=r(31, 64))):
+            with pytest.raises(ValueError):
+                call(**bad)
+        with pytest.raises(RuntimeError):
+            call(r(6, n).cpu())
