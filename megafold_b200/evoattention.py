@@ -75,8 +75,22 @@ def TritonEvoformer(Q, K, V, res_mask, pair_bias):
     return _lib.native().evo_attention(Q, K, V, res_mask, pair_bias)
 
 
-class EvoformerAttention:
-    """The operator under the reference's class name: ``EvoformerAttention.apply`` is ``TritonEvoformer``.  The autograd
-    function behind it is native (csrc/torch_ops.cpp)."""
+class EvoformerAttention(torch.autograd.Function):
+    """The operator under the reference's class name: ``EvoformerAttention.apply`` is ``TritonEvoformer``, whose autograd
+    function is native (csrc/torch_ops.cpp).  ``forward`` and ``backward`` are its two halves, for subclasses."""
 
-    apply = staticmethod(TritonEvoformer)
+    @staticmethod
+    def forward(ctx, Q, K, V, res_mask, pair_bias):
+        o, lse = evo_attention_forward(Q, K, V, res_mask, pair_bias)
+        ctx.save_for_backward(Q, K, V, res_mask, pair_bias, o, lse)
+        return o
+
+    @staticmethod
+    def backward(ctx, dO):
+        Q, K, V, res_mask, pair_bias, o, lse = ctx.saved_tensors
+        dq, dk, dv, d_bias = evo_attention_backward(dO, Q, K, V, res_mask, pair_bias, o, lse)
+        return dq, dk, dv, None, d_bias
+
+    @classmethod
+    def apply(cls, *args):
+        return TritonEvoformer(*args) if cls is EvoformerAttention else super().apply(*args)

@@ -28,14 +28,33 @@ def layernorm_linear_backward(dy, x, linear_weight, ln_weight, ln_bias, mean, rs
     return tuple(_lib.native().lnl_backward(dy, x, linear_weight, ln_weight, ln_bias, mean, rstd, has_linear_bias, flags))
 
 
-class LayernormLinearFunction:
+class LayernormLinearFunction(torch.autograd.Function):
     """``apply(X, linear_weight, linear_bias, WEIGHT, BIAS, has_layernorm_bias, has_linear_bias,
     supported_configs)``; the last argument (the reference's Triton tile configs) is ignored.  Under autocast the
     operands are converted to bf16, as the reference's ``custom_fwd(cast_inputs=torch.bfloat16)`` does; the gradients
-    come back in the types of the arguments.  The autograd function is native (csrc/torch_ops.cpp)."""
+    come back in the types of the arguments.  The autograd function is native (csrc/torch_ops.cpp); ``forward`` and
+    ``backward`` are its two halves, for subclasses."""
 
     @staticmethod
-    def apply(X, linear_weight, linear_bias, WEIGHT, BIAS, has_layernorm_bias=True, has_linear_bias=False, supported_configs=None):
+    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    def forward(ctx, X, linear_weight, linear_bias, WEIGHT, BIAS, has_layernorm_bias=True, has_linear_bias=False, supported_configs=None):
+        ln_b, lin_b = BIAS if has_layernorm_bias else None, linear_bias if has_linear_bias else None
+        y, mean, rstd = layernorm_linear_forward(X, linear_weight, lin_b, WEIGHT, ln_b)
+        ctx.save_for_backward(X, linear_weight, lin_b, WEIGHT, ln_b, mean, rstd)
+        return y
+
+    @staticmethod
+    @torch.amp.custom_bwd(device_type="cuda")
+    def backward(ctx, dOUT):
+        X, w, b, ln_w, ln_b, mean, rstd = ctx.saved_tensors
+        dx, dw, db, d_ln_w, d_ln_b = layernorm_linear_backward(dOUT, X, w, ln_w, ln_b, mean, rstd, b is not None)
+        grads = (g if g is None else g.to(t.dtype) for g, t in ((dx, X), (dw, w), (db, b), (d_ln_w, ln_w), (d_ln_b, ln_b)))
+        return (*grads, None, None, None)
+
+    @classmethod
+    def apply(cls, X, linear_weight, linear_bias, WEIGHT, BIAS, has_layernorm_bias=True, has_linear_bias=False, supported_configs=None):
+        if cls is not LayernormLinearFunction:
+            return super().apply(X, linear_weight, linear_bias, WEIGHT, BIAS, has_layernorm_bias, has_linear_bias, supported_configs)
         return _lib.native().lnl(X, linear_weight, linear_bias if has_linear_bias else None, WEIGHT, BIAS if has_layernorm_bias else None)
 
 

@@ -10,6 +10,7 @@ overwrites its saved input, :49-52).
 """
 from __future__ import annotations
 
+import torch
 from torch import nn
 
 from . import _lib
@@ -19,12 +20,27 @@ __all__ = ["FusedSwiGLUFunction", "FusedSwiGLU", "FusedTransition", "TransitionF
            "transition_forward", "transition_backward"]
 
 
-class FusedSwiGLUFunction:
-    """``apply(x [..., 2 * inner])``; the autograd function is native (csrc/torch_ops.cpp)."""
+class FusedSwiGLUFunction(torch.autograd.Function):
+    """``apply(x [..., 2 * inner])``; the autograd function is native (csrc/torch_ops.cpp).  ``forward`` and ``backward``
+    are its two halves, for subclasses."""
 
     @staticmethod
-    def apply(input):
+    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    def forward(ctx, input):
+        ctx.save_for_backward(input)
         return _lib.native().swiglu(input)
+
+    @staticmethod
+    @torch.amp.custom_bwd(device_type="cuda")
+    def backward(ctx, grad_output):
+        x = ctx.saved_tensors[0].detach().requires_grad_(True)
+        with torch.enable_grad():
+            y = _lib.native().swiglu(x)
+        return torch.autograd.grad(y, x, grad_output.to(y.dtype))[0]
+
+    @classmethod
+    def apply(cls, input):
+        return _lib.native().swiglu(input) if cls is FusedSwiGLUFunction else super().apply(input)
 
 
 class FusedSwiGLU(nn.Module):
@@ -42,12 +58,28 @@ def transition_backward(dy, x, ln_weight, ln_bias, w1, w2, mean, rstd, flags: in
     return tuple(_lib.native().transition_backward(dy, x, ln_weight, ln_bias, w1, w2, mean, rstd, flags))
 
 
-class TransitionFunction:
+class TransitionFunction(torch.autograd.Function):
     """``apply(x, ln_weight | None, ln_bias | None, w1 [dim, 2*inner], w2 [dim, inner])``; the autograd function is native
-    (csrc/torch_ops.cpp)."""
+    (csrc/torch_ops.cpp).  ``forward`` and ``backward`` are its two halves, for subclasses."""
 
     @staticmethod
-    def apply(x, ln_weight, ln_bias, w1, w2):
+    @torch.amp.custom_fwd(device_type="cuda", cast_inputs=torch.bfloat16)
+    def forward(ctx, x, ln_weight, ln_bias, w1, w2):
+        y, mean, rstd = transition_forward(x, ln_weight, ln_bias, w1, w2)
+        ctx.save_for_backward(x, ln_weight, ln_bias, w1, w2, mean, rstd)
+        return y
+
+    @staticmethod
+    @torch.amp.custom_bwd(device_type="cuda")
+    def backward(ctx, dy):
+        x, ln_weight, ln_bias, w1, w2, mean, rstd = ctx.saved_tensors
+        grads = transition_backward(dy, x, ln_weight, ln_bias, w1, w2, mean, rstd)
+        return tuple(g if g is None else g.to(t.dtype) for g, t in zip(grads, (x, ln_weight, ln_bias, w1, w2)))
+
+    @classmethod
+    def apply(cls, x, ln_weight, ln_bias, w1, w2):
+        if cls is not TransitionFunction:
+            return super().apply(x, ln_weight, ln_bias, w1, w2)
         return _lib.native().transition(x, ln_weight, ln_bias, w1, w2)
 
 

@@ -88,3 +88,10 @@ def test_row_sharded_bias_gradient_is_all_reduced(tmp_path):
         torch.testing.assert_close(got["o"], o[:, s:e], rtol=1e-5, atol=1e-6)
         torch.testing.assert_close(got["dq"], dq[:, s:e], rtol=1e-5, atol=1e-6)
         torch.testing.assert_close(got["dbias"], db, rtol=1e-5, atol=1e-5)     # full sum on every rank
+
+
+def test_operator_classes_are_autograd_functions():
+    from megafold_b200.fused_transition import TransitionFunction
+    for cls in (mfb.EvoformerAttention, mfb.LayernormLinearFunction, mfb.FusedSwiGLUFunction, TransitionFunction):
+        assert issubclass(cls, torch.autograd.Function)
+        assert all(callable(getattr(cls, n)) for n in ("forward", "backward", "apply"))
