@@ -158,11 +158,14 @@ class _Attn(nn.Module):
 
 
 class PairformerBlock(nn.Module):
+    native_ok = True           # False: always composed from the operators
+    _default_ops = None        # what the block put into ``ops`` itself: other operators are injected ones
+
     def __init__(self, dim_pair=128, dim_single=384, tri_heads=4, tri_dim_head=32, single_heads=16, single_dim_head=24,
                  expansion=4, group=None, ops=None, device=None, dtype=None):
         super().__init__()
         kw = dict(device=device, dtype=dtype)
-        self.group, self.ops, self.native_ok = group, ops, ops is None
+        self.group, self.ops = group, ops
         self.tri_start = _Attn(dim_pair, tri_heads, tri_dim_head, dim_pair, **kw)
         self.tri_end = _Attn(dim_pair, tri_heads, tri_dim_head, dim_pair, **kw)
         self.single_attn = _Attn(dim_single, single_heads, single_dim_head, dim_pair, **kw)
@@ -195,14 +198,14 @@ class PairformerBlock(nn.Module):
         """One GPU holds all rows and everything has one type: the attentions run as single native functions (projection,
         attention, gate, output projection, residual; csrc/torch_ops.cpp), the ending-node one on strides instead of a
         transposed copy.  Otherwise, and with injected operators, they are composed from the pieces above."""
-        return (self.native_ok and _world(self.group) == 1 and x.is_cuda and x.shape[0] == x.shape[1] and not torch.is_autocast_enabled("cuda")
+        return (self.native_ok and self.ops is self._default_ops and _world(self.group) == 1 and x.is_cuda and x.shape[0] == x.shape[1] and not torch.is_autocast_enabled("cuda")
                 and all(t.dtype == x.dtype for t in (single, *self.parameters()))
                 and all(a.inner % 8 == 0 for a in (self.tri_start, self.tri_end, self.single_attn)))
 
     def _forward_whole(self, x, single, mask):
         from . import _lib
         native = _lib.native()
-        mask = mask.contiguous()
+        mask = mask.view(x.shape[1]).contiguous()
         for a, swap in ((self.tri_start, False), (self.tri_end, True)):
             x = native.triangle(x, a.ln_w, a.ln_b, a.w_qkvg, a.b_qkvg, a.w_out, a.pair_ln_w, a.pair_ln_b, a.w_pair_bias, mask, a.heads, swap)
         x = x + native.transition(x, self.tr_ln_w, self.tr_ln_b, self.tr_w1, self.tr_w2)
@@ -214,7 +217,7 @@ class PairformerBlock(nn.Module):
     def forward(self, pair_rows, single, mask):
         """pair_rows [n_local, L, dim_pair] (this rank's rows), single [L, dim_single] (replicated), mask bool [L]."""
         if self.ops is None:
-            self.ops = cuda_ops()
+            self.ops = self._default_ops = cuda_ops()
         if self._whole(pair_rows, single):
             return self._forward_whole(pair_rows, single, mask)
         L = pair_rows.shape[1]

@@ -67,3 +67,25 @@ def test_many_heads(heads, dim_head, dtype):
     got = go(block, *rest)
     block.native_ok, block.ops = False, cuda_ops()
     close(got, go(block, *rest), block, 1e-2 if dtype != torch.float32 else 1e-4)
+
+
+def test_mask_of_any_shape_with_a_value_per_token():
+    block, pair, single, mask, d = make(40)
+    want = go(block, pair, single, mask, d)
+    for m in (mask[None], mask.view(40, 1), torch.stack([mask, ~mask], 1)[:, 0]):
+        assert torch.equal(block(pair, single, m)[0], want[0])
+
+
+def test_injected_operators_are_used():
+    """Operators set on a block that has already run with its own, and a block restored from a state without the newer fields."""
+    from types import SimpleNamespace
+    from megafold_b200.pairformer_block import cuda_ops
+    block, pair, single, mask, _ = make(40)
+    want = block(pair, single, mask)
+    ops, seen = cuda_ops(), []
+    block.ops = SimpleNamespace(lnl=ops.lnl, transition=ops.transition, attention=lambda *a: (seen.append(1), ops.attention(*a))[1])
+    x, s = block(pair, single, mask)
+    assert len(seen) == 3
+    block.ops = None
+    block.__dict__.pop("native_ok", None)
+    assert torch.equal(block(pair, single, mask)[0], want[0]) and len(seen) == 3
