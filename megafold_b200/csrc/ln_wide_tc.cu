@@ -214,8 +214,8 @@ ln_wide_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ C
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const float b = __uint_as_float(hg[2 * e + q]);
+          // exp(-b) beyond 2^126 divides to 0, and an infinite b to NaN, which the product with the value carries on
           g[q] = __fdividef(b, 1.f + __expf(-b)) * __uint_as_float(hv[2 * e + q]);
-          if (b < -80.f) g[q] = 0.f;                 // 1 + exp(-b) beyond the range of __fdividef; silu is below 1e-33 there
         }
         out[e] = Pack2<T>::pack(g[0], g[1]);
       }
