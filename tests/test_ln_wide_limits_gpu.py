@@ -35,3 +35,30 @@ def test_swiglu_of_non_finite_products(what):
         assert bool(torch.isnan(want).all())
     ok = ~torch.isnan(want)
     torch.testing.assert_close(y[ok].float(), want[ok].float(), rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("K", [192, 256, 384])
+def test_normalised_values_beyond_fp16(K):
+    """|LN(x)| up to 80000 in fp16, where the products with small weights are ordinary numbers."""
+    M, N = 140, 72
+    g = torch.Generator(device="cuda").manual_seed(K)
+    r = lambda *s: torch.randn(*s, device="cuda", generator=g)      # noqa: E731
+    x = (0.01 * r(M, K)).half()
+    x[torch.arange(M), torch.randint(K, (M,), device="cuda", generator=g)] = 30.0      # one element of sqrt(K) standard deviations
+    gain = torch.full((K,), 80000 / K ** 0.5, device="cuda").half()
+    w = (1e-3 * r(K, N)).half()
+    y, *_ = mfb.layernorm_linear_forward(x, w, None, gain, None)
+    assert _lib.last_path() == "tcgen05"
+    want, *_ = mfb.layernorm_linear_forward(x, w, None, gain, None, flags=FORCE)
+    assert bool(torch.isfinite(want).all())
+    torch.testing.assert_close(y, want, rtol=2e-3, atol=2e-3 * float(want.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_nan_rows_stay_nan(dtype):
+    """A row of x with a NaN or an infinity is NaN in the result, the rows beside it are not touched."""
+    r = torch.randn(140, 256, device="cuda").to(dtype)
+    r[3, 7], r[131, 0] = float("nan"), float("inf")
+    w, gain = (torch.randn(256, 64, device="cuda") / 16).to(dtype), torch.ones(256, device="cuda").to(dtype)
+    y, *_ = mfb.layernorm_linear_forward(r, w, None, gain, None)
+    assert bool(torch.isnan(y[[3, 131]]).all()) and bool(torch.isfinite(y[[i for i in range(140) if i not in (3, 131)]]).all())
