@@ -328,8 +328,10 @@ int lnl_fwd_wide(const mf_lnl_fwd_args& a, cudaStream_t st) {
   return dispatch<0>(a.K, WideArgs{a.M, a.N, 0, a.dtype, a.eps, a.x, a.ln_w, a.ln_b, a.w, a.b, a.y, a.mean, a.rstd}, st);
 }
 
+// The workspace, which TMA writes, needs the alignment that the CUDA-core path, with a workspace of the same size, does without.
 bool transition_fwd_wide_supported(const mf_transition_fwd_args& a) {
-  const uintptr_t al = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w1) | reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.y);
+  const uintptr_t al = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w1) | reinterpret_cast<uintptr_t>(a.w2) | reinterpret_cast<uintptr_t>(a.y) |
+                       reinterpret_cast<uintptr_t>(a.workspace);
   return wide_ok(a.M, a.dim, a.dtype) && a.ln_w && a.inner % 32 == 0 && (al & 15) == 0;
 }
 size_t transition_fwd_wide_workspace(const mf_transition_fwd_args& a) { return align_up((size_t)a.M * a.inner * dtype_size(a.dtype), 256); }

@@ -62,3 +62,24 @@ def test_nan_rows_stay_nan(dtype):
     w, gain = (torch.randn(256, 64, device="cuda") / 16).to(dtype), torch.ones(256, device="cuda").to(dtype)
     y, *_ = mfb.layernorm_linear_forward(r, w, None, gain, None)
     assert bool(torch.isnan(y[[3, 131]]).all()) and bool(torch.isfinite(y[[i for i in range(140) if i not in (3, 131)]]).all())
+
+
+@pytest.mark.parametrize("offset,path", [(0, "tcgen05"), (2, "simt"), (8, "simt"), (16, "tcgen05")])
+def test_transition_workspace_at_any_address(offset, path):
+    """mf_transition_fwd with a workspace that is aligned for its elements only."""
+    import ctypes as C
+    M, dim, inner = 130, 256, 64
+    x, w1, w2 = (torch.randn(*s, device="cuda").bfloat16() for s in ((M, dim), (dim, 2 * inner), (dim, inner)))
+    lw = torch.ones(dim, device="cuda").bfloat16()
+    want, mean, rstd = mfb.transition_forward(x, lw, None, w1, w2)
+    y = torch.empty_like(x)
+    a = _lib.TransitionFwdArgs()
+    a.M, a.dim, a.inner, a.dtype, a.eps = M, dim, inner, _lib.MF_BF16, 1e-5
+    a.x, a.ln_w, a.w1, a.w2, a.y, a.mean, a.rstd = (t.data_ptr() for t in (x, lw, w1, w2, y, mean, rstd))
+    need = _lib.lib().mf_transition_fwd_workspace_bytes(C.byref(a))
+    ws = torch.empty(need + 64, dtype=torch.uint8, device="cuda")
+    a.workspace, a.workspace_bytes = ws.data_ptr() + offset, need
+    assert _lib.lib().mf_transition_fwd_workspace_bytes(C.byref(a)) == need
+    _lib.check(_lib.lib().mf_transition_fwd(C.byref(a), _lib.stream_ptr("cuda")), "mf_transition_fwd")
+    assert _lib.last_path() == path
+    torch.testing.assert_close(y.float(), want.float(), rtol=2e-2, atol=2e-2 * float(want.float().abs().max()))
