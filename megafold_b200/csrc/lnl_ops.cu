@@ -770,7 +770,8 @@ int transition_bwd_tc(const mf_transition_bwd_args& a, cudaStream_t st) {
 // scratch (g and dh: 3 KB per row at inner = 512); the weight gradients accumulate over the ranges, the partial column
 // sums of every range are reduced together at the end.  A range costs about 20 us of its own (filling and draining three
 // kernels, adding the split weight gradients up): [262144, 128] in one took 463 us, in two 509, in four 603, although g
-// and dh would stay in L2 with more.  kTransitionChunkRows keeps the scratch at 0.8 GB for inner = 512.
+// and dh would stay in L2 with more.  A range has kTransitionChunkRows rows, rounded up to whole waves where there are several,
+// at most: 0.8 GB of scratch for inner = 512.
 constexpr int64_t kTransitionChunkRows = 262144;
 struct TransitionChunks { int n; int64_t rows; };
 TransitionChunks transition_chunks(int64_t M) {
@@ -779,6 +780,7 @@ TransitionChunks transition_chunks(int64_t M) {
   if (c.n < 1) c.n = 1;
   const int64_t wave = 128 * (int64_t)tcx::sm_count(), even = (M + c.n - 1) / c.n;
   c.rows = c.n == 1 ? (M + 127) / 128 * 128 : (even + wave - 1) / wave * wave;
+  if (c.n > 1) c.n = (int)((M + c.rows - 1) / c.rows);        // rounding up may have made the last range empty
   return c;
 }
 size_t transition_bwd_fused_bytes(const mf_transition_bwd_args& a) {
@@ -803,7 +805,6 @@ int transition_bwd_fused_path(const mf_transition_bwd_args& a, cudaStream_t st) 
   int part_rows = 0;
   for (int c = 0; c < ch.n; ++c) {
     const int64_t m0 = (int64_t)c * ch.rows, rows = (m0 + ch.rows < M ? ch.rows : M - m0);
-    if (rows <= 0) break;
     mf_transition_bwd_args ac = a;
     ac.M = rows;
     ac.x = static_cast<const T*>(a.x) + m0 * K;
