@@ -463,6 +463,11 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       ++item_local;
     }
   }
+  if (*abort_flag) {
+    if (officer_kv) { drain_ring(&bar.q_full, cq.item_local, 1); drain_ring(bar.k_full, gk, C::KS); drain_ring(bar.v_full, gv, kVS); }
+    if (BM == kTma && officer_b) drain_ring(bar.b_full, cb_next, kBC);
+  }
+  if (BM == kStaged) cp_async_wait<0>();
 
   tc_fence_before();
   __syncthreads();

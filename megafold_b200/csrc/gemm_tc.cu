@@ -124,6 +124,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
         }
       }
     }
+    drain_ring(bar.full, cnt, kStages);
   } else if (warp == 1) {
     // ------------------------------------------------------------------------------------ MMA issuer
     // Run by the whole warp, one elected lane issuing: with a single lane's branch and run-time descriptors an MMA took 100

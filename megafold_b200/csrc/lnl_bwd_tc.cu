@@ -200,6 +200,7 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
         tma_load_2d(a + kSlabB, &mw, &bar.full[st], s * 64, 0);
       }
     }
+    drain_ring(bar.full, cnt, kStages);
     } else if (warp == kRowWarps) {
     // ---------------------------------------------------------------------------------------- MMA issuer
     // Run by the whole warp, one elected lane issuing: with a single lane's branch and run-time descriptors an MMA took 100

@@ -259,10 +259,12 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
     }
   } else if (warp == 9 + kNormWarps && lane == 0) {
     // ------------------------------------------------------------------------------------ TMA producer of X and W tiles
-    uint32_t w_cnt = 0;
+    uint32_t w_cnt = 0, n_x = 0;
     auto load_x = [&](int t_local) {
       const int buf = t_local % kAStages;
       if (t_local >= kAStages) wait_or_flag(&bar.a_empty[buf], ((t_local / kAStages) - 1) & 1, abort_flag);
+      if (*abort_flag) return;
+      ++n_x;
       const int row0 = (int)(((int64_t)blockIdx.x + (int64_t)t_local * gridDim.x) * kRows);
       mbar_expect_tx(&bar.x_full[buf], A_BYTES);
 #pragma unroll
@@ -281,6 +283,8 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
         tma_load_2d(sW + ws * W_BYTES + K * 128, &mw, &bar.w_full[ws], nt * kNT + 64, 0);
       }
     }
+    drain_ring(bar.x_full, n_x, kAStages);
+    drain_ring(bar.w_full, w_cnt, kWStages);
   }
   }
 

@@ -61,6 +61,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return false;
 }
 
+// Waits (bounded) for the last of the `requested` copies that went through a ring of `depth` barriers.  Whoever requests copies
+// does this before it leaves: after a wait that expired nobody else waits for them, and none may land once the CTA's shared
+// memory belongs to another.  (Otherwise they have long landed.)
+__device__ __forceinline__ void drain_ring(uint64_t* full, uint32_t requested, uint32_t depth) {
+  for (uint32_t back = 1; back <= depth && back <= requested; ++back) mbar_wait(&full[(requested - back) % depth], ((requested - back) / depth) & 1);
+}
+
 // ---- TMA -------------------------------------------------------------------------------------
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -196,7 +196,9 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
     uint64_t* xr_full = &bar.xr_full[quarter];
     uint8_t* xr = sXR + quarter * 32 * 128;                // my 32 rows of the first 64 columns; the others are kRows * 128 further
     auto row_of = [&](int t) { return ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows; };
+    uint32_t n_raw = 0;
     auto load_raw = [&](int t) {                           // (lane 0) my rows of tile t for the write-out
+      ++n_raw;
       mbar_expect_tx(xr_full, 2 * 32 * 128);
       for (int q = 0; q < K / 64; ++q) tma_load_2d(xr + q * (kRows * 128), &mxr, xr_full, q * 64, (int)row_of(t) + quarter * 32);
     };
@@ -275,7 +277,7 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       }
       __syncwarp();
     }
-    if (lane == 0) bulk_wait_group<0>();
+    if (lane == 0) { drain_ring(xr_full, n_raw, 1); bulk_wait_group<0>(); }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     auto dead = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };      // the MMA roles are run by whole warps
@@ -347,16 +349,18 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       bulk_wait_group<0>();
     } else if (warp == kWorkWarps + 5 && lane == 0) {
       // -------------------------------------------------------------------------------- TMA producer
-      uint32_t ch_cnt = 0;
+      uint32_t ch_cnt = 0, n_x = 0, n_dy = 0;
       auto load_rows = [&](int t) {           // (the normalising warps have taken tile t - 1)
         const int row0 = (int)(((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows);
         if (t > 0) wait_or_flag(&bar.x_empty, (t - 1) & 1, abort_flag);
         if (*abort_flag) return;
+        ++n_x;
         mbar_expect_tx(&bar.x_full, A_BYTES);
         tma_load_2d(sX, &mx, &bar.x_full, 0, row0);
         tma_load_2d(sX + kRows * 128, &mx, &bar.x_full, 64, row0);
         if (t > 0) wait_or_flag(&bar.dy_empty, (t - 1) & 1, abort_flag);
         if (*abort_flag) return;
+        ++n_dy;
         mbar_expect_tx(&bar.dy_full, A_BYTES);
         tma_load_2d(sDY, &mdy, &bar.dy_full, 0, row0);
         tma_load_2d(sDY + kRows * 128, &mdy, &bar.dy_full, 64, row0);
@@ -375,6 +379,9 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           tma_load_2d(w + 2 * WB, &mw2, &bar.w_full[ws], c * kHC, 0);           // W2[:, chunk]
         }
       }
+      drain_ring(&bar.x_full, n_x, 1);
+      drain_ring(&bar.dy_full, n_dy, 1);
+      drain_ring(bar.w_full, ch_cnt, kWS);
     }
   }
 

@@ -321,9 +321,11 @@ transition_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       }
     } else if (warp == kWorkWarps + 5 && lane == 0) {
       // ---------------------------------------------------------------------------------- TMA producer of X and W1
-      uint32_t ch_cnt = 0;
+      uint32_t ch_cnt = 0, n_x = 0;
       auto load_x = [&](int t) {           // (the normalising warps hold the rows of tile t - 1 in registers)
         if (t > 0) wait_or_flag(&bar.x_empty, (t - 1) & 1, abort_flag);
+        if (*abort_flag) return;
+        ++n_x;
         const int row0 = (int)(((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows);
         mbar_expect_tx(&bar.x_full, A_BYTES);
 #pragma unroll
@@ -342,6 +344,8 @@ transition_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           tma_load_2d(w + W1B, &mw1, &bar.w1_full[ws], p.inner + c * kHC, 0);   // gate columns of W1
         }
       }
+      drain_ring(&bar.x_full, n_x, 1);
+      drain_ring(bar.w1_full, ch_cnt, kWStages);
     } else if (warp == kWorkWarps + 7 && lane == 0) {
       // ---------------------------------------------------------------------------------- TMA producer of the W2 blocks
       uint32_t ch_cnt = 0;
@@ -353,6 +357,7 @@ transition_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           mbar_expect_tx(&bar.w2_full[ws], W2B);
           tma_load_2d(sW + ws * W_BYTES + 2 * W1B, &mw2, &bar.w2_full[ws], c * kHC, 0);      // W2[:, chunk]
         }
+      drain_ring(bar.w2_full, ch_cnt, kWStages);
     }
   }
 
