@@ -22,6 +22,9 @@ from .evoattention import evo_attention_backward, evo_attention_forward
 
 __all__ = ["evoformer_fwd_bwd_host", "HostPipeline"]
 
+# how a call runs; whoever can do one can do those before it
+ISSUE, RECORD, REPLAY = 0, 1, 2
+
 
 def _row_spans(n_rows, chunks):
     """Row chunks for the pipeline: about ``chunks`` full-size chunks in the middle, and short ones at both ends,
@@ -71,37 +74,52 @@ class HostPipeline:
         before it is downloaded (the collective is part of the replayed graph; every rank must call in step)."""
         host = dict(q=q, k=k, v=v, d_out=d_out, mask=res_mask, bias=pair_bias)
         self.group = group
-        key = tuple(t.data_ptr() for t in host.values())
         cur = torch.cuda.current_stream(self.device)
+        # what the recorded copies and the collective depend on
+        key = (group, *((t.data_ptr(), t.dtype, tuple(t.shape), t.stride()) for t in host.values()))
         if self.graph is not None and key == self.graph_key:
+            mode = REPLAY
+        else:
+            mode = RECORD if self.use_graph and key == self.last_key and all(t.is_pinned() for t in host.values()) else ISSUE
+        self.last_key = key
+        if group is not None:
+            mode = self._least(mode)                 # a rank whose buffers come back does not run ahead of one whose do not
+        if mode == RECORD:
+            mode = REPLAY if self._record(host, key, cur) else ISSUE
+        if mode == REPLAY:
             self.graph.replay()                      # on the current stream
-            cur.synchronize()
-            return self.out
-        again, self.last_key = key == self.last_key, key
-        if self.use_graph and again and all(t.is_pinned() for t in host.values()):
-            try:
-                self.s_cap.wait_stream(cur)
-                g = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(g, stream=self.s_cap):
-                    self._schedule(host, self.s_cap)
-                self.graph, self.graph_key = g, key
-                cur.wait_stream(self.s_cap)
-            except Exception as e:                   # capture not possible here: keep the direct schedule
-                warnings.warn(f"CUDA graph capture of the host pipeline failed ({type(e).__name__}: {e}); issuing the schedule directly")
-                self.use_graph = False
-                self.graph = None
-                torch.cuda.synchronize(self.device)
-            if group is not None:                    # every rank replays, or none does
-                import torch.distributed as dist
-                ok = torch.tensor([1 if self.graph is not None else 0], device=self.device)
-                dist.all_reduce(ok, op=dist.ReduceOp.MIN, group=group)
-                if not int(ok):
-                    self.graph, self.use_graph = None, False
-            if self.graph is not None:
-                return self.run(q, k, v, res_mask, pair_bias, d_out, group)
-        self._schedule(host, cur)
+        else:
+            self._schedule(host, cur)
         cur.synchronize()
         return self.out
+
+    def _least(self, value):
+        """The smallest of the ranks' values: each step of the group's ranks has to be the same on all of them."""
+        import torch.distributed as dist
+        on = self.device if dist.get_backend(self.group) == "nccl" else "cpu"
+        t = torch.tensor([value], device=on)
+        dist.all_reduce(t, op=dist.ReduceOp.MIN, group=self.group)
+        return int(t)
+
+    def _record(self, host, key, cur):
+        """Records the schedule for these buffers; False where a rank could not."""
+        self.graph = None
+        try:
+            self.s_cap.wait_stream(cur)
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=self.s_cap):
+                self._schedule(host, self.s_cap)
+            self.graph, self.graph_key = g, key
+            cur.wait_stream(self.s_cap)
+        except Exception as e:                       # capture not possible here: keep the direct schedule
+            warnings.warn(f"CUDA graph capture of the host pipeline failed ({type(e).__name__}: {e}); issuing the schedule directly")
+            torch.cuda.synchronize(self.device)
+        done = int(self.graph is not None)
+        if self.group is not None:                   # every rank replays, or none does
+            done = self._least(done)
+        if not done:
+            self.graph, self.use_graph = None, False
+        return bool(done)
 
     def _schedule(self, host, cur):
         """Enqueue one step: the three streams fork from ``cur`` and join it again at the end."""
