@@ -15,7 +15,6 @@ import torch
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libmegafold_b200_trace.so" if os.environ.get("MF_TRACE") == "1" else "libmegafold_b200.so")
-NATIVE_PATH = os.path.join(_PKG, "_native.so")
 
 MF_F32, MF_BF16, MF_F16, MF_U8 = 0, 1, 2, 3
 MF_FLAG_FORCE_SIMT = 1
@@ -149,11 +148,12 @@ def native():
         return _native
     with _lock:
         if _native is None:
-            if not os.path.exists(NATIVE_PATH):
-                from . import build as _build
+            from . import build as _build
+            path = _build.native_path()
+            if not os.path.exists(path):
                 _build.build()
             lib()
-            spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE_PATH)
+            spec = importlib.util.spec_from_file_location(__package__ + "._native", path)
             module = importlib.util.module_from_spec(spec)
             spec.loader.exec_module(module)
             module.load(LIB_PATH)

@@ -4,7 +4,7 @@
 
 The library is plain CUDA C++ behind a C ABI (include/megafold_b200.h); it links the static CUDA
 runtime only, so it loads on hosts without a GPU driver (entry points then fail with MF_ERR_CUDA).  The torch functions over it
-are a second shared object (_native.so), which needs the torch it was built against.
+are a second shared object (native_path()), which needs the torch it was built against.
 """
 from __future__ import annotations
 
@@ -21,7 +21,6 @@ ROOT = os.path.dirname(PKG)
 # regular library; megafold_b200._lib loads it when MF_TRACE=1 is set there too.
 TRACE = os.environ.get("MF_TRACE") == "1"
 LIB = os.path.join(PKG, "libmegafold_b200_trace.so" if TRACE else "libmegafold_b200.so")
-NATIVE = os.path.join(PKG, "_native.so")          # torch functions over the library (csrc/torch_ops.cpp)
 OBJ_DIR = os.path.join(PKG, "build_trace" if TRACE else "build")
 
 SOURCES = ["api.cu", "evo_simt.cu", "evo_tc.cu", "evo_tc_fwd.cu", "evo_fwd_ws.cu", "evo_bwd_ws.cu", "lnl_ops.cu", "lnl_tc.cu", "transition_tc.cu", "gemm_tc.cu", "transition_bwd_tc.cu", "cast.cu", "lnl_bwd_tc.cu", "ln_wide_tc.cu", "block_ops.cu"]
@@ -54,7 +53,14 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def _native_command(src: str):
+def native_path() -> str:
+    """The torch functions over the library (csrc/torch_ops.cpp).  They fit the interpreter and the torch they were built
+    against only, so both are part of the name: another torch finds no file and builds its own."""
+    import torch
+    return os.path.join(PKG, f"_native.{sys.implementation.cache_tag}-torch-{torch.__version__}.so")
+
+
+def _native_command(src: str, target: str):
     """g++ of one translation unit against the installed torch; the result is imported by file name."""
     import sysconfig
 
@@ -64,7 +70,7 @@ def _native_command(src: str):
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     # the C++ runtime has to be the one torch uses: a second, static copy crashes when it formats an error message
     return ["g++", "-shared", "-fPIC", "-O2", "-std=c++17", "-fvisibility=hidden",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), src, "-o", NATIVE,
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), src, "-o", target,
             f"-L{lib}", f"-Wl,-rpath,{lib}", "-lc10", "-ltorch_cpu", "-ltorch", "-ltorch_python", "-lc10_cuda", "-lstdc++", "-ldl"]
 
 
@@ -87,13 +93,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return p.stdout + p.stderr
 
     native_src = os.path.join(CSRC, "torch_ops.cpp")
-    if force or _stale(NATIVE, [native_src, os.path.join(ROOT, "include", "megafold_b200.h"), os.path.abspath(__file__)]):
-        jobs.insert(0, _native_command(native_src))
+    native = native_path()
+    if force or _stale(native, [native_src, os.path.join(ROOT, "include", "megafold_b200.h"), os.path.abspath(__file__)]):
+        jobs.insert(0, _native_command(native_src, native))
     with ThreadPoolExecutor(max_workers=5) as ex:
         for out in ex.map(run, jobs):
             if verbose and out.strip():
                 print(out)
-    jobs = [c for c in jobs if NATIVE not in c]
+    jobs = [c for c in jobs if native not in c]
     objs = [os.path.join(OBJ_DIR, s.replace(".cu", ".o")) for s in SOURCES]
     if force or jobs or _stale(LIB, objs):
         run([nvcc, "-shared", "-o", LIB, *objs, "-Xcompiler", "-fPIC", "-cudart", "static", "-ldl"])

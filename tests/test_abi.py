@@ -61,3 +61,22 @@ def test_cpu_tensors_are_rejected():
         mfb.LayernormLinear(8, 4)(torch.zeros(3, 8))
     with pytest.raises(RuntimeError, match="CUDA"):
         mfb.FusedTransition(8)(torch.zeros(3, 8))
+
+
+def test_another_torch_gets_torch_functions_of_its_own(monkeypatch):
+    """The extension is bound to the torch it was built against: with another one it is built anew, not loaded."""
+    import torch
+    from megafold_b200 import build
+    _lib.native()
+
+    class Built(Exception):
+        pass
+
+    def fake_build(*a, **k):
+        raise Built
+
+    monkeypatch.setattr(torch, "__version__", "0.0.0+other")
+    monkeypatch.setattr(_lib, "_native", None)
+    monkeypatch.setattr(build, "build", fake_build)
+    with pytest.raises(Built):
+        _lib.native()

@@ -16,7 +16,7 @@ def kernels():
             yield os.path.basename(path), text
 
 
-@pytest.mark.parametrize("name,text", kernels(), ids=[n for n, _ in kernels()])
+@pytest.mark.parametrize("name,text", list(kernels()), ids=[n for n, _ in kernels()])
 def test_every_requested_copy_is_awaited_before_exit(name, text):
     pointers = re.findall(r"uint64_t\* (\w+) = &bar\.(\w+)", text)
 
