@@ -519,10 +519,13 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   p.items_per_stream = (p.n_items + 2 * grid - 1) / (2 * grid);
   const size_t smem = 1024 + 2 * (size_t)kStreamBytes + 2048 + kXTileB;
   constexpr auto kern = evo_fwd_ws_kernel<T, TB, EXACT>;
-  static const int regs = [] {
+  static std::atomic<int> built_with{0};           // asked for once; a query that fails is made again
+  int regs = built_with.load(std::memory_order_relaxed);
+  if (!regs) {
     cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, kern) == cudaSuccess ? fa.numRegs : -1;
-  }();
+    MF_CUDA(cudaFuncGetAttributes(&fa, kern));
+    built_with.store(regs = fa.numRegs, std::memory_order_relaxed);
+  }
   MF_REQUIRE(regs == kLaunchRegs, MF_ERR_CUDA, "evo_fwd_ws_kernel was built with %d registers per thread, %d expected", regs, kLaunchRegs);
   if (int e = opt_in_smem<kern>(smem)) return e;
   kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p MF_TRACE_ARG);

@@ -476,7 +476,8 @@ bool lnl_bwd_core_tc_ok(int64_t M, int K, int N, int dtype, bool has_ln, const v
   return (al & 15) == 0;
 }
 
-// The fused LayerNorm-backward row pass over M rows; returns the number of blocks (= rows of `part`, [blocks][2 K]).
+// The fused LayerNorm-backward row pass over M rows; returns the number of blocks (= rows of `part`, [blocks][2 K]), or an
+// error, which is negative.
 template <typename T>
 int launch_ln_bwd_rows(const float* dyln, const T* x, const T* gain, const T* shift, const float* mean, const float* rstd,
                        T* dx, DxAdd<T> add, T* xln, float* part, int64_t M, int K, cudaStream_t st) {
@@ -529,6 +530,7 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
         if (r) return r;
       }
       const int blocks = launch_ln_bwd_rows<T>(dyln, x, gain, shift, mean, rstd, dx, add, xln, part, M, K, st);
+      if (blocks < 0) return blocks;
       if (db && N <= 2048) {
         const int64_t rows = (M + blocks - 1) / blocks;           // the same blocks of rows as the pass above
         float* dpart = ws.take<float>((size_t)kRowBlocks * N);
