@@ -241,7 +241,7 @@ int mf_lnl_bwd_add(const mf_lnl_bwd_args* args, const void* add1, const void* ad
   MF_REQUIRE(((uintptr_t)a.workspace & 255) == 0, MF_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   int r = check_device(); if (r) return r;
   r = lnl_bwd(a, add1, add2, static_cast<cudaStream_t>(stream));
-  if (r == MF_OK) set_last_path(lnl_bwd_runs_on_tc(a) ? "tcgen05" : "simt");
+  if (r == MF_OK) set_last_path(lnl_bwd_runs_on_tc(a, add1, add2) ? "tcgen05" : "simt");
   return r;
 }
 

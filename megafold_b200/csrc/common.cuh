@@ -166,7 +166,7 @@ int lnl_fwd_tc(const mf_lnl_fwd_args& a, cudaStream_t st);
 bool lnl_fwd_wide_supported(const mf_lnl_fwd_args& a);
 int lnl_fwd_wide(const mf_lnl_fwd_args& a, cudaStream_t st);
 int lnl_bwd(const mf_lnl_bwd_args& a, const void* add1, const void* add2, cudaStream_t st);   // picks tensor-core GEMMs when lnl_bwd_runs_on_tc
-bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a);
+bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a, const void* add1, const void* add2);
 bool transition_bwd_runs_on_tc(const mf_transition_bwd_args& a);
 bool transition_bwd_fused_ok(const mf_transition_bwd_args& a);
 int transition_bwd_fused_blocks(int64_t M);

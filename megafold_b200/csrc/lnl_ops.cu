@@ -630,12 +630,15 @@ size_t lnl_bwd_workspace(const mf_lnl_bwd_args& a) {
   const size_t tc = lnl_bwd_use_tc(a) ? lnl_bwd_core_bytes(a.M, a.K, a.N, true, true, a.dtype) : 0;
   return simt > tc ? simt : tc;
 }
-bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a) { return lnl_bwd_use_tc(a); }
+// the kernels that add gradients to dx read them 16 bytes at a time, like the other operands
+bool lnl_bwd_runs_on_tc(const mf_lnl_bwd_args& a, const void* add1, const void* add2) {
+  return lnl_bwd_use_tc(a) && ((reinterpret_cast<uintptr_t>(add1) | reinterpret_cast<uintptr_t>(add2)) & 15) == 0;
+}
 bool transition_bwd_runs_on_tc(const mf_transition_bwd_args& a) { return transition_bwd_use_tc(a); }
 
 int lnl_bwd(const mf_lnl_bwd_args& a, const void* add1, const void* add2, cudaStream_t st) {
   Carver ws(a.workspace);
-  const bool tc = lnl_bwd_use_tc(a) && ((reinterpret_cast<uintptr_t>(add1) | reinterpret_cast<uintptr_t>(add2)) & 15) == 0;
+  const bool tc = lnl_bwd_runs_on_tc(a, add1, add2);
   if (!add1) { add1 = add2; add2 = nullptr; }
   MF_DISPATCH_FLOAT(a.dtype, T, {
     int r = lnl_bwd_core<T>(a.M, a.K, a.N, static_cast<const T*>(a.x), static_cast<const T*>(a.ln_w),

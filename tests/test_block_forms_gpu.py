@@ -89,3 +89,42 @@ def test_injected_operators_are_used():
     block.ops = None
     block.__dict__.pop("native_ok", None)
     assert torch.equal(block(pair, single, mask)[0], want[0]) and len(seen) == 3
+
+
+def at_offset(t):
+    """The same values at an address that is a multiple of 2 bytes only."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    flat[1:] = t.detach().reshape(-1)
+    return flat[1:].view(t.shape)
+
+
+def test_inputs_at_any_address():
+    block, pair, single, mask, d = make(40)
+    want = go(block, pair, single, mask, d)
+    got = go(block, at_offset(pair).requires_grad_(True), at_offset(single).requires_grad_(True), mask, [at_offset(t) for t in d])
+    close(got, want, block)
+
+
+@pytest.mark.parametrize("K", [128, 384])
+def test_added_gradients_at_any_address(K):
+    """mf_lnl_bwd_add with an addend that cannot be read in 16-byte pieces: its values, and the family of kernels it reports."""
+    import ctypes as C
+    from megafold_b200 import _lib
+    M, N = 150, 64
+    x, dy, add = (torch.randn(M, n, device="cuda").bfloat16() for n in (K, N, K))
+    w, lw = torch.randn(K, N, device="cuda").bfloat16(), torch.ones(K, device="cuda").bfloat16()
+    _, mean, rstd = mfb.layernorm_linear_forward(x, w, None, lw, None)
+    got = {}
+    for name, addend in (("tcgen05", add), ("simt", at_offset(add))):
+        a = _lib.LnlBwdArgs()
+        a.M, a.K, a.N, a.dtype = M, K, N, _lib.MF_BF16
+        dx, dw, dlw = torch.empty_like(x), torch.empty(K, N, device="cuda"), torch.empty(K, device="cuda")
+        a.x, a.ln_w, a.w, a.dy, a.mean, a.rstd = (t.data_ptr() for t in (x, lw, w, dy, mean, rstd))
+        a.dx, a.dw, a.d_ln_w = dx.data_ptr(), dw.data_ptr(), dlw.data_ptr()
+        ws = _lib.workspace(_lib.lib().mf_lnl_bwd_workspace_bytes(C.byref(a)), "cuda")
+        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+        _lib.check(_lib.lib().mf_lnl_bwd_add(C.byref(a), addend.data_ptr(), None, _lib.stream_ptr("cuda")), "mf_lnl_bwd_add")
+        assert _lib.last_path() == name
+        got[name] = dx, dw, dlw
+    for a, b in zip(*got.values()):
+        torch.testing.assert_close(a.float(), b.float(), rtol=2e-2, atol=2e-2 * float(b.float().abs().max()))
