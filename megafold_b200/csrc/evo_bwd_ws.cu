@@ -1067,8 +1067,7 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
   const int64_t n_dq = (int64_t)a.B * a.N * a.L * a.H * a.D;
 
   float alpha[2];
-  // with a copied 16-bit bias the forward pass took both terms of sqrt(D) (evo_fwd_ws.cu): so does the probability here
-  const int n_alpha = split_alpha(a.D, bt_dtype, alpha, !pl.bias_direct && sizeof(TB) == 2);
+  const int n_alpha = split_alpha(a.D, bt_dtype, alpha, false);
   // With one row per bias (N = 1, single-representation attention) and d_pair_bias in the q/k/v type, dS is the answer:
   // the dQ/dK/dV kernel writes it and the d_pair_bias kernel is not needed.
   const bool dbias_direct = a.N == 1 && a.dbias_dtype == a.dtype;
