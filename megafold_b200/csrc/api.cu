@@ -84,10 +84,6 @@ int check_evo_common(const A& a) {
 
 using namespace mf;
 
-extern "C" {
-
-}  // extern "C"
-
 namespace mf {
 namespace {
 

@@ -458,11 +458,11 @@ void fill_common(EvoP& p, const A& a) {
   p.nt = (a.L + kTile - 1) / kTile;
 }
 
-// Ranges of the N rows that a tile of d_pair_bias is summed in: enough blocks for four on each of 148 SMs, at least two
+// Ranges of the N rows that a tile of d_pair_bias is summed in: enough blocks for four on each SM, at least two
 // rows each (a block of one row would write its tile for less work than reading it back costs).
 int bias_ranges(int B, int N, int L, int H) {
   const int64_t nt = (L + kTile - 1) / kTile, tiles = (int64_t)B * H * nt * nt;
-  int64_t r = (592 + tiles - 1) / tiles;
+  int64_t r = (4 * tcx::sm_count() + tiles - 1) / tiles;
   if (r > (N + 1) / 2) r = (N + 1) / 2;
   return (int)(r < 1 ? 1 : r);
 }

@@ -85,7 +85,7 @@ int launch_gemm_simt(const char* name, int64_t M, int N, int64_t K, int splits, 
 
 // number of slices of a reduction of length `red` for an output of `tiles` 64x64 tiles
 inline int pick_splits(int64_t tiles, int64_t red) {
-  int64_t s = (592 + tiles - 1) / tiles;
+  int64_t s = (4 * tcx::sm_count() + tiles - 1) / tiles;
   int64_t cap = red / 256; if (cap < 1) cap = 1;
   if (s > cap) s = cap;
   if (s > 128) s = 128;

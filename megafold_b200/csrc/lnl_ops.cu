@@ -259,12 +259,6 @@ __global__ void ln_apply_kernel(const T* __restrict__ x, const T* __restrict__ g
   *reinterpret_cast<uint2*>(xln + m * K + k) = *reinterpret_cast<const uint2*>(o);
 }
 
-template <typename T>
-__global__ void cast_rows_kernel(const float* __restrict__ src, T* __restrict__ dst, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = from_f<T>(src[i]);
-}
-
 // partial column sums: part[z, c] = sum over the rows of slice z of f(m, c)
 template <class F>
 __global__ void colsum_partial_kernel(F f, float* __restrict__ part, int64_t M, int ncols, int64_t rows_per_slice) {
@@ -499,8 +493,7 @@ int launch_ln_bwd_rows(const float* dyln, const T* x, const T* gain, const T* sh
 template <typename T>
 int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* shift, const T* w, const T* dy,
                  const float* mean, const float* rstd, T* dx, DxAdd<T> add, float* dw, float* db, float* d_ln_w, float* d_ln_b,
-                 Carver& ws, bool tc, int dtype, cudaStream_t st, const T* xln_ready = nullptr,
-                 const float* dyln_ready = nullptr) {
+                 Carver& ws, bool tc, int dtype, cudaStream_t st, const T* xln_ready = nullptr) {
   int r;
   float* col_scratch = ws.take<float>((size_t)kColSlices * (K > N ? K : N));
   if constexpr (sizeof(T) == 2) {
@@ -521,14 +514,12 @@ int lnl_bwd_core(int64_t M, int K, int N, const T* x, const T* gain, const T* sh
       return gemm_tc(GemmTcArgs{x, dy, dw, K, N, M, dtype, 1, 1, 2, 0, mean, rstd, gain, shift}, st);
     }
     if (tc) {
-      float* dyln = dyln_ready ? const_cast<float*>(dyln_ready) : ws.take<float>((size_t)M * K);
+      float* dyln = ws.take<float>((size_t)M * K);
       T* xln = xln_ready ? nullptr : ws.take<T>((size_t)M * K);
       float* part = ws.take<float>((size_t)kRowBlocks * 2 * K);
-      if (!dyln_ready) {
-        // dyln[M,K] = dy @ w^T  (A = dy [M,N], B = w [K,N], both with the reduction index contiguous)
-        r = gemm_tc(GemmTcArgs{dy, w, dyln, M, K, N, dtype, 0, 0, 1}, st);
-        if (r) return r;
-      }
+      // dyln[M,K] = dy @ w^T  (A = dy [M,N], B = w [K,N], both with the reduction index contiguous)
+      r = gemm_tc(GemmTcArgs{dy, w, dyln, M, K, N, dtype, 0, 0, 1}, st);
+      if (r) return r;
       const int blocks = launch_ln_bwd_rows<T>(dyln, x, gain, shift, mean, rstd, dx, add, xln, part, M, K, st);
       if (blocks < 0) return blocks;
       if (db && N <= 2048) {

@@ -59,7 +59,7 @@ constexpr int kWS = 3;                           // weight stages: a stage is re
 struct TbP {
   int64_t M; int inner, n_mt, n_ch;
   uint32_t ab_fmt;
-  const void *x, *gamma, *beta;
+  const void *gamma, *beta;
   const float *mean, *rstd;
   float* part;                                   // [gridDim.x][2 K]
   int* status;
@@ -457,7 +457,7 @@ int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, flo
   p.n_mt = (int)((a.M + kRows - 1) / kRows);
   p.n_ch = a.inner / kHC;
   p.ab_fmt = a.dtype == MF_BF16 ? 1u : 0u;
-  p.x = a.x; p.gamma = a.ln_w; p.beta = a.ln_b; p.mean = a.mean; p.rstd = a.rstd;
+  p.gamma = a.ln_w; p.beta = a.ln_b; p.mean = a.mean; p.rstd = a.rstd;
   p.part = part;
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");

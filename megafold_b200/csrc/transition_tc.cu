@@ -43,7 +43,7 @@ struct TrP {
   float eps;
   uint32_t ab_fmt;
   int has_ln;
-  const void *x, *gamma, *beta;
+  const void *gamma, *beta;
   float *mean, *rstd;
   int* status;
 };
@@ -54,17 +54,6 @@ struct Bars {
   uint64_t h_full[2], h_empty[2], g_full[2], g_empty[2], y_full, y_empty;
 };
 
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, const void* src, int c0, int c1) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(src)), "r"(c0), "r"(c1) : "memory");
-}
-__device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void bulk_wait_group_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-template <int N> __device__ __forceinline__ void bulk_wait_group() {
-  asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -395,7 +384,7 @@ int launch_tr(const mf_transition_fwd_args& a, cudaStream_t st) {
   p.eps = a.eps;
   p.ab_fmt = a.dtype == MF_BF16 ? 1u : 0u;
   p.has_ln = a.ln_w != nullptr;
-  p.x = a.x; p.gamma = a.ln_w; p.beta = a.ln_b;
+  p.gamma = a.ln_w; p.beta = a.ln_b;
   p.mean = a.mean; p.rstd = a.rstd;
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
