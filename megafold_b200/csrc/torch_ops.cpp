@@ -121,6 +121,7 @@ Tensor or_none(const OptTensor& t) { return t ? *t : Tensor(); }
 
 // The values themselves where a negation is still pending (the imaginary part of a conjugate, say): kernels read memory.
 Tensor plain(const Tensor& t) { return t.defined() && t.is_neg() ? t.resolve_neg() : t; }
+const Tensor& plain(const Tensor& t, Tensor& hold) { return t.defined() && t.is_neg() ? (hold = t.resolve_neg()) : t; }      // no copy of the handle
 
 // ---- conversions -------------------------------------------------------------------------------------------------
 // Brings each tensor to its wanted type (and to contiguous memory), all of them in one launch: mixed-precision calls
@@ -133,7 +134,7 @@ void cast_batch(std::initializer_list<Cast> list) {
   Tensor any;
   for (const Cast& c : list) {
     if (!c.t->defined()) continue;
-    *c.t = plain(*c.t);
+    if (c.t->is_neg()) *c.t = c.t->resolve_neg();
     if (!c.t->is_contiguous()) *c.t = c.t->contiguous();
     if (c.t->scalar_type() == c.to) continue;
     const auto from = c.t->scalar_type();
@@ -187,7 +188,9 @@ void fill_common(A& a, const Tensor& q, const Tensor& k, const Tensor& v, const 
 }
 
 std::tuple<Tensor, Tensor> evo_forward(const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& mask_, const OptTensor& bias_, int64_t flags) {
-  const Tensor q = plain(q_), k = plain(k_), v = plain(v_), mask = plain(or_none(mask_)), bias = plain(or_none(bias_));
+  const Tensor mask_t = or_none(mask_), bias_t = or_none(bias_);
+  Tensor hold[5];
+  const Tensor &q = plain(q_, hold[0]), &k = plain(k_, hold[1]), &v = plain(v_, hold[2]), &mask = plain(mask_t, hold[3]), &bias = plain(bias_t, hold[4]);
   require_cuda({&q, &k, &v, &mask, &bias});
   const auto s = check_shapes(q, k, v, mask_, bias_);
   const c10::cuda::CUDAGuard guard(q.device());
@@ -205,7 +208,9 @@ std::tuple<Tensor, Tensor> evo_forward(const Tensor& q_, const Tensor& k_, const
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> evo_backward(const Tensor& d_o_, const Tensor& q_, const Tensor& k_, const Tensor& v_, const OptTensor& mask_,
                                                         const OptTensor& bias_, const Tensor& o_, const Tensor& lse, int64_t flags, int64_t event) {
-  const Tensor q = plain(q_), k = plain(k_), v = plain(v_), mask = plain(or_none(mask_)), bias = plain(or_none(bias_));
+  const Tensor mask_t = or_none(mask_), bias_t = or_none(bias_);
+  Tensor hold[5];
+  const Tensor &q = plain(q_, hold[0]), &k = plain(k_, hold[1]), &v = plain(v_, hold[2]), &mask = plain(mask_t, hold[3]), &bias = plain(bias_t, hold[4]);
   require_cuda({&d_o_, &q, &k, &v, &mask, &bias, &o_, &lse});
   const auto s = check_shapes(q, k, v, mask_, bias_);
   const c10::cuda::CUDAGuard guard(q.device());
