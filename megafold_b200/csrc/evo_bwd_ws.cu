@@ -232,7 +232,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < 2; ++i) {
@@ -260,7 +260,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = tmem_base_s;
+  const uint32_t tm0 = uniform(tmem_base_s);
   const int nt = p.n_t;
   const bool dbuf = p.dbuf != 0;
   // TMEM: team t's scores S''^T at t*128 + [0,64), dP^T at t*128 + [64,128) (P^T / dS^T are packed over them);
@@ -718,7 +718,7 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < 3; ++i) {
@@ -738,7 +738,7 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = tmem_base_s;
+  const uint32_t tm0 = uniform(tmem_base_s);
   const int nt = p.n_t;
   // unit = ((b * H + h) * nt + jt) * nt + it, split `sp` of the rows
   struct Unit { int b, h, jt, it, n0, n1; };

@@ -116,7 +116,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int s = warp >> 2;                    // stream = warpgroup
   const int wg_tid = tid & 127;
   const bool leader = wg_tid == 0;

@@ -63,7 +63,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
   __shared__ __align__(16) float gain_s[LN ? kBM : 4], shift_s[LN ? kBM : 4];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < kStages; ++i) { mbar_init(&bar.full[i], 1); mbar_init(&bar.empty[i], 1); mbar_init(&bar.ready[i], 4); }
@@ -76,7 +76,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = tmem_base_s;
+  const uint32_t tm0 = uniform(tmem_base_s);
   const int n_items = p.m_tiles * p.n_tiles * p.k_splits;
   auto decode = [&](int item, int& mt, int& nt, int& s0, int& s1) {
     const int ks = item % p.k_splits, rest = item / p.k_splits;

@@ -66,7 +66,7 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
   __shared__ float gam_s[K], bet_s[K];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < 2; ++i) {
@@ -86,7 +86,7 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = tmem_base_s;
+  const uint32_t tm0 = uniform(tmem_base_s);
   // Register re-partition (the CTA is launched with 128 per thread): the issuer warpgroup keeps 40, the epilogue
   // warpgroups get 152 and the normalising warpgroup 168; 256 * 152 + 128 * 168 + 128 * 40 = 512 * 128 exactly.
   static_assert(256 * 152 + 128 * 168 + 128 * 40 <= kThreads * 128, "setmaxnreg budget");

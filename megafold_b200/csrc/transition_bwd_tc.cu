@@ -97,7 +97,7 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
   __shared__ float sum_s[4][2 * K];            // gain and shift sums over the rows of each row warp
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     mbar_init(&bar.x_full, 1); mbar_init(&bar.x_empty, 4); mbar_init(&bar.dy_full, 1); mbar_init(&bar.dy_empty, 4);
@@ -122,7 +122,7 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = tmem_base_s;
+  const uint32_t tm0 = uniform(tmem_base_s);
   // TMEM columns: two buffers of (H value 32 | H gate 32 | DG 32); dyln accumulator 128; LN(X) 64; dY 64; two dh of 32
   const uint32_t tHD = tm0, tACC = tm0 + 192, tA = tm0 + 320, tDY = tm0 + 384, tDH = tm0 + 448;
   const int my_tiles = p.n_mt > (int)blockIdx.x ? (p.n_mt - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;

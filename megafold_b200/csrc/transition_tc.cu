@@ -79,7 +79,7 @@ transition_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
   __shared__ __align__(16) float gam_s[K], bet_s[K];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     mbar_init(&bar.x_full, 1); mbar_init(&bar.x_empty, 4);
@@ -105,7 +105,7 @@ transition_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = tmem_base_s;
+  const uint32_t tm0 = uniform(tmem_base_s);
   // H: two buffers of (value 64 | gate 64); G: two of 32 (64 packed); Y: K columns; A: K / 2
   const uint32_t tH = tm0, tG = tm0 + 256, tY = tm0 + 320, tA = tm0 + 448;
   const int my_tiles = p.n_mt > (int)blockIdx.x ? (p.n_mt - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
