@@ -66,6 +66,7 @@ struct BwdWsP {
   int B, N, L, H, D;
   int n_t, n_items, lpad;
   int ksplit;            // work items per (b, n, h): the key tiles are split into this many ranges
+  int step[4];           // the grid size as (range, h, n, b) digits: from one item of a CTA to its next
   int dq_stream;         // dQ leaves the SM block by block (more query tiles than TMEM holds)
   int dbuf;              // dK/dV accumulators double-buffered over the key tiles
   float* dq_acc;         // fp32 [B,N,L,H,D] accumulator of dQ when ksplit > 1 or dq_stream
@@ -78,6 +79,28 @@ struct BwdWsP {
   void* dbias_direct;                       // N == 1 and a 16-bit d_pair_bias: dS is the answer, written by this kernel
   void *dq, *dk, *dv; TokenStrides gs;
   int* status;
+};
+
+// Work item of a CTA: a range of the key tiles of (b, n, h).  The first one is taken apart by divisions, the others are
+// stepped to: six divisions per item and role, executed once in 30000 cycles and so each time from a cold instruction cache,
+// took 1000 cycles.
+struct Item {
+  int sp, h, n, b;
+  __device__ __forceinline__ Item(int item, const BwdWsP& p) {
+    sp = item % p.ksplit;
+    const int bnh = item / p.ksplit, bn = bnh / p.H;
+    h = bnh - bn * p.H; b = bn / p.N; n = bn - b * p.N;
+  }
+  __device__ __forceinline__ void step(const BwdWsP& p) {
+    sp += p.step[0]; h += p.step[1]; n += p.step[2]; b += p.step[3];
+    if (sp >= p.ksplit) { sp -= p.ksplit; ++h; }
+    if (h >= p.H) { h -= p.H; ++n; }
+    if (n >= p.N) { n -= p.N; ++b; }
+  }
+  __device__ __forceinline__ int bn(const BwdWsP& p) const { return b * p.N + n; }
+  __device__ __forceinline__ int bnh(const BwdWsP& p) const { return bn(p) * p.H + h; }
+  __device__ __forceinline__ int jt0(const BwdWsP& p) const { return p.ksplit == 1 ? 0 : sp * p.n_t / p.ksplit; }
+  __device__ __forceinline__ int jt1(const BwdWsP& p) const { return p.ksplit == 1 ? p.n_t : (sp + 1) * p.n_t / p.ksplit; }
 };
 
 struct Bars {
@@ -268,11 +291,6 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   // (each accumulator has 32 columns per head half: dK = [0, 32 NH), dV = [32 NH, 64 NH) of a set)
   const uint32_t tKV = tm0 + 256, tDQ = tm0 + 256 + (dbuf ? 128 : 64) * NH;
   const uint32_t kv_set = dbuf ? 64 * NH : 0;    // column distance between the two dK|dV accumulator sets
-  // work item = (b, n, h, range of key tiles)
-  auto item_range = [&](int item, int& jt0, int& jt1) {
-    const int sp = item % p.ksplit;
-    jt0 = sp * nt / p.ksplit; jt1 = (sp + 1) * nt / p.ksplit;
-  };
 
   if (warp < kComputeWarps) {
     // ============================================================================ compute warps
@@ -290,25 +308,10 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     const int kv_which = NH == 1 ? w : (w >> 1), kv_hh = NH == 1 ? 0 : (w & 1);
     auto store_kv = [&](uint32_t kc, int j, int b, int n, int h) {
       tc_fence_after();
-      uint32_t o32[32];
-      tmem_ld32(tKV + (kc & 1) * kv_set + kv_which * 32 * NH + kv_hh * 32 + lane_addr, o32);
-      tmem_ld_wait();
+      T* out = static_cast<T*>(kv_which == 0 ? p.dk : p.dv) + p.gs.at(b, n, j) + h * p.D + kv_hh * 32;
+      store_rows(tKV + (kc & 1) * kv_set + kv_which * 32 * NH + kv_hh * 32 + lane_addr, kv_which == 0 ? p.scale : 1.f, out, p.gs.l, j,
+                 *abort_flag ? 0 : p.L, p.D - kv_hh * 32);
       tc_fence_before();
-      if (j < p.L && !*abort_flag) {
-        const float sc = kv_which == 0 ? p.scale : 1.f;
-        T* orow = static_cast<T*>(kv_which == 0 ? p.dk : p.dv) + p.gs.at(b, n, j) + h * p.D + kv_hh * 32;
-#pragma unroll
-        for (int d8 = 0; d8 < 4; ++d8) {
-          if (kv_hh * 32 + d8 * 8 < p.D) {
-            uint4 v;
-            v.x = Pack2<T>::pack(__uint_as_float(o32[d8 * 8]) * sc, __uint_as_float(o32[d8 * 8 + 1]) * sc);
-            v.y = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 2]) * sc, __uint_as_float(o32[d8 * 8 + 3]) * sc);
-            v.z = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 4]) * sc, __uint_as_float(o32[d8 * 8 + 5]) * sc);
-            v.w = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 6]) * sc, __uint_as_float(o32[d8 * 8 + 7]) * sc);
-            *reinterpret_cast<uint4*>(orow + d8 * 8) = v;
-          }
-        }
-      }
     };
     // rows of a dQ accumulator (TMEM lane = query) added, scaled, to the fp32 dQ rows in global memory
     auto add_dq = [&](uint32_t tacc, int it2, int hh, int b, int n, int h) {
@@ -337,14 +340,14 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     int item_no = 0;
     int pend_j = -1; uint32_t pend_kc = 0; int pend_b = 0, pend_n = 0, pend_h = 0;   // deferred dK/dV write-out
     int dqp_it = -1; uint32_t dqp_g = 0; int dqp_b = 0, dqp_n = 0, dqp_h = 0;        // deferred streamed dQ
-    int special_next = blockIdx.x < p.n_items ? p.flags[blockIdx.x / p.ksplit] : 0;
+    Item at(blockIdx.x, p);
+    int special_next = p.flags[at.bnh(p)];
     for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++item_no) {
-      const int bnh = item / p.ksplit;
-      int jt0, jt1; item_range(item, jt0, jt1);
-      const int h = bnh % p.H, bn = bnh / p.H, n = bn % p.N, b = bn / p.N;
+      const int h = at.h, n = at.n, b = at.b, jt0 = at.jt0(p), jt1 = at.jt1(p);
       const int sbuf = item_no & 1;
       const bool special = special_next != 0;      // every key of the row is masked: the item takes the careful path
-      if (item + (int)gridDim.x < p.n_items) special_next = p.flags[(item + (int)gridDim.x) / p.ksplit];
+      at.step(p);
+      if (item + (int)gridDim.x < p.n_items) special_next = p.flags[at.bnh(p)];
       for (int jt = jt0; jt < jt1; ++jt, ++kv_cnt) {
         const int j = jt * kT + r;
         const float p_uniform = j < p.L ? p.inv_L : 0.f;       // careful path: P of a fully masked row
@@ -443,25 +446,10 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             add_dq(tDQ + it * 32 * NH, it, hh, b, n, h);
           } else {
             tc_fence_after();
-            uint32_t o32[32];
-            tmem_ld32(tDQ + it * 32 * NH + hh * 32 + lane_addr, o32);
-            tmem_ld_wait();
-            tc_fence_before();
             const int i = it * kT + r;
-            if (i < p.L && !*abort_flag) {
-              T* orow = static_cast<T*>(p.dq) + p.gs.at(b, n, i) + h * p.D + hh * 32;
-#pragma unroll
-              for (int d8 = 0; d8 < 4; ++d8) {
-                if (hh * 32 + d8 * 8 < p.D) {
-                  uint4 v;
-                  v.x = Pack2<T>::pack(__uint_as_float(o32[d8 * 8]) * p.scale, __uint_as_float(o32[d8 * 8 + 1]) * p.scale);
-                  v.y = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 2]) * p.scale, __uint_as_float(o32[d8 * 8 + 3]) * p.scale);
-                  v.z = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 4]) * p.scale, __uint_as_float(o32[d8 * 8 + 5]) * p.scale);
-                  v.w = Pack2<T>::pack(__uint_as_float(o32[d8 * 8 + 6]) * p.scale, __uint_as_float(o32[d8 * 8 + 7]) * p.scale);
-                  *reinterpret_cast<uint4*>(orow + d8 * 8) = v;
-                }
-              }
-            }
+            T* out = static_cast<T*>(p.dq) + p.gs.at(b, n, i) + h * p.D + hh * 32;
+            store_rows(tDQ + it * 32 * NH + hh * 32 + lane_addr, p.scale, out, p.gs.l, i, *abort_flag ? 0 : p.L, p.D - hh * 32);
+            tc_fence_before();
           }
         }
       }
@@ -488,9 +476,9 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       const uint32_t id_kv = idesc_f16(128, 32, p.fmt, 0, 1);
       MF_TRACE_DECL(tr, 2, blockIdx.x == 0 && lane == 0);
       uint32_t g = 0, kv = 0, qslot = 0;
-      for (int item = blockIdx.x; item < p.n_items && !dead(); item += gridDim.x) {
-        int jt0, jt1; item_range(item, jt0, jt1);
-        for (int jt = jt0; jt < jt1 && !dead(); ++jt, ++kv) {
+      Item at(blockIdx.x, p);
+      for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, at.step(p)) {
+        for (int jt = at.jt0(p), jt1 = at.jt1(p); jt < jt1; ++jt, ++kv) {
           if (!dbuf && kv > 0) wait_or_flag(&bar.kv_drained, (kv - 1) & 1, abort_flag);
           const uint32_t tdk = tKV + (kv & 1) * kv_set, tdv = tdk + 32 * NH;
           for (int it = 0; it < nt && !dead(); ++it, ++g) {
@@ -531,11 +519,12 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       const uint32_t ds_base = desc_lo(smem_u32(sDS), kAtomB);
       uint32_t g = 0, kv = 0;
       int item_no = 0;
-      for (int item = blockIdx.x; item < p.n_items && !dead(); item += gridDim.x, ++item_no) {
-        int jt0, jt1; item_range(item, jt0, jt1);
+      Item at(blockIdx.x, p);
+      for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++item_no, at.step(p)) {
+        const int jt0 = at.jt0(p), jt1 = at.jt1(p);
         // the on-chip dQ accumulators of the previous item must have been read out before they start afresh
         if (!DQS && item_no > 0) wait_or_flag(&bar.item_done[(item_no - 1) & 1], ((item_no - 1) >> 1) & 1, abort_flag);
-        for (int jt = jt0; jt < jt1 && !dead(); ++jt, ++kv) {
+        for (int jt = jt0; jt < jt1; ++jt, ++kv) {
           const uint32_t k_lo = kv_base + (kv % NKV) * kStage16;
           for (int it = 0; it < nt && !dead(); ++it, ++g) {
             wait_or_flag(&bar.ds_written[g & 1], (g >> 1) & 1, abort_flag);
@@ -570,9 +559,9 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       const bool two_terms = p.n_alpha > 1;
       MF_TRACE_DECL(tr, 3, blockIdx.x == 0 && lane == 0);
       uint32_t g = 0, kv = 0, bslot = 0, buse = 0, qslot = 0, quse = 0;
-      for (int item = blockIdx.x; item < p.n_items && !dead(); item += gridDim.x) {
-        int jt0, jt1; item_range(item, jt0, jt1);
-        for (int jt = jt0; jt < jt1 && !dead(); ++jt, ++kv) {
+      Item at(blockIdx.x, p);
+      for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, at.step(p)) {
+        for (int jt = at.jt0(p), jt1 = at.jt1(p); jt < jt1; ++jt, ++kv) {
           wait_or_flag(&bar.kv_full[kv % NKV], (kv / NKV) & 1, abort_flag);
           const uint32_t k_lo = kv_base + (kv % NKV) * kStage16, v_lo = k_lo + kOp2, xk_lo = k_lo + kTerm16;
           for (int it = 0; it < nt && !dead(); ++it, ++g) {
@@ -618,12 +607,10 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     } else if (warp == kComputeWarps + 1) {
       // ========================================================================== TMA producer, in order of need
       uint32_t g = 0, kv = 0, bslot = 0, buse = 0, nbt = 0, qslot = 0, quse = 0;
-      int item_no = 0;
-      for (int item = blockIdx.x; item < p.n_items && !dead(); item += gridDim.x, ++item_no) {
-        const int bnh = item / p.ksplit;
-        int jt0, jt1; item_range(item, jt0, jt1);
-        const int h = bnh % p.H, bn = bnh / p.H, n = bn % p.N, b = bn / p.N;
-        for (int jt = jt0; jt < jt1 && !dead(); ++jt, ++kv) {
+      Item at(blockIdx.x, p);
+      for (int item = blockIdx.x; item < p.n_items && !dead(); item += gridDim.x, at.step(p)) {
+        const int h = at.h, n = at.n, b = at.b, bn = at.bn(p), bnh = at.bnh(p);
+        for (int jt = at.jt0(p), jt1 = at.jt1(p); jt < jt1 && !dead(); ++jt, ++kv) {
           if (kv >= (uint32_t)NKV) wait_or_flag(&bar.kv_empty[kv % NKV], ((kv / NKV) - 1) & 1, abort_flag);
           if (dead()) break;
           if (elect_one()) {
@@ -1108,6 +1095,9 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
     p.B = a.B; p.N = a.N; p.L = a.L; p.H = a.H; p.D = a.D;
     p.n_t = pl.nt; p.lpad = lpad; p.ksplit = pl.ksplit; p.dq_stream = pl.dq_stream; p.dbuf = pl.dbuf;
     p.n_items = a.B * a.N * a.H * pl.ksplit;
+    int grid = sm_count();
+    if (grid > p.n_items) grid = p.n_items;
+    p.step[0] = grid % pl.ksplit; p.step[1] = grid / pl.ksplit % a.H; p.step[2] = grid / pl.ksplit / a.H % a.N; p.step[3] = grid / pl.ksplit / a.H / a.N;
     p.dq_acc = dq_acc;
     p.scale = 1.0f / sqrtf((float)a.D); p.c1 = kLog2e * p.scale; p.inv_L = 1.0f / a.L;
     p.fmt = a.dtype == MF_BF16 ? 1u : 0u; p.bfmt = bt_dtype == MF_BF16 ? 1u : 0u;
@@ -1118,8 +1108,6 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
     p.dq = a.dq; p.dk = a.dk; p.dv = a.dv; p.gs = token_strides(lay.d_qkv);
     p.status = status;
     const size_t smem = Geo<NH>::kMainSmem;
-    int grid = sm_count();
-    if (grid > p.n_items) grid = p.n_items;
     if (pl.dq_stream) {
       constexpr auto kern = evo_bwd_ws_kernel<T, TT, true, NH>;
       if (int e = opt_in_smem<kern>(smem)) return e;

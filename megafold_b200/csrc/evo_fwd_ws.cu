@@ -167,39 +167,11 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     T* o_done = nullptr;
     float* lse_done = nullptr;
     auto wait_step = [&](uint32_t v) { wait_or_flag(&bar.step_done[v & 1], (v >> 1) & 1, abort_flag); tc_fence_after(); };
-    // O / l and the log-sum-exp of the item before, whose last product is complete.  Four lanes exchange their 16-byte pieces,
-    // so that a store instruction writes whole rows of eight tokens instead of a piece of 32.
+    // O / l and the log-sum-exp of the item before, whose last product is complete
     auto write_out = [&]() {
-      const float inv = 1.f / l_done;
-      uint32_t w[4][4];                            // [piece of eight columns][word]
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        uint32_t o16[16];
-        tmem_ld16(tO + hf * 16, o16);
-        tmem_ld_wait();
-#pragma unroll
-        for (int e = 0; e < 8; ++e) w[hf * 2 + e / 4][e % 4] = Pack2<T>::pack(__uint_as_float(o16[2 * e]) * inv, __uint_as_float(o16[2 * e + 1]) * inv);
-      }
-      const int q = lane & 3;
-#pragma unroll
-      for (int s2 = 2; s2 > 0; s2 >>= 1) {         // 4 x 4 transposition over lanes q
-        const bool up = q & s2;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c & s2) continue;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[c][e] : w[c + s2][e], s2);
-            if (up) w[c][e] = got; else w[c + s2][e] = got;
-          }
-        }
-      }
-      if (*abort_flag) return;
-      T* piece = o_done + q * 8;
-#pragma unroll
-      for (int c = 0; c < 4; ++c)                  // w[c]: piece q of row i_done - q + c
-        if (i_done - q + c < p.L && q * 8 < p.D)
-          *reinterpret_cast<uint4*>(piece + (c - q) * p.os.l) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+      const bool gone = *abort_flag;
+      store_rows(tO, 1.f / l_done, o_done, p.os.l, i_done, gone ? 0 : p.L, p.D);
+      if (gone) return;
       // a row whose keys are all masked has every logit at the mask term (about -1e30): uniform attention over its L
       // keys; its log-sum-exp is stored as -FLT_MAX, the value the backward kernels recognise
       if (i_done < p.L) *lse_done = m_done <= -1e28f ? -FLT_MAX : (m_done * p.c1 + lg2f(l_done)) * kLn2;

@@ -136,6 +136,41 @@ template <> struct Pack2<float> {   // only so that code templated on the bias t
   static __device__ __forceinline__ float2 unpack(uint32_t u) { return make_float2(__uint_as_float(u), 0.f); }
 };
 
+// 32 fp32 columns of a TMEM accumulator, scaled, to rows of a 16-bit tensor.  Called by a whole warp; a lane holds row `i` (nothing
+// is written where i >= L), whose first `left` columns (a multiple of 8) start at `out`, rows being `stride` elements apart.  Four
+// lanes exchange their 16-byte pieces, so that a store instruction writes whole rows of eight tokens: with every lane writing
+// its own row each instruction touches 32 lines, and the twelve warps that write out dQ took 2500 cycles.
+template <typename T>
+__device__ __forceinline__ void store_rows(uint32_t tacc, float sc, T* out, int64_t stride, int i, int L, int left) {
+  uint32_t w[4][4];                            // [piece of eight columns][word]
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    uint32_t o16[16];
+    tmem_ld16(tacc + hf * 16, o16);
+    tmem_ld_wait();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[hf * 2 + e / 4][e % 4] = Pack2<T>::pack(__uint_as_float(o16[2 * e]) * sc, __uint_as_float(o16[2 * e + 1]) * sc);
+  }
+  const int q = threadIdx.x & 3;
+#pragma unroll
+  for (int s2 = 2; s2 > 0; s2 >>= 1) {         // 4 x 4 transposition over lanes q
+    const bool up = q & s2;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c & s2) continue;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[c][e] : w[c + s2][e], s2);
+        if (up) w[c][e] = got; else w[c + s2][e] = got;
+      }
+    }
+  }
+  T* piece = out + q * 8;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)                  // w[c]: piece q of row i - q + c
+    if (i - q + c < L && q * 8 < left) *reinterpret_cast<uint4*>(piece + (c - q) * stride) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+}
+
 // 3-D and 4-D tiled TMA loads
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
