@@ -7,7 +7,7 @@
 //   P^T   = 2^(c1 * S''^T)                              dS^T   = P^T dP''^T                 term is itself a product with
 //   alpha * I, and the key mask, the log-sum-exp and delta enter through one more K = 16 product: evo_tc_common.cuh)
 //
-// evo_bwd_ws_kernel (dQ, dK, dV).  A persistent CTA owns a (b, n, h) - or a range of its key tiles - and walks the
+// evo_bwd_ws_kernel (dQ, dK, dV).  A persistent CTA (768 threads) owns a (b, n, h) - or a range of its key tiles - and walks the
 // key tiles j and, inside, the query tiles i in HALF blocks of [128 keys x 64 queries].  Two teams of eight compute
 // warps take alternate half blocks, each with its own score buffers in TMEM, so that the tensor pipe works on one
 // team's products while the other team exponentiates.  A thread (key row, 32 query columns) writes packed 16-bit
@@ -57,10 +57,13 @@ template <int NH> struct Geo {
 };
 static_assert(Geo<2>::kMainSmem + 1024 <= 227 * 1024 && Geo<1>::kMainSmem + 1024 <= 227 * 1024, "shared memory of the main kernel");
 static_assert(Geo<2>::kDbSmem + 1024 <= 227 * 1024 && Geo<1>::kDbSmem + 1024 <= 227 * 1024, "shared memory of the dBias kernel");
-// registers per thread: at launch (640 threads) / compute warps / helper warps after setmaxnreg.  The raise of the
-// compute warps can only draw on what the helper warps release inside the CTA - otherwise it never returns.
+constexpr int kMainThreads = kThreads + 128;      // the main kernel has four write-out warps besides
+// registers per thread: at launch / compute warps / helper (and write-out) warps after setmaxnreg.  The raise of the
+// compute warps can only draw on what the others release inside the CTA - otherwise it never returns.
 constexpr int kLaunchRegs = 96, kComputeRegs = 104, kHelperRegs = 64;
 static_assert(kComputeWarps * 32 * kComputeRegs + 128 * kHelperRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
+constexpr int kMainLaunchRegs = 80, kMainComputeRegs = 96, kMainHelperRegs = 48;
+static_assert(kComputeWarps * 32 * kMainComputeRegs + 256 * kMainHelperRegs <= kMainThreads * kMainLaunchRegs, "setmaxnreg budget");
 
 struct BwdWsP {
   int B, N, L, H, D;
@@ -107,9 +110,9 @@ struct Bars {
   uint64_t kv_full[2], kv_empty[2], qd_full[3], qd_empty[3], bt_full[3], bt_empty[3];
   uint64_t sd_ready[2], written[2], buf_free[2];
   uint64_t ds_written[2], dq_done[2];        // per block parity: dS^T tile complete in shared memory / its dQ product complete
-  uint64_t kv_done;                          // the dK / dV accumulation of a key tile is complete
-  uint64_t item_done[2];                     // the compute warps have read the item's on-chip dQ accumulators
-  uint64_t kv_drained, dq_drained[2];
+  uint64_t kv_done[2], kv_drained[2];        // by parity: the dK / dV accumulation of a key tile is complete / has been read out
+  uint64_t item_done[2];                     // the item's on-chip dQ accumulators have been read out
+  uint64_t dq_drained[2];
 };
 
 // 1-D bulk copy global -> shared, completion counted in bytes on `bar` (addresses and size multiples of 16 bytes)
@@ -237,7 +240,7 @@ __device__ __forceinline__ void p_and_ds(const uint32_t (&sr)[16], const uint32_
 }
 
 template <typename T, typename TB, bool DQS, int NH>      // DQS: dQ streamed block by block through global memory
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kMainThreads, 1)
 evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                   const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mg,
                   const __grid_constant__ CUtensorMap mbt, const BwdWsP p MF_TRACE_PARAM) {
@@ -263,20 +266,19 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       mbar_init(&bar.sd_ready[i], 1); mbar_init(&bar.written[i], kComputeWarps / 2);
       mbar_init(&bar.buf_free[i], 1);
       mbar_init(&bar.ds_written[i], kComputeWarps); mbar_init(&bar.dq_done[i], 1);
-      mbar_init(&bar.item_done[i], kComputeWarps);
-      mbar_init(&bar.dq_drained[i], 4 * NH);
+      mbar_init(&bar.item_done[i], 4);
+      mbar_init(&bar.dq_drained[i], 4);
+      mbar_init(&bar.kv_done[i], 1); mbar_init(&bar.kv_drained[i], 4);
     }
     for (int i = 0; i < 3; ++i) {
       mbar_init(&bar.qd_full[i], 1); mbar_init(&bar.qd_empty[i], 1); mbar_init(&bar.bt_full[i], 1); mbar_init(&bar.bt_empty[i], 1);
     }
-    mbar_init(&bar.kv_done, 1);
-    mbar_init(&bar.kv_drained, 8 * NH);
     mbar_fence_init();
     prefetch_tmap(&mq); prefetch_tmap(&mk); prefetch_tmap(&mv); prefetch_tmap(&mg); prefetch_tmap(&mbt);
   }
-  write_alpha_identity<TB>(sI, p.alpha[0], tid, kThreads);
-  write_alpha_identity<TB>(sI + 1024, p.alpha[1], tid, kThreads);
-  write_xc_tile(sXC, tid, kThreads);
+  write_alpha_identity<TB>(sI, p.alpha[0], tid, kMainThreads);
+  write_alpha_identity<TB>(sI + 1024, p.alpha[1], tid, kMainThreads);
+  write_xc_tile(sXC, tid, kMainThreads);
   fence_async_smem();
   if (warp == 0) { tmem_alloc(&tmem_base_s, 512); tmem_relinquish(); }
   tc_fence_before();
@@ -294,61 +296,23 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
 
   if (warp < kComputeWarps) {
     // ============================================================================ compute warps
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kComputeRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kMainComputeRegs));
     const int team = warp >> 3;                       // takes the half blocks with (half == team)
     const int ch = (warp >> 2) & 1;                   // which 32 of the half block's 64 query columns
-    const int w = warp >> 2;                          // 0..3: role in the write-out of accumulators
     const int r = (warp & 3) * 32 + lane;             // TMEM lane = key row inside the tile
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tST = tm0 + team * 128 + ch * 32 + lane_addr, tDP = tST + 64;
     MF_TRACE_DECL(tr, team, blockIdx.x == 0 && (warp == 0 || warp == 8) && lane == 0);
 
-    // dK (scaled) and dV rows of key `j` from accumulator set `kc`: the warps with w < 2 NH take one (dK or dV, head
-    // half) each
-    const int kv_which = NH == 1 ? w : (w >> 1), kv_hh = NH == 1 ? 0 : (w & 1);
-    auto store_kv = [&](uint32_t kc, int j, int b, int n, int h) {
-      tc_fence_after();
-      T* out = static_cast<T*>(kv_which == 0 ? p.dk : p.dv) + p.gs.at(b, n, j) + h * p.D + kv_hh * 32;
-      store_rows(tKV + (kc & 1) * kv_set + kv_which * 32 * NH + kv_hh * 32 + lane_addr, kv_which == 0 ? p.scale : 1.f, out, p.gs.l, j,
-                 *abort_flag ? 0 : p.L, p.D - kv_hh * 32);
-      tc_fence_before();
-    };
-    // rows of a dQ accumulator (TMEM lane = query) added, scaled, to the fp32 dQ rows in global memory
-    auto add_dq = [&](uint32_t tacc, int it2, int hh, int b, int n, int h) {
-      tc_fence_after();
-      uint32_t o32[32];
-      tmem_ld32(tacc + hh * 32 + lane_addr, o32);
-      tmem_ld_wait();
-      tc_fence_before();
-      const int i = it2 * kT + r;
-      if (i < p.L && !*abort_flag) {
-        float* arow = p.dq_acc + ((((int64_t)b * p.N + n) * p.L + i) * p.H + h) * p.D + hh * 32;
-#pragma unroll
-        for (int d4 = 0; d4 < 8; ++d4)
-          if (hh * 32 + d4 * 4 < p.D)
-            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(arow + d4 * 4),
-                         "f"(__uint_as_float(o32[d4 * 4]) * p.scale), "f"(__uint_as_float(o32[d4 * 4 + 1]) * p.scale),
-                         "f"(__uint_as_float(o32[d4 * 4 + 2]) * p.scale), "f"(__uint_as_float(o32[d4 * 4 + 3]) * p.scale) : "memory");
-      }
-    };
-
-    // streamed dQ: which warps drain the accumulator of block g2, and which head half each takes
-    const int dq_hh = NH == 1 ? 0 : (w & 1);
-    auto dq_mine = [&](uint32_t g2) { return NH == 1 ? w == (int)(g2 & 3) : (w >> 1) == (int)(g2 & 1); };
     uint32_t g = 0;                 // full blocks seen by this CTA (both teams count every block)
-    uint32_t kv_cnt = 0;            // (item, j) pairs so far
-    int item_no = 0;
-    int pend_j = -1; uint32_t pend_kc = 0; int pend_b = 0, pend_n = 0, pend_h = 0;   // deferred dK/dV write-out
-    int dqp_it = -1; uint32_t dqp_g = 0; int dqp_b = 0, dqp_n = 0, dqp_h = 0;        // deferred streamed dQ
     Item at(blockIdx.x, p);
     int special_next = p.flags[at.bnh(p)];
-    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++item_no) {
-      const int h = at.h, n = at.n, b = at.b, jt0 = at.jt0(p), jt1 = at.jt1(p);
-      const int sbuf = item_no & 1;
+    for (int item = blockIdx.x; item < p.n_items; item += gridDim.x) {
+      const int h = at.h, b = at.b, jt0 = at.jt0(p), jt1 = at.jt1(p);
       const bool special = special_next != 0;      // every key of the row is masked: the item takes the careful path
       at.step(p);
       if (item + (int)gridDim.x < p.n_items) special_next = p.flags[at.bnh(p)];
-      for (int jt = jt0; jt < jt1; ++jt, ++kv_cnt) {
+      for (int jt = jt0; jt < jt1; ++jt) {
         const int j = jt * kT + r;
         const float p_uniform = j < p.L ? p.inv_L : 0.f;       // careful path: P of a fully masked row
         for (int it = 0; it < nt; ++it, ++g) {
@@ -401,66 +365,11 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           __syncwarp();
           if (lane == 0) mbar_arrive(&bar.ds_written[g & 1]);
           tr(6);
-          // ---- streamed dQ: the product of the previous block sits in accumulator (g - 1) & 1; the four warps with
-          // w == (g - 1) & 3 add it to global memory and hand the accumulator back
-          if constexpr (DQS) {
-            if (dqp_it >= 0 && dq_mine(dqp_g)) {
-              wait_or_flag(&bar.dq_done[dqp_g & 1], (dqp_g >> 1) & 1, abort_flag);
-              add_dq(tDQ + (dqp_g & 1) * 32 * NH, dqp_it, dq_hh, dqp_b, dqp_n, dqp_h);
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&bar.dq_drained[dqp_g & 1]);
-            }
-            dqp_it = it; dqp_g = g; dqp_b = b; dqp_n = n; dqp_h = h;
-          }
-          // ---- dK_j, dV_j of the key tile that finished one block ago (warps 0-7)
-          if (pend_j >= 0 && w < 2 * NH) {
-            wait_or_flag(&bar.kv_done, pend_kc & 1, abort_flag);
-            store_kv(pend_kc, pend_j, pend_b, pend_n, pend_h);
-            if (!dbuf) { __syncwarp(); if (lane == 0) mbar_arrive(&bar.kv_drained); }
-          }
-          pend_j = -1;
-          if (it == nt - 1) { pend_j = j; pend_kc = kv_cnt; pend_b = b; pend_n = n; pend_h = h; }
         }
       }
-      // ---- end of the item: the last key tile's dK/dV, the last streamed dQ, or every query tile's dQ
-      tr(7);
-      if (pend_j >= 0 && w < 2 * NH) {
-        wait_or_flag(&bar.kv_done, pend_kc & 1, abort_flag);
-        store_kv(pend_kc, pend_j, pend_b, pend_n, pend_h);
-        if (!dbuf) { __syncwarp(); if (lane == 0) mbar_arrive(&bar.kv_drained); }
-      }
-      pend_j = -1;
-      const uint32_t gl = g - 1;
-      wait_or_flag(&bar.dq_done[gl & 1], (gl >> 1) & 1, abort_flag);
-      if constexpr (DQS) {
-        if (dqp_it >= 0 && dq_mine(dqp_g)) {
-          add_dq(tDQ + (dqp_g & 1) * 32 * NH, dqp_it, dq_hh, dqp_b, dqp_n, dqp_h);
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bar.dq_drained[dqp_g & 1]);
-        }
-        dqp_it = -1;
-      } else {
-        for (int u = w; u < nt * NH; u += 4) {          // one (query tile, head half) accumulator per turn
-          const int it = u / NH, hh = u - it * NH;
-          if (p.ksplit > 1) {
-            add_dq(tDQ + it * 32 * NH, it, hh, b, n, h);
-          } else {
-            tc_fence_after();
-            const int i = it * kT + r;
-            T* out = static_cast<T*>(p.dq) + p.gs.at(b, n, i) + h * p.D + hh * 32;
-            store_rows(tDQ + it * 32 * NH + hh * 32 + lane_addr, p.scale, out, p.gs.l, i, *abort_flag ? 0 : p.L, p.D - hh * 32);
-            tc_fence_before();
-          }
-        }
-      }
-      // this item's on-chip dQ accumulators have been read out by this warp
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.item_done[sbuf]);
-      tr(8);
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kHelperRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMainHelperRegs));
     // The helper roles are run by whole warps (one elected lane issues: see mma_ss_el); every exit decision is a warp vote.
     auto dead = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };
     constexpr uint32_t hi64 = desc_hi(512, kSw64), hi128 = desc_hi(1024, kSw128);
@@ -474,12 +383,14 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       //   dV_j += P^T dO_i,  dK_j += dS^T Q_i   (A = packed P^T / dS^T in TMEM, B = the dO / Q rows of the half, MN-major;
       //   one group of four products per head half, into that half's 32 accumulator columns)
       const uint32_t id_kv = idesc_f16(128, 32, p.fmt, 0, 1);
+      const uint32_t n_set = dbuf ? 2 : 1;
       MF_TRACE_DECL(tr, 2, blockIdx.x == 0 && lane == 0);
       uint32_t g = 0, kv = 0, qslot = 0;
       Item at(blockIdx.x, p);
       for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, at.step(p)) {
         for (int jt = at.jt0(p), jt1 = at.jt1(p); jt < jt1; ++jt, ++kv) {
-          if (!dbuf && kv > 0) wait_or_flag(&bar.kv_drained, (kv - 1) & 1, abort_flag);
+          // the accumulators have been read out since their last key tile (the one before, or with two sets the one before that)
+          if (kv >= n_set) wait_or_flag(&bar.kv_drained[(kv - n_set) & 1], ((kv - n_set) >> 1) & 1, abort_flag);
           const uint32_t tdk = tKV + (kv & 1) * kv_set, tdv = tdk + 32 * NH;
           for (int it = 0; it < nt && !dead(); ++it, ++g) {
             const uint32_t q_lo = qd_base + qslot * kStage16, do_lo = q_lo + kOp2;
@@ -507,9 +418,81 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
               tr(22);
             }
             tc_commit_el(&bar.qd_empty[qslot]);
-            if (it == nt - 1) tc_commit_el(&bar.kv_done);
+            if (it == nt - 1) tc_commit_el(&bar.kv_done[kv & 1]);
             if (++qslot == NQ) qslot = 0;
           }
+        }
+      }
+    } else if (warp >= kComputeWarps + 4) {
+      // ========================================================================== write-out warps: accumulators to global memory
+      // The compute warps did this beside their blocks: a fifth of their time, with the wait for the last products at each
+      // item's end (forward + backward [1, 384, 384, 4, 32] 359 us, 338 now; at 768 2577 and 2508).
+      const int r = (warp & 3) * 32 + lane;             // TMEM lane: key row (dK, dV) or query row (dQ) inside the tile
+      const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+      MF_TRACE_DECL(tr, 4, blockIdx.x == 0 && warp == kComputeWarps + 4 && lane == 0);
+      uint32_t g = 0, kv = 0;
+      int item_no = 0;
+      Item at(blockIdx.x, p);
+      for (int item = blockIdx.x; item < p.n_items; item += gridDim.x, ++item_no, at.step(p)) {
+        // rows of a dQ accumulator added, scaled, to the fp32 dQ rows in global memory
+        auto add_dq = [&](uint32_t tacc, int it2, int hh) {
+          uint32_t o32[32];
+          tmem_ld32(tacc + hh * 32 + lane_addr, o32);
+          tmem_ld_wait();
+          const int i = it2 * kT + r;
+          if (i < p.L && !*abort_flag) {
+            float* arow = p.dq_acc + (((int64_t)at.bn(p) * p.L + i) * p.H + at.h) * p.D + hh * 32;
+#pragma unroll
+            for (int d4 = 0; d4 < 8; ++d4)
+              if (hh * 32 + d4 * 4 < p.D)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(arow + d4 * 4),
+                             "f"(__uint_as_float(o32[d4 * 4]) * p.scale), "f"(__uint_as_float(o32[d4 * 4 + 1]) * p.scale),
+                             "f"(__uint_as_float(o32[d4 * 4 + 2]) * p.scale), "f"(__uint_as_float(o32[d4 * 4 + 3]) * p.scale) : "memory");
+          }
+        };
+        for (int jt = at.jt0(p), jt1 = at.jt1(p); jt < jt1; ++jt, ++kv) {
+          for (int it = 0; it < nt; ++it, ++g) {
+            if constexpr (DQS) {                        // streamed dQ: the product of every block
+              wait_or_flag(&bar.dq_done[g & 1], (g >> 1) & 1, abort_flag);
+              tc_fence_after();
+#pragma unroll 1
+              for (int hh = 0; hh < NH; ++hh) add_dq(tDQ + (g & 1) * 32 * NH, it, hh);
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bar.dq_drained[g & 1]);
+            }
+          }
+          // dK_j (scaled) and dV_j
+          wait_or_flag(&bar.kv_done[kv & 1], (kv >> 1) & 1, abort_flag);
+          tc_fence_after();
+          const int j = jt * kT + r;
+          const int64_t row = p.gs.at(at.b, at.n, j) + at.h * p.D;
+#pragma unroll 1
+          for (int u = 0; u < 2 * NH; ++u) {            // (dK or dV, head half)
+            const int hh = u & (NH - 1);
+            const bool is_dk = u < NH;
+            store_rows(tKV + (kv & 1) * kv_set + u * 32 + lane_addr, is_dk ? p.scale : 1.f, static_cast<T*>(is_dk ? p.dk : p.dv) + row + hh * 32,
+                       p.gs.l, j, *abort_flag ? 0 : p.L, p.D - hh * 32);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar.kv_drained[kv & 1]);
+        }
+        if constexpr (!DQS) {                           // every query tile's dQ
+          const uint32_t gl = g - 1;
+          wait_or_flag(&bar.dq_done[gl & 1], (gl >> 1) & 1, abort_flag);
+          tc_fence_after();
+#pragma unroll 1
+          for (int u = 0; u < nt * NH; ++u) {           // (query tile, head half)
+            const int it = NH == 1 ? u : u >> 1, hh = u & (NH - 1), i = it * kT + r;
+            if (p.ksplit > 1) add_dq(tDQ + it * 32 * NH, it, hh);
+            else
+              store_rows(tDQ + u * 32 + lane_addr, p.scale, static_cast<T*>(p.dq) + p.gs.at(at.b, at.n, i) + at.h * p.D + hh * 32, p.gs.l, i,
+                         *abort_flag ? 0 : p.L, p.D - hh * 32);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar.item_done[item_no & 1]);
         }
       }
     } else if (warp == kComputeWarps + 3) {
@@ -1111,11 +1094,11 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
     if (pl.dq_stream) {
       constexpr auto kern = evo_bwd_ws_kernel<T, TT, true, NH>;
       if (int e = opt_in_smem<kern>(smem)) return e;
-      kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
+      kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     } else {
       constexpr auto kern = evo_bwd_ws_kernel<T, TT, false, NH>;
       if (int e = opt_in_smem<kern>(smem)) return e;
-      kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
+      kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     }
     MF_LAUNCHED("evo_bwd_ws_kernel");
     if (a.dbias_ready_event && dbias_direct) MF_CUDA(cudaEventRecord(static_cast<cudaEvent_t>(a.dbias_ready_event), st));
