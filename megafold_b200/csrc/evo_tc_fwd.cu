@@ -119,7 +119,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int s = warp >> 2;                    // stream = warpgroup
   const int wg_tid = tid & 127;
-  const bool leader = wg_tid == 0;
+  const bool leader = (warp & 3) == 0;
   if (tid == 0) {
     abort_s = 0;
     for (int q = 0; q < 2; ++q) {
@@ -151,7 +151,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   const int r = (warp & 3) * 32 + lane;                              // TMEM lane = query row in the tile
   const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t tS = tmem_base_s + s * 256 + lane_addr, tP = tS + 128, tO = tS + 192;
-  const uint32_t tS0 = tmem_base_s + s * 256;                      // lane 0 addresses for the MMA issuer
+  const uint32_t tS0 = uniform(tmem_base_s) + s * 256;                      // lane 0 addresses for the MMA issuer
   const uint32_t id_s = idesc_f16(128, kKT, p.ab_fmt, 0, 0);
   const uint32_t id_o = idesc_f16(128, DP, p.ab_fmt, 0, 1);
 
@@ -245,15 +245,15 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     const uint32_t q_lo = desc_lo(smem_u32(sQ), 16), k_lo = desc_lo(smem_u32(sK + (g % C::KS) * C::TILEB), 16);
 #pragma unroll
     for (int ks = 0; ks < DP / 16; ++ks)
-      mma_ss_lh(tS0, q_lo + ks * 2, desc_hi(C::SBO, C::SW), k_lo + ks * 2, desc_hi(C::SBO, C::SW), id_s, ks > 0);
-    tc_commit(&bar.s_ready);
+      mma_ss_el(tS0, q_lo + ks * 2, desc_hi(C::SBO, C::SW), k_lo + ks * 2, desc_hi(C::SBO, C::SW), id_s, ks > 0);
+    tc_commit_el(&bar.s_ready);
   };
   auto issue_pv = [&](int g) {    // O_tile(g) = P V(g)
     const uint32_t v_lo = desc_lo(smem_u32(sV + (g % kVS) * C::TILEB), 16);
 #pragma unroll
     for (int ks = 0; ks < kKT / 16; ++ks)
-      mma_ts_lh(tS0 + 192, tS0 + 128 + ks * 8, v_lo + ks * (16 * C::ROWB / 16), desc_hi(C::SBO, C::SW), id_o, ks > 0);
-    tc_commit(&bar.pv_done);
+      mma_ts_el(tS0 + 192, tS0 + 128 + ks * 8, v_lo + ks * (16 * C::ROWB / 16), desc_hi(C::SBO, C::SW), id_o, ks > 0);
+    tc_commit_el(&bar.pv_done);
   };
 
   if (g_total > 0) {
@@ -316,7 +316,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         wait_or_flag(&bar.q_full, item_local & 1, abort_flag);
         wait_or_flag(&bar.k_full[g % C::KS], (g / C::KS) & 1, abort_flag);
         tc_fence_after();
-        if (!*abort_flag) issue_s(g);
+        if (!__any_sync(0xffffffffu, *abort_flag)) issue_s(g);
       }
     }
     // ------------------------------------------------------------------ S(g) -> registers
@@ -336,7 +336,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       if (t + 1 < p.n_kt) {
         wait_or_flag(&bar.k_full[(g + 1) % C::KS], ((g + 1) / C::KS) & 1, abort_flag);
         tc_fence_after();
-        if (!*abort_flag) issue_s(g + 1);
+        if (!__any_sync(0xffffffffu, *abort_flag)) issue_s(g + 1);
       }
     }
     if (officer_kv) {
@@ -433,7 +433,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     if (leader) {
       wait_or_flag(&bar.v_full[g % kVS], (g / kVS) & 1, abort_flag);
       tc_fence_after();
-      if (!*abort_flag) issue_pv(g);
+      if (!__any_sync(0xffffffffu, *abort_flag)) issue_pv(g);
     }
     if (officer_kv) pump_v(g);          // P V(g-1) and earlier are known complete
     if (officer_b) pump_b();

@@ -222,11 +222,12 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
     }
   } else {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-  if (warp == 8 + kNormWarps && lane == 0) {
-    // ------------------------------------------------------------------------------------ MMA issuer
+  if (warp == 8 + kNormWarps) {
+    // ------------------------------------------------------------------------------------ MMA issuer (the whole warp: see mma_ss_el)
+    auto dead = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };
     const uint32_t idesc = idesc_f16(128, kNT, p.ab_fmt, 0, 1);     // A K-major, B MN-major
     uint32_t acc_cnt = 0, w_cnt = 0;
-    for (int t = 0; t < my_tiles && !*abort_flag; ++t) {
+    for (int t = 0; t < my_tiles && !dead(); ++t) {
       const int buf = t % kAStages;
       wait_or_flag(&bar.a_full[buf], (t / kAStages) & 1, abort_flag);
       const uint32_t a_lo = desc_lo(smem_u32(sA + buf * A_BYTES), 16);
@@ -235,16 +236,16 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
         wait_or_flag(&bar.w_full[ws], (w_cnt / kWStages) & 1, abort_flag);
         if (acc_cnt >= 2) wait_or_flag(&bar.acc_empty[ab], ((acc_cnt >> 1) - 1) & 1, abort_flag);
         tc_fence_after();
-        if (*abort_flag) break;
+        if (dead()) break;
         const uint32_t w_lo = desc_lo(smem_u32(sW + ws * W_BYTES), K * 128);
 #pragma unroll
         for (int ks = 0; ks < K / 16; ++ks)
-          mma_ss_lh(tm0 + ab * kNT, a_lo + (ks >> 2) * (kRows * 128 / 16) + (ks & 3) * 2, desc_hi(1024, kSw128),
+          mma_ss_el(tm0 + ab * kNT, a_lo + (ks >> 2) * (kRows * 128 / 16) + (ks & 3) * 2, desc_hi(1024, kSw128),
                     w_lo + ks * (2048 / 16), desc_hi(1024, kSw128), idesc, ks > 0);
-        tc_commit(&bar.acc_full[ab]);
-        tc_commit(&bar.w_empty[ws]);
+        tc_commit_el(&bar.acc_full[ab]);
+        tc_commit_el(&bar.w_empty[ws]);
       }
-      tc_commit(&bar.a_empty[buf]);
+      tc_commit_el(&bar.a_empty[buf]);
     }
   } else if (warp == 9 + kNormWarps && lane == 0) {
     // ------------------------------------------------------------------------------------ TMA producer of X and W tiles
