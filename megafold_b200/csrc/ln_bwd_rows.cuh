@@ -97,26 +97,30 @@ __device__ __forceinline__ void ln_bwd_row(const uint32_t (&dy)[CW], const uint4
   emit(o);
 }
 
-// The same for a thread that has all 128 columns of its row in registers.  at(c): where the raw columns 8 c .. 8 c + 7 of the
-// row lie in shared memory; dx replaces them.  sums: the gain and shift sums of the warp's rows so far, [2][128].
+// The same for two threads a row of 128 columns: thread `part` has the 32-column quarters part and part + 2 in registers (dy:
+// 32 columns of each).  at(q, c): where the raw columns 8 c .. 8 c + 7 of its q-th quarter lie in shared memory; dx replaces
+// them.  sums: the gain and shift sums of the 32 rows so far, [2][128].  red: [2 parts][4][128] float4; `barrier`: a named barrier
+// of the two warps that share 32 rows.
 template <typename T, typename At>
-__device__ __forceinline__ void ln_bwd_whole_row(uint32_t (&dy)[128], float mu, float rs, const float* gam, float* sums, int lane, At at) {
+__device__ __forceinline__ void ln_bwd_half_row(uint32_t (&dy)[64], float mu, float rs, const float* gam, float* sums, float4 (*red)[4][128],
+                                                int part, int row, int lane, int barrier, At at) {
   const float2 mm = make_float2(mu, mu), rr = make_float2(rs, rs);
   auto xhat = [&](uint32_t u) { return mul2(sub2(Pack2<T>::unpack(u), mm), rr); };
   auto grad_of = [&](int k) { return make_float2(__uint_as_float(dy[k]), __uint_as_float(dy[k + 1])); };
+  const float* g_of[2] = {gam + part * 32, gam + part * 32 + 64};
   // sums of four neighbouring columns, of groups i, i + 16 and i + 8, i + 24, then a tree over i: the butterfly's order
   float a1[8], a2[8];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {              // groups 2 j and 2 j + 1 of each quarter
-    float q1[4][2], q2[4][2];
+    float q1[2][2], q2[2][2];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const uint4 raw = *at(q * 4 + j);
+    for (int q = 0; q < 2; ++q) {
+      const uint4 raw = *at(q, j);
       const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int k = q * 32 + j * 8 + h * 4;
-        const float4 g = *reinterpret_cast<const float4*>(gam + k);
+        const int c = j * 8 + h * 4, k = q * 32 + c;
+        const float4 g = *reinterpret_cast<const float4*>(g_of[q] + c);
         const float2 w0 = mul2(grad_of(k), make_float2(g.x, g.y)), w1 = mul2(grad_of(k + 2), make_float2(g.z, g.w)), h0 = xhat(u[2 * h]), h1 = xhat(u[2 * h + 1]);
         q1[q][h] = __fmaf_rn(h1.y, w1.y, __fmaf_rn(h1.x, w1.x, __fmaf_rn(h0.y, w0.y, __fmul_rn(h0.x, w0.x))));
         q2[q][h] = __fadd_rn(__fadd_rn(__fadd_rn(w0.x, w0.y), w1.x), w1.y);
@@ -124,10 +128,23 @@ __device__ __forceinline__ void ln_bwd_whole_row(uint32_t (&dy)[128], float mu, 
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      a1[2 * j + h] = __fadd_rn(__fadd_rn(q1[0][h], q1[2][h]), __fadd_rn(q1[1][h], q1[3][h]));
-      a2[2 * j + h] = __fadd_rn(__fadd_rn(q2[0][h], q2[2][h]), __fadd_rn(q2[1][h], q2[3][h]));
+      a1[2 * j + h] = __fadd_rn(q1[0][h], q1[1][h]);
+      a2[2 * j + h] = __fadd_rn(q2[0][h], q2[1][h]);
     }
   }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    red[part][i][row] = make_float4(a1[4 * i], a1[4 * i + 1], a1[4 * i + 2], a1[4 * i + 3]);
+    red[part][2 + i][row] = make_float4(a2[4 * i], a2[4 * i + 1], a2[4 * i + 2], a2[4 * i + 3]);
+  }
+  named_sync(barrier, 64);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const float4 x = red[part ^ 1][i][row], y = red[part ^ 1][2 + i][row];
+    a1[4 * i] = __fadd_rn(a1[4 * i], x.x); a1[4 * i + 1] = __fadd_rn(a1[4 * i + 1], x.y); a1[4 * i + 2] = __fadd_rn(a1[4 * i + 2], x.z); a1[4 * i + 3] = __fadd_rn(a1[4 * i + 3], x.w);
+    a2[4 * i] = __fadd_rn(a2[4 * i], y.x); a2[4 * i + 1] = __fadd_rn(a2[4 * i + 1], y.y); a2[4 * i + 2] = __fadd_rn(a2[4 * i + 2], y.z); a2[4 * i + 3] = __fadd_rn(a2[4 * i + 3], y.w);
+  }
+  named_sync(barrier, 64);                   // both have read before the next tile writes
 #pragma unroll
   for (int h = 4; h > 0; h >>= 1)
 #pragma unroll
@@ -140,21 +157,21 @@ __device__ __forceinline__ void ln_bwd_whole_row(uint32_t (&dy)[128], float mu, 
     return (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, s);
   };
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 2; ++q) {
     float vg[16], vs[16];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       float p[2][8];
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        uint4* slot = at(q * 4 + half * 2 + j);
+        uint4* slot = at(q, half * 2 + j);
         const uint4 raw = *slot;
         const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
         uint32_t o[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int k = q * 32 + half * 16 + j * 8 + e * 2;
-          const float2 g = *reinterpret_cast<const float2*>(gam + k), h = xhat(u[e]), d = grad_of(k);
+          const int c = half * 16 + j * 8 + e * 2, k = q * 32 + c;
+          const float2 g = *reinterpret_cast<const float2*>(g_of[q] + c), h = xhat(u[e]), d = grad_of(k);
           const float2 t = make_float2(__fadd_rn(__fmul_rn(c1, h.x), c2), __fadd_rn(__fmul_rn(c1, h.y), c2));      // (packed, the two would be fused)
           const float2 z = mul2(fma2(d, g, make_float2(-t.x, -t.y)), rr);
           o[e] = Pack2<T>::pack(z.x, z.y);
@@ -173,8 +190,8 @@ __device__ __forceinline__ void ln_bwd_whole_row(uint32_t (&dy)[128], float mu, 
     for (int s = 8; s > 0; s >>= 1)
 #pragma unroll
       for (int i = 0; i < s; ++i) { vg[i] = fold(vg[i], vg[i + s], s); vs[i] = fold(vs[i], vs[i + s], s); }
-    sums[q * 32 + lane] += vg[0];
-    sums[128 + q * 32 + lane] += vs[0];
+    sums[(part + 2 * q) * 32 + lane] += vg[0];
+    sums[128 + (part + 2 * q) * 32 + lane] += vs[0];
   }
 }
 

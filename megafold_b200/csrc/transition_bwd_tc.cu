@@ -17,22 +17,22 @@
 //                TMEM; g, dh in registers with one MUFU op per element; dh packed to TMEM (A operand of the dyln product,
 //                column order inside a chunk: [value 0-15 | gate 0-15 | value 16-31 | gate 16-31]), dh and g to shared-memory
 //                tiles that are TMA-stored.
-//   warps 16-19  rows: LayerNorm of the next X tile (thread per row, saved statistics) to TMEM, dY beside it; then this
+//   warps 16-23  rows, two threads a row: LayerNorm of the next X tile (saved statistics) to TMEM, dY beside it; then this
 //                tile's dyln row into registers, which frees the accumulator at once, and the LayerNorm backward of it while
 //                the workers are in the next tile.  dx replaces the raw row of x in shared memory and is TMA-stored.
-//   warp 20      MMAs of H(c) = A W1blocks (8 x N=64, the two blocks as the two swizzle atoms of one MN-major B operand)
+//   warp 24      MMAs of H(c) = A W1blocks (8 x N=64, the two blocks as the two swizzle atoms of one MN-major B operand)
 //                and DG(c) = dY W2block (8 x N=32) into one of two TMEM buffers.
-//   warp 21      TMA loads: X and dY tiles, per chunk the W1 value / gate blocks and the W2 block ([128 rows][32 columns],
-//                64-byte swizzle; three stages).
-//   warp 22      MMAs of dyln += dh(c) [W1 value block; W1 gate block]^T (4 x N=128; the same shared-memory blocks read
+//   warp 25      TMA loads: per chunk the W1 value / gate blocks and the W2 block ([128 rows][32 columns], 64-byte swizzle).
+//   warp 26      MMAs of dyln += dh(c) [W1 value block; W1 gate block]^T (4 x N=128; the same shared-memory blocks read
 //                K-major) once the workers have written dh(c).
-//   warp 23      TMA stores of the dh and g tiles of every chunk.
+//   warp 27      TMA stores of the dh and g tiles of every chunk.
 // (The workers doing the LayerNorm backward between two tiles, four threads a row, held up the dyln products, and with them
-// the weight stages, for 14000 cycles a tile: 341 us.)
+// the weight stages, for 14000 cycles a tile: 341 us.  One thread a row took 14000 to 20000 cycles for it, beside some 13000
+// for the LayerNorm of the next tile and its waits: as long as a tile, 286 us.)
 // dh is stored in that column order, a panel [M][64] per chunk; dW1 computed from it has its columns in the same order and is
 // put back by a small kernel.  (Panels, of g too: a chunk of a tile is one run of 16 KB.  128-byte pieces at the pitch of a
 // whole row took 25 us more.)
-// [262144, 128], inner 512: 303 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
+// [262144, 128], inner 512: 250 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
 // Every wait is bounded; on expiry the CTA raises a flag, drains and reports through mf_async_status().
 #include "ln_bwd_rows.cuh"
 
@@ -44,17 +44,20 @@ constexpr int kRows = 128;
 constexpr int K = 128;               // dim
 constexpr int kHC = 32;              // hidden (value) columns per chunk
 constexpr int kWorkWarps = 16;       // two teams of eight
-constexpr int kThreads = (kWorkWarps + 8) * 32;
+constexpr int kRowWarps = 8, kFirstIssuer = kWorkWarps + kRowWarps;         // row warps: two per 32 rows: the 32-column quarters 0 and 2, 1 and 3
+constexpr int kThreads = (kWorkWarps + kRowWarps + 4) * 32;
 // registers per thread: at launch / workers / row warps / issuers after setmaxnreg (the raises draw on the drop)
-constexpr int kLaunchRegs = 80, kWorkRegs = 72, kRowRegs = 160, kIssueRegs = 32;
-static_assert(kWorkWarps * 32 * kWorkRegs + 128 * kRowRegs + 128 * kIssueRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
+constexpr int kLaunchRegs = 72, kWorkRegs = 64, kRowRegs = 96, kIssueRegs = 56;
+static_assert(kWorkWarps * 32 * kWorkRegs + kRowWarps * 32 * kRowRegs + 128 * kIssueRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 constexpr int A_BYTES = kRows * K * 2;          // 32 KB: X or dY tile, two 64-column atoms
 constexpr int WB = K * 64;                       // 8 KB: one [128 rows][32 columns] weight block
-constexpr int W_BYTES = 3 * WB;                  // W1 value | W1 gate | W2
 constexpr int DH_BYTES = kRows * 128;            // [128 rows][64 columns] 16 bit
 constexpr int G_BYTES = kRows * 64;              // [128 rows][32 columns] 16 bit
-constexpr int kWS = 3;                           // weight stages: a stage is released only by the dyln GEMM of its chunk,
-                                                 // one chunk after its H / DG GEMMs, so two stages would stall the TMA refill
+// Weight stages.  The W1 blocks of a chunk (value | gate) are held from its H products to its dyln product, about 6000 cycles with
+// the copy, the W2 block only to its DG product.  With three stages of all three blocks a chunk took 2100 cycles, the time of
+// that loop by three (1600 now); the room came from X and dY, which take turns in one buffer.
+constexpr int kW1S = 4, kW2S = 3;
+constexpr int kSlabB = 32 * 64;                   // a row warp's [32 rows][32 columns] piece of X, dY or dx, 64-byte swizzle
 
 struct TbP {
   int64_t M; int inner, n_mt, n_ch;
@@ -66,9 +69,9 @@ struct TbP {
 };
 
 struct Bars {
-  uint64_t x_full, x_empty, dy_full, dy_empty, a_full, a_empty;
-  uint64_t w_full[kWS], w_empty[kWS];
-  uint64_t xr_full[4], hd_full[2], hd_empty[2], dh_full[2], dh_empty[2], st_done[2], acc_full, acc_empty;
+  uint64_t x_full[kRowWarps], dy_full[kRowWarps], a_full, a_empty;
+  uint64_t w1_full[kW1S], w1_empty[kW1S], w2_full[kW2S], w2_empty[kW2S];
+  uint64_t xr_full[kRowWarps], hd_full[2], hd_empty[2], dh_full[2], dh_empty[2], st_done[2], acc_full, acc_empty;
 };
 
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -79,18 +82,19 @@ __device__ __forceinline__ float tanh_approx(float x) {
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mdy,
+transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy,
                          const __grid_constant__ CUtensorMap mw1, const __grid_constant__ CUtensorMap mw2,
                          const __grid_constant__ CUtensorMap mdh, const __grid_constant__ CUtensorMap mg,
-                         const __grid_constant__ CUtensorMap mxr, const __grid_constant__ CUtensorMap mdx, const TbP p) {
+                         const __grid_constant__ CUtensorMap mx, const __grid_constant__ CUtensorMap mdx, const TbP p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sX = smem;                          // raw rows of X
-  uint8_t* sDY = sX + A_BYTES;                 // rows of dY
-  uint8_t* sW = sDY + A_BYTES;                 // [kWS] weight stages
-  uint8_t* sDH = sW + kWS * W_BYTES;           // [2] dh tiles
+  uint8_t* sX = smem;                          // raw rows of X, then rows of dY
+  uint8_t* sW1 = sX + A_BYTES;                 // [kW1S] value | gate blocks
+  uint8_t* sW2 = sW1 + kW1S * 2 * WB;          // [kW2S]
+  uint8_t* sDH = sW2 + kW2S * WB;              // [2] dh tiles
   uint8_t* sG = sDH + 2 * DH_BYTES;            // [2] g tiles
   uint8_t* sXR = sG + 2 * G_BYTES;             // rows of X once more, then rows of dx
+  float4 (*red)[4][128] = reinterpret_cast<float4 (*)[4][128]>(sXR + A_BYTES);      // [2] row sums, exchanged by the row warps
 
   __shared__ Bars bar;
   __shared__ __align__(16) float gam_s[K], bet_s[K];
@@ -100,17 +104,17 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
-    mbar_init(&bar.x_full, 1); mbar_init(&bar.x_empty, 4); mbar_init(&bar.dy_full, 1); mbar_init(&bar.dy_empty, 4);
-    mbar_init(&bar.a_full, 4); mbar_init(&bar.a_empty, 1);
+    mbar_init(&bar.a_full, kRowWarps); mbar_init(&bar.a_empty, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bar.hd_full[i], 1); mbar_init(&bar.hd_empty[i], 8);
       mbar_init(&bar.dh_full[i], 8); mbar_init(&bar.dh_empty[i], 1); mbar_init(&bar.st_done[i], 1);
     }
-    for (int i = 0; i < kWS; ++i) { mbar_init(&bar.w_full[i], 1); mbar_init(&bar.w_empty[i], 1); }
-    mbar_init(&bar.acc_full, 1); mbar_init(&bar.acc_empty, 4);
-    for (int i = 0; i < 4; ++i) mbar_init(&bar.xr_full[i], 1);
+    for (int i = 0; i < kW1S; ++i) { mbar_init(&bar.w1_full[i], 1); mbar_init(&bar.w1_empty[i], 1); }
+    for (int i = 0; i < kW2S; ++i) { mbar_init(&bar.w2_full[i], 1); mbar_init(&bar.w2_empty[i], 1); }
+    mbar_init(&bar.acc_full, 1); mbar_init(&bar.acc_empty, kRowWarps);
+    for (int i = 0; i < kRowWarps; ++i) { mbar_init(&bar.xr_full[i], 1); mbar_init(&bar.x_full[i], 1); mbar_init(&bar.dy_full[i], 1); }
     mbar_fence_init();
-    prefetch_tmap(&mx); prefetch_tmap(&mdy); prefetch_tmap(&mw1); prefetch_tmap(&mw2); prefetch_tmap(&mdh); prefetch_tmap(&mg); prefetch_tmap(&mxr); prefetch_tmap(&mdx);
+    prefetch_tmap(&mx); prefetch_tmap(&mdy); prefetch_tmap(&mw1); prefetch_tmap(&mw2); prefetch_tmap(&mdh); prefetch_tmap(&mg); prefetch_tmap(&mdx);
   }
   for (int k = tid; k < K; k += kThreads) {
     gam_s[k] = to_f(static_cast<const T*>(p.gamma)[k]);
@@ -189,18 +193,34 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.dh_full[team]);
     }
-  } else if (warp < kWorkWarps + 4) {
+  } else if (warp < kWorkWarps + kRowWarps) {
     // ---------------------------------------------------------------------------------- row warps
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
-    const int quarter = warp & 3;
-    uint64_t* xr_full = &bar.xr_full[quarter];
-    uint8_t* xr = sXR + quarter * 32 * 128;                // my 32 rows of the first 64 columns; the others are kRows * 128 further
+    const int quarter = warp & 3, part = (warp >> 2) & 1, me = part * 4 + quarter;      // rows 32 quarter .., columns 32 part .. and 64 + 32 part ..
+    uint64_t* xr_full = &bar.xr_full[me];
+    uint64_t* x_full = &bar.x_full[me];
+    uint64_t* dy_full = &bar.dy_full[me];
+    uint8_t* xr = sXR + me * 2 * kSlabB;
+    uint8_t* xd = sX + me * 2 * kSlabB;
     auto row_of = [&](int t) { return ((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows; };
-    uint32_t n_raw = 0;
-    auto load_raw = [&](int t) {                           // (lane 0) my rows of tile t for the write-out
+    auto slot = [&](uint8_t* slab, int q, int c) { return reinterpret_cast<uint4*>(slab + q * kSlabB + swz_offset(lane, c, 64)); };
+    uint32_t n_raw = 0, n_x = 0, n_dy = 0;
+    // (lane 0) my pieces of tile t: X and dY, in turn into one slab, each requested once the other is in registers; X once more
+    // for the write-out
+    auto load_x = [&](int t) {
+      ++n_x;
+      mbar_expect_tx(x_full, 2 * kSlabB);
+      for (int q = 0; q < 2; ++q) tma_load_2d(xd + q * kSlabB, &mx, x_full, q * 64 + part * 32, (int)row_of(t) + quarter * 32);
+    };
+    auto load_dy = [&](int t) {
+      ++n_dy;
+      mbar_expect_tx(dy_full, 2 * kSlabB);
+      for (int q = 0; q < 2; ++q) tma_load_2d(xd + q * kSlabB, &mdy, dy_full, q * 64 + part * 32, (int)row_of(t) + quarter * 32);
+    };
+    auto load_raw = [&](int t) {
       ++n_raw;
-      mbar_expect_tx(xr_full, 2 * 32 * 128);
-      for (int q = 0; q < K / 64; ++q) tma_load_2d(xr + q * (kRows * 128), &mxr, xr_full, q * 64, (int)row_of(t) + quarter * 32);
+      mbar_expect_tx(xr_full, 2 * kSlabB);
+      for (int q = 0; q < 2; ++q) tma_load_2d(xr + q * kSlabB, &mx, xr_full, q * 64 + part * 32, (int)row_of(t) + quarter * 32);
     };
     // LN(X) and dY of tile t to TMEM
     auto normalise = [&](int t) {
@@ -208,94 +228,102 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
       const bool ok = row < p.M;
       const float mu = ok ? p.mean[row] : 0.f, rs = ok ? p.rstd[row] : 0.f;     // saved by the forward pass
       const float2 mm = make_float2(mu, mu), rr = make_float2(rs, rs);
-      wait_or_flag(&bar.x_full, t & 1, abort_flag);
-      uint32_t o[K / 2];
+      wait_or_flag(x_full, t & 1, abort_flag);
+      uint32_t o[2][16];
 #pragma unroll
-      for (int c = 0; c < K / 8; ++c) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(sX + (c >> 3) * (kRows * 128) + swz_offset(row_l, c & 7, 128));
-        const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+      for (int q = 0; q < 2; ++q)
 #pragma unroll
-        for (int e = 0; e < 4; e += 2) {
-          const int k = c * 8 + e * 2;
-          const float4 ga = *reinterpret_cast<const float4*>(gam_s + k), be = *reinterpret_cast<const float4*>(bet_s + k);
-          const float2 y0 = fma2(mul2(sub2(Pack2<T>::unpack(u[e]), mm), rr), make_float2(ga.x, ga.y), make_float2(be.x, be.y));
-          const float2 y1 = fma2(mul2(sub2(Pack2<T>::unpack(u[e + 1]), mm), rr), make_float2(ga.z, ga.w), make_float2(be.z, be.w));
-          o[c * 4 + e] = ok ? Pack2<T>::pack(y0.x, y0.y) : 0u; o[c * 4 + e + 1] = ok ? Pack2<T>::pack(y1.x, y1.y) : 0u;
+        for (int c = 0; c < 4; ++c) {
+          const uint4 raw = *slot(xd, q, c);
+          const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            const int k = q * 64 + part * 32 + c * 8 + e * 2;
+            const float4 ga = *reinterpret_cast<const float4*>(gam_s + k), be = *reinterpret_cast<const float4*>(bet_s + k);
+            const float2 y0 = fma2(mul2(sub2(Pack2<T>::unpack(u[e]), mm), rr), make_float2(ga.x, ga.y), make_float2(be.x, be.y));
+            const float2 y1 = fma2(mul2(sub2(Pack2<T>::unpack(u[e + 1]), mm), rr), make_float2(ga.z, ga.w), make_float2(be.z, be.w));
+            o[q][c * 4 + e] = ok ? Pack2<T>::pack(y0.x, y0.y) : 0u; o[q][c * 4 + e + 1] = ok ? Pack2<T>::pack(y1.x, y1.y) : 0u;
+          }
         }
-      }
+      fence_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.x_empty);
+      if (lane == 0 && !*abort_flag) load_dy(t);
+      __syncwarp();
       if (t > 0) wait_or_flag(&bar.a_empty, (t - 1) & 1, abort_flag);      // the H / DG products of the previous tile
       tc_fence_after();
 #pragma unroll
-      for (int q = 0; q < K / 64; ++q) tmem_st32(tA + q * 32 + lane_addr, *reinterpret_cast<uint32_t (*)[32]>(o + q * 32));
-      wait_or_flag(&bar.dy_full, t & 1, abort_flag);
+      for (int q = 0; q < 2; ++q) tmem_st16(tA + q * 32 + part * 16 + lane_addr, o[q]);
+      wait_or_flag(dy_full, t & 1, abort_flag);
 #pragma unroll
-      for (int c = 0; c < K / 8; ++c) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(sDY + (c >> 3) * (kRows * 128) + swz_offset(row_l, c & 7, 128));
-        o[c * 4] = raw.x; o[c * 4 + 1] = raw.y; o[c * 4 + 2] = raw.z; o[c * 4 + 3] = raw.w;
-      }
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const uint4 raw = *slot(xd, q, c);
+          o[q][c * 4] = raw.x; o[q][c * 4 + 1] = raw.y; o[q][c * 4 + 2] = raw.z; o[q][c * 4 + 3] = raw.w;
+        }
+      fence_async_smem();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bar.dy_empty);
+      if (lane == 0 && t + 1 < my_tiles && !*abort_flag) load_x(t + 1);
+      __syncwarp();
 #pragma unroll
-      for (int q = 0; q < K / 64; ++q) tmem_st32(tDY + q * 32 + lane_addr, *reinterpret_cast<uint32_t (*)[32]>(o + q * 32));
+      for (int q = 0; q < 2; ++q) tmem_st16(tDY + q * 32 + part * 16 + lane_addr, o[q]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.a_full);
     };
     if (my_tiles > 0) {
-      if (lane == 0) load_raw(0);
+      if (lane == 0) { load_x(0); load_raw(0); }
+      __syncwarp();
       normalise(0);
     }
     for (int t = 0; t < my_tiles; ++t) {
       if (t + 1 < my_tiles) normalise(t + 1);
-      if (__any_sync(0xffffffffu, *abort_flag)) break;
       const int64_t row = row_of(t) + row_l;
       const bool ok = row < p.M;
       const float mu = ok ? p.mean[row] : 0.f, rs = ok ? p.rstd[row] : 0.f;
       wait_or_flag(xr_full, t & 1, abort_flag);
       wait_or_flag(&bar.acc_full, t & 1, abort_flag);
+      if (named_sync_or(1 + quarter, 64, *abort_flag)) break;          // the two warps that exchange sums leave together
       tc_fence_after();
-      uint32_t dy[K];
+      uint32_t dy[64];
 #pragma unroll
-      for (int q = 0; q < K / 32; ++q) tmem_ld32(tACC + q * 32 + lane_addr, *reinterpret_cast<uint32_t (*)[32]>(dy + q * 32));
+      for (int q = 0; q < 2; ++q) tmem_ld32(tACC + q * 64 + part * 32 + lane_addr, *reinterpret_cast<uint32_t (*)[32]>(dy + q * 32));
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.acc_empty);
-      ln_bwd_whole_row<T>(dy, mu, rs, gam_s, sum_s[quarter], lane,
-                          [&](int c) { return reinterpret_cast<uint4*>(xr + (c >> 3) * (kRows * 128) + swz_offset(lane, c & 7, 128)); });
+      ln_bwd_half_row<T>(dy, mu, rs, gam_s, sum_s[quarter], red, part, row_l, lane, 1 + quarter, [&](int q, int c) { return slot(xr, q, c); });
       fence_async_smem();
       __syncwarp();
       if (lane == 0) {
         if (row_of(t) + quarter * 32 < p.M)                 // never past the last row
-          for (int q = 0; q < K / 64; ++q) tma_store_2d(&mdx, xr + q * (kRows * 128), q * 64, (int)row_of(t) + quarter * 32);
+          for (int q = 0; q < 2; ++q) tma_store_2d(&mdx, xr + q * kSlabB, q * 64 + part * 32, (int)row_of(t) + quarter * 32);
         bulk_commit_group();
         bulk_wait_group_read<0>();
         if (t + 1 < my_tiles) load_raw(t + 1);
       }
       __syncwarp();
     }
-    if (lane == 0) { drain_ring(xr_full, n_raw, 1); bulk_wait_group<0>(); }
+    if (lane == 0) { drain_ring(xr_full, n_raw, 1); drain_ring(x_full, n_x, 1); drain_ring(dy_full, n_dy, 1); bulk_wait_group<0>(); }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kIssueRegs));
     auto dead = [&] { return __any_sync(0xffffffffu, *abort_flag) != 0; };      // the MMA roles are run by whole warps
-    if (warp == kWorkWarps + 4) {
+    if (warp == kFirstIssuer + 0) {
       // -------------------------------------------------------------------------------- MMA issuer: H and DG
       const uint32_t id_h = idesc_f16(128, 64, p.ab_fmt, 0, 1);     // B = W1 value|gate blocks MN-major, N = 64
       const uint32_t id_g = idesc_f16(128, 32, p.ab_fmt, 0, 1);     // A = dY, B = W2 block MN-major, N = 32
-      uint32_t ch_cnt = 0;
+      uint32_t ch_cnt = 0, s1 = 0, u1 = 0, s2 = 0, u2 = 0;          // stages and how often they have been used
       for (int t = 0; t < my_tiles; ++t) {
         wait_or_flag(&bar.a_full, t & 1, abort_flag);
         for (int c = 0; c < nch; ++c, ++ch_cnt) {
-          const int hb = ch_cnt & 1, ws = ch_cnt % kWS;
-          wait_or_flag(&bar.w_full[ws], (ch_cnt / kWS) & 1, abort_flag);
+          const int hb = ch_cnt & 1;
+          wait_or_flag(&bar.w1_full[s1], u1 & 1, abort_flag);
+          wait_or_flag(&bar.w2_full[s2], u2 & 1, abort_flag);
           if (ch_cnt >= 2) wait_or_flag(&bar.hd_empty[hb], ((ch_cnt >> 1) - 1) & 1, abort_flag);
           tc_fence_after();
           if (dead()) break;
-          const uint32_t w = smem_u32(sW + ws * W_BYTES);
-          const uint32_t wh_lo = desc_lo(w, WB), wg_lo = desc_lo(w + 2 * WB, 16);
+          const uint32_t wh_lo = desc_lo(smem_u32(sW1), WB) + s1 * (2 * WB / 16), wg_lo = desc_lo(smem_u32(sW2), 16) + s2 * (WB / 16);
 #pragma unroll
           for (int ks = 0; ks < K / 16; ++ks)      // H value | gate: the two blocks are the two atoms along N (LBO = WB)
             mma_ts_el(tHD + hb * 96, tA + ks * 8, wh_lo + ((ks * 1024) >> 4), desc_hi(512, kSw64), id_h, ks > 0);
@@ -303,15 +331,18 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           for (int ks = 0; ks < K / 16; ++ks)      // DG
             mma_ts_el(tHD + hb * 96 + 64, tDY + ks * 8, wg_lo + ((ks * 1024) >> 4), desc_hi(512, kSw64), id_g, ks > 0);
           tc_commit_el(&bar.hd_full[hb]);
+          tc_commit_el(&bar.w2_empty[s2]);
+          if (++s1 == kW1S) { s1 = 0; ++u1; }
+          if (++s2 == kW2S) { s2 = 0; ++u2; }
         }
         if (dead()) break;
         tc_commit_el(&bar.a_empty);      // the H / DG products of this tile are all issued: LN(X) and dY are free when they complete
       }
-    } else if (warp == kWorkWarps + 6) {
+    } else if (warp == kFirstIssuer + 2) {
       // -------------------------------------------------------------------------------- second MMA issuer: the dyln products
       // (one warp issuing both would wait for the workers' dh of one chunk before it could start the next chunk's H)
       const uint32_t id_a = idesc_f16(128, 128, p.ab_fmt, 0, 0);    // B = W1 blocks K-major, N = dim
-      uint32_t ch_cnt = 0;
+      uint32_t ch_cnt = 0, s1 = 0;
       for (int t = 0; t < my_tiles; ++t) {
         for (int c = 0; c < nch; ++c, ++ch_cnt) {                   // dyln (+)= dh(c) [W1v; W1g](c)^T
           const int hb = ch_cnt & 1;
@@ -319,18 +350,19 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           if (c == 0 && t > 0) wait_or_flag(&bar.acc_empty, (t - 1) & 1, abort_flag);
           tc_fence_after();
           if (dead()) break;
-          const uint32_t w_lo = desc_lo(smem_u32(sW + (ch_cnt % kWS) * W_BYTES), 16);
+          const uint32_t w_lo = desc_lo(smem_u32(sW1), 16) + s1 * (2 * WB / 16);
 #pragma unroll
           for (int ks = 0; ks < 4; ++ks)
             // k-step ks covers dh columns ks*16 .. +15: value (ks even) or gate (ks odd) columns (ks / 2) * 16 .. of the chunk
             mma_ts_el(tACC, tDH + hb * 32 + ks * 8, w_lo + (((ks & 1) * WB + (ks >> 1) * 32) >> 4), desc_hi(512, kSw64), id_a, c > 0 || ks > 0);
           tc_commit_el(&bar.dh_empty[hb]);
-          tc_commit_el(&bar.w_empty[ch_cnt % kWS]);
+          tc_commit_el(&bar.w1_empty[s1]);
+          if (++s1 == kW1S) s1 = 0;
         }
         if (dead()) break;
         tc_commit_el(&bar.acc_full);
       }
-    } else if (warp == kWorkWarps + 7 && lane == 0) {
+    } else if (warp == kFirstIssuer + 3 && lane == 0) {
       // -------------------------------------------------------------------------------- TMA stores of the dh / g tiles
       uint32_t ch_cnt = 0;
       for (int t = 0; t < my_tiles && !*abort_flag; ++t) {
@@ -342,46 +374,33 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_co
           tma_store_3d(&mdh, sDH + hb * DH_BYTES, 0, row0, c);               // rows >= M are clipped
           tma_store_3d(&mg, sG + hb * G_BYTES, (c & 1) * kHC, row0, c >> 1);
           bulk_commit_group();
-          bulk_wait_group_read<1>();
-          if (ch_cnt > 0) mbar_arrive(&bar.st_done[hb ^ 1]);                   // the chunk before this one has been read
+          bulk_wait_group_read<0>();
+          mbar_arrive(&bar.st_done[hb]);                                       // the tiles have been read
         }
       }
       bulk_wait_group<0>();
-    } else if (warp == kWorkWarps + 5 && lane == 0) {
+    } else if (warp == kFirstIssuer + 1 && lane == 0) {
       // -------------------------------------------------------------------------------- TMA producer
-      uint32_t ch_cnt = 0, n_x = 0, n_dy = 0;
-      auto load_rows = [&](int t) {           // (the normalising warps have taken tile t - 1)
-        const int row0 = (int)(((int64_t)blockIdx.x + (int64_t)t * gridDim.x) * kRows);
-        if (t > 0) wait_or_flag(&bar.x_empty, (t - 1) & 1, abort_flag);
-        if (*abort_flag) return;
-        ++n_x;
-        mbar_expect_tx(&bar.x_full, A_BYTES);
-        tma_load_2d(sX, &mx, &bar.x_full, 0, row0);
-        tma_load_2d(sX + kRows * 128, &mx, &bar.x_full, 64, row0);
-        if (t > 0) wait_or_flag(&bar.dy_empty, (t - 1) & 1, abort_flag);
-        if (*abort_flag) return;
-        ++n_dy;
-        mbar_expect_tx(&bar.dy_full, A_BYTES);
-        tma_load_2d(sDY, &mdy, &bar.dy_full, 0, row0);
-        tma_load_2d(sDY + kRows * 128, &mdy, &bar.dy_full, 64, row0);
-      };
-      if (my_tiles > 0) load_rows(0);
+      uint32_t n1 = 0, n2 = 0, s1 = 0, u1 = 0, s2 = 0, u2 = 0;
       for (int t = 0; t < my_tiles && !*abort_flag; ++t) {
-        for (int c = 0; c < nch; ++c, ++ch_cnt) {
-          if (c == (nch > 2 ? 2 : nch - 1) && t + 1 < my_tiles) load_rows(t + 1);
-          const int ws = ch_cnt % kWS;
-          uint8_t* w = sW + ws * W_BYTES;
-          if (ch_cnt >= kWS) wait_or_flag(&bar.w_empty[ws], ((ch_cnt / kWS) - 1) & 1, abort_flag);
+        for (int c = 0; c < nch; ++c) {
+          if (u1 > 0) wait_or_flag(&bar.w1_empty[s1], (u1 - 1) & 1, abort_flag);
           if (*abort_flag) break;
-          mbar_expect_tx(&bar.w_full[ws], W_BYTES);
-          tma_load_2d(w, &mw1, &bar.w_full[ws], c * kHC, 0);                    // value columns of W1
-          tma_load_2d(w + WB, &mw1, &bar.w_full[ws], p.inner + c * kHC, 0);     // gate columns of W1
-          tma_load_2d(w + 2 * WB, &mw2, &bar.w_full[ws], c * kHC, 0);           // W2[:, chunk]
+          mbar_expect_tx(&bar.w1_full[s1], 2 * WB);
+          tma_load_2d(sW1 + s1 * 2 * WB, &mw1, &bar.w1_full[s1], c * kHC, 0);                    // value columns of W1
+          tma_load_2d(sW1 + s1 * 2 * WB + WB, &mw1, &bar.w1_full[s1], p.inner + c * kHC, 0);     // gate columns of W1
+          ++n1;
+          if (++s1 == kW1S) { s1 = 0; ++u1; }
+          if (u2 > 0) wait_or_flag(&bar.w2_empty[s2], (u2 - 1) & 1, abort_flag);
+          if (*abort_flag) break;
+          mbar_expect_tx(&bar.w2_full[s2], WB);
+          tma_load_2d(sW2 + s2 * WB, &mw2, &bar.w2_full[s2], c * kHC, 0);                        // W2[:, chunk]
+          ++n2;
+          if (++s2 == kW2S) { s2 = 0; ++u2; }
         }
       }
-      drain_ring(&bar.x_full, n_x, 1);
-      drain_ring(&bar.dy_full, n_dy, 1);
-      drain_ring(bar.w_full, ch_cnt, kWS);
+      drain_ring(bar.w1_full, n1, kW1S);
+      drain_ring(bar.w2_full, n2, kW2S);
     }
   }
 
@@ -421,16 +440,14 @@ int transition_bwd_fused_blocks(int64_t M) {
 
 // g [panels of 64 columns][M][64], dh [inner/32][M][64] (chunk-ordered columns), dx, and per block the column sums part [blocks][2 * 128]
 int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, float* part, cudaStream_t st) {
-  CUtensorMap mx, mdy, mw1, mw2, mdh, mg, mxr, mdx;
+  CUtensorMap mx, mdy, mw1, mw2, mdh, mg, mdx;
   int r;
   {
     const int64_t dims[2] = {K, a.M}, str[2] = {1, K};
-    const int box[2] = {64, kRows};
-    if ((r = make_tiled_map(&mx, a.x, a.dtype, 2, dims, str, box, 128))) return r;
-    if ((r = make_tiled_map(&mdy, a.dy, a.dtype, 2, dims, str, box, 128))) return r;
-    const int slab[2] = {64, 32};                // half of a row warp's rows
-    if ((r = make_tiled_map(&mxr, a.x, a.dtype, 2, dims, str, slab, 128))) return r;
-    if ((r = make_tiled_map(&mdx, a.dx, a.dtype, 2, dims, str, slab, 128))) return r;
+    const int slab[2] = {32, 32};                // half of a row warp's piece
+    if ((r = make_tiled_map(&mx, a.x, a.dtype, 2, dims, str, slab, 64))) return r;
+    if ((r = make_tiled_map(&mdy, a.dy, a.dtype, 2, dims, str, slab, 64))) return r;
+    if ((r = make_tiled_map(&mdx, a.dx, a.dtype, 2, dims, str, slab, 64))) return r;
   }
   {
     const int64_t dims[2] = {2 * (int64_t)a.inner, K}, str[2] = {1, 2 * (int64_t)a.inner};
@@ -462,16 +479,16 @@ int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, flo
   p.status = status_word();
   MF_REQUIRE(p.status, MF_ERR_CUDA, "could not allocate the device status word");
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
-  constexpr size_t smem = 1024 + 3 * (size_t)A_BYTES + kWS * (size_t)W_BYTES + 2 * (size_t)DH_BYTES + 2 * (size_t)G_BYTES;
+  constexpr size_t smem = 1024 + 2 * (size_t)A_BYTES + (2 * kW1S + kW2S) * (size_t)WB + 2 * (size_t)DH_BYTES + 2 * (size_t)G_BYTES + 2 * 4 * 128 * sizeof(float4);
   const int grid = transition_bwd_fused_blocks(a.M);
   if (a.dtype == MF_BF16) {
     constexpr auto kern = transition_bwd_tc_kernel<__nv_bfloat16>;
     if (int e = opt_in_smem<kern>(smem)) return e;
-    kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, mxr, mdx, p);
+    kern<<<grid, kThreads, smem, st>>>(mdy, mw1, mw2, mdh, mg, mx, mdx, p);
   } else {
     constexpr auto kern = transition_bwd_tc_kernel<__half>;
     if (int e = opt_in_smem<kern>(smem)) return e;
-    kern<<<grid, kThreads, smem, st>>>(mx, mdy, mw1, mw2, mdh, mg, mxr, mdx, p);
+    kern<<<grid, kThreads, smem, st>>>(mdy, mw1, mw2, mdh, mg, mx, mdx, p);
   }
   MF_LAUNCHED("transition_bwd_tc_kernel");
   return MF_OK;
