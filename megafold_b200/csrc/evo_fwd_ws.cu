@@ -26,8 +26,10 @@
 // exponentials; P overwrites the scores, since TMEM has no room beside them (3 x (2 x 64 + 32) columns).  Step v of a stream's
 // products is P V of block v - 2 and the scores of block v, one sequence into one buffer with one completion barrier: it
 // says that the scores are there and that the operand buffers of that parity are free again.  The maximum is that of 128
-// keys: with one per block of 64 the same call takes 91 us, but rows that need rescaling at every new maximum (kExactStep)
-// wait for the last product twice as often ([1, 467, 467, 4, 32]: 217 us instead of 203).
+// keys: with one per block of 64 the same call takes 90 us, but other last bits come out, on which the shift gradients of a
+// block's pair-bias LayerNorms depend (they are 0 up to rounding), and rows that need rescaling at every new maximum
+// (kExactStep) wait for the last product twice as often ([1, 467, 467, 4, 32]: 217 us instead of 203).  For the bits' sake the
+// exponent stays a difference and a product as well: one fused step for both takes 85 instead of 90 us.
 // Measured, [1, 384, 384, 4, 32] bf16 / [1, 467, 467, 4, 32] bf16 (copied bias): 135 / 294 us with two streams of 128-key tiles
 // (208 registers a thread, every logit in a register), 115 / 254 with three streams and one score buffer each, 98 / 263 with
 // two buffers of 64 keys, 90 / 217 with the operands of the products in uniform registers, 94 / 203 with pairs, as now.

@@ -116,7 +116,10 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
-  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
+  // A 16-bit bias read element by element is the one form that is slower with uniform operands (the compiler then spills three times as much in the
+  // loop over its columns: [4, 1, 322, 8, 48] 38 -> 42 us; staged and TMA forms [4, 1, 384, 32, 64] 48 -> 44 and 43 -> 39).
+  constexpr bool kUniform = BM != kDirect || sizeof(TB) != 2;
+  const int tid = threadIdx.x, warp = kUniform ? uniform(tid >> 5) : tid >> 5, lane = tid & 31;
   const int s = warp >> 2;                    // stream = warpgroup
   const int wg_tid = tid & 127;
   const bool leader = (warp & 3) == 0;
@@ -151,7 +154,7 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   const int r = (warp & 3) * 32 + lane;                              // TMEM lane = query row in the tile
   const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t tS = tmem_base_s + s * 256 + lane_addr, tP = tS + 128, tO = tS + 192;
-  const uint32_t tS0 = uniform(tmem_base_s) + s * 256;                      // lane 0 addresses for the MMA issuer
+  const uint32_t tS0 = (kUniform ? uniform(tmem_base_s) : tmem_base_s) + s * 256;                      // lane 0 addresses for the MMA issuer
   const uint32_t id_s = idesc_f16(128, kKT, p.ab_fmt, 0, 0);
   const uint32_t id_o = idesc_f16(128, DP, p.ab_fmt, 0, 1);
 

@@ -68,7 +68,7 @@ ln_wide_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ C
   __shared__ float part_s[2][kRows];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = blockIdx.x * kRows, b0 = blockIdx.y * p.R;
   const int nb = p.n_blocks - b0 < p.R ? p.n_blocks - b0 : p.R;      // my blocks of columns
   if (tid == 0) {
@@ -89,7 +89,7 @@ ln_wide_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = uniform(tmem_base_s);
+  const uint32_t tm0 = tmem_base_s;
 
   // block u of the 2 nb passes over W (hi terms, then lo terms)
   int loaded = 0;                                    // blocks requested (thread 0)
