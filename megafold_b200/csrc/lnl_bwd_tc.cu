@@ -69,7 +69,7 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
   __shared__ __align__(128) uint8_t ones_s[16 * 32];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < kStages; ++i) { mbar_init(&bar.full[i], 1); mbar_init(&bar.empty[i], 1); }
@@ -86,7 +86,7 @@ lnl_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy, const __grid_constant
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tAcc = uniform(tmem_base_s), tDb = tAcc + 2 * K;
+  const uint32_t tAcc = tmem_base_s, tDb = tmem_base_s + 2 * K;
   const int my_tiles = (p.n_mt - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int ns = p.n_slabs;
 
