@@ -17,22 +17,23 @@
 // 2^(m_old - m_new) when the running maximum has grown by more than 8 (rare after the first pair; P then stays
 // below 2^8, far inside the 16-bit range), or at all (kExactStep).  Only O and the log-sum-exp reach global memory.
 //
-// Bound: no single unit.  The exponentials, one per logit at 16 a clock and SM, are 50 of the 94 us that [1, 384, 384, 4, 32]
+// Bound: no single unit.  The exponentials, one per logit at 16 a clock and SM, are 50 of the 89 us that [1, 384, 384, 4, 32]
 // bf16 takes (256 clocks a warp and 32 logits of its rows; one warp per scheduler needs 11.4 cycles an element in this loop
 // with the unit free to it, two 9.3, three 8.9, where 8 saturate it), the issue slots are half used, and with either the
 // exponentials or half of the products left out the time falls by 3 % only: what counts is how many softmax warps have work.
-// So there are three streams, which leaves a thread 120 registers: the logits are read twice (a TMEM read of 128 columns
+// So there are three streams, which leaves a thread 128 registers: the logits are read twice (a TMEM read of 128 columns
 // takes 25 cycles).  A stream has two score buffers of 64 keys, so that the products of a block run under the other one's
 // exponentials; P overwrites the scores, since TMEM has no room beside them (3 x (2 x 64 + 32) columns).  Step v of a stream's
 // products is P V of block v - 2 and the scores of block v, one sequence into one buffer with one completion barrier: it
 // says that the scores are there and that the operand buffers of that parity are free again.  The maximum is that of 128
 // keys: with one per block of 64 the same call takes 90 us, but other last bits come out, on which the shift gradients of a
 // block's pair-bias LayerNorms depend (they are 0 up to rounding), and rows that need rescaling at every new maximum
-// (kExactStep) wait for the last product twice as often ([1, 467, 467, 4, 32]: 217 us instead of 203).  For the bits' sake the
+// (kExactStep) wait for the last product twice as often ([1, 467, 467, 4, 32]: 217 us where pairs take 203).  For the bits' sake the
 // exponent stays a difference and a product as well: one fused step for both takes 85 instead of 90 us.
 // Measured, [1, 384, 384, 4, 32] bf16 / [1, 467, 467, 4, 32] bf16 (copied bias): 135 / 294 us with two streams of 128-key tiles
 // (208 registers a thread, every logit in a register), 115 / 254 with three streams and one score buffer each, 98 / 263 with
-// two buffers of 64 keys, 90 / 217 with the operands of the products in uniform registers, 94 / 203 with pairs, as now.
+// two buffers of 64 keys, 90 / 217 with the operands of the products in uniform registers, 94 / 203 with pairs, 89 / 197 with 128 / 40 registers
+// a softmax / helper thread instead of 120 / 56, as now.
 // Taken back: loading the next block's logits between the exponentials (109), separate warps for the bias copies and the
 // mask terms (108: more warps for the same issue slots), nanosleep in the waits of the helper warps (99), streams started
 // a third of a block apart (100; all against 98).
@@ -95,7 +96,7 @@ __device__ __forceinline__ void step_item(ItemPos& x, const FwdWsP& p) {      //
   if (++x.qt == p.n_qt) { x.qt = 0; if (++x.h == p.H) { x.h = 0; if (++x.n == p.N) { x.n = 0; ++x.b; } } }
 }
 
-constexpr int kLaunchRegs = 96, kSoftmaxRegs = 120, kHelperRegs = 56;      // registers per thread: at launch / after setmaxnreg
+constexpr int kLaunchRegs = 96, kSoftmaxRegs = 128, kHelperRegs = 40;      // registers per thread: at launch / after setmaxnreg
 static_assert(kLaunchRegs * kThreads <= 65536, "register file");
 static_assert(kStreams * 128 * kSoftmaxRegs + 256 * kHelperRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 
