@@ -46,8 +46,9 @@ constexpr int kHC = 32;              // hidden (value) columns per chunk
 constexpr int kWorkWarps = 16;       // two teams of eight
 constexpr int kRowWarps = 8, kFirstIssuer = kWorkWarps + kRowWarps;         // row warps: two per 32 rows: the 32-column quarters 0 and 2, 1 and 3
 constexpr int kThreads = (kWorkWarps + kRowWarps + 4) * 32;
-// registers per thread: at launch / workers / row warps / issuers after setmaxnreg (the raises draw on the drop)
-constexpr int kLaunchRegs = 72, kWorkRegs = 64, kRowRegs = 96, kIssueRegs = 56;
+// registers per thread: at launch / workers / row warps / issuers after setmaxnreg (the raises draw on the drop).  With 64 / 96 / 56 the
+// row warps spilled: [100000, 128], inner 512, forward + backward 236 us, 231 with 64 / 104 / 40, 227 with these.
+constexpr int kLaunchRegs = 72, kWorkRegs = 56, kRowRegs = 120, kIssueRegs = 40;
 static_assert(kWorkWarps * 32 * kWorkRegs + kRowWarps * 32 * kRowRegs + 128 * kIssueRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 constexpr int A_BYTES = kRows * K * 2;          // 32 KB: X or dY tile, two 64-column atoms
 constexpr int WB = K * 64;                       // 8 KB: one [128 rows][32 columns] weight block
