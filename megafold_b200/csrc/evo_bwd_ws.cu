@@ -106,12 +106,18 @@ struct Item {
   __device__ __forceinline__ int jt1(const BwdWsP& p) const { return p.ksplit == 1 ? p.n_t : (sp + 1) * p.n_t / p.ksplit; }
 };
 
+// A parity wait tells a phase from the one before it only: asked for phase m while m - 1 is open it takes m - 2 for it and returns
+// at once.  So a role that waits on a barrier waits for every phase of it, in turn, and the phase before the one asked for
+// is known to be complete, whatever the other roles do.  That is why dQ on chip has a barrier of its own: the write-out warps
+// would use one phase of dq_done an item, and nothing that they wait for says how far the dQ products have come (the compute
+// warps hand P and dS over before they wait for the product of two blocks ago).  None of the barriers can run ahead of a waiter
+// either, since the role that completes a phase waits, directly or through the copies, for what the waiter does after the phase before it.
 struct Bars {
   uint64_t kv_full[2], kv_empty[2], qd_full[3], qd_empty[3], bt_full[3], bt_empty[3];
   uint64_t sd_ready[2], written[2], buf_free[2];
   uint64_t ds_written[2], dq_done[2];        // per block parity: dS^T tile complete in shared memory / its dQ product complete
   uint64_t kv_done[2], kv_drained[2];        // by parity: the dK / dV accumulation of a key tile is complete / has been read out
-  uint64_t item_done[2];                     // the item's on-chip dQ accumulators have been read out
+  uint64_t item_dq, item_done[2];            // the item's on-chip dQ accumulators are complete / have been read out
   uint64_t dq_drained[2];
 };
 
@@ -270,6 +276,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       mbar_init(&bar.dq_drained[i], 4);
       mbar_init(&bar.kv_done[i], 1); mbar_init(&bar.kv_drained[i], 4);
     }
+    mbar_init(&bar.item_dq, 1);
     for (int i = 0; i < 3; ++i) {
       mbar_init(&bar.qd_full[i], 1); mbar_init(&bar.qd_empty[i], 1); mbar_init(&bar.bt_full[i], 1); mbar_init(&bar.bt_empty[i], 1);
     }
@@ -451,16 +458,14 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           }
         };
         for (int jt = at.jt0(p), jt1 = at.jt1(p); jt < jt1; ++jt, ++kv) {
-          for (int it = 0; it < nt; ++it, ++g) {
-            if constexpr (DQS) {                        // streamed dQ: the product of every block
-              wait_or_flag(&bar.dq_done[g & 1], (g >> 1) & 1, abort_flag);
-              tc_fence_after();
+          for (int it = 0; DQS && it < nt; ++it, ++g) {               // streamed dQ: the product of every block
+            wait_or_flag(&bar.dq_done[g & 1], (g >> 1) & 1, abort_flag);
+            tc_fence_after();
 #pragma unroll 1
-              for (int hh = 0; hh < NH; ++hh) add_dq(tDQ + (g & 1) * 32 * NH, it, hh);
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&bar.dq_drained[g & 1]);
-            }
+            for (int hh = 0; hh < NH; ++hh) add_dq(tDQ + (g & 1) * 32 * NH, it, hh);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar.dq_drained[g & 1]);
           }
           // dK_j (scaled) and dV_j
           wait_or_flag(&bar.kv_done[kv & 1], (kv >> 1) & 1, abort_flag);
@@ -479,8 +484,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           if (lane == 0) mbar_arrive(&bar.kv_drained[kv & 1]);
         }
         if constexpr (!DQS) {                           // every query tile's dQ
-          const uint32_t gl = g - 1;
-          wait_or_flag(&bar.dq_done[gl & 1], (gl >> 1) & 1, abort_flag);
+          wait_or_flag(&bar.item_dq, item_no & 1, abort_flag);
           tc_fence_after();
 #pragma unroll 1
           for (int u = 0; u < nt * NH; ++u) {           // (query tile, head half)
@@ -526,6 +530,7 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             if (it == nt - 1) tc_commit_el(&bar.kv_empty[kv % NKV]);
           }
         }
+        if (!DQS && !dead()) tc_commit_el(&bar.item_dq);
       }
     } else if (warp == kComputeWarps + 2) {
       // ========================================================================== score issuer: per half block
