@@ -526,11 +526,11 @@ evo_bwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
 #pragma unroll
               for (int ks = 1; ks < 8; ++ks) mma_ss_el(tacc + hh * 32, a_lo + ks * (2048 / 16), hi128, kh + ks * 64, hi64, id_q, true);
             }
+            if (!DQS && jt == jt1 - 1 && it == nt - 1) tc_commit_el(&bar.item_dq);
             tc_commit_el(&bar.dq_done[g & 1]);
             if (it == nt - 1) tc_commit_el(&bar.kv_empty[kv % NKV]);
           }
         }
-        if (!DQS && !dead()) tc_commit_el(&bar.item_dq);
       }
     } else if (warp == kComputeWarps + 2) {
       // ========================================================================== score issuer: per half block
