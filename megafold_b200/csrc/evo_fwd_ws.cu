@@ -76,6 +76,12 @@ struct FwdWsP {
   void* o; TokenStrides os; float* lse; int* status;
 };
 
+// A parity wait tells a phase from the one before it only: asked for phase m while m - 1 is open it takes m - 2 for it and returns
+// at once.  So every role waits for each phase of a barrier in turn.  The softmax warps need the second step of each pair of
+// blocks: with an even number of blocks an item these are the steps of one parity, 1, 3, 5, ...; with an odd number (ODD) the parity
+// changes from item to item and they wait for the first step of a pair as well.  A kernel of its own, since code for it in the loop
+// cost the even numbers 1 %; [1, 448, 448, 4, 32] 161.5 -> 162.5 us, [1, 264, 264, 4, 32] 59.8 -> 60.3.  (Commits of one warp that arrive in the
+// order in which they were issued would do too; that order is not promised.)
 struct StreamBars {                      // [parity of the block; of the item for Q]
   uint64_t q_full[2], k_full[2], v_full[2];      // Q tile / K, bias and mask-term tiles / V tile
   uint64_t step_done[2];                 // step v: P V of block v - 2 and the scores of block v are complete
@@ -100,7 +106,7 @@ constexpr int kLaunchRegs = 96, kSoftmaxRegs = 128, kHelperRegs = 40;      // re
 static_assert(kLaunchRegs * kThreads <= 65536, "register file");
 static_assert(kStreams * 128 * kSoftmaxRegs + 256 * kHelperRegs <= kThreads * kLaunchRegs, "setmaxnreg budget");
 
-template <typename T, typename TB, bool EXACT>      // EXACT: see kExactStep
+template <typename T, typename TB, bool EXACT, bool ODD>      // EXACT: see kExactStep; ODD: an odd number of key blocks, see StreamBars
 __global__ void __maxnreg__(kLaunchRegs)
 evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                   const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mb, const FwdWsP p MF_TRACE_PARAM) {
@@ -188,6 +194,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         const uint32_t tS = tbase + (u & 1) * kB + lane_addr, tN = tbase + (~u & 1) * kB + lane_addr;
         const bool two = t + 1 < n_kb;
         tr(1);
+        if (ODD) wait_step(u);
         wait_step(u + 1);                          // scores of both blocks, and every earlier product: O may be read and rescaled
         tr(2);
         // ---------------------------------------------------------------- pass 1: the maximum.  Bias and key mask are
@@ -443,7 +450,7 @@ evo_fwd_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   if (warp == 0) tmem_dealloc(tmem_base_s, 512);
 }
 
-template <typename T, typename TB, bool EXACT>
+template <typename T, typename TB, bool EXACT, bool ODD>
 int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   CUtensorMap mq, mk, mv, mb;
   int r;
@@ -475,7 +482,7 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   int grid = sm_count();
   if (grid > p.n_items) grid = p.n_items;
   const size_t smem = 1024 + kStreams * (size_t)kStreamBytes + 2048 + kXTileB;
-  constexpr auto kern = evo_fwd_ws_kernel<T, TB, EXACT>;
+  constexpr auto kern = evo_fwd_ws_kernel<T, TB, EXACT, ODD>;
   static std::atomic<int> built_with{0};           // asked for once; a query that fails is made again
   int regs = built_with.load(std::memory_order_relaxed);
   if (!regs) {
@@ -490,11 +497,11 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   return MF_OK;
 }
 
-template <bool EXACT>
+template <bool EXACT, bool ODD>
 int dispatch(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st) {
   if (a.dtype == MF_BF16)
-    return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16, EXACT>(a, lay, st) : launch_fwd_ws<__nv_bfloat16, __half, EXACT>(a, lay, st);
-  return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16, EXACT>(a, lay, st) : launch_fwd_ws<__half, __half, EXACT>(a, lay, st);
+    return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__nv_bfloat16, __nv_bfloat16, EXACT, ODD>(a, lay, st) : launch_fwd_ws<__nv_bfloat16, __half, EXACT, ODD>(a, lay, st);
+  return a.bias_dtype == MF_BF16 ? launch_fwd_ws<__half, __nv_bfloat16, EXACT, ODD>(a, lay, st) : launch_fwd_ws<__half, __half, EXACT, ODD>(a, lay, st);
 }
 
 }  // namespace
@@ -525,7 +532,9 @@ int evo_fwd_ws(const mf_evo_fwd_args& args, const mf_evo_layout& lay, void* work
     a.bias_strides[3] = 1; a.bias_strides[2] = row; a.bias_strides[1] = row * a.L;
     a.bias_strides[0] = args.bias_strides[0] == 0 ? 0 : row * a.L * a.H;
   }
-  return copied ? dispatch<true>(a, lay, st) : dispatch<false>(a, lay, st);
+  const bool odd = (a.L + kB - 1) / kB % 2 != 0;
+  if (copied) return odd ? dispatch<true, true>(a, lay, st) : dispatch<true, false>(a, lay, st);
+  return odd ? dispatch<false, true>(a, lay, st) : dispatch<false, false>(a, lay, st);
 }
 
 }  // namespace mf

@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("N,L,H,D", [(1, 1, 1, 32), (2, 64, 1, 8), (1, 65, 3, 32), (37, 72, 4, 24), (149, 128, 1, 32), (3, 129, 1, 16), (5, 192, 30, 32),
-                                     (2, 200, 2, 32), (1, 320, 5, 24), (4, 456, 1, 32)])
+                                     (2, 200, 2, 32), (1, 320, 5, 24), (4, 456, 1, 32),
+                                     # six or more items a CTA: a stream goes from item to item, with an odd and an even number of blocks
+                                     (1001, 64, 1, 32), (333, 72, 3, 8), (251, 192, 2, 32), (151, 320, 2, 24), (113, 384, 3, 32)])
 @pytest.mark.parametrize("rising", [False, True])
 def test_streams_and_blocks(dtype, N, L, H, D, rising):
     g = torch.Generator(device="cuda").manual_seed(N + L)
