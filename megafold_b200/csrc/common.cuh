@@ -53,9 +53,11 @@ inline int after_launch(const char* name) {
   do { int r__ = ::mf::after_launch(name); if (r__ != MF_OK) return r__; } while (0)
 
 // Dynamic shared memory beyond 48 KB has to be asked for once per kernel and device; the call costs the host about as much
-// as a launch, so what has been granted is remembered.
+// as a launch, so what has been granted is remembered.  `regs`: registers per thread that a kernel with setmaxnreg shares out.
+// __launch_bounds__ is an upper bound only, and a raise beyond what the CTA was launched with never returns: a build that
+// gives the kernel fewer (they are handed out in eights) is an error here.
 template <auto Kernel>
-int opt_in_smem(size_t bytes) {
+int opt_in_smem(size_t bytes, int regs = 0) {
   static std::atomic<int> granted[64];
   static std::mutex mu;
   int dev = 0;
@@ -63,6 +65,11 @@ int opt_in_smem(size_t bytes) {
   if (dev >= 0 && dev < 64 && granted[dev].load(std::memory_order_acquire) >= (int)bytes) return MF_OK;
   std::lock_guard<std::mutex> lk(mu);
   if (dev >= 0 && dev < 64 && granted[dev].load(std::memory_order_relaxed) >= (int)bytes) return MF_OK;
+  if (regs) {
+    cudaFuncAttributes fa;
+    MF_CUDA(cudaFuncGetAttributes(&fa, Kernel));
+    MF_REQUIRE((fa.numRegs + 7) / 8 * 8 >= regs, MF_ERR_CUDA, "a kernel was built with %d registers per thread, %d expected", fa.numRegs, regs);
+  }
   MF_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
   if (dev >= 0 && dev < 64) granted[dev].store((int)bytes, std::memory_order_release);
   return MF_OK;

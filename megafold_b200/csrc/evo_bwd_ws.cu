@@ -1064,7 +1064,7 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
     int grid = sm_count();
     if (grid > p.n_units) grid = p.n_units;
     constexpr auto kern = evo_dbias_ws_kernel<T, TT, NH>;
-    if (int e = opt_in_smem<kern>(smem)) return e;
+    if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
     kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     MF_LAUNCHED("evo_dbias_ws_kernel");
     if (!pl.part_direct) {
@@ -1098,11 +1098,11 @@ int launch_bwd_ws(const mf_evo_bwd_args& a, const mf_evo_layout& lay, cudaStream
     const size_t smem = Geo<NH>::kMainSmem;
     if (pl.dq_stream) {
       constexpr auto kern = evo_bwd_ws_kernel<T, TT, true, NH>;
-      if (int e = opt_in_smem<kern>(smem)) return e;
+      if (int e = opt_in_smem<kern>(smem, kMainLaunchRegs)) return e;
       kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     } else {
       constexpr auto kern = evo_bwd_ws_kernel<T, TT, false, NH>;
-      if (int e = opt_in_smem<kern>(smem)) return e;
+      if (int e = opt_in_smem<kern>(smem, kMainLaunchRegs)) return e;
       kern<<<grid, kMainThreads, smem, st>>>(mq, mk, mv, mg, mbt, p MF_TRACE_ARG);
     }
     MF_LAUNCHED("evo_bwd_ws_kernel");

@@ -483,15 +483,7 @@ int launch_fwd_ws(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream
   if (grid > p.n_items) grid = p.n_items;
   const size_t smem = 1024 + kStreams * (size_t)kStreamBytes + 2048 + kXTileB;
   constexpr auto kern = evo_fwd_ws_kernel<T, TB, EXACT, ODD>;
-  static std::atomic<int> built_with{0};           // asked for once; a query that fails is made again
-  int regs = built_with.load(std::memory_order_relaxed);
-  if (!regs) {
-    cudaFuncAttributes fa;
-    MF_CUDA(cudaFuncGetAttributes(&fa, kern));
-    built_with.store(regs = fa.numRegs, std::memory_order_relaxed);
-  }
-  MF_REQUIRE(regs == kLaunchRegs, MF_ERR_CUDA, "evo_fwd_ws_kernel was built with %d registers per thread, %d expected", regs, kLaunchRegs);
-  if (int e = opt_in_smem<kern>(smem)) return e;
+  if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
   kern<<<grid, kThreads, smem, st>>>(mq, mk, mv, mb, p MF_TRACE_ARG);
   MF_LAUNCHED("evo_fwd_ws_kernel");
   return MF_OK;

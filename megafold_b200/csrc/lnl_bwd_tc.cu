@@ -274,7 +274,7 @@ int launch(const LnlBwdRowsArgs& a, int grid, cudaStream_t st) {
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
   constexpr size_t smem = 1024 + kRowWarps * 32 * (size_t)K / 2 + kStages * (size_t)(kSlabB + K * 128) + 128 * (size_t)K * 2;
   constexpr auto kern = lnl_bwd_tc_kernel<K, T>;
-  if (int e = opt_in_smem<kern>(smem)) return e;
+  if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
   kern<<<grid, kThreads, smem, st>>>(mdy, mw, mdx, p);
   MF_LAUNCHED("lnl_bwd_tc_kernel");
   return MF_OK;

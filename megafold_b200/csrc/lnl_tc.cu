@@ -30,6 +30,7 @@ constexpr int kNT = 128;            // output columns per MMA group
 constexpr int kWorkers = 256;
 constexpr int kNormWarps = 4;         // warps 8-11 normalise rows; warp 12 issues MMAs, warp 13 TMA loads
 constexpr int kThreads = 512;          // four warpgroups: two of epilogue warps, one of normalising warps, one of issuers
+constexpr int kLaunchRegs = 128;       // registers per thread at launch, re-partitioned inside the kernel
 constexpr int kWStages = 2;
 constexpr int kAStages = 3;         // X tiles in flight (TMA prefetch two tiles ahead)
 
@@ -87,9 +88,9 @@ lnl_fwd_tc_kernel(const __grid_constant__ CUtensorMap mx, const __grid_constant_
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
   const uint32_t tm0 = uniform(tmem_base_s);
-  // Register re-partition (the CTA is launched with 128 per thread): the issuer warpgroup keeps 40, the epilogue
+  // Register re-partition (the CTA is launched with kLaunchRegs per thread): the issuer warpgroup keeps 40, the epilogue
   // warpgroups get 152 and the normalising warpgroup 168; 256 * 152 + 128 * 168 + 128 * 40 = 512 * 128 exactly.
-  static_assert(256 * 152 + 128 * 168 + 128 * 40 <= kThreads * 128, "setmaxnreg budget");
+  static_assert(256 * 152 + 128 * 168 + 128 * 40 <= kThreads * kLaunchRegs, "setmaxnreg budget");
   // (each setmaxnreg sits inside its role's branch: the compiler allocates registers per region)
   const int my_tiles = p.n_mt > (int)blockIdx.x ? (p.n_mt - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
@@ -316,7 +317,7 @@ int launch_lnl(const mf_lnl_fwd_args& a, cudaStream_t st) {
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
   const size_t smem = 1024 + kAStages * (size_t)kRows * K * 2 + kWStages * (size_t)K * kNT * 2 + 2 * (size_t)kRows * kNT * 2;
   constexpr auto kern = lnl_fwd_tc_kernel<K, T>;
-  if (int e = opt_in_smem<kern>(smem)) return e;
+  if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
   int grid = sm_count();
   if (grid > p.n_mt) grid = p.n_mt;
   kern<<<grid, kThreads, smem, st>>>(mx, mw, my, p);

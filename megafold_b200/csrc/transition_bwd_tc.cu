@@ -484,11 +484,11 @@ int transition_bwd_fused(const mf_transition_bwd_args& a, void* g, void* dh, flo
   const int grid = transition_bwd_fused_blocks(a.M);
   if (a.dtype == MF_BF16) {
     constexpr auto kern = transition_bwd_tc_kernel<__nv_bfloat16>;
-    if (int e = opt_in_smem<kern>(smem)) return e;
+    if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
     kern<<<grid, kThreads, smem, st>>>(mdy, mw1, mw2, mdh, mg, mx, mdx, p);
   } else {
     constexpr auto kern = transition_bwd_tc_kernel<__half>;
-    if (int e = opt_in_smem<kern>(smem)) return e;
+    if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
     kern<<<grid, kThreads, smem, st>>>(mdy, mw1, mw2, mdh, mg, mx, mdx, p);
   }
   MF_LAUNCHED("transition_bwd_tc_kernel");

@@ -391,7 +391,7 @@ int launch_tr(const mf_transition_fwd_args& a, cudaStream_t st) {
   MF_REQUIRE(tc_async_status() == 0, MF_ERR_CUDA, "an earlier tensor-core kernel gave up on a bounded wait; results are invalid");
   const size_t smem = 1024 + 2 * (size_t)kRows * K * 2 + kWStages * (size_t)(3 * K * 128);
   constexpr auto kern = transition_fwd_tc_kernel<K, T>;
-  if (int e = opt_in_smem<kern>(smem)) return e;
+  if (int e = opt_in_smem<kern>(smem, kLaunchRegs)) return e;
   int grid = sm_count();
   if (grid > p.n_mt) grid = p.n_mt;
   kern<<<grid, kThreads, smem, st>>>(mx, mw1, mw2, my, p);
