@@ -138,36 +138,24 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {
 // ---- descriptors ------------------------------------------------------------------------------------
 enum Swizzle : uint32_t { kSwNone = 0, kSw128 = 2, kSw64 = 4, kSw32 = 6 };
 
-// Shared-memory matrix descriptor (64 bit): start address >> 4 in [0,14), leading byte offset >> 4 in
-// [16,30), stride byte offset >> 4 in [32,46), descriptor version 1 in [46,48), swizzle mode in [61,64).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes, Swizzle sw) {
-  return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16) |
-         ((uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32) | (1ull << 46) | ((uint64_t)sw << 61);
-}
 // Instruction descriptor for kind::f16 with fp32 accumulation.  ab_fmt: 0 = f16, 1 = bf16.
 // a_mn / b_mn: 1 when the operand is MN-major (the non-reduction index is contiguous in shared memory).
 __host__ __device__ constexpr uint32_t idesc_f16(uint32_t M, uint32_t N, uint32_t ab_fmt, uint32_t a_mn, uint32_t b_mn) {
   return (1u << 4) | (ab_fmt << 7) | (ab_fmt << 10) | (a_mn << 15) | (b_mn << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-      : "memory");
-}
-// The same with the descriptors given as (low, high) words.  The issuing thread's own instruction stream bounds how
-// fast MMAs can be issued, so loops keep the high words (stride, version, swizzle: constants) and a base low word in
-// registers and step the address field by adding (bytes >> 4) to the low word: one integer add per operand and MMA.
+// Shared-memory matrix descriptor (64 bit): start address >> 4 in [0,14), leading byte offset >> 4 in
+// [16,30), stride byte offset >> 4 in [32,46), descriptor version 1 in [46,48), swizzle mode in [61,64), as (low, high) words.
+// The issuing thread's own instruction stream bounds how fast MMAs can be issued, so loops keep the high words (stride,
+// version, swizzle: constants) and a base low word in registers and step the address field by adding (bytes >> 4) to the low
+// word: one integer add per operand and MMA.
 __host__ __device__ constexpr uint32_t desc_hi(uint32_t sbo_bytes, Swizzle sw) {
   return ((sbo_bytes >> 4) & 0x3FFF) | (1u << 14) | ((uint32_t)sw << 29);
 }
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr & 0x3FFFFu) >> 4) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
 }
+// D[tmem] (+)= A[smem] * B[smem]; issued by ONE thread.
 __device__ __forceinline__ void mma_ss_lh(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                           uint32_t idesc, bool accumulate) {
   asm volatile(
@@ -179,29 +167,9 @@ __device__ __forceinline__ void mma_ss_lh(uint32_t d_tmem, uint32_t a_lo, uint32
       ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"((uint32_t)accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"((uint32_t)accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void mma_ts_lh(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, bool accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"((uint32_t)accumulate)
-      : "memory");
-}
-
-// The same two, called by ALL 32 lanes of a converged warp; one elected lane issues.  With the whole warp running the
-// issue loop the descriptor arithmetic stays warp-uniform, which more than halves the instructions per MMA compared
-// with a single-lane branch (measured: ~18 instead of ~45 cycles per issued MMA).
+// The same with A in shared memory (ss) or TMEM (ts), called by ALL 32 lanes of a converged warp; one elected lane issues.
+// With the whole warp running the issue loop the descriptor arithmetic stays warp-uniform, which more than halves the
+// instructions per MMA compared with a single-lane branch (measured: ~18 instead of ~45 cycles per issued MMA).
 __device__ __forceinline__ void mma_ss_el(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                           uint32_t idesc, bool accumulate) {
   asm volatile(
