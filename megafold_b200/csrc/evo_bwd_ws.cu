@@ -693,7 +693,10 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
 
-  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
+  // With one head half uniform operands only make the compute warps spill more (24 bytes stored, 16 without): [1, 384, 384, 4, 32] 73.2 us
+  // for this kernel, 71.9 without, at 512 183.5 and 180.0 (at 96 8.1 and 8.3); with two halves [4, 1, 384, 32, 64] 34.2 and 36.1.
+  constexpr bool kUniform = NH > 1;
+  const int tid = threadIdx.x, warp = kUniform ? uniform(tid >> 5) : tid >> 5, lane = tid & 31;
   if (tid == 0) {
     abort_s = 0;
     for (int i = 0; i < 3; ++i) {
@@ -713,7 +716,7 @@ evo_dbias_ws_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constan
   __syncthreads();
   tc_fence_after();
   volatile int* abort_flag = &abort_s;
-  const uint32_t tm0 = uniform(tmem_base_s);
+  const uint32_t tm0 = kUniform ? uniform(tmem_base_s) : tmem_base_s;
   const int nt = p.n_t;
   // unit = ((b * H + h) * nt + jt) * nt + it, split `sp` of the rows
   struct Unit { int b, h, jt, it, n0, n1; };
