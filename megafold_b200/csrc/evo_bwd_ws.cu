@@ -106,12 +106,10 @@ struct Item {
   __device__ __forceinline__ int jt1(const BwdWsP& p) const { return p.ksplit == 1 ? p.n_t : (sp + 1) * p.n_t / p.ksplit; }
 };
 
-// A parity wait tells a phase from the one before it only: asked for phase m while m - 1 is open it takes m - 2 for it and returns
-// at once.  So a role that waits on a barrier waits for every phase of it, in turn, and the phase before the one asked for
-// is known to be complete, whatever the other roles do.  That is why dQ on chip has a barrier of its own: the write-out warps
-// would use one phase of dq_done an item, and nothing that they wait for says how far the dQ products have come (the compute
-// warps hand P and dS over before they wait for the product of two blocks ago).  None of the barriers can run ahead of a waiter
-// either, since the role that completes a phase waits, directly or through the copies, for what the waiter does after the phase before it.
+// Every role waits for each phase of a barrier in turn (see tc.cuh).  That is why dQ on chip has a barrier of its own, item_dq: the
+// write-out warps would use one phase of dq_done an item, and nothing that they wait for says how far the dQ products have
+// come (the compute warps hand P and dS over before they wait for the product of two blocks ago).  The issuer starts an item's dQ
+// behind item_done of the item before, so that item_dq cannot run ahead.
 struct Bars {
   uint64_t kv_full[2], kv_empty[2], qd_full[3], qd_empty[3], bt_full[3], bt_empty[3];
   uint64_t sd_ready[2], written[2], buf_free[2];
@@ -670,7 +668,7 @@ struct DbP {
   int* status;
 };
 
-struct DbBars {
+struct DbBars {                              // every role waits for each phase of a barrier in turn (see tc.cuh)
   uint64_t op_full[3], op_empty[3];          // Q, dO, K, V, XQ, XK of one row n
   uint64_t bt_full, bt_free;                 // the unit's two bias atoms
   uint64_t sd_ready[2], loaded[2];

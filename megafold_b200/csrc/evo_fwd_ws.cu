@@ -62,7 +62,7 @@ constexpr float kRescaleStep = 8.f;          // O is rescaled only when the runn
 // tile's probabilities relative to the running maximum and the bias as it is.  For them the step is 0 and sqrt(D) keeps its
 // second term, so that they are as close to the exact result as there: the largest probability of a row is then exactly 1.
 // Distance from 64 bits at [1, 200, 467, 4, 32] bf16: 2.25e-3 with the step of 8 (2.04e-3 the general kernel and now),
-// fp16 at 323: 3.02e-4 with it, 2.81e-4 without but with one term, 2.54e-4 now.  It cost 7 % at [1, 467, 467, 4, 32];
+// fp16 at 323: 3.02e-4 with it, 2.81e-4 without but with one term, 2.54e-4 now.  It costs 8 % at [1, 467, 467, 4, 32] (182 -> 197 us);
 // a template parameter, because a step read from the arguments cost the other lengths 1.5 %.
 constexpr float kExactStep = 0.f;
 
@@ -76,8 +76,7 @@ struct FwdWsP {
   void* o; TokenStrides os; float* lse; int* status;
 };
 
-// A parity wait tells a phase from the one before it only: asked for phase m while m - 1 is open it takes m - 2 for it and returns
-// at once.  So every role waits for each phase of a barrier in turn.  The softmax warps need the second step of each pair of
+// Every role waits for each phase of a barrier in turn (see tc.cuh).  The softmax warps need the second step of each pair of
 // blocks: with an even number of blocks an item these are the steps of one parity, 1, 3, 5, ...; with an odd number (ODD) the parity
 // changes from item to item and they wait for the first step of a pair as well.  A kernel of its own, since code for it in the loop
 // cost the even numbers 1 %; [1, 448, 448, 4, 32] 161.5 -> 162.5 us, [1, 264, 264, 4, 32] 59.8 -> 60.3.  (Commits of one warp that arrive in the
@@ -503,7 +502,7 @@ int dispatch(const mf_evo_fwd_args& a, const mf_evo_layout& lay, cudaStream_t st
 static bool shape_ok(const mf_evo_fwd_args& a) { return a.D <= 32 && a.L <= 2048 && (a.bias_dtype == MF_BF16 || a.bias_dtype == MF_F16); }
 
 // A bias whose rows TMA cannot address (a chain of odd length) is copied to a 16-byte pitch when the caller gives the
-// scratch for it: an exact copy in 3 us.  At [1, 467, 467, 4, 32] the call takes 295 us, where the general kernel that reads
+// scratch for it: an exact copy in 3 us.  At [1, 467, 467, 4, 32] the call takes 197 us, where the general kernel that reads
 // such a bias in place takes 1263, and the same kernel on the copied bias 457.
 size_t evo_fwd_ws_workspace(const mf_evo_fwd_args& a) {
   if (!shape_ok(a) || bias_tma_ok(a.bias, a.bias_dtype, a.bias_strides, a.B, a.H)) return 0;

@@ -4,8 +4,8 @@
 //
 // A persistent CTA (one per SM, 256 threads) runs TWO independent streams, one per warpgroup.  A stream walks a
 // contiguous range of work items (b, n, h, 128-query tile) and, per item, the key tiles (128 keys, 64 for DP = 64).  Inside a stream every
-// thread owns one query row (= one TMEM lane); three "officer" threads of the warpgroup also issue the stream's
-// tcgen05.mma instructions (thread 0), its Q/K/V TMA loads (thread 32) and its bias TMA loads (thread 64):
+// thread owns one query row (= one TMEM lane); "officers" of the warpgroup also issue the stream's
+// tcgen05.mma instructions (warp 0, through an elected lane), its Q/K/V TMA loads (thread 32) and its bias TMA loads (thread 64):
 //
 //   wait S(t) in TMEM -> tcgen05.ld the whole row of the tile into registers -> group barrier ->
 //   S(t+1) = Q K(t+1)^T is issued at once (the S buffer is free again: registers double-buffer it)
@@ -168,8 +168,8 @@ evo_fwd_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   const int g_total = n_my * p.n_kt;
   const int per_bn = p.H * p.n_qt;
 
-  // ---- TMA bookkeeping.  Three "officer" threads per stream share the issue work so that none of it
-  // piles up on one warp: thread 0 issues the MMAs, thread 32 the Q/K/V loads, thread 64 the bias loads.
+  // ---- TMA bookkeeping.  Three "officers" per stream share the issue work so that none of it piles up on
+  // one warp: warp 0 issues the MMAs, thread 32 the Q/K/V loads, thread 64 the bias loads.
   // A cursor walks (item, key tile) incrementally: no divisions on the hot path.
   struct Cursor {
     int qt, h, n, b, t, item_local;

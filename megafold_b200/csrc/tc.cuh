@@ -23,6 +23,10 @@ __device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xf
 __device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 
 // ---- mbarrier ------------------------------------------------------------------------------
+// A parity wait tells a phase from the one before it only.  Asked for phase m while m - 1 is open it takes m - 2 for it and returns
+// at once; asked for m once m + 1 is complete it waits for m + 2.  So a role that waits on a barrier waits for every phase
+// of it, in turn: then the phase before the one asked for is known to be complete, whatever the other roles do.  And whoever
+// completes a phase first waits, directly or through the copies, for what the waiter does after the phase before it.
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

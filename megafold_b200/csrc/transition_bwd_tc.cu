@@ -32,7 +32,7 @@
 // dh is stored in that column order, a panel [M][64] per chunk; dW1 computed from it has its columns in the same order and is
 // put back by a small kernel.  (Panels, of g too: a chunk of a tile is one run of 16 KB.  128-byte pieces at the pitch of a
 // whole row took 25 us more.)
-// [262144, 128], inner 512: 250 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
+// [262144, 128], inner 512: 245 us; with one team, operands in shared memory and dyln in HBM 322 us, and 68 for the row pass.
 // Every wait is bounded; on expiry the CTA raises a flag, drains and reports through mf_async_status().
 #include "ln_bwd_rows.cuh"
 
@@ -99,7 +99,7 @@ transition_bwd_tc_kernel(const __grid_constant__ CUtensorMap mdy,
 
   __shared__ Bars bar;
   __shared__ __align__(16) float gam_s[K], bet_s[K];
-  __shared__ float sum_s[4][2 * K];            // gain and shift sums over the rows of each row warp
+  __shared__ float sum_s[4][2 * K];            // gain and shift sums over each quarter of a tile's rows
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
